@@ -314,11 +314,11 @@ int launch_simple(DeviceCtx& c, int slot, const CUtensorMap& mq, const CUtensorM
     return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 
-template <int H, bool M>
+template <int H, int M>
 int launch_pipelined(DeviceCtx& c, int slot, const CUtensorMap& mq, const CUtensorMap& mk,
                      const CUtensorMap& mv, const CUtensorMap& my, const CUtensorMap& mm, const Params& p,
                      uint32_t n_ctas, cudaStream_t st, bool overlap) {
-    constexpr int smem = fa::PipeCfg<H, M>::kSmemBytes;
+    constexpr int smem = fa::PipeCfg<H, M != fa::kNoMask>::kSmemBytes;
     auto kern = fa::fa_fwd_pipelined<H, M>;
     if (!(c.attr_done.load(std::memory_order_acquire) & (1u << slot))) {   // setting it twice is harmless
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -457,7 +457,6 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                 p.n_items = p.q_pairs * p.R * B;
                 p.scale_log2 = static_cast<float>(1.4426950408889634 / std::sqrt(static_cast<double>(H)));
                 p.mask_to_score = static_cast<float>(std::sqrt(static_cast<double>(H)));
-                p.mask_tma = 0;
 #ifdef FA_CYCLES
                 p.cycles = g_cycles_buf;
 #endif
@@ -494,12 +493,12 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                     CUtensorMap my;
                     rc = make_map(&my, y, B, L, F, H, 32);
                     bool done = false;
-                    // mask tiles through TMA when every mask row starts on a 16-byte boundary; else the
-                    // softmax threads (of the kernel on single CTAs) read their rows straight from global memory
+                    // mask tiles through TMA when every mask row starts on a 16-byte boundary; else two of the
+                    // warps (of the kernel on single CTAs) copy them with cp.async
                     CUtensorMap mm = mq;
-                    p.mask_tma = (mask && mask_rows_aligned(mask, L)) ? 1u : 0u;
-                    if (rc == FA_B200_OK && p.mask_tma) rc = make_mask_map(&mm, mask, B, L);
-                    if (rc == FA_B200_OK && use_pair_kernel(H, mask != nullptr, p.mask_tma != 0u, p.q_pairs, p.R * B,
+                    const bool mask_tma = mask && mask_rows_aligned(mask, L);
+                    if (rc == FA_B200_OK && mask_tma) rc = make_mask_map(&mm, mask, B, L);
+                    if (rc == FA_B200_OK && use_pair_kernel(H, mask != nullptr, mask_tma, p.q_pairs, p.R * B,
                                                             static_cast<uint32_t>(c->sm_count), sch.tail_steps, flags)) {
                         // K as halves of a tile: boxes of 64 keys x 64 columns
                         CUtensorMap mkh;
@@ -513,14 +512,15 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                         }
                     }
                     if (rc == FA_B200_OK && !done) {
-                        if (mask) {
-                            if (rc == FA_B200_OK)
-                                rc = H == 128 ? launch_pipelined<128, true>(*c, 10, mq, mk, mv, my, mm, p, sch.grid, st, overlap)
-                                              : launch_pipelined<64, true>(*c, 11, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
-                        } else {
-                            rc = H == 128 ? launch_pipelined<128, false>(*c, 8, mq, mk, mv, my, mq, p, sch.grid, st, overlap)
-                                          : launch_pipelined<64, false>(*c, 9, mq, mk, mv, my, mq, p, sch.grid, st, overlap);
-                        }
+                        if (mask_tma)
+                            rc = H == 128 ? launch_pipelined<128, fa::kMaskTma>(*c, 10, mq, mk, mv, my, mm, p, sch.grid, st, overlap)
+                                          : launch_pipelined<64, fa::kMaskTma>(*c, 11, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
+                        else if (mask)
+                            rc = H == 128 ? launch_pipelined<128, fa::kMaskCopied>(*c, 14, mq, mk, mv, my, mm, p, sch.grid, st, overlap)
+                                          : launch_pipelined<64, fa::kMaskCopied>(*c, 15, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
+                        else
+                            rc = H == 128 ? launch_pipelined<128, fa::kNoMask>(*c, 8, mq, mk, mv, my, mm, p, sch.grid, st, overlap)
+                                          : launch_pipelined<64, fa::kNoMask>(*c, 9, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
                     }
                 } else if (mask) {
                     switch (H) {
@@ -679,7 +679,6 @@ int fa_b200_attention_forward_noalloc(const void* q, const void* k, const void* 
         p.n_items = p.q_pairs * p.R * B;
         p.scale_log2 = static_cast<float>(1.4426950408889634 / std::sqrt(static_cast<double>(H)));
         p.mask_to_score = static_cast<float>(std::sqrt(static_cast<double>(H)));
-        p.mask_tma = 0;
         p.full_rounds = p.tail_items = p.tail_steps = p.tail_grid = 0;
         p.part_slots = 0;
         p.part_o = nullptr;

@@ -47,7 +47,6 @@ struct Params {
     uint32_t n_items;     // q_pairs * R * B: work items of the pipelined kernel
     float scale_log2;     // log2(e) / sqrt(H)
     float mask_to_score;  // sqrt(H): mask value m enters as s + m*sqrt(H) before the folded scale
-    uint32_t mask_tma;    // pipelined kernel with a mask: 1 = mask tiles come through TMA (rows 16-byte aligned)
     // schedule of the pipelined kernel (see Plan) and the scratch of a divided tail round
     uint32_t full_rounds;  // rounds of whole items: item = cta + k * grid
     uint32_t tail_items;   // items after the full rounds whose key steps are divided among the CTAs
@@ -422,6 +421,105 @@ __device__ __forceinline__ void add_mask_tile_row(float (&s)[kTile], uint32_t sm
     }
 }
 
+// Mask rows that TMA cannot fetch (row starts on no 16-byte boundary): one or two otherwise idle warps copy the tile
+// with cp.async, whole aligned words of every row into the layout that TMA gives an aligned tile.  A row that starts
+// in the middle of a 4-byte word (odd L, or a base on an odd element) lies two bytes further on in its 256 bytes, with
+// its last key in a word of its own (`sextra`, one per row); add_mask_tile_row_shifted puts that right.  Copies of
+// 8 bytes where every row starts on an 8-byte boundary.
+// Why copies of this kind: a thread that reads its own row value by value makes each load of a warp touch 32
+// lines; here the 32 lanes of a copy read 128 (256) consecutive bytes.  Measured on B=4 R=12 L=1021 H=64:
+// 217 us a call with loads by the threads themselves, 88 us with these copies.
+struct MaskRows {
+    uint64_t base, end;   // first byte of the mask, first byte behind it
+    bool wide;            // every row starts on an 8-byte boundary
+    bool shifted;         // some rows start in the middle of a word
+};
+__device__ __forceinline__ MaskRows mask_rows(const Params& p) {
+    MaskRows m;
+    m.base = reinterpret_cast<uint64_t>(p.mask);
+    m.end = m.base + 2ull * p.B * p.L * p.L;
+    m.wide = (((p.L * 2u) | static_cast<uint32_t>(m.base)) & 7u) == 0u;
+    m.shifted = (((p.L * 2u) | static_cast<uint32_t>(m.base)) & 2u) != 0u;
+    return m;
+}
+// 0 or 16: how many bits into its first 4-byte word a mask row starts (the same for every key tile)
+__device__ __forceinline__ uint32_t mask_row_shift(const Params& p, uint32_t batch, uint32_t q_row) {
+    return (((static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p.mask)) >> 1) + (batch * p.L + q_row) * p.L) & 1u) * 16u;
+}
+// Rows [r0, r0 + kRows) of the tile whose first row is q0 and whose first key is key0, eight at a time.  Nothing
+// outside the mask is read; what lies beyond the end of a row (the next row's first keys) is not used by anybody, and
+// rows below the last one are left as they are.
+template <uint32_t kRows>
+__device__ __forceinline__ void copy_mask_rows(const Params& p, const MaskRows& m, uint32_t smask, uint32_t sextra,
+                                               uint32_t batch, uint32_t q0, uint32_t key0, uint32_t r0, uint32_t lane) {
+    const uint64_t first = m.base + 2ull * ((static_cast<uint64_t>(batch) * p.L + q0 + r0) * p.L + key0);
+    const uint64_t pitch = 2ull * p.L;
+    const uint32_t n = q0 + r0 < p.L ? min(kRows, p.L - q0 - r0) : 0u;
+#pragma unroll 1
+    for (uint32_t g = 0; g < n; g += 8u) {
+        const uint64_t at = first + g * pitch;
+        const uint32_t box = smask + (r0 + g) * 128u;
+        if ((at & ~3ull) >= m.base && at + 7u * pitch + 260u <= m.end) {
+            if (m.wide) {
+                const uint32_t dst = box + (lane >> 4) * (kTile * 128) + (lane & 1u) * 8u, piece = (lane >> 1) & 7u;
+#pragma unroll
+                for (uint32_t r = 0; r < 8u; ++r)
+                    cp_async_8(dst + r * 128u + ((piece ^ r) << 4), at + r * pitch + lane * 8u);
+            } else {
+                const uint32_t dst = box + (lane & 3u) * 4u, piece = lane >> 2;
+#pragma unroll
+                for (uint32_t r = 0; r < 8u; ++r) {
+                    const uint64_t src = ((at + r * pitch) & ~3ull) + lane * 4u;
+                    cp_async_4(dst + r * 128u + ((piece ^ r) << 4), src);
+                    cp_async_4(dst + r * 128u + ((piece ^ r) << 4) + kTile * 128, src + 128u);
+                }
+                if (m.shifted && lane < 8u)
+                    cp_async_4(sextra + (r0 + g + lane) * 4u, ((at + lane * pitch) & ~3ull) + 256u);
+            }
+        } else {
+            // the first or the last rows of the whole mask: word by word
+            for (uint32_t r = 0; r < 8u && g + r < n; ++r) {
+                const uint64_t row = (at + r * pitch) & ~3ull;
+                for (uint32_t w = lane; w <= 64u; w += 32u) {
+                    const uint64_t src = row + w * 4u;
+                    const uint32_t dst = w == 64u ? sextra + (r0 + g + r) * 4u
+                                                  : box + (w >> 5) * (kTile * 128) + r * 128u + ((((w >> 2) & 7u) ^ r) << 4) +
+                                                        (w & 3u) * 4u;
+                    if (src < m.base)   // the mask begins in the middle of this word
+                        st_shared_u16(dst + 2u, *reinterpret_cast<const uint16_t*>(src + 2u));
+                    else if (src < m.end)
+                        cp_async_4_part(dst, src, m.end - src < 4u ? static_cast<uint32_t>(m.end - src) : 4u);
+                }
+            }
+        }
+    }
+}
+
+// add_mask_tile_row for a tile that copy_mask_rows has brought in and whose row may start `sh` (0 or 16) bits into its
+// first word; `extra` is the word behind the row's 64.
+__device__ __forceinline__ void add_mask_tile_row_shifted(float (&s)[kTile], uint32_t smask, uint32_t row, float to_score,
+                                                          uint32_t sh, uint32_t extra) {
+    const uint64_t ts2 = pack_f32x2(to_score, to_score);
+    uint32_t w[4], nx[4];
+    ld_shared_v4(smask + row * 128u + ((row & 7u) << 4), w);
+#pragma unroll
+    for (int c = 0; c < 16; ++c) {
+        if (c < 15)
+            ld_shared_v4(smask + ((c + 1) / 8) * (kTile * 128) + row * 128u + ((static_cast<uint32_t>((c + 1) % 8) ^ (row & 7u)) << 4), nx);
+        else
+            nx[0] = extra;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const uint32_t v = __funnelshift_r(w[e], e < 3 ? w[e < 3 ? e + 1 : 3] : nx[0], sh);
+            const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&v));
+            const int i = c * 8 + 2 * e;
+            unpack_f32x2(fma_f32x2(pack_f32x2(f.x, f.y), ts2, pack_f32x2(s[i], s[i + 1])), s[i], s[i + 1]);
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) w[e] = nx[e];
+    }
+}
+
 // What every mask row start of a call is aligned to: rows are L fp16 values apart from the base address.
 __device__ __forceinline__ uint32_t mask_row_alignment(const Params& p) {
     const uint32_t bits = (p.L * 2u) | static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p.mask));
@@ -608,6 +706,10 @@ fa_fwd_simple(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 #endif
 
 // ============================================================================ pipelined kernel
+// How the tiles of the additive mask come into shared memory: by TMA (every row starts on a 16-byte boundary), or
+// copied by warps of the CTA (copy_mask_rows).
+enum : int { kNoMask = 0, kMaskTma = 1, kMaskCopied = 2 };
+
 template <int H, bool kHasMask = false>
 struct PipeCfg {
     using G = TileGeom<H>;
@@ -621,8 +723,9 @@ struct PipeCfg {
     static constexpr int kQBytes = 2 * G::kTileBytes;  // two query tiles
     static constexpr int kRingBytes = kStages * G::kTileBytes;
     static constexpr int kMaskBytes = kHasMask ? kTile * kTile * 2 : 0;   // one 128 x 128 fp16 mask tile (two boxes of 64 keys)
+    static constexpr int kMaskExtraBytes = kHasMask ? kTile * 4 : 0;      // one word per row, see copy_mask_rows
     static constexpr int kStageBytes = 4 * 32 * 128;   // epilogue staging: per warp 32 rows x 64 fp16
-    static constexpr int kSmemBytes = kQBufs * kQBytes + kRingBytes + kMaskBytes + kStageBytes + 1024;  // + alignment slack
+    static constexpr int kSmemBytes = kQBufs * kQBytes + kRingBytes + kMaskBytes + kStageBytes + kMaskExtraBytes + 1024;  // + alignment slack
     static constexpr uint32_t kTmemCols = 512;
     // TMEM columns.  P (fp16, 64 columns per tile) has columns of its own instead of overwriting its
     // S: the next Q K^T of a tile then does not have to wait for the P V that reads P, only for the
@@ -638,6 +741,8 @@ struct PipeCfg {
     // Two MMA-issuing warps (one for Q K^T, one for P V) or one for both.  Measured: two win at
     // H = 128 (-3 % SM clocks), one, with its early barriers tested ahead, at H = 64 (-5 %).
     static constexpr bool kTwoIssuers = H == 128;
+    // Warps that copy the mask tiles TMA cannot fetch: 15, and 14 where it does not issue MMAs.
+    static constexpr uint32_t kMaskCopyWarps = kTwoIssuers ? 1 : 2;
     // How many 32-key chunks of exponentials a softmax thread takes into registers before it needs
     // the P buffer to be free of the previous step's P V.  Measured at H = 128: 1 (-2.4 %; 2 and 3
     // spill); at H = 64 holding any back costs more than it hides.
@@ -974,13 +1079,14 @@ __device__ __forceinline__ void merge_parts(const Params& p, uint32_t tail_item,
 // warps 0-3: softmax of query tile 0; 4-7: softmax of tile 1 (each also rescales its O rows in
 // the rare steps whose reference maximum moves); 8-11: epilogue (Y = O / l, or the hand-over and
 // merge of a partial segment); 12: MMA issue (one elected lane) and TMEM owner; 13: TMA producer
-// (one lane); 14: second MMA issuing warp at H = 128 (12 issues Q K^T, 14 issues P V); 15: idle.
+// (one lane); 14: second MMA issuing warp at H = 128 (12 issues Q K^T, 14 issues P V); 15: mask
+// tiles.
 //
 // Per tile and key step: Q K^T -> S; the softmax warps read S into registers and say so (SFREE),
 // which lets the next Q K^T into the S buffer; they write P into the tile's P columns once the
 // previous step's P V has read them (PV); P V accumulates into O.  Nothing of a tile's next Q K^T
-// waits for its P V.  With kHasMask the softmax warps add the additive mask row (read with 16-byte
-// loads) to the scores they have just read.
+// waits for its P V.  With kHasMask the softmax warps add their row of the mask tile, which warp 15 (and 14 where it
+// issues nothing) has brought into shared memory, to the scores they have just read.
 //
 // Barrier phases (the parity to wait for is the low bit of the index):
 //   per global step g:  S_i (MMA -> softmax), SFREE (softmax -> MMA; at H = 128 one barrier whose
@@ -994,11 +1100,12 @@ __device__ __forceinline__ void merge_parts(const Params& p, uint32_t tail_item,
 // for the previous kernel and at its end, and its SM clock count in between, in Params::cycles (a
 // diagnostic: the clock count compares versions of the kernel independently of the clock the GPU happens
 // to run at, the timer shows the gaps between launches; absent from normal builds).
-template <int H, bool kHasMask>
+template <int H, int kMask>
 __global__ void __launch_bounds__(512, 1)
 fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmY,
                  const __grid_constant__ CUtensorMap tmM, const Params p) {
+    constexpr bool kHasMask = kMask != kNoMask;
     using G = TileGeom<H>;
     using C = PipeCfg<H, kHasMask>;
     constexpr int NS = C::kStages;
@@ -1049,6 +1156,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t sRing = smem_base + C::kQBufs * C::kQBytes;   // NS tiles
     const uint32_t sMask = sRing + C::kRingBytes;    // one mask tile (instances with a mask only)
     const uint32_t sStage = sMask + C::kMaskBytes;   // epilogue staging, 4 KiB per epilogue warp
+    const uint32_t sMaskExtra = sStage + C::kStageBytes;   // a word per mask row (instances with a mask only)
     const uint32_t bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8u * i; };
     // Segment k's query tiles: buffer k mod kQBufs; its barriers complete one phase per use of that buffer.
@@ -1097,7 +1205,10 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const bool per_warp = (i == BAR_P0 || i == BAR_P1 || i == BAR_SFREE0 || i == BAR_SFREE1 ||
                                    i == BAR_A0 || i == BAR_A1 || i == BAR_EPI || i == BAR_MEMPTY0 || i == BAR_MEMPTY1 ||
                                    i == BAR_OFREE0 || i == BAR_OFREE1);
-            mbar_init(bar(i), per_warp ? 4u : 1u);
+            uint32_t count = per_warp ? 4u : 1u;
+            // mask tiles by cp.async: every lane of a copying warp when its copies have landed, and one for the warp
+            if (kMask == kMaskCopied && (i == BAR_MFULL0 || i == BAR_MFULL1)) count = 33u * C::kMaskCopyWarps;
+            mbar_init(bar(i), count);
         }
         abort_flag = 0;
 #pragma unroll
@@ -1106,7 +1217,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         prefetch_tensormap(&tmQ);
         prefetch_tensormap(&tmK);
         prefetch_tensormap(&tmV);
-        if constexpr (kHasMask) prefetch_tensormap(&tmM);
+        if constexpr (kMask == kMaskTma) prefetch_tensormap(&tmM);
     }
 #ifdef FA_DEBUG
     dbg_begin(p, ctl, smem_base, C::kSmemBytes - 1024);
@@ -1159,15 +1270,10 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const Seg sg = get_seg(pl_s, t0, p, k);
             m = -INFINITY;
             l = 0.f;
-            // with a mask: the row of mask[batch] this thread adds to its scores
-            const __half* mask_row = nullptr;
-            uint32_t mask_vec = 2;
-            if constexpr (kHasMask) {
-                const uint32_t q_row = ((sg.item % q_pairs) * 2u + i) * kTile + row;
-                const uint32_t batch = (sg.item / q_pairs) / p.R;
-                if (q_row < p.L) mask_row = p.mask + (static_cast<size_t>(batch) * p.L + q_row) * p.L;
-                mask_vec = mask_row_alignment(p);
-            }
+            // how far into its first word this thread's mask row starts
+            uint32_t mask_sh = 0;
+            if constexpr (kMask == kMaskCopied)
+                mask_sh = mask_row_shift(p, (sg.item / q_pairs) / p.R, ((sg.item % q_pairs) * 2u + i) * kTile + row);
             for (uint32_t jj = 0; jj < sg.len; ++jj, ++g) {
                 const uint32_t j = sg.j0 + jj;
                 mbar_wait(bar(BAR_S0 + i), g & 1u, ctl, kRoleSoftmax | (BAR_S0 + i));
@@ -1190,17 +1296,15 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     }
                 }
                 if constexpr (kHasMask) {
-                    if (p.mask_tma != 0u) {
-                        // The mask tile of this tile and step, brought in by TMA into the one mask buffer; it is
-                        // handed back as soon as it has been read.
-                        mbar_wait(bar(BAR_MFULL0 + i), g & 1u, ctl, kRoleSoftmax | (BAR_MFULL0 + i));
+                    // The mask tile of this tile and step, brought in by TMA or by the copying warps into the one
+                    // mask buffer; it is handed back as soon as it has been read.
+                    mbar_wait(bar(BAR_MFULL0 + i), g & 1u, ctl, kRoleSoftmax | (BAR_MFULL0 + i));
+                    if constexpr (kMask == kMaskCopied)
+                        add_mask_tile_row_shifted(s, sMask, row, p.mask_to_score, mask_sh, ld_shared_u32(sMaskExtra + row * 4u));
+                    else
                         add_mask_tile_row(s, sMask, row, p.mask_to_score);
-                        __syncwarp();
-                        if (lane == 0) mbar_arrive(bar(BAR_MEMPTY0 + i));
-                    } else if (mask_row != nullptr) {
-                        add_mask_row(s, mask_row + static_cast<size_t>(j) * kTile,
-                                     min(static_cast<int>(p.L - j * kTile), kTile), p.mask_to_score, mask_vec);
-                    }
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(bar(BAR_MEMPTY0 + i));
                 }
                 if (ragged) mask_tail(s, static_cast<int>(p.L - j * kTile));
                 if (first) m = row_max(s);   // first key tile of the segment: the reference is its row maximum
@@ -1734,7 +1838,35 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     }
                 }
             }
-        } else if (kHasMask && warp == 15 && p.mask_tma != 0u && elect_one()) {
+        } else if (kMask == kMaskCopied && warp >= 16u - C::kMaskCopyWarps) {
+            // -------------------------------------------------------------- copies of mask tiles that TMA cannot fetch
+            // The same order as below; each copying warp takes its share of the 128 rows.
+            constexpr uint32_t kRows = kTile / C::kMaskCopyWarps;
+            const uint32_t r0 = (15u - warp) * kRows;
+            const MaskRows mr = mask_rows(p);
+            uint32_t g = 0;
+            bool stop = false;
+            for (uint32_t k = 0; k < nseg && !stop; ++k) {
+                const Seg sg = get_seg(pl_s, t0, p, k);
+                const uint32_t batch = (sg.item / q_pairs) / p.R, q0 = (sg.item % q_pairs) * 2u * kTile;
+                for (uint32_t jj = 0; jj < sg.len && !stop; ++jj, ++g) {
+                    for (uint32_t i = 0; i < 2; ++i) {
+                        bool ok = true;
+                        if (i == 1) ok = mbar_wait(bar(BAR_MEMPTY0), g & 1u, ctl, kRoleProducer | BAR_MEMPTY0);
+                        else if (g > 0) ok = mbar_wait(bar(BAR_MEMPTY1), (g - 1u) & 1u, ctl, kRoleProducer | BAR_MEMPTY1);
+                        if (__any_sync(0xffffffffu, !ok)) {
+                            stop = true;
+                            break;
+                        }
+                        copy_mask_rows<kRows>(p, mr, sMask, sMaskExtra, batch, q0 + i * kTile, (sg.j0 + jj) * kTile, r0, lane);
+                        cp_async_arrive(bar(BAR_MFULL0 + i));
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar(BAR_MFULL0 + i));
+                    }
+                }
+            }
+            cp_async_wait_all();
+        } else if (kMask == kMaskTma && warp == 15 && elect_one()) {
             // -------------------------------------------------------------- TMA producer of the mask tiles
             // One buffer, filled for tile 0 and tile 1 of every key step in turn, each time as soon as the softmax
             // warps of the tile before have read it: tile 1 of step g follows tile 0 of step g, tile 0 of step g
