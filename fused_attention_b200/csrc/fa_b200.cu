@@ -214,13 +214,11 @@ int validate(const void* q, const void* k, const void* v, const void* mask, cons
     return FA_B200_OK;
 }
 
-// 1 = simple kernel, 2 = pipelined kernel.
+// 1 = simple kernel, 2 = pipelined kernel (or the one on pairs of CTAs, see use_pair_kernel).
 int select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool has_mask, uint32_t flags,
                   int sm_count) {
     if (flags & FA_B200_FLAG_FORCE_SIMPLE) return 1;
     if (flags & (FA_B200_FLAG_FORCE_PIPELINED | FA_B200_FLAG_FORCE_PAIR)) return 2;
-    (void)has_mask;   // both kernels take the additive mask
-    if (H < 64) return 1;
     // The pipelined kernel works on items of two query tiles (256 rows) on persistent CTAs.  It wins
     // as soon as there are enough items to occupy a good part of the SMs (measured: 39 vs 57 us on
     // B=64 R=16 L=197 H=64); a single partial tile or a handful of items goes to the simple kernel,
@@ -228,9 +226,13 @@ int select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool has_mask,
     // With few items the two are level up to about five key steps (7-14 us, mostly launch); from
     // there on the pipelined kernel wins however few items there are (measured: B=1 R=16 L=1024 H=128
     // 20.5 vs 24.6 us, B=1 R=4 L=2048 32.8 vs 41.9 us, B=1 R=2 L=4096 57 vs 79 us).
+    // At H = 16 and 32, where a tile is cheap to load, they are level up to two key steps only (H = 32, B=1 R=4 L=256
+    // 7.7 vs 7.4 us, L=512 8.5 vs 9.2 us; H = 16, B=8 R=16 L=1024 49.0 vs 67.6 us).
+    // With a mask the pipelined kernel is ahead from the second tile on: its other warps bring the mask in
+    // (H = 32, B=1 R=4 L=129 9.7 vs 11.6 us, L=256 7.7 vs 10.1 us, L=1024 17.6 vs 34.9 us).
     const uint64_t pairs = static_cast<uint64_t>((L + 255) / 256) * (F / H) * B;
     if (L <= 128) return 1;
-    if (L > 5 * 128) return 2;
+    if (has_mask || L > (H >= 64 ? 5u : 2u) * 128u) return 2;
     if (pairs * 2 < static_cast<uint64_t>(sm_count)) return 1;
     return 2;
 }
@@ -314,12 +316,12 @@ int launch_simple(DeviceCtx& c, int slot, const CUtensorMap& mq, const CUtensorM
     return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 
-template <int H, int M>
+template <int H, int kMask>
 int launch_pipelined(DeviceCtx& c, int slot, const CUtensorMap& mq, const CUtensorMap& mk,
                      const CUtensorMap& mv, const CUtensorMap& my, const CUtensorMap& mm, const Params& p,
                      uint32_t n_ctas, cudaStream_t st, bool overlap) {
-    constexpr int smem = fa::PipeCfg<H, M != fa::kNoMask>::kSmemBytes;
-    auto kern = fa::fa_fwd_pipelined<H, M>;
+    constexpr int smem = fa::PipeCfg<H, kMask != fa::kNoMask>::kSmemBytes;
+    auto kern = fa::fa_fwd_pipelined<H, kMask>;
     if (!(c.attr_done.load(std::memory_order_acquire) & (1u << slot))) {   // setting it twice is harmless
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return static_cast<int>(e);
@@ -328,6 +330,15 @@ int launch_pipelined(DeviceCtx& c, int slot, const CUtensorMap& mq, const CUtens
     const dim3 grid(n_ctas, 1, 1);   // persistent: at most one CTA per SM
     const cudaError_t e = launch_kernel(kern, grid, 512, smem, st, overlap, mq, mk, mv, my, mm, p);
     return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+}
+// The instance for a call with or without a mask; `slot`, slot + 1 and slot + 2 are its attribute bits.
+template <int H>
+int launch_pipelined(DeviceCtx& c, int slot, const void* mask, bool mask_tma, const CUtensorMap& mq, const CUtensorMap& mk,
+                     const CUtensorMap& mv, const CUtensorMap& my, const CUtensorMap& mm, const Params& p,
+                     uint32_t n_ctas, cudaStream_t st, bool overlap) {
+    if (mask == nullptr) return launch_pipelined<H, fa::kNoMask>(c, slot, mq, mk, mv, my, mm, p, n_ctas, st, overlap);
+    if (mask_tma) return launch_pipelined<H, fa::kMaskTma>(c, slot + 1, mq, mk, mv, my, mm, p, n_ctas, st, overlap);
+    return launch_pipelined<H, fa::kMaskCopied>(c, slot + 2, mq, mk, mv, my, mm, p, n_ctas, st, overlap);
 }
 
 // The split-scratch buffer of `st` on this device: the one it already has, else a free one, else none.
@@ -375,7 +386,7 @@ int launch_pair(DeviceCtx& c, const CUtensorMap& mq, const CUtensorMap& mkh, con
                 const CUtensorMap& my, const CUtensorMap& mm, const Params& p, uint32_t n_quad_items,
                 cudaStream_t st, bool overlap, bool* launched) {
     constexpr int smem = fa::PairCfgT<kHasMask>::kSmemBytes;
-    constexpr int slot = kHasMask ? 13 : 12;
+    constexpr int slot = kHasMask ? 9 : 8;
     auto kern = fa::fa_fwd_pair<kHasMask>;
     *launched = false;
     if (!(c.attr_done.load(std::memory_order_acquire) & (1u << slot))) {
@@ -512,15 +523,12 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                         }
                     }
                     if (rc == FA_B200_OK && !done) {
-                        if (mask_tma)
-                            rc = H == 128 ? launch_pipelined<128, fa::kMaskTma>(*c, 10, mq, mk, mv, my, mm, p, sch.grid, st, overlap)
-                                          : launch_pipelined<64, fa::kMaskTma>(*c, 11, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
-                        else if (mask)
-                            rc = H == 128 ? launch_pipelined<128, fa::kMaskCopied>(*c, 14, mq, mk, mv, my, mm, p, sch.grid, st, overlap)
-                                          : launch_pipelined<64, fa::kMaskCopied>(*c, 15, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
-                        else
-                            rc = H == 128 ? launch_pipelined<128, fa::kNoMask>(*c, 8, mq, mk, mv, my, mm, p, sch.grid, st, overlap)
-                                          : launch_pipelined<64, fa::kNoMask>(*c, 9, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
+                        switch (H) {
+                            case 16: rc = launch_pipelined<16>(*c, 14, mask, mask_tma, mq, mk, mv, my, mm, p, sch.grid, st, overlap); break;
+                            case 32: rc = launch_pipelined<32>(*c, 17, mask, mask_tma, mq, mk, mv, my, mm, p, sch.grid, st, overlap); break;
+                            case 64: rc = launch_pipelined<64>(*c, 20, mask, mask_tma, mq, mk, mv, my, mm, p, sch.grid, st, overlap); break;
+                            default: rc = launch_pipelined<128>(*c, 23, mask, mask_tma, mq, mk, mv, my, mm, p, sch.grid, st, overlap); break;
+                        }
                     }
                 } else if (mask) {
                     switch (H) {
@@ -981,7 +989,8 @@ int fa_b200_describe_schedule(uint32_t B, uint32_t L, uint32_t F, uint32_t head_
     if (rc != FA_B200_OK) return rc;
     const uint32_t n = (L + fa::kTile - 1) / fa::kTile;
     const uint32_t n_items = ((L + 2 * fa::kTile - 1) / (2 * fa::kTile)) * (F / head_dim) * B;
-    const int which = select_kernel(B, L, F, head_dim, false, flags, static_cast<int>(sm_count));
+    // (head_dim 16 and 32: reported as one CTA per query tile, see the header)
+    const int which = head_dim < 64 ? 1 : select_kernel(B, L, F, head_dim, false, flags, static_cast<int>(sm_count));
     out[0] = static_cast<uint32_t>(which);
     out[5] = n;
     if (which != 2) {
@@ -1021,7 +1030,7 @@ int fa_b200_select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t head_dim,
         (void)cudaGetLastError();
         sms = 148;
     }
-    const int which = select_kernel(B, L, F, head_dim, has_mask != 0, flags, sms);
+    const int which = head_dim < 64 ? 1 : select_kernel(B, L, F, head_dim, has_mask != 0, flags, sms);
     if (which != 2) return which;
     const uint32_t n = (L + fa::kTile - 1) / fa::kTile, q_pairs = (L + 2 * fa::kTile - 1) / (2 * fa::kTile);
     const Schedule s = make_schedule(q_pairs * (F / head_dim) * B, n, static_cast<uint32_t>(sms),

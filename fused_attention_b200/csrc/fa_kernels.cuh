@@ -8,7 +8,7 @@
 //                               (2 softmax warpgroups, 1 epilogue warpgroup, 1 or 2 MMA warps, 1 TMA
 //                               warp, 1 warp for the mask tiles); K/V stream through a shared-memory
 //                               ring; the softmax of one tile overlaps the MMAs of the other.
-//                               H in {64, 128}.
+//                               Every head_dim.
 // fa_pair.cuh holds a third, fa_fwd_pair<kHasMask>: the same roles on pairs of CTAs at H = 128.
 //
 // What they replace in the reference (include/fused_attn.cuh): attention_kernel (605-858) and the
@@ -714,24 +714,24 @@ template <int H, bool kHasMask = false>
 struct PipeCfg {
     using G = TileGeom<H>;
     // ring slots of one K or V tile each; with a mask a quarter of the ring makes room for one mask tile
-    static constexpr int kStages = (H == 128 ? 4 : 8) * (kHasMask ? 3 : 4) / 4;
-    // Buffers for the two query tiles of a segment.  With two of them (H = 64, where they fit) the next segment's
+    static constexpr int kStages = (H == 128 ? 4 : 8) * (kHasMask && H >= 64 ? 3 : 4) / 4;   // (tiles of H < 64 leave room for both)
+    // Buffers for the two query tiles of a segment.  With two of them (H <= 64, where they fit) the next segment's
     // query tiles, and behind them its K and V tiles, are on their way while this segment still multiplies: the
     // producer no longer stops at every segment boundary until the last Q K^T has let go of the one buffer.
     // Measured: 1 to 1.5 % fewer SM clocks per CTA on shapes of two to sixteen key steps per segment.
-    static constexpr int kQBufs = H == 64 ? 2 : 1;
+    static constexpr int kQBufs = H <= 64 ? 2 : 1;
     static constexpr int kQBytes = 2 * G::kTileBytes;  // two query tiles
     static constexpr int kRingBytes = kStages * G::kTileBytes;
     static constexpr int kMaskBytes = kHasMask ? kTile * kTile * 2 : 0;   // one 128 x 128 fp16 mask tile (two boxes of 64 keys)
     static constexpr int kMaskExtraBytes = kHasMask ? kTile * 4 : 0;      // one word per row, see copy_mask_rows
-    static constexpr int kStageBytes = 4 * 32 * 128;   // epilogue staging: per warp 32 rows x 64 fp16
+    static constexpr int kStageBytes = 4 * 32 * 128;   // epilogue staging: per warp 32 rows x up to 64 fp16
     static constexpr int kSmemBytes = kQBufs * kQBytes + kRingBytes + kMaskBytes + kStageBytes + kMaskExtraBytes + 1024;  // + alignment slack
     static constexpr uint32_t kTmemCols = 512;
     // TMEM columns.  P (fp16, 64 columns per tile) has columns of its own instead of overwriting its
     // S: the next Q K^T of a tile then does not have to wait for the P V that reads P, only for the
     // softmax warps to have read S, and a tile's softmax passes follow one another without its MMAs
     // in between.
-    //   H = 64:   S0 [0,128)  S1 [128,256)  O0 [256,320)  P0 [320,384)  O1 [384,448)  P1 [448,512)
+    //   H <= 64:  S0 [0,128)  S1 [128,256)  O0 [256,320)  P0 [320,384)  O1 [384,448)  P1 [448,512) (O: the first H of 64)
     //   H = 128:  S  [0,128) shared by the two tiles, which use it in turn (scores only live from the
     //             Q K^T until the softmax warps have read them), P0 [128,192)  P1 [192,256)
     //             O0 [256,384)  O1 [384,512)
@@ -917,14 +917,15 @@ __device__ __forceinline__ void merge_two(const Params& p, uint32_t tail_item, u
     const bool first = mine == 0u;   // parts are added in the order of the key axis
     const float w0 = first ? w_m : w_o, w1 = first ? w_o : w_m;
     const float inv_l = 1.f / fmaf(w1, first ? ml_o.y : l_mine, fmaf(w0, first ? l_mine : ml_o.y, 0.f));
+    constexpr int W = H < 32 ? H : 32;   // columns at a time
 #pragma unroll
-    for (int q = 0; q < H / 32; ++q) {
-        float o[32];
-        tmem_ld32(tO + q * 32, o);
+    for (int q = 0; q < H / W; ++q) {
+        float o[W];
+        tmem_ld<W>(tO + q * W, o);
         tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-            const float xs[4] = {x[q * 8 + c].x, x[q * 8 + c].y, x[q * 8 + c].z, x[q * 8 + c].w};
+        for (int c = 0; c < W / 4; ++c) {
+            const float xs[4] = {x[q * (W / 4) + c].x, x[q * (W / 4) + c].y, x[q * (W / 4) + c].z, x[q * (W / 4) + c].w};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float a0 = first ? o[4 * c + e] : xs[e], a1 = first ? xs[e] : o[4 * c + e];
@@ -933,13 +934,13 @@ __device__ __forceinline__ void merge_two(const Params& p, uint32_t tail_item, u
         }
         if (row_valid) {
 #pragma unroll
-            for (int e = 0; e < 32; e += 8) {
+            for (int e = 0; e < W; e += 8) {
                 uint4 wv;
                 wv.x = pack_half2(o[e], o[e + 1]);
                 wv.y = pack_half2(o[e + 2], o[e + 3]);
                 wv.z = pack_half2(o[e + 4], o[e + 5]);
                 wv.w = pack_half2(o[e + 6], o[e + 7]);
-                *reinterpret_cast<uint4*>(y_row + q * 32 + e) = wv;
+                *reinterpret_cast<uint4*>(y_row + q * W + e) = wv;
             }
         }
     }
@@ -980,33 +981,34 @@ __device__ __forceinline__ void merge_parts(const Params& p, uint32_t tail_item,
         if (pp < po.parts) l_all = fmaf(w[pp], lp[pp], l_all);
     }
     const float inv_l = 1.f / l_all;
+    constexpr int W = H < 64 ? H : 64, W2 = W < 32 ? W : 32;   // columns at a time: in flight, from TMEM
     if (po.parts == 3u && mine < 3u) {
         // Three parts, one of them in TMEM: half a row of both others in flight at a time.  In key order
         // the parts are (o, a, b), (a, o, b) or (a, b, o) with o the one in TMEM.
         const uint32_t sa = mine == 0u ? slot[1] : slot[0], sb = mine == 2u ? slot[1] : slot[2];
 #pragma unroll 1
-        for (int half = 0; half < H / 64; ++half) {
-            float xa[64], xb[64];
-            const float4* pa = p.part_o + part_o_index<H>(sa, tile, row) + (half * 16) * kTile;
-            const float4* pb = p.part_o + part_o_index<H>(sb, tile, row) + (half * 16) * kTile;
+        for (int half = 0; half < H / W; ++half) {
+            float xa[W], xb[W];
+            const float4* pa = p.part_o + part_o_index<H>(sa, tile, row) + (half * (W / 4)) * kTile;
+            const float4* pb = p.part_o + part_o_index<H>(sb, tile, row) + (half * (W / 4)) * kTile;
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
+            for (int c = 0; c < W / 4; ++c) {
                 const float4 v = __ldcg(pa + c * kTile);
                 xa[4 * c] = v.x; xa[4 * c + 1] = v.y; xa[4 * c + 2] = v.z; xa[4 * c + 3] = v.w;
             }
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
+            for (int c = 0; c < W / 4; ++c) {
                 const float4 v = __ldcg(pb + c * kTile);
                 xb[4 * c] = v.x; xb[4 * c + 1] = v.y; xb[4 * c + 2] = v.z; xb[4 * c + 3] = v.w;
             }
 #pragma unroll
-            for (int sub = 0; sub < 2; ++sub) {
-                float o[32];
-                tmem_ld32(tO + half * 64 + sub * 32, o);
+            for (int sub = 0; sub < W / W2; ++sub) {
+                float o[W2];
+                tmem_ld<W2>(tO + half * W + sub * W2, o);
                 tmem_wait_ld();
 #pragma unroll
-                for (int e = 0; e < 32; ++e) {
-                    const float a = xa[sub * 32 + e], bq = xb[sub * 32 + e];
+                for (int e = 0; e < W2; ++e) {
+                    const float a = xa[sub * W2 + e], bq = xb[sub * W2 + e];
                     const float v0 = mine == 0u ? o[e] : a;
                     const float v1 = mine == 0u ? a : (mine == 1u ? o[e] : bq);
                     const float v2 = mine == 2u ? o[e] : bq;
@@ -1014,13 +1016,13 @@ __device__ __forceinline__ void merge_parts(const Params& p, uint32_t tail_item,
                 }
                 if (row_valid) {
 #pragma unroll
-                    for (int e = 0; e < 32; e += 8) {
+                    for (int e = 0; e < W2; e += 8) {
                         uint4 wv;
                         wv.x = pack_half2(o[e], o[e + 1]);
                         wv.y = pack_half2(o[e + 2], o[e + 3]);
                         wv.z = pack_half2(o[e + 4], o[e + 5]);
                         wv.w = pack_half2(o[e + 6], o[e + 7]);
-                        *reinterpret_cast<uint4*>(y_row + half * 64 + sub * 32 + e) = wv;
+                        *reinterpret_cast<uint4*>(y_row + half * W + sub * W2 + e) = wv;
                     }
                 }
             }
@@ -1030,41 +1032,41 @@ __device__ __forceinline__ void merge_parts(const Params& p, uint32_t tail_item,
     // Every part from scratch (an epilogue warp's part was the last of its item): half a row of two
     // parts in flight at a time, the third, if there is one, behind them.
 #pragma unroll 1
-    for (int half = 0; half < H / 64; ++half) {
-        float xa[64], xb[64];
-        const float4* pa = p.part_o + part_o_index<H>(slot[0], tile, row) + (half * 16) * kTile;
-        const float4* pb = p.part_o + part_o_index<H>(slot[1], tile, row) + (half * 16) * kTile;
+    for (int half = 0; half < H / W; ++half) {
+        float xa[W], xb[W];
+        const float4* pa = p.part_o + part_o_index<H>(slot[0], tile, row) + (half * (W / 4)) * kTile;
+        const float4* pb = p.part_o + part_o_index<H>(slot[1], tile, row) + (half * (W / 4)) * kTile;
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
+        for (int c = 0; c < W / 4; ++c) {
             const float4 v = __ldcg(pa + c * kTile);
             xa[4 * c] = v.x; xa[4 * c + 1] = v.y; xa[4 * c + 2] = v.z; xa[4 * c + 3] = v.w;
         }
 #pragma unroll
-        for (int c = 0; c < 16; ++c) {
+        for (int c = 0; c < W / 4; ++c) {
             const float4 v = __ldcg(pb + c * kTile);
             xb[4 * c] = v.x; xb[4 * c + 1] = v.y; xb[4 * c + 2] = v.z; xb[4 * c + 3] = v.w;
         }
 #pragma unroll
-        for (int e = 0; e < 64; ++e) xa[e] = fmaf(w[1], xb[e], fmaf(w[0], xa[e], 0.f));
+        for (int e = 0; e < W; ++e) xa[e] = fmaf(w[1], xb[e], fmaf(w[0], xa[e], 0.f));
         if (po.parts > 2u) {
-            const float4* pc = p.part_o + part_o_index<H>(slot[2], tile, row) + (half * 16) * kTile;
+            const float4* pc = p.part_o + part_o_index<H>(slot[2], tile, row) + (half * (W / 4)) * kTile;
 #pragma unroll
-            for (int c = 0; c < 16; ++c) {
+            for (int c = 0; c < W / 4; ++c) {
                 const float4 v = __ldcg(pc + c * kTile);
                 xb[4 * c] = v.x; xb[4 * c + 1] = v.y; xb[4 * c + 2] = v.z; xb[4 * c + 3] = v.w;
             }
 #pragma unroll
-            for (int e = 0; e < 64; ++e) xa[e] = fmaf(w[2], xb[e], xa[e]);
+            for (int e = 0; e < W; ++e) xa[e] = fmaf(w[2], xb[e], xa[e]);
         }
         if (row_valid) {
 #pragma unroll
-            for (int e = 0; e < 64; e += 8) {
+            for (int e = 0; e < W; e += 8) {
                 uint4 wv;
                 wv.x = pack_half2(xa[e] * inv_l, xa[e + 1] * inv_l);
                 wv.y = pack_half2(xa[e + 2] * inv_l, xa[e + 3] * inv_l);
                 wv.z = pack_half2(xa[e + 4] * inv_l, xa[e + 5] * inv_l);
                 wv.w = pack_half2(xa[e + 6] * inv_l, xa[e + 7] * inv_l);
-                *reinterpret_cast<uint4*>(y_row + half * 64 + e) = wv;
+                *reinterpret_cast<uint4*>(y_row + half * W + e) = wv;
             }
         }
     }
@@ -1508,17 +1510,18 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const int32_t row0 = static_cast<int32_t>((q_pair * 2u + i) * kTile + wq * 32u);
                 if (!sg.partial) {
                     const float inv_l = 1.f / l_row;
+                    constexpr int W = G::kBoxCols;   // columns of one staging buffer and store
 #pragma unroll
-                    for (int half = 0; half < H / 64; ++half) {
+                    for (int half = 0; half < H / W; ++half) {
                         // the previous store out of this staging buffer must have read it completely
                         if (lane == 0) bulk_wait_read_all();
                         __syncwarp();
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) {   // 16 columns at a time keeps this role within 64 registers
+                        for (int c = 0; c < W / 16; ++c) {   // 16 columns at a time keeps this role within 64 registers
                             float o[16];
-                            tmem_ld16(tO + half * 64 + c * 16, o);
+                            tmem_ld16(tO + half * W + c * 16, o);
                             tmem_wait_ld();
-                            if (half == H / 64 - 1 && c == 3) {
+                            if (half == H / W - 1 && c == W / 16 - 1) {
                                 // the whole O tile has left TMEM: the MMA warp may overwrite it
                                 tc_fence_before();
                                 __syncwarp();
@@ -1530,15 +1533,16 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                                 const uint32_t w1 = pack_half2(o[v4 * 8 + 2] * inv_l, o[v4 * 8 + 3] * inv_l);
                                 const uint32_t w2 = pack_half2(o[v4 * 8 + 4] * inv_l, o[v4 * 8 + 5] * inv_l);
                                 const uint32_t w3 = pack_half2(o[v4 * 8 + 6] * inv_l, o[v4 * 8 + 7] * inv_l);
-                                // logical 16-byte chunk c*2+v4 of row `lane`, 128-byte swizzle
-                                const uint32_t chunk = static_cast<uint32_t>(c * 2 + v4) ^ (lane & 7u);
-                                st_shared_v4(stage + lane * 128u + chunk * 16u, w0, w1, w2, w3);
+                                // logical 16-byte chunk c*2+v4 of row `lane`; the swizzle of rows of kSwz bytes takes
+                                // the chunk's low bits with the bits of the address from bit 7 on
+                                const uint32_t chunk = static_cast<uint32_t>(c * 2 + v4) ^ ((lane * G::kSwz >> 7) & (G::kSwz / 16u - 1u));
+                                st_shared_v4(stage + lane * G::kSwz + chunk * 16u, w0, w1, w2, w3);
                             }
                         }
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0 && row0 < static_cast<int32_t>(p.L)) {   // rows past L are clipped by the store
-                            tma_store_3d(&tmY, stage, static_cast<int32_t>(head * H + half * 64), row0,
+                            tma_store_3d(&tmY, stage, static_cast<int32_t>(head * H + half * W), row0,
                                          static_cast<int32_t>(batch));
                             bulk_commit_group();
                         }

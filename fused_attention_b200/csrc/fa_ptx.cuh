@@ -423,6 +423,12 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
         : "r"(taddr)
         : "memory");
 }
+template <int N>
+__device__ __forceinline__ void tmem_ld(uint32_t taddr, float* v) {
+    static_assert(N == 16 || N == 32, "columns per load");
+    if constexpr (N == 32) tmem_ld32(taddr, v);
+    else tmem_ld16(taddr, v);
+}
 __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float* v) {
     FA_DBG_TMEM(taddr, 32u);
     asm volatile(

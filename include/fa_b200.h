@@ -210,7 +210,8 @@ int fa_b200_debug_cycles(void* device_buffer_of_256_u64);
 
 /*
  * Which kernel the default heuristics pick for a shape: returns 1 for the one-tile-per-CTA
- * kernel, 2 for the warp-specialised kernel, 3 for the warp-specialised kernel on pairs of CTAs
+ * kernel (and always for head_dim 16 and 32, which the flags cannot force onto another one; by
+ * default they are served by either), 2 for the warp-specialised kernel, 3 for the warp-specialised kernel on pairs of CTAs
  * (head_dim 128, whole work items; a mask is taken to start on a 16-byte boundary, its rows then
  * do so whenever L is a multiple of 8), negative status on invalid arguments.
  * No counterpart in the reference.
@@ -220,7 +221,8 @@ int fa_b200_select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t head_dim,
 
 /*
  * How the warp-specialised kernel would spread a call's work over its CTAs on a device with
- * `sm_count` SMs: out[0] = kernel (1, 2 or 3, as fa_b200_select_kernel; for 3 a work item is 512 query
+ * `sm_count` SMs (head_dim 64 and 128; smaller ones are described as one CTA per query tile):
+ * out[0] = kernel (1, 2 or 3, as fa_b200_select_kernel; for 3 a work item is 512 query
  * rows and out[1] CTAs form out[1]/2 pairs, nothing is divided), out[1] = CTAs launched,
  * out[2] = rounds of whole work items (a work item is 256 query rows of one (batch, head) against
  * all keys; CTA c takes items c, c + out[1], ...), out[3] = work items of the last, partial round

@@ -32,7 +32,7 @@ def assert_close(y, expected):
     assert m["max_abs"] <= MAX_ABS_TOL and m["mean_abs"] <= MEAN_ABS_TOL, m
 
 
-@pytest.mark.parametrize("H", [64, 128])
+@pytest.mark.parametrize("H", [16, 32, 64, 128])
 @pytest.mark.parametrize("L", [1, 2, 127, 129, 131, 255, 257, 388, 390, 391, 1021])
 @pytest.mark.parametrize("offset", [0, 1, 2, 3, 4])
 def test_mask_rows_that_tma_cannot_fetch(H, L, offset):
@@ -45,4 +45,4 @@ def test_mask_rows_that_tma_cannot_fetch(H, L, offset):
     store = torch.full((offset + mask.numel(),), float("nan"), dtype=torch.float16, device="cuda")
     on_gpu = store[offset:].view_as(mask)
     on_gpu.copy_(mask)
-    assert_close(run(q, k, v, H, on_gpu, ONE), oracle(q, k, v, H, mask))
+    assert_close(run(q, k, v, H, on_gpu, ONE if H >= 64 else 0), oracle(q, k, v, H, mask))
