@@ -1336,7 +1336,9 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     // row's maximum, which is what costs 64 instructions per row and step).
                     float mx = m;
                     bool moved = false;
-                    if (__any_sync(0xffffffffu, sum > kLazyRescaleSum)) {
+                    // (A row that has had nothing but -inf so far takes the maximum of its first finite scores as its
+                    // reference, as a row without a mask takes that of its first tile.)
+                    if (__any_sync(0xffffffffu, sum > kLazyRescaleSum || (kHasMask && m == -INFINITY))) {
                         mx = row_max(s);
                         moved = (mx - m) * c > kLazyRescaleLog2;
                     }

@@ -46,3 +46,17 @@ def test_mask_rows_that_tma_cannot_fetch(H, L, offset):
     on_gpu = store[offset:].view_as(mask)
     on_gpu.copy_(mask)
     assert_close(run(q, k, v, H, on_gpu, ONE if H >= 64 else 0), oracle(q, k, v, H, mask))
+
+
+@pytest.mark.parametrize("H,flags", [(32, 0), (64, ONE), (128, ONE), (128, _lib.FLAG_FORCE_PAIR)])
+def test_rows_whose_first_tiles_are_masked_and_whose_scores_are_far_below_zero(H, flags):
+    """Left padding of more than a key tile, and scores around -40 in the exp2 domain: against a reference of 0 instead
+    of the row's own maximum every P would be lost in fp16."""
+    B, L = 2, 520
+    q, k, v = make_inputs(B, L, 2 * H, 1.0, 7)
+    q = q.abs() * 0 + 1.0
+    k = k * 0.25 - 28.0 / H ** 0.5                     # q.k / sqrt(H) around -28
+    mask = torch.zeros(B, L, L, dtype=torch.float16)
+    mask[0, :, :130] = float("-inf")
+    mask[1, :, :400] = float("-inf")
+    assert_close(run(q, k, v, H, mask.cuda(), flags), oracle(q, k, v, H, mask))
