@@ -17,6 +17,7 @@
 
 #include "fa_b200.h"
 #include "fa_kernels.cuh"
+#include "fa_mask_plan.cuh"
 #include "fa_pair.cuh"
 
 namespace {
@@ -149,8 +150,8 @@ int ensure_ctx(int device, DeviceCtx** out) {
 
 // 3-D map {F, L, B} over a contiguous [B, L, F] fp16 array; box = 128 rows x min(H, 64) columns.
 int make_map(CUtensorMap* map, const void* base, uint32_t B, uint32_t L, uint32_t F, uint32_t H,
-             uint32_t box_rows = static_cast<uint32_t>(fa::kTile)) {
-    const uint32_t box_cols = H < 64 ? H : 64;
+             uint32_t box_rows = static_cast<uint32_t>(fa::kTile), uint32_t max_cols = 64) {
+    const uint32_t box_cols = H < max_cols ? H : max_cols;
     const cuuint64_t dims[3] = {F, L, B};
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(F) * 2ull,
                                    static_cast<cuuint64_t>(F) * 2ull * L};
@@ -165,11 +166,11 @@ int make_map(CUtensorMap* map, const void* base, uint32_t B, uint32_t L, uint32_
     return r == CUDA_SUCCESS ? FA_B200_OK : FA_B200_ERR_DRIVER;
 }
 
-// 3-D map {L keys, L rows, B} over a contiguous [B, L, L] fp16 mask; box = 128 rows x 64 keys.  Needs rows that
-// start on 16-byte boundaries (L a multiple of 8, base aligned); the caller checks.
-int make_mask_map(CUtensorMap* map, const void* base, uint32_t B, uint32_t L) {
+// 3-D map {L keys, L rows, B} over a [B, L, L] fp16 mask whose rows are `pitch` elements apart; box = 128 rows x 64
+// keys.  Needs rows that start on 16-byte boundaries (pitch a multiple of 8, base aligned); the caller checks.
+int make_mask_map(CUtensorMap* map, const void* base, uint32_t B, uint32_t L, uint32_t pitch) {
     const cuuint64_t dims[3] = {L, L, B};
-    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(L) * 2ull, static_cast<cuuint64_t>(L) * 2ull * L};
+    const cuuint64_t strides[2] = {static_cast<cuuint64_t>(pitch) * 2ull, static_cast<cuuint64_t>(pitch) * 2ull * L};
     const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(fa::kTile), 1};
     const cuuint32_t estr[3] = {1, 1, 1};
     const CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box,
@@ -320,7 +321,7 @@ template <int H, int kMask>
 int launch_pipelined(DeviceCtx& c, int slot, const CUtensorMap& mq, const CUtensorMap& mk,
                      const CUtensorMap& mv, const CUtensorMap& my, const CUtensorMap& mm, const Params& p,
                      uint32_t n_ctas, cudaStream_t st, bool overlap) {
-    constexpr int smem = fa::PipeCfg<H, kMask != fa::kNoMask>::kSmemBytes;
+    constexpr int smem = fa::PipeCfg<H, kMask>::kSmemBytes;
     auto kern = fa::fa_fwd_pipelined<H, kMask>;
     if (!(c.attr_done.load(std::memory_order_acquire) & (1u << slot))) {   // setting it twice is harmless
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -331,14 +332,17 @@ int launch_pipelined(DeviceCtx& c, int slot, const CUtensorMap& mq, const CUtens
     const cudaError_t e = launch_kernel(kern, grid, 512, smem, st, overlap, mq, mk, mv, my, mm, p);
     return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
-// The instance for a call with or without a mask; `slot`, slot + 1 and slot + 2 are its attribute bits.
+// The instance for what the mask is (fa::kNoMask ...); `slot` ... slot + 3 are its attribute bits.
 template <int H>
-int launch_pipelined(DeviceCtx& c, int slot, const void* mask, bool mask_tma, const CUtensorMap& mq, const CUtensorMap& mk,
+int launch_pipelined(DeviceCtx& c, int slot, int mask_kind, const CUtensorMap& mq, const CUtensorMap& mk,
                      const CUtensorMap& mv, const CUtensorMap& my, const CUtensorMap& mm, const Params& p,
                      uint32_t n_ctas, cudaStream_t st, bool overlap) {
-    if (mask == nullptr) return launch_pipelined<H, fa::kNoMask>(c, slot, mq, mk, mv, my, mm, p, n_ctas, st, overlap);
-    if (mask_tma) return launch_pipelined<H, fa::kMaskTma>(c, slot + 1, mq, mk, mv, my, mm, p, n_ctas, st, overlap);
-    return launch_pipelined<H, fa::kMaskCopied>(c, slot + 2, mq, mk, mv, my, mm, p, n_ctas, st, overlap);
+    switch (mask_kind) {
+        case fa::kNoMask: return launch_pipelined<H, fa::kNoMask>(c, slot, mq, mk, mv, my, mm, p, n_ctas, st, overlap);
+        case fa::kMaskTma: return launch_pipelined<H, fa::kMaskTma>(c, slot + 1, mq, mk, mv, my, mm, p, n_ctas, st, overlap);
+        case fa::kMaskCopied: return launch_pipelined<H, fa::kMaskCopied>(c, slot + 2, mq, mk, mv, my, mm, p, n_ctas, st, overlap);
+        default: return launch_pipelined<H, fa::kMaskPlanned>(c, slot + 3, mq, mk, mv, my, mm, p, n_ctas, st, overlap);
+    }
 }
 
 // The split-scratch buffer of `st` on this device: the one it already has, else a free one, else none.
@@ -386,7 +390,7 @@ int launch_pair(DeviceCtx& c, const CUtensorMap& mq, const CUtensorMap& mkh, con
                 const CUtensorMap& my, const CUtensorMap& mm, const Params& p, uint32_t n_quad_items,
                 cudaStream_t st, bool overlap, bool* launched) {
     constexpr int smem = fa::PairCfgT<kHasMask>::kSmemBytes;
-    constexpr int slot = kHasMask ? 9 : 8;
+    constexpr int slot = kHasMask ? 9 : 8;   // (the simple kernel's instances are 0 ... 7)
     auto kern = fa::fa_fwd_pair<kHasMask>;
     *launched = false;
     if (!(c.attr_done.load(std::memory_order_acquire) & (1u << slot))) {
@@ -427,6 +431,69 @@ int launch_pair(DeviceCtx& c, const CUtensorMap& mq, const CUtensorMap& mkh, con
     const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, mq, mkh, mv, my, mm, p);
     *launched = true;
     return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+}
+
+// Whether a masked call of the pipelined kernel is planned (fa_mask_plan.cuh).  The plan is a launch and a pass over the
+// mask, K and V ahead of the attention kernel, 6 us at least, and 13 in all where it finds that too little can be left
+// out; what it saves is up to half of the key steps where there is more than one round of them.  Measured, us without
+// and with a plan, causal masks:
+//   H = 64: B=8 R=12 L=512 21.8 / 24.2, B=32 R=12 L=512 58 / 73, B=8 R=16 L=1024 70 / 65, B=8 R=32 L=2048 430 / 320
+//   H = 32: B=8 R=16 L=2048 255 / 160
+//   H = 128: B=4 R=32 L=1024 77 / 97, B=2 R=32 L=2048 141 / 138, B=4 R=32 L=2048 291 / 254, B=1 R=40 L=4096 385 / 227
+// so from sixteen key tiles and some fifty key steps per SM on.  Where TMA cannot fetch the rows the plan's copy also
+// spares every head the copies inside the kernel, and it pays much sooner:
+//   H = 64: B=32 R=16 L=201 36 / 46, B=1 R=8 L=301 15 / 18, B=32 R=12 L=301 82 / 63, B=2 R=8 L=511 26 / 21,
+//           B=4 R=12 L=1021 72 / 38;   H = 128: B=1 R=8 L=301 25 / 19, B=2 R=32 L=1021 125 / 51
+bool use_mask_plan(uint32_t H, uint32_t n_items, uint32_t n, uint32_t B, uint32_t q_pairs, bool mask_tma, uint32_t sms, uint32_t flags) {
+    if ((flags & FA_B200_FLAG_FORCE_PAIR) || n > fa::kPlanMaxTiles || static_cast<uint64_t>(B) * q_pairs > fa::kPlanMaxGroups) return false;
+    const uint64_t steps = static_cast<uint64_t>(n_items) * n;
+    if (mask_tma) return n >= 16u && steps >= 48ull * sms;
+    return n >= 4u || (n == 3u && (H == 128 || steps >= 4ull * sms));
+}
+
+// Launches the kernel that plans a masked call, into the scratch of the call's stream (a planned call is not divided,
+// so the scratch is free): on return p's plan_ fields are set, and the mask's rows are at *mask_rows, *mask_pitch
+// elements apart.  *planned stays false when the copy of the mask does not fit.
+int plan_mask(DeviceCtx& c, const SplitScratch& scratch, const void* k, const void* v, bool mask_tma,
+              Params& p, cudaStream_t st, bool overlap, const void** mask_rows, uint32_t* mask_pitch, bool* planned) {
+    const uint32_t n = p.n_kv_tiles, groups = p.B * p.q_pairs, pitch = (p.L + 7u) & ~7u;
+    auto up = [](size_t x) { return (x + 255u) & ~static_cast<size_t>(255u); };
+    const size_t copy_bytes = mask_tma ? 0 : up(static_cast<size_t>(p.B) * p.L * pitch * 2u);
+    const size_t order_at = copy_bytes + 256, bad_at = order_at + up(groups * 4ull), list_at = bad_at + up(static_cast<size_t>(p.B) * n * 4u);
+    const size_t cls_at = list_at + up(static_cast<size_t>(groups) * n * 2u), bytes = cls_at + up(static_cast<size_t>(p.B) * n * n);
+    const uint64_t jobs = static_cast<uint64_t>(p.B) * n * 2u * ((p.F + fa::kPlanCols - 1u) / fa::kPlanCols), tiles = static_cast<uint64_t>(p.B) * n * n;
+    if (bytes > split_o_bytes(c.sm_count) || jobs > 0x7FFFFFFFull) return FA_B200_OK;
+    char* base = reinterpret_cast<char*>(scratch.o);
+    fa::PlanArgs a;
+    a.mask = p.mask;
+    a.k = static_cast<const __half*>(k);
+    a.v = static_cast<const __half*>(v);
+    a.copy = mask_tma ? nullptr : reinterpret_cast<__half*>(base);
+    a.head = reinterpret_cast<uint32_t*>(base + copy_bytes);
+    a.ticket = scratch.cnt;
+    a.order = reinterpret_cast<uint32_t*>(base + order_at);
+    a.bad = reinterpret_cast<uint32_t*>(base + bad_at);
+    a.list = reinterpret_cast<uint16_t*>(base + list_at);
+    a.cls = reinterpret_cast<uint8_t*>(base + cls_at);
+    a.B = p.B;
+    a.L = p.L;
+    a.F = p.F;
+    a.n = n;
+    a.q_pairs = p.q_pairs;
+    a.copy_pitch = pitch;
+    a.stamp = p.launch_id;
+    a.dense_allowed = mask_tma ? 1u : 0u;
+    const uint64_t most = static_cast<uint64_t>(fa::kPlanCtasPerSm) * c.sm_count, wide = tiles > jobs ? tiles : jobs;
+    cudaError_t e = launch_kernel(fa::fa_mask_plan, dim3(static_cast<unsigned>(wide < most ? wide : most)), fa::kPlanThreads, 0, st, overlap, a);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) return static_cast<int>(e);
+    p.plan_head = a.head;
+    p.plan_order = a.order;
+    p.plan_list = a.list;
+    *mask_rows = mask_tma ? static_cast<const void*>(p.mask) : a.copy;
+    *mask_pitch = mask_tma ? p.L : pitch;
+    *planned = true;
+    return FA_B200_OK;
 }
 
 // Device-pointer launch on `st`.  Caller holds no lock.
@@ -481,16 +548,28 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                 p.part_o = nullptr;
                 p.part_ml = nullptr;
                 p.part_cnt = nullptr;
+                p.plan_head = nullptr;
+                p.plan_order = nullptr;
+                p.plan_list = nullptr;
                 const int which = select_kernel(B, L, F, H, mask != nullptr, flags, c->sm_count);
                 const bool overlap = (flags & FA_B200_FLAG_NO_OVERLAP) == 0;
                 if (which == 2) {
                     // Dividing the last round needs scratch that no other launch is using: the buffer that
                     // belongs to this stream.  A stream that is being captured gets none (the recorded launch
                     // could later be replayed next to anything).
-                    const SplitScratch* scratch = nullptr;
-                    if (!(flags & (FA_B200_FLAG_NO_SPLIT | FA_B200_FLAG_FORCE_PAIR))) scratch = scratch_for_stream(*c, st);
-                    const Schedule sch = make_schedule(p.n_items, p.n_kv_tiles, static_cast<uint32_t>(c->sm_count),
-                                                       scratch != nullptr);
+                    // (Planning a mask needs the same scratch, and a planned call is not divided.)
+                    const uint32_t sms = static_cast<uint32_t>(c->sm_count);
+                    const bool mask_tma = mask && mask_rows_aligned(mask, L);
+                    const bool want_plan = mask && use_mask_plan(H, p.n_items, p.n_kv_tiles, B, p.q_pairs, mask_tma, sms, flags);
+                    const bool want_split = !(flags & (FA_B200_FLAG_NO_SPLIT | FA_B200_FLAG_FORCE_PAIR));
+                    const SplitScratch* scratch = want_plan || want_split ? scratch_for_stream(*c, st) : nullptr;
+                    const bool pair = use_pair_kernel(H, mask != nullptr, mask_tma, p.q_pairs, p.R * B, sms, 0, flags);
+                    const void* mask_at = mask;
+                    uint32_t mask_pitch = L;
+                    bool planned = false;
+                    if (want_plan && scratch != nullptr)
+                        rc = plan_mask(*c, *scratch, k, v, mask_tma, p, st, overlap, &mask_at, &mask_pitch, &planned);
+                    const Schedule sch = make_schedule(p.n_items, p.n_kv_tiles, sms, want_split && scratch != nullptr && !planned);
                     p.full_rounds = sch.full_rounds;
                     p.tail_items = sch.tail_items;
                     p.tail_steps = sch.tail_steps;
@@ -502,15 +581,30 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                     }
                     // Y as a TMA store target: boxes of 32 rows x 64 columns (one epilogue warp each)
                     CUtensorMap my;
-                    rc = make_map(&my, y, B, L, F, H, 32);
-                    bool done = false;
-                    // mask tiles through TMA when every mask row starts on a 16-byte boundary; else two of the
-                    // warps (of the kernel on single CTAs) copy them with cp.async
+                    if (rc == FA_B200_OK) rc = make_map(&my, y, B, L, F, H, 32);
+                    // mask tiles through TMA when every mask row (or row of the plan's copy) starts on a 16-byte
+                    // boundary; else two of the warps (of the kernel on single CTAs) copy them with cp.async
                     CUtensorMap mm = mq;
-                    const bool mask_tma = mask && mask_rows_aligned(mask, L);
-                    if (rc == FA_B200_OK && mask_tma) rc = make_mask_map(&mm, mask, B, L);
-                    if (rc == FA_B200_OK && use_pair_kernel(H, mask != nullptr, mask_tma, p.q_pairs, p.R * B,
-                                                            static_cast<uint32_t>(c->sm_count), sch.tail_steps, flags)) {
+                    if (rc == FA_B200_OK && (mask_tma || planned)) rc = make_mask_map(&mm, mask_at, B, L, mask_pitch);
+                    auto launch_single = [&](int kind) {
+                        switch (H) {
+                            case 16: return launch_pipelined<16>(*c, 12, kind, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
+                            case 32: return launch_pipelined<32>(*c, 16, kind, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
+                            case 64: return launch_pipelined<64>(*c, 20, kind, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
+                            default: return launch_pipelined<128>(*c, 24, kind, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
+                        }
+                    };
+                    // What the mask holds is known on the device only: where the plan may find that too little can be
+                    // left out, the kernel that the call would have without a plan is launched behind the planned one,
+                    // and the plan says which of them finds work (the other leaves at once, 4 to 6 us).
+                    if (rc == FA_B200_OK && planned) {
+                        const CUtensorMap wide = my;   // (fa::PipeCfg::kStoreCols of the planned kernel at head_dim 128)
+                        if (H == 128) rc = make_map(&my, y, B, L, F, H, 32, fa::PipeCfg<128, fa::kMaskPlanned>::kStoreCols);
+                        if (rc == FA_B200_OK) rc = launch_single(fa::kMaskPlanned);
+                        my = wide;
+                    }
+                    bool done = false;
+                    if (rc == FA_B200_OK && pair && sch.tail_steps == 0) {
                         // K as halves of a tile: boxes of 64 keys x 64 columns
                         CUtensorMap mkh;
                         rc = make_map(&mkh, k, B, L, F, H, 64);
@@ -522,14 +616,8 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                                       : launch_pair<false>(*c, mq, mkh, mv, my, mm, pp, quads, st, overlap, &done);
                         }
                     }
-                    if (rc == FA_B200_OK && !done) {
-                        switch (H) {
-                            case 16: rc = launch_pipelined<16>(*c, 14, mask, mask_tma, mq, mk, mv, my, mm, p, sch.grid, st, overlap); break;
-                            case 32: rc = launch_pipelined<32>(*c, 17, mask, mask_tma, mq, mk, mv, my, mm, p, sch.grid, st, overlap); break;
-                            case 64: rc = launch_pipelined<64>(*c, 20, mask, mask_tma, mq, mk, mv, my, mm, p, sch.grid, st, overlap); break;
-                            default: rc = launch_pipelined<128>(*c, 23, mask, mask_tma, mq, mk, mv, my, mm, p, sch.grid, st, overlap); break;
-                        }
-                    }
+                    if (rc == FA_B200_OK && !done && (!planned || mask_tma))
+                        rc = launch_single(mask == nullptr ? fa::kNoMask : (mask_tma ? fa::kMaskTma : fa::kMaskCopied));
                 } else if (mask) {
                     switch (H) {
                         case 16: rc = launch_simple<16, true>(*c, 4, mq, mk, mv, p, st, overlap); break;
@@ -692,6 +780,9 @@ int fa_b200_attention_forward_noalloc(const void* q, const void* k, const void* 
         p.part_o = nullptr;
         p.part_ml = nullptr;
         p.part_cnt = nullptr;
+        p.plan_head = nullptr;
+        p.plan_order = nullptr;
+        p.plan_list = nullptr;
 #ifdef FA_CYCLES
         p.cycles = nullptr;
 #endif

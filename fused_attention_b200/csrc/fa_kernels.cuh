@@ -56,6 +56,10 @@ struct Params {
     float2* part_ml;       // [2 * grid slots][2 tiles][128 rows] {reference maximum, row sum}
     uint32_t* part_cnt;    // [tail item][2 tiles][4 warps] parts counted in; zero between launches
     uint32_t part_slots;   // scratch slots behind part_o / part_ml (two per CTA of the largest grid)
+    // what the mask leaves to do (fa_mask_plan.cuh), or null: {1 = the planned kernel runs, 0 = the kernel behind it}
+    const uint32_t* plan_head;
+    const uint32_t* plan_order;   // pairs of query tiles of a batch entry, longest first: index | key steps << kPlanLenShift
+    const uint16_t* plan_list;    // [pair][n_kv_tiles]: the key steps that are left, see kStepShift0
 #ifdef FA_CYCLES
     unsigned long long* cycles;  // 64 records (launch_id % 64) of CTA 0: {globaltimer at entry, globaltimer after the
                                  // wait for the previous kernel, globaltimer at the end, clock64 from that wait to the end}
@@ -313,11 +317,13 @@ __device__ __forceinline__ void store_o_row(uint32_t tO, float inv_l, __half* ds
 
 // One O row from TMEM, multiplied by `inv_l` and converted to fp16, into a staging area in shared memory from
 // where TMA stores it: for a thread with registers to spare (a softmax thread), the whole row in one round trip.
-// The area holds, per 64 columns, one box of the Y map (32 rows of 128 bytes with the 128-byte swizzle: 16-byte
-// piece c of row r at piece c ^ (r & 7)); `stage` is 1024-byte aligned, `lane` the row within the box.
-template <int H>
+// The area holds, per kCols columns, one box of the Y map (32 rows of 2 * kCols bytes with the swizzle of that span:
+// the piece's low bits are taken with the bits of the address from bit 7 on); `stage` is 1024-byte aligned, `lane` the
+// row within the box.
+template <int H, int kCols = 64>
 __device__ __forceinline__ void stage_o_row(uint32_t tO, float inv_l, uint32_t stage, uint32_t lane) {
-    static_assert(H % 64 == 0, "boxes of 64 columns");
+    static_assert(H % kCols == 0 && (kCols == 64 || kCols == 32 || kCols == 16), "whole boxes");
+    constexpr uint32_t kRow = kCols * 2;
     float o[H];
 #pragma unroll
     for (int c0 = 0; c0 < H; c0 += 32) tmem_ld32(tO + c0, o + c0);
@@ -328,8 +334,8 @@ __device__ __forceinline__ void stage_o_row(uint32_t tO, float inv_l, uint32_t s
         const uint32_t w1 = pack_half2(o[i + 2] * inv_l, o[i + 3] * inv_l);
         const uint32_t w2 = pack_half2(o[i + 4] * inv_l, o[i + 5] * inv_l);
         const uint32_t w3 = pack_half2(o[i + 6] * inv_l, o[i + 7] * inv_l);
-        const uint32_t piece = static_cast<uint32_t>((i % 64) / 8) ^ (lane & 7u);
-        st_shared_v4(stage + static_cast<uint32_t>(i / 64) * 4096u + lane * 128u + piece * 16u, w0, w1, w2, w3);
+        const uint32_t piece = static_cast<uint32_t>((i % kCols) / 8) ^ ((lane * kRow >> 7) & (kRow / 16u - 1u));
+        st_shared_v4(stage + static_cast<uint32_t>(i / kCols) * (32u * kRow) + lane * kRow + piece * 16u, w0, w1, w2, w3);
     }
 }
 
@@ -402,13 +408,14 @@ __device__ __forceinline__ void add_mask_row(float (&s)[kTile], const __half* mr
 // The same from a mask tile that TMA has brought into shared memory: two boxes of 128 rows x 64 keys, rows of
 // 128 bytes with the 128-byte swizzle (16-byte chunk c of row r lies at chunk c ^ (r & 7)).  Keys and rows
 // beyond the end of the sequence were filled with zeros.
+template <int kBox0 = 0, int kBox1 = 2>   // the boxes [kBox0, kBox1); kBox0 lies at smask
 __device__ __forceinline__ void add_mask_tile_row(float (&s)[kTile], uint32_t smask, uint32_t row, float to_score) {
 #pragma unroll
-    for (int b = 0; b < 2; ++b) {
+    for (int b = kBox0; b < kBox1; ++b) {
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
             uint32_t w[4];
-            ld_shared_v4(smask + b * (kTile * 128) + row * 128u + ((static_cast<uint32_t>(c) ^ (row & 7u)) * 16u), w);
+            ld_shared_v4(smask + (b - kBox0) * (kTile * 128) + row * 128u + ((static_cast<uint32_t>(c) ^ (row & 7u)) * 16u), w);
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
                 const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
@@ -708,13 +715,32 @@ fa_fwd_simple(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 // ============================================================================ pipelined kernel
 // How the tiles of the additive mask come into shared memory: by TMA (every row starts on a 16-byte boundary), or
 // copied by warps of the CTA (copy_mask_rows).
-enum : int { kNoMask = 0, kMaskTma = 1, kMaskCopied = 2 };
+// kMaskPlanned: by TMA, and only what fa_mask_plan.cuh has found to be left: work items have key steps of their own
+// number, listed in Params::plan_list, and for a step that needs no mask tile none is fetched.
+enum : int { kNoMask = 0, kMaskTma = 1, kMaskCopied = 2, kMaskPlanned = 3 };
+constexpr uint32_t kPlanLenShift = 20;
+// an entry of a list: key tile, and what the mask is there for query tile 0 and 1 of the pair
+constexpr uint32_t kStepShift0 = 12, kStepShift1 = 14;
+constexpr uint32_t kStepNoMask = 0, kStepMask = 1, kStepAllNeg = 2;   // zero; a tile of its own; -inf throughout
 
-template <int H, bool kHasMask = false>
+template <int H, int kMask = kNoMask>
 struct PipeCfg {
     using G = TileGeom<H>;
-    // ring slots of one K or V tile each; with a mask a quarter of the ring makes room for one mask tile
-    static constexpr int kStages = (H == 128 ? 4 : 8) * (kHasMask && H >= 64 ? 3 : 4) / 4;   // (tiles of H < 64 leave room for both)
+    static constexpr bool kHasMask = kMask != kNoMask;
+    // How many boxes of 64 keys of a mask tile the mask buffer holds: both, or one after the other.  At H = 128, where
+    // the ring has four slots, a planned call, most of whose steps need no mask tile, has better use for the room of the
+    // second (causal B=4 R=32 L=2048: 163 us with four slots and one box, 174 us with three and two).  At H = 64 the
+    // eight slots can spare it (causal B=4 R=12 L=1021: 20.8 us with six slots and two boxes, 23.8 with eight and one),
+    // and the tiles of H < 64 leave room for everything.
+    static constexpr int kMaskBoxes = (kMask == kMaskPlanned && H == 128) ? 1 : 2;
+    // A mask buffer per query tile, or one that the two tiles use in turn (H = 128, where there is room for no more).
+    // With one the way of a mask tile from L2 is waited for twice a step: H = 64, B=8 R=32 L=2048, dense mask 513 us with
+    // one buffer and six ring slots, 450 us with two and four (B=8 R=12 L=512 22.4 and 21.0).  At H < 64, where a step's
+    // 64 KB of mask are most of what an SM takes from L2, the second buffer gains nothing (B=8 R=16 L=1024 68 and 72 us)
+    // unless the tiles are copied by warps (152 and 130 us).
+    static constexpr int kMaskBufs = H == 64 || (H < 64 && kMask == kMaskCopied) ? 2 : 1;
+    // ring slots of one K or V tile each; a whole mask tile takes the room of one (H = 128) or two of them (H = 64)
+    static constexpr int kStages = H == 128 ? (kHasMask && kMaskBoxes == 2 ? 3 : 4) : (kHasMask && H == 64 ? 4 : 8);
     // Buffers for the two query tiles of a segment.  With two of them (H <= 64, where they fit) the next segment's
     // query tiles, and behind them its K and V tiles, are on their way while this segment still multiplies: the
     // producer no longer stops at every segment boundary until the last Q K^T has let go of the one buffer.
@@ -722,10 +748,14 @@ struct PipeCfg {
     static constexpr int kQBufs = H <= 64 ? 2 : 1;
     static constexpr int kQBytes = 2 * G::kTileBytes;  // two query tiles
     static constexpr int kRingBytes = kStages * G::kTileBytes;
-    static constexpr int kMaskBytes = kHasMask ? kTile * kTile * 2 : 0;   // one 128 x 128 fp16 mask tile (two boxes of 64 keys)
-    static constexpr int kMaskExtraBytes = kHasMask ? kTile * 4 : 0;      // one word per row, see copy_mask_rows
-    static constexpr int kStageBytes = 4 * 32 * 128;   // epilogue staging: per warp 32 rows x up to 64 fp16
-    static constexpr int kSmemBytes = kQBufs * kQBytes + kRingBytes + kMaskBytes + kStageBytes + kMaskExtraBytes + 1024;  // + alignment slack
+    static constexpr int kMaskBoxBytes = kTile * 64 * 2;                  // 128 rows x 64 keys
+    static constexpr int kMaskBytes = kHasMask ? kMaskBoxes * kMaskBoxBytes : 0;   // one buffer
+    static constexpr int kMaskExtraBytes = kMask == kMaskCopied ? kTile * 4 : 0;  // of one buffer:     // one word per row, see copy_mask_rows
+    // Columns of one TMA store of Y: with the mask's box the whole ring leaves room for staging buffers of 32 only.
+    static constexpr int kStoreCols = kMaskBoxes == 1 ? 32 : G::kBoxCols;
+    static constexpr int kStageWarpBytes = kMaskBoxes == 1 ? 2048 : 4096;   // per epilogue warp 32 rows x kStoreCols fp16
+    static constexpr int kStageBytes = 4 * kStageWarpBytes;
+    static constexpr int kSmemBytes = kQBufs * kQBytes + kRingBytes + kMaskBufs * kMaskBytes + kStageBytes + kMaskBufs * kMaskExtraBytes + 1024;  // + alignment slack
     static constexpr uint32_t kTmemCols = 512;
     // TMEM columns.  P (fp16, 64 columns per tile) has columns of its own instead of overwriting its
     // S: the next Q K^T of a tile then does not have to wait for the P V that reads P, only for the
@@ -810,6 +840,7 @@ struct Seg {
     uint32_t item;       // work item: q_pair = item % q_pairs, (batch, head) = item / q_pairs
     uint32_t j0, len;    // key steps [j0, j0 + len)
     bool partial;        // fewer than all n key steps
+    uint32_t list;       // kMaskPlanned: where the item's entries of Params::plan_list begin
 };
 // Of a tail segment k (k >= t0 = number of whole segments): index of its item among the tail items; this
 // CTA's scratch slot for the part (two per CTA).  Looked up where they are needed rather than kept in
@@ -832,13 +863,42 @@ __device__ __forceinline__ Seg get_seg(PlanRef& pl, uint32_t t0, const Params& p
         s.j0 = 0;
         s.len = p.n_kv_tiles;
         s.partial = false;
+        s.list = 0;
     } else {
         const uint32_t t = k - t0;   // 0 or 1
         s.j0 = t ? 0u : pl.t_j00;
         s.len = t ? pl.t_len1 : pl.t_len0;
         s.item = p.full_rounds * gridDim.x + pl.t_item0 + t;
         s.partial = s.len != p.n_kv_tiles;
+        s.list = 0;
     }
+    return s;
+}
+
+// kMaskPlanned.  Items are numbered pair of query tiles (longest first) by head; CTA c takes item c of the first round
+// of gridDim.x items, item gridDim.x - 1 - c of the second, and so on in turn, so that a CTA that has a long item of
+// one round has a short one of the next (B=4 R=32 L=2048, causal: 64 key steps for the busiest CTA, 62.3 on average).
+struct Planned {
+    uint32_t pair, head, len;   // len 0: there is no such item
+};
+__device__ __forceinline__ uint32_t planned_count(const Params& p) {
+    const uint32_t full = p.n_items / gridDim.x, rest = p.n_items % gridDim.x;
+    return full + (((full & 1u) ? gridDim.x - 1u - blockIdx.x : blockIdx.x) < rest ? 1u : 0u);
+}
+__device__ __forceinline__ Planned planned_item(const Params& p, uint32_t k) {
+    const uint32_t idx = k * gridDim.x + ((k & 1u) ? gridDim.x - 1u - blockIdx.x : blockIdx.x);
+    if (idx >= p.n_items) return Planned{0u, 0u, 0u};
+    const uint32_t o = __ldg(p.plan_order + idx / p.R);
+    return Planned{o & ((1u << kPlanLenShift) - 1u), idx % p.R, o >> kPlanLenShift};
+}
+__device__ __forceinline__ Seg planned_seg(const Params& p, uint32_t k) {
+    const Planned it = planned_item(p, k);
+    Seg s;
+    s.item = (it.pair / p.q_pairs * p.R + it.head) * p.q_pairs + it.pair % p.q_pairs;
+    s.j0 = 0;
+    s.len = it.len;
+    s.partial = false;
+    s.list = it.pair * p.n_kv_tiles;
     return s;
 }
 
@@ -1107,9 +1167,9 @@ __global__ void __launch_bounds__(512, 1)
 fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                  const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmY,
                  const __grid_constant__ CUtensorMap tmM, const Params p) {
-    constexpr bool kHasMask = kMask != kNoMask;
+    constexpr bool kHasMask = kMask != kNoMask, kPlanned = kMask == kMaskPlanned;
     using G = TileGeom<H>;
-    using C = PipeCfg<H, kHasMask>;
+    using C = PipeCfg<H, kMask>;
     constexpr int NS = C::kStages;
     enum {
         BAR_QFULL0 = 0, BAR_QFULL1,  // TMA -> MMA: query tile landed
@@ -1123,9 +1183,9 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         BAR_A0, BAR_A1,              // softmax -> epilogue: final row sums in shared memory (4)
         BAR_OFREE0, BAR_OFREE1,      // epilogue -> MMA, softmax: O tile read out (4 arrivals)
         BAR_EPI,                     // epilogue -> softmax: the epilogue warps are through (4 arrivals)
-        BAR_MFULL0, BAR_MFULL1,      // TMA -> softmax of tile i: its mask tile of this key step landed (one buffer,
-                                     // filled for the two tiles in turn; a barrier per tile, one phase per key step,
-                                     // so that a tile can never take the other tile's phase for its own)
+        BAR_MFULL0, BAR_MFULL1,      // TMA -> softmax of tile i: its mask tile of this key step landed (a barrier per tile,
+                                     // one phase per mask tile or box, also where the two tiles share one buffer, so
+                                     // that a tile can never take the other tile's phase for its own)
         BAR_MEMPTY0, BAR_MEMPTY1,    // softmax of tile i -> TMA: the mask tile has been read (4 arrivals)
         BAR_FINAL,                   // MMA -> itself: every MMA retired
         BAR_FINAL2,                  // the same for the second issuing warp
@@ -1152,13 +1212,29 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t q_pairs = p.q_pairs;
     __shared__ Plan plan_smem;
     volatile Plan& pl_s = plan_smem;
+    auto seg_of = [&](uint32_t t_first, uint32_t k) {
+        if constexpr (kPlanned) return planned_seg(p, k);
+        else return get_seg(pl_s, t_first, p, k);
+    };
+    // key tile of step jj of a segment (with what the mask is there, if it is planned)
+    auto step_of = [&](const Seg& sg, uint32_t jj) -> uint32_t {
+        if constexpr (kPlanned) return __ldg(p.plan_list + sg.list + jj);
+        else return sg.j0 + jj;
+    };
+    auto step_tile = [](uint32_t e) -> uint32_t { return kPlanned ? e & ((1u << kStepShift0) - 1u) : e; };
+    // what the mask is at a step for query tile i
+    auto step_mask = [](uint32_t e, uint32_t i) -> uint32_t {
+        return kPlanned ? (e >> (i ? kStepShift1 : kStepShift0)) & 3u : (kHasMask ? kStepMask : kStepNoMask);
+    };
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t sQ = smem_base;                   // two tiles per buffer
     const uint32_t sRing = smem_base + C::kQBufs * C::kQBytes;   // NS tiles
-    const uint32_t sMask = sRing + C::kRingBytes;    // one mask tile (instances with a mask only)
-    const uint32_t sStage = sMask + C::kMaskBytes;   // epilogue staging, 4 KiB per epilogue warp
+    const uint32_t sMask = sRing + C::kRingBytes;    // mask buffers (instances with a mask only)
+    const uint32_t sStage = sMask + C::kMaskBufs * C::kMaskBytes;   // epilogue staging, 4 KiB per epilogue warp
     const uint32_t sMaskExtra = sStage + C::kStageBytes;   // a word per mask row (instances with a mask only)
+    auto mask_addr = [&](uint32_t i) { return sMask + (C::kMaskBufs == 2 ? i * C::kMaskBytes : 0u); };   // of query tile i
+    auto mask_extra_addr = [&](uint32_t i) { return sMaskExtra + (C::kMaskBufs == 2 ? i * C::kMaskExtraBytes : 0u); };
     const uint32_t bar0 = smem_u32(bars);
     auto bar = [&](int i) { return bar0 + 8u * i; };
     // Segment k's query tiles: buffer k mod kQBufs; its barriers complete one phase per use of that buffer.
@@ -1174,7 +1250,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // thread has found its way into its role's loop (measured: the first copy goes out ~1000 clocks sooner).
     int32_t first_col0 = 0, first_batch = 0, first_q_row0 = 0, first_key0 = 0;
     bool first_known = false;
-    if (tid == 13 * 32) {
+    if (!kPlanned && tid == 13 * 32) {
         // The plan of this CTA, and a request for the tiles it needs first to be brought into L2.  In a
         // launch that overlaps the previous kernel of the stream this CTA may be here long before that
         // kernel completes; a prefetch returns nothing to the SM, and L2 is where that kernel's writes
@@ -1219,7 +1295,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         prefetch_tensormap(&tmQ);
         prefetch_tensormap(&tmK);
         prefetch_tensormap(&tmV);
-        if constexpr (kMask == kMaskTma) prefetch_tensormap(&tmM);
+        if constexpr (kMask == kMaskTma || kPlanned) prefetch_tensormap(&tmM);
     }
 #ifdef FA_DEBUG
     dbg_begin(p, ctl, smem_base, C::kSmemBytes - 1024);
@@ -1245,7 +1321,23 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         load_tile<H>(sQ, &tmQ, bar(BAR_QFULL0), first_col0, first_q_row0, first_batch);
         load_tile<H>(sRing, &tmK, bar(BAR_FULL), first_col0, first_key0, first_batch);
     }
-    if (tid == 15 * 32) leave_early_if_launch_failed(ctl);   // warp 15 has no other work
+    if (tid == 15 * 32) leave_early_if_launch_failed(ctl);
+    if constexpr (kMask == kMaskTma) {   // the planned kernel before this one has taken the call: no segments here
+        if (p.plan_head != nullptr && tid == 13 * 32 && __ldg(p.plan_head) != 0u) plan_smem = Plan{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+        if (p.plan_head != nullptr) __syncthreads();
+    }
+    if constexpr (kPlanned) {
+        // the lists were written by the kernel before this one, so this CTA's plan is made behind the wait for it
+        if (warp == 13) {
+            const bool runs = __ldg(p.plan_head) != 0u;   // else the kernel launched behind this one takes the call
+            const uint32_t mine = planned_count(p);
+            uint32_t sum = 0;
+            for (uint32_t k = lane; k < mine; k += 32u) sum += planned_item(p, k).len;
+            sum = __reduce_add_sync(0xffffffffu, sum);
+            if (lane == 0) plan_smem = runs ? Plan{mine, 0u, mine, sum, 0u, 0u, 0u, 0u} : Plan{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+        }
+        __syncthreads();
+    }
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
     const uint32_t nseg = pl_s.nseg, ntail = pl_s.ntail, t0 = nseg - ntail;   // t0: first tail segment
 #ifdef FA_CYCLES
@@ -1267,9 +1359,10 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t tO = tmem_base + lane_off + (i ? C::kColO1 : C::kColO0);
         const float c = p.scale_log2;
         uint32_t g = 0;   // global step
+        uint32_t gm = 0;  // mask tiles (or boxes) taken so far
         float m = -INFINITY, l = 0.f;
         for (uint32_t k = 0; k < nseg; ++k) {
-            const Seg sg = get_seg(pl_s, t0, p, k);
+            const Seg sg = seg_of(t0, k);
             m = -INFINITY;
             l = 0.f;
             // how far into its first word this thread's mask row starts
@@ -1277,7 +1370,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             if constexpr (kMask == kMaskCopied)
                 mask_sh = mask_row_shift(p, (sg.item / q_pairs) / p.R, ((sg.item % q_pairs) * 2u + i) * kTile + row);
             for (uint32_t jj = 0; jj < sg.len; ++jj, ++g) {
-                const uint32_t j = sg.j0 + jj;
+                const uint32_t step = step_of(sg, jj), j = step_tile(step);
                 mbar_wait(bar(BAR_S0 + i), g & 1u, ctl, kRoleSoftmax | (BAR_S0 + i));
                 tc_fence_after();
                 __syncwarp();
@@ -1298,15 +1391,29 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     }
                 }
                 if constexpr (kHasMask) {
-                    // The mask tile of this tile and step, brought in by TMA or by the copying warps into the one
-                    // mask buffer; it is handed back as soon as it has been read.
-                    mbar_wait(bar(BAR_MFULL0 + i), g & 1u, ctl, kRoleSoftmax | (BAR_MFULL0 + i));
-                    if constexpr (kMask == kMaskCopied)
-                        add_mask_tile_row_shifted(s, sMask, row, p.mask_to_score, mask_sh, ld_shared_u32(sMaskExtra + row * 4u));
-                    else
-                        add_mask_tile_row(s, sMask, row, p.mask_to_score);
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(bar(BAR_MEMPTY0 + i));
+                    const uint32_t what = step_mask(step, i);
+                    if (what == kStepMask) {
+                        // The mask tile of this tile and step, brought in by TMA or by the copying warps; its buffer is handed back as soon as it has been read.
+                        mbar_wait(bar(BAR_MFULL0 + i), gm & 1u, ctl, kRoleSoftmax | (BAR_MFULL0 + i));
+                        ++gm;
+                        if constexpr (C::kMaskBoxes == 1) {   // the second box follows the first in the same place
+                            add_mask_tile_row<0, 1>(s, mask_addr(i), row, p.mask_to_score);
+                            __syncwarp();
+                            if (lane == 0) mbar_arrive(bar(BAR_MEMPTY0 + i));
+                            mbar_wait(bar(BAR_MFULL0 + i), gm & 1u, ctl, kRoleSoftmax | (BAR_MFULL0 + i));
+                            ++gm;
+                            add_mask_tile_row<1, 2>(s, mask_addr(i), row, p.mask_to_score);
+                        } else if constexpr (kMask == kMaskCopied)
+                            add_mask_tile_row_shifted(s, mask_addr(i), row, p.mask_to_score, mask_sh,
+                                                      ld_shared_u32(mask_extra_addr(i) + row * 4u));
+                        else
+                            add_mask_tile_row(s, mask_addr(i), row, p.mask_to_score);
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(bar(BAR_MEMPTY0 + i));
+                    } else if (what == kStepAllNeg) {
+#pragma unroll
+                        for (int e = 0; e < kTile; ++e) s[e] += -INFINITY;
+                    }
                 }
                 if (ragged) mask_tail(s, static_cast<int>(p.L - j * kTile));
                 if (first) m = row_max(s);   // first key tile of the segment: the reference is its row maximum
@@ -1352,7 +1459,9 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         float nmc2 = -m * c;
                         if constexpr (kHasMask) nmc2 = (m == -INFINITY) ? 0.f : nmc2;
                         float unused[4];
-                        l = l * alpha + exp_chunks<0, 4, false>(s, c, nmc2, tP, unused);
+                        // (the sum in the order of the common path: it does not matter on which of them a row took its reference)
+                        const float sum2 = exp_chunks<0, C::kHeldChunks, false>(s, c, nmc2, tP, unused);
+                        l = l * alpha + (sum2 + exp_chunks<C::kHeldChunks, 4, false>(s, c, nmc2, tP, unused));
                         // (This wait returns at once.  It is here because with a branch point at this
                         // place of the rare path the compiler allocates the common path without spills.)
                         if (g > 0) mbar_wait(bar(BAR_PV0 + i), (g - 1u) & 1u, ctl, kRoleSoftmax | (BAR_PV0 + i));
@@ -1389,8 +1498,8 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // CTA's scratch slot and counts itself in (and adds up after all if that made it the last).
         const uint32_t wq = warp & 3u;
         bool last_is_whole = C::kSoftmaxWritesLast && nseg > 0u;
-        if (ntail > 0u) {   // the CTA's last segment is a tail segment
-            const Seg sg = get_seg(pl_s, t0, p, nseg - 1u);
+        if (!kPlanned && ntail > 0u) {   // the CTA's last segment is a tail segment
+            const Seg sg = seg_of(t0, nseg - 1u);
             if (sg.partial) {
                 last_is_whole = false;
                 const uint32_t tail_item = seg_tail_item(pl_s, t0, nseg - 1u);
@@ -1439,31 +1548,31 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             // both tiles at once (each thread has its row sum, and the registers to take the whole O row in one
             // round trip), instead of handing the two tiles to the four epilogue warps one after the other.
             // Staging area: the tile's own query buffer, which its last Q K^T has long let go of.
-            const Seg sg = get_seg(pl_s, t0, p, nseg - 1u);
+            const Seg sg = seg_of(t0, nseg - 1u);
             const uint32_t bh = sg.item / q_pairs;
             const int32_t row0 = static_cast<int32_t>(((sg.item % q_pairs) * 2u + i) * kTile + wq * 32u);
-            const uint32_t stage = q_addr(nseg - 1u, i) + wq * static_cast<uint32_t>((H / 64) * 4096);
+            const uint32_t stage = q_addr(nseg - 1u, i) + wq * static_cast<uint32_t>(32 * H * 2);
             mbar_wait(bar(BAR_PV0 + i), (g - 1u) & 1u, ctl, kRoleSoftmax | (BAR_PV0 + i));
             tc_fence_after();
             __syncwarp();
-            stage_o_row<H>(tO, 1.f / l, stage, lane);
+            stage_o_row<H, C::kStoreCols>(tO, 1.f / l, stage, lane);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0 && row0 < static_cast<int32_t>(p.L)) {
 #pragma unroll
-                for (int half = 0; half < H / 64; ++half)
-                    tma_store_3d(&tmY, stage + half * 4096u, static_cast<int32_t>((bh % p.R) * H + half * 64), row0,
-                                 static_cast<int32_t>(bh / p.R));
+                for (int half = 0; half < H / C::kStoreCols; ++half)
+                    tma_store_3d(&tmY, stage + half * (64u * C::kStoreCols), static_cast<int32_t>((bh % p.R) * H + half * C::kStoreCols),
+                                 row0, static_cast<int32_t>(bh / p.R));
                 bulk_commit_group();
             }
             if (lane == 0) bulk_wait_read_all();   // the staging area is this CTA's until TMA has read it
         }
         // A part that the epilogue warps put into scratch (the first tail segment of a CTA that has two) and
         // that turned out to be the last of its item: added up here, every part read from scratch.
-        if (ntail == 2u) {
+        if (!kPlanned && ntail == 2u) {
             mbar_wait_relaxed(bar(BAR_EPI), 0, ctl, kRoleSoftmax | BAR_EPI, 100);
             if (deferred[i][wq] != 0u) {
-                const Seg sg = get_seg(pl_s, t0, p, t0);
+                const Seg sg = seg_of(t0, t0);
                 const uint32_t q_row = ((sg.item % q_pairs) * 2u + i) * kTile + row;
                 const uint32_t bh = sg.item / q_pairs;
                 __half* y_row = p.y + (static_cast<size_t>(bh / p.R) * p.L + q_row) * p.F + (bh % p.R) * H;
@@ -1488,10 +1597,10 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         const uint32_t row = tid & 127u;
         const uint32_t wq = warp & 3u;
         const uint32_t lane_off = (wq * 32u) << 16;
-        const uint32_t stage = sStage + wq * 4096u;
+        const uint32_t stage = sStage + wq * C::kStageWarpBytes;
         uint32_t g_end = 0;   // global steps up to and including the current segment
         for (uint32_t k = 0; k < nseg; ++k) {
-            const Seg sg = get_seg(pl_s, t0, p, k);
+            const Seg sg = seg_of(t0, k);
             // the softmax warps finish a final part themselves, and with kSoftmaxWritesLast a final whole item too
             if (k + 1u == nseg && (sg.partial || C::kSoftmaxWritesLast)) break;
             g_end += sg.len;
@@ -1512,7 +1621,8 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const int32_t row0 = static_cast<int32_t>((q_pair * 2u + i) * kTile + wq * 32u);
                 if (!sg.partial) {
                     const float inv_l = 1.f / l_row;
-                    constexpr int W = G::kBoxCols;   // columns of one staging buffer and store
+                    constexpr int W = C::kStoreCols;   // columns of one staging buffer and store
+                    constexpr uint32_t kRow = W * 2;
 #pragma unroll
                     for (int half = 0; half < H / W; ++half) {
                         // the previous store out of this staging buffer must have read it completely
@@ -1535,10 +1645,10 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                                 const uint32_t w1 = pack_half2(o[v4 * 8 + 2] * inv_l, o[v4 * 8 + 3] * inv_l);
                                 const uint32_t w2 = pack_half2(o[v4 * 8 + 4] * inv_l, o[v4 * 8 + 5] * inv_l);
                                 const uint32_t w3 = pack_half2(o[v4 * 8 + 6] * inv_l, o[v4 * 8 + 7] * inv_l);
-                                // logical 16-byte chunk c*2+v4 of row `lane`; the swizzle of rows of kSwz bytes takes
+                                // logical 16-byte chunk c*2+v4 of row `lane`; the swizzle of rows of kRow bytes takes
                                 // the chunk's low bits with the bits of the address from bit 7 on
-                                const uint32_t chunk = static_cast<uint32_t>(c * 2 + v4) ^ ((lane * G::kSwz >> 7) & (G::kSwz / 16u - 1u));
-                                st_shared_v4(stage + lane * G::kSwz + chunk * 16u, w0, w1, w2, w3);
+                                const uint32_t chunk = static_cast<uint32_t>(c * 2 + v4) ^ ((lane * kRow >> 7) & (kRow / 16u - 1u));
+                                st_shared_v4(stage + lane * kRow + chunk * 16u, w0, w1, w2, w3);
                             }
                         }
                         fence_proxy_async_smem();
@@ -1614,7 +1724,11 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const uint32_t steps = pl.steps;   // global steps of this CTA
             // ring item 2g is the K tile of global step g, item 2g+1 its V tile
             // (k, j, len): segment of the step a loop is working on, its position in it, its length
-            uint32_t k = 0, j = 0, len = seg_len(pl, p, 0);
+            auto seg_len_of = [&](uint32_t kk) {
+                if constexpr (kPlanned) return planned_item(p, kk).len;
+                else return seg_len(pl, p, kk);
+            };
+            uint32_t k = 0, j = 0, len = seg_len_of(0);
             if (steps > 0 && warp == 12) {
                 // S tiles of the very first step
                 mwait(bar_qfull(0, 0), 0, code_qfull(0, 0));
@@ -1646,7 +1760,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     // after them (mbar_poll_begin).
                     for (uint32_t q = 1; q < steps; ++q) {
                         bool new_seg = false;            // step q opens segment k
-                        if (++j == len) { j = 0; ++k; len = seg_len(pl, p, k); new_seg = true; }
+                        if (++j == len) { j = 0; ++k; len = seg_len_of(k); new_seg = true; }
                         const bool last_of_seg = j + 1 == len;   // a segment's last Q K^T is its last use of the query tile
                         const uint32_t tk = 2 * q;
                         if (!(polled && mbar_poll_end<0>())) wait_full(tk);
@@ -1701,7 +1815,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                             tc_commit(bar(BAR_PV1));
                             free_slot(tv);
                         }
-                        if (++j == len) { j = 0; ++k; len = seg_len(pl, p, k); }
+                        if (++j == len) { j = 0; ++k; len = seg_len_of(k); }
                     }
                 }
             } else {
@@ -1717,7 +1831,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     const bool more = g + 1 < steps;            // a next global step exists
                     const bool next_new_seg = j + 1 == len;     // ... and it opens segment k + 1
                     // is the next step the last of its segment (its Q K^T the last use of the query tile)?
-                    const bool next_last_of_seg = next_new_seg ? seg_len(pl, p, k + 1u) == 1u : j + 2 == len;
+                    const bool next_last_of_seg = next_new_seg ? seg_len_of(k + 1u) == 1u : j + 2 == len;
                     const uint32_t acc = j > 0 ? 1u : 0u;
                     const uint32_t kn = next_new_seg ? k + 1u : k;   // the segment of the next step
                     {
@@ -1779,7 +1893,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         tc_commit(bar(BAR_PV1));
                         free_slot(tv);
                     }
-                    if (++j == len) { j = 0; ++k; len = seg_len(pl, p, k); }
+                    if (++j == len) { j = 0; ++k; len = seg_len_of(k); }
                 }
             }
             // Every MMA this warp issued has to retire before the CTA releases tensor memory and shared
@@ -1795,7 +1909,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             bool stop = false;
             uint32_t q_asked[2] = {0, 0};   // for how many segments query tile tt has been asked for
             for (; k < nseg && !stop; ++k) {
-                const Seg sg = get_seg(pl_s, t0, p, k);
+                const Seg sg = seg_of(t0, k);
 #ifdef FA_DEBUG
                 if (!dbg_ok(sg.item < p.n_items && sg.len >= 1u && sg.j0 + sg.len <= p.n_kv_tiles &&
                             (k < t0 || (seg_slot(t0, k) < p.part_slots && seg_tail_item(pl_s, t0, k) < p.tail_items)),
@@ -1805,8 +1919,10 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const int32_t col0 = static_cast<int32_t>((bh % p.R) * H);
                 const int32_t batch = static_cast<int32_t>(bh / p.R);
                 const int32_t q_row0 = static_cast<int32_t>(q_pair * 2u * kTile);
+                uint32_t key_tile = 0;
                 for (uint32_t tt = 0; tt < 2 * sg.len; ++tt, ++t) {
-                    const bool asked_already = t == 0u;   // query tile 0 and K tile 0 of the first segment: see above
+                    if ((tt & 1u) == 0u) key_tile = step_tile(step_of(sg, tt >> 1));
+                    const bool asked_already = !kPlanned && t == 0u;   // query tile 0 and K tile 0 of the first segment: see above
                     if (tt < 2) {
                         // query tile tt of this segment, once the buffer's previous user has let go of it
                         if (k >= static_cast<uint32_t>(C::kQBufs) &&
@@ -1822,7 +1938,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                                    kRoleProducer | (BAR_EMPTY + slot))) { stop = true; break; }
                     if (!asked_already)
                         load_tile<H>(sRing + slot * G::kTileBytes, (tt & 1u) ? &tmV : &tmK, bar(BAR_FULL + slot),
-                                     col0, static_cast<int32_t>((sg.j0 + (tt >> 1)) * kTile), batch);
+                                     col0, static_cast<int32_t>(key_tile * kTile), batch);
                 }
             }
             if (abort_flag != 0u) {
@@ -1853,18 +1969,19 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             uint32_t g = 0;
             bool stop = false;
             for (uint32_t k = 0; k < nseg && !stop; ++k) {
-                const Seg sg = get_seg(pl_s, t0, p, k);
+                const Seg sg = seg_of(t0, k);
                 const uint32_t batch = (sg.item / q_pairs) / p.R, q0 = (sg.item % q_pairs) * 2u * kTile;
                 for (uint32_t jj = 0; jj < sg.len && !stop; ++jj, ++g) {
                     for (uint32_t i = 0; i < 2; ++i) {
                         bool ok = true;
-                        if (i == 1) ok = mbar_wait(bar(BAR_MEMPTY0), g & 1u, ctl, kRoleProducer | BAR_MEMPTY0);
+                        if (C::kMaskBufs == 2) ok = g == 0 || mbar_wait(bar(BAR_MEMPTY0 + i), (g - 1u) & 1u, ctl, kRoleProducer | (BAR_MEMPTY0 + i));
+                        else if (i == 1) ok = mbar_wait(bar(BAR_MEMPTY0), g & 1u, ctl, kRoleProducer | BAR_MEMPTY0);
                         else if (g > 0) ok = mbar_wait(bar(BAR_MEMPTY1), (g - 1u) & 1u, ctl, kRoleProducer | BAR_MEMPTY1);
                         if (__any_sync(0xffffffffu, !ok)) {
                             stop = true;
                             break;
                         }
-                        copy_mask_rows<kRows>(p, mr, sMask, sMaskExtra, batch, q0 + i * kTile, (sg.j0 + jj) * kTile, r0, lane);
+                        copy_mask_rows<kRows>(p, mr, mask_addr(i), mask_extra_addr(i), batch, q0 + i * kTile, (sg.j0 + jj) * kTile, r0, lane);
                         cp_async_arrive(bar(BAR_MFULL0 + i));
                         __syncwarp();
                         if (lane == 0) mbar_arrive(bar(BAR_MFULL0 + i));
@@ -1872,34 +1989,39 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 }
             }
             cp_async_wait_all();
-        } else if (kMask == kMaskTma && warp == 15 && elect_one()) {
+        } else if ((kMask == kMaskTma || kPlanned) && warp == 15 && elect_one()) {
             // -------------------------------------------------------------- TMA producer of the mask tiles
-            // One buffer, filled for tile 0 and tile 1 of every key step in turn, each time as soon as the softmax
-            // warps of the tile before have read it: tile 1 of step g follows tile 0 of step g, tile 0 of step g
-            // follows tile 1 of step g - 1.  Boxes that lie beyond the end of the sequence (keys or rows) arrive
-            // as zeros.
-            uint32_t g = 0;   // global step
-            uint32_t asked[2] = {0, 0};   // for how many key steps tile i's mask tile has been asked for
+            // Tile 0 and tile 1 of every key step in turn (where the step needs them; box by box where a buffer holds one
+            // box), each as soon as the softmax warps that had the buffer before have read it.  Boxes that lie beyond the end of the
+            // sequence (keys or rows) arrive as zeros.
+            uint32_t asked[2] = {0, 0};   // mask tiles (or boxes) asked for so far for tile i
+            uint32_t before = 0;          // the tile that was asked for last
             bool stop = false;
             for (uint32_t k = 0; k < nseg && !stop; ++k) {
-                const Seg sg = get_seg(pl_s, t0, p, k);
+                const Seg sg = seg_of(t0, k);
                 const int32_t batch = static_cast<int32_t>((sg.item / q_pairs) / p.R);
                 const int32_t q_row0 = static_cast<int32_t>((sg.item % q_pairs) * 2u * kTile);
-                for (uint32_t jj = 0; jj < sg.len && !stop; ++jj, ++g) {
-                    const int32_t key0 = static_cast<int32_t>((sg.j0 + jj) * kTile);
+                for (uint32_t jj = 0; jj < sg.len && !stop; ++jj) {
+                    const uint32_t step = step_of(sg, jj);
+                    const int32_t key0 = static_cast<int32_t>(step_tile(step) * kTile);
                     for (uint32_t i = 0; i < 2; ++i) {
-                        bool ok = true;
-                        if (i == 1) ok = mbar_wait(bar(BAR_MEMPTY0), g & 1u, ctl, kRoleProducer | BAR_MEMPTY0);
-                        else if (g > 0) ok = mbar_wait(bar(BAR_MEMPTY1), (g - 1u) & 1u, ctl, kRoleProducer | BAR_MEMPTY1);
-                        if (!ok) {
-                            stop = true;
-                            break;
+                        if (step_mask(step, i) != kStepMask) continue;
+                        if (C::kMaskBufs == 2) before = i;   // the buffer's last user is the tile itself
+                        for (int box = 0; box < 2 && !stop; box += C::kMaskBoxes) {
+                            if (asked[before] > 0u && !mbar_wait(bar(BAR_MEMPTY0 + before), (asked[before] - 1u) & 1u, ctl,
+                                                                 kRoleProducer | (BAR_MEMPTY0 + before))) {
+                                stop = true;
+                                break;
+                            }
+                            mbar_expect_tx(bar(BAR_MFULL0 + i), C::kMaskBytes);
+#pragma unroll
+                            for (int u = 0; u < C::kMaskBoxes; ++u)
+                                tma_load_3d(mask_addr(i) + u * C::kMaskBoxBytes, &tmM, bar(BAR_MFULL0 + i), key0 + (box + u) * 64,
+                                            q_row0 + static_cast<int32_t>(i * kTile), batch);
+                            ++asked[i];
+                            before = i;
                         }
-                        mbar_expect_tx(bar(BAR_MFULL0 + i), C::kMaskBytes);
-                        tma_load_3d(sMask, &tmM, bar(BAR_MFULL0 + i), key0, q_row0 + static_cast<int32_t>(i * kTile), batch);
-                        tma_load_3d(sMask + kTile * 128, &tmM, bar(BAR_MFULL0 + i), key0 + 64,
-                                    q_row0 + static_cast<int32_t>(i * kTile), batch);
-                        asked[i] = g + 1u;
+                        if (stop) break;
                     }
                 }
             }

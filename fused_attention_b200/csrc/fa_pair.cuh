@@ -121,8 +121,8 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
     const uint32_t cluster = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
     const uint32_t n = p.n_kv_tiles;
     const uint32_t q_quads = (p.q_pairs + 1u) >> 1;     // blocks of 512 query rows per (batch, head)
-    const uint32_t n_items = q_quads * p.R * p.B;
-    const uint32_t my_items = cluster < n_items ? (n_items - cluster + n_clusters - 1u) / n_clusters : 0u;
+    uint32_t n_items = q_quads * p.R * p.B;
+    uint32_t my_items = cluster < n_items ? (n_items - cluster + n_clusters - 1u) / n_clusters : 0u;
 
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
     const uint32_t sQ = smem_base;                   // two tiles
@@ -169,6 +169,8 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
     tc_fence_after();
     grid_dep_wait();
     grid_dep_launch();
+    // A mask that leaves enough out: the planned kernel has done the work (fa_mask_plan.cuh), nothing is left here.
+    if (kHasMask && p.plan_head != nullptr && *p.plan_head != 0u) n_items = my_items = 0u;
     if (tid == 15 * 32) leave_early_if_launch_failed(ctl);
     const uint32_t tmem_base = __shfl_sync(0xffffffffu, tmem_slot, 0);
 #ifdef FA_CYCLES
@@ -256,7 +258,9 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
                         float nmc2 = -m * c;
                         if constexpr (kHasMask) nmc2 = (m == -INFINITY) ? 0.f : nmc2;
                         float unused[4];
-                        l = l * alpha + exp_chunks<0, 4, false>(s, c, nmc2, tP, unused);
+                        // (the sum in the order of the common path: it does not matter on which of them a row took its reference)
+                        const float sum2 = exp_chunks<0, C::kHeldChunks, false>(s, c, nmc2, tP, unused);
+                        l = l * alpha + (sum2 + exp_chunks<C::kHeldChunks, 4, false>(s, c, nmc2, tP, unused));
                         if (g > 0) mbar_wait(bar(BAR_PV0 + i), (g - 1u) & 1u, ctl, kRoleSoftmax | (BAR_PV0 + i));
                         tc_fence_after();
                         __syncwarp();

@@ -60,3 +60,80 @@ def test_rows_whose_first_tiles_are_masked_and_whose_scores_are_far_below_zero(H
     mask[0, :, :130] = float("-inf")
     mask[1, :, :400] = float("-inf")
     assert_close(run(q, k, v, H, mask.cuda(), flags), oracle(q, k, v, H, mask))
+
+
+def _recorded(q, k, v, H, mask, flags):
+    """The same call recorded into a CUDA graph and replayed: a stream that is being captured gets no plan."""
+    fa.attention_forward(H, 32, q, k, v, mask, flags=flags)          # set-up outside the capture
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = fa.attention_forward(H, 32, q, k, v, mask, flags=flags)
+    graph.replay()
+    torch.cuda.synchronize()
+    return y
+
+
+def _block_mask(B, L, kind):
+    """Masks whose 128 x 128 tiles are of every kind: -inf throughout, zero throughout, neither."""
+    gen = torch.Generator().manual_seed(B * L)
+    rows, keys = torch.arange(L)[:, None], torch.arange(L)[None, :]
+    m = torch.zeros(B, L, L)
+    if kind == "causal":
+        m[:, (keys > rows)] = float("-inf")
+    elif kind == "padding":
+        for b in range(B):
+            m[b, :, max(1, L * (b + 1) // (B + 1)):] = float("-inf")
+    elif kind == "left_padding":
+        for b in range(B):
+            m[b, :, :L * (b + 1) // (B + 2)] = float("-inf")
+    elif kind == "band":
+        m[:, ((keys - rows).abs() > 100)] = float("-inf")
+    elif kind == "dense":
+        m = 0.5 * torch.randn(B, L, L, generator=gen)
+    else:
+        for b in range(B):                     # every tile of a kind of its own; whole pairs of query tiles without a key
+            for i in range(0, L, 128):
+                for j in range(0, L, 128):
+                    pick = int(torch.randint(0, 4, (1,), generator=gen))
+                    tile = m[b, i:i + 128, j:j + 128]
+                    if pick == 0 or (b == 0 and i < 256):
+                        tile.fill_(float("-inf"))
+                    elif pick == 1:
+                        tile.copy_(torch.randn(tile.shape, generator=gen))
+                    elif pick == 2:
+                        tile[::3] = float("-inf")
+    return m.half()
+
+
+@pytest.mark.parametrize("B,R,L,H", [(4, 40, 301, 32), (3, 50, 265, 16), (5, 80, 201, 64), (2, 32, 1021, 64), (2, 20, 1101, 128),
+                                     (1, 2, 515, 64), (2, 30, 1928, 64), (2, 30, 2048, 32), (3, 20, 1944, 128), (2, 30, 2048, 128)])
+@pytest.mark.parametrize("kind", ["causal", "padding", "left_padding", "band", "dense", "tiles"])
+def test_planned_masks(B, R, L, H, kind):
+    """Calls that are planned: key tiles that the mask takes away are left out, tiles that are zero or -inf are not
+    fetched, rows on no 16-byte boundary are copied.  The same bits as without a plan, and the oracle's values."""
+    q, k, v = make_inputs(B, L, R * H, 1.0, L)
+    mask = _block_mask(B, L, kind)
+    dev = [t.cuda() for t in (q, k, v, mask)]
+    y = fa.attention_forward(H, 32, *dev, flags=_lib.FLAG_SYNC)
+    assert torch.equal(torch.nan_to_num(y, nan=9.0), torch.nan_to_num(_recorded(*dev[:3], H, dev[3], _lib.FLAG_NO_SPLIT), nan=9.0))
+    cols = slice((R - 1) * H, R * H)
+    assert_close(y[..., cols].float().cpu(), oracle(*(t[..., cols].contiguous() for t in (q, k, v)), H, mask))
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+@pytest.mark.parametrize("where", ["k", "v", "q"])
+@pytest.mark.parametrize("B,R,L", [(2, 30, 2048), (3, 40, 515)])
+def test_masked_keys_that_are_not_finite_are_not_left_out(where, value, B, R, L):
+    """0 * inf and inf - inf are NaN: a masked key with an infinity or a NaN in K or V reaches the result with a plan
+    exactly as it does without one."""
+    H = 64
+    q, k, v = (t.cuda() for t in make_inputs(B, L, R * H, 1.0, L))
+    mask = torch.zeros(B, L, L, dtype=torch.float16)
+    mask[:, :, 200:] = float("-inf")
+    mask = mask.cuda()
+    {"q": q, "k": k, "v": v}[where][1, 450, 7 * H + 3] = value
+    y = fa.attention_forward(H, 32, q, k, v, mask, flags=_lib.FLAG_SYNC)
+    plain = _recorded(q, k, v, H, mask, _lib.FLAG_NO_SPLIT)
+    assert torch.equal(torch.isnan(y), torch.isnan(plain)) and bool(torch.isnan(y).any())
+    assert torch.equal(torch.nan_to_num(y, nan=9.0), torch.nan_to_num(plain, nan=9.0))
