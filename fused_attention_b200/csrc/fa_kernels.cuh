@@ -1398,6 +1398,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         ++gm;
                         if constexpr (C::kMaskBoxes == 1) {   // the second box follows the first in the same place
                             add_mask_tile_row<0, 1>(s, mask_addr(i), row, p.mask_to_score);
+                            fence_proxy_async_smem();   // the row has been read before the next box may land on it
                             __syncwarp();
                             if (lane == 0) mbar_arrive(bar(BAR_MEMPTY0 + i));
                             mbar_wait(bar(BAR_MFULL0 + i), gm & 1u, ctl, kRoleSoftmax | (BAR_MFULL0 + i));
@@ -1408,6 +1409,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                                                       ld_shared_u32(mask_extra_addr(i) + row * 4u));
                         else
                             add_mask_tile_row(s, mask_addr(i), row, p.mask_to_score);
+                        fence_proxy_async_smem();   // the row has been read before the next tile may land on it
                         __syncwarp();
                         if (lane == 0) mbar_arrive(bar(BAR_MEMPTY0 + i));
                     } else if (what == kStepAllNeg) {

@@ -216,6 +216,7 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
                     // this tile's mask tile of this step; its buffer is handed back as soon as it has been read
                     mbar_wait(bar(BAR_MFULL0 + i), g & 1u, ctl, kRoleSoftmax | (BAR_MFULL0 + i));
                     add_mask_tile_row(s, sMask + i * C::kMaskTileBytes, row, p.mask_to_score);
+                    fence_proxy_async_smem();   // the row has been read before the next tile may land on it
                     __syncwarp();
                     if (lane == 0) mbar_arrive(bar(BAR_MEMPTY0 + i));
                 }
