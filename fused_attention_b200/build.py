@@ -49,7 +49,7 @@ def _stale(target: str, sources: list[str]) -> bool:
 
 
 def lib_sources() -> list[str]:
-    return [os.path.join(CSRC, f) for f in ("fa_b200.cu", "fa_kernels.cuh", "fa_mask_plan.cuh", "fa_pair.cuh", "fa_ptx.cuh")] + [
+    return [os.path.join(CSRC, f) for f in ("fa_b200.cu", "fa_kernels.cuh", "fa_mask_plan.cuh", "fa_pair.cuh", "fa_ptx.cuh", "fa_small.cuh")] + [
         os.path.join(ROOT, "include", "fa_b200.h")]
 
 

@@ -19,6 +19,7 @@
 #include "fa_kernels.cuh"
 #include "fa_mask_plan.cuh"
 #include "fa_pair.cuh"
+#include "fa_small.cuh"
 
 namespace {
 
@@ -47,6 +48,7 @@ struct DeviceCtx {
     int cc_major = 0, cc_minor = 0, sm_count = 0, smem_optin = 0;
     uint32_t* status = nullptr;   // device memory: {first failure code, reporting CTA count, id of the launch that reported, -}
     std::atomic<uint32_t> attr_done{0};   // bit per kernel instance whose smem attribute is set
+    std::atomic<uint64_t> small_attr_done{0};   // the same for the instances of the kernel for short sequences
     std::atomic<int> pair_clusters{-1};    // how many CTA pairs of fa_fwd_pair the device holds at once (-1: not asked yet)
     std::atomic<int> pair_clusters_mask{-1};   // the same for the instance with a mask
     // Scratch of launches that divide their last round of work items (fa::Plan): one buffer per stream,
@@ -215,7 +217,23 @@ int validate(const void* q, const void* k, const void* v, const void* mask, cons
     return FA_B200_OK;
 }
 
-// 1 = simple kernel, 2 = pipelined kernel (or the one on pairs of CTAs, see use_pair_kernel).
+// Whether a call goes to the kernel for short sequences (fa_small.cuh): by length, head_dim and mask alone, never by how
+// many problems there are.  Measured, us on the kernel that would have the call otherwise and on this one:
+//   H = 16 and 32: ahead up to 160 keys: H = 32, B=256 R=8 L=49 29 / 12 (with a mask 44 / 12), L=121 32 / 26, L=144
+//   58 / 54 (88 / 68), B=64 R=8 L=144 18.5 / 15.0.
+//   H = 64: B=256 R=8 L=49 31 / 11, L=121 41 / 39, but L=128, where the 128-row tile wastes nothing, B=32 R=16 10.1 /
+//   11.2, and behind that (L=144) 62 / 85, the scores of ten key tiles leaving the SM too few warps; with a mask L=121
+//   95 / 61, L=128 62 / 56, L=144 102 / 92, L=129 119 / 133 (a row that starts anywhere costs its reader twice the loads).
+//   H = 128: B=64 R=16 L=50 21 / 11, L=100 16 / 23; with a mask that TMA cannot fetch L=121 141 / 109.
+bool use_small_kernel(uint32_t H, uint32_t L, bool has_mask) {
+    const bool even_rows = (L & 7u) == 0u;
+    if (H <= 32) return L <= 160;
+    if (H == 64) return has_mask ? L <= 128 || (L <= 160 && even_rows) : L < 128;
+    return L <= 64 || (has_mask && !even_rows && L <= 128);
+}
+
+// 0 = the kernel for short sequences, 1 = simple kernel, 2 = pipelined kernel (or the one on pairs of CTAs, see
+// use_pair_kernel).
 int select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool has_mask, uint32_t flags,
                   int sm_count) {
     if (flags & FA_B200_FLAG_FORCE_SIMPLE) return 1;
@@ -232,6 +250,7 @@ int select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool has_mask,
     // With a mask the pipelined kernel is ahead from the second tile on: its other warps bring the mask in
     // (H = 32, B=1 R=4 L=129 9.7 vs 11.6 us, L=256 7.7 vs 10.1 us, L=1024 17.6 vs 34.9 us).
     const uint64_t pairs = static_cast<uint64_t>((L + 255) / 256) * (F / H) * B;
+    if (use_small_kernel(H, L, has_mask)) return 0;
     if (L <= 128) return 1;
     if (has_mask || L > (H >= 64 ? 5u : 2u) * 128u) return 2;
     if (pairs * 2 < static_cast<uint64_t>(sm_count)) return 1;
@@ -496,6 +515,36 @@ int plan_mask(DeviceCtx& c, const SplitScratch& scratch, const void* k, const vo
     return FA_B200_OK;
 }
 
+// The kernel for short sequences: L at most 160 (128 at head_dim 128).
+template <int H, int KT, bool M>
+int launch_small(DeviceCtx& c, const fa::SmallArgs& a, cudaStream_t st, bool overlap) {
+    auto kern = fa::fa_fwd_small<H, KT, M>;
+    const uint32_t smem = fa::SmallCfg<H, KT>::smem_bytes(a.L, M);
+    const uint64_t bit = 1ull << ((H == 16 ? 0 : H == 32 ? 10 : H == 64 ? 20 : 30) + (KT / 2 - 1) * 2 + (M ? 1 : 0));
+    if (smem > 48u * 1024u && !(c.small_attr_done.load(std::memory_order_acquire) & bit)) {   // setting it twice is harmless
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                   static_cast<int>(fa::SmallCfg<H, KT>::smem_bytes(KT * 16, M)));
+        if (e != cudaSuccess) return static_cast<int>(e);
+        c.small_attr_done.fetch_or(bit, std::memory_order_release);
+    }
+    const cudaError_t e = launch_kernel(kern, dim3(a.R * a.B), KT * 32, smem, st, overlap, a);
+    return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
+}
+template <int H, bool M>
+int launch_small(DeviceCtx& c, const fa::SmallArgs& a, cudaStream_t st, bool overlap) {
+    switch ((a.L + 31u) / 32u) {   // key tiles of 16, two at a time
+        case 1: return launch_small<H, 2, M>(c, a, st, overlap);
+        case 2: return launch_small<H, 4, M>(c, a, st, overlap);
+        case 3: return launch_small<H, 6, M>(c, a, st, overlap);
+        case 4: return launch_small<H, 8, M>(c, a, st, overlap);
+        default: return launch_small<H, H == 128 || (H == 64 && !M) ? 8 : 10, M>(c, a, st, overlap);
+    }
+}
+template <int H>
+int launch_small(DeviceCtx& c, const fa::SmallArgs& a, cudaStream_t st, bool overlap) {
+    return a.mask ? launch_small<H, true>(c, a, st, overlap) : launch_small<H, false>(c, a, st, overlap);
+}
+
 // Device-pointer launch on `st`.  Caller holds no lock.
 int forward_device(const void* q, const void* k, const void* v, const void* mask, void* y, uint32_t B,
                    uint32_t L, uint32_t F, uint32_t H, int device, cudaStream_t st, uint32_t flags) {
@@ -618,6 +667,15 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                     }
                     if (rc == FA_B200_OK && !done && (!planned || mask_tma))
                         rc = launch_single(mask == nullptr ? fa::kNoMask : (mask_tma ? fa::kMaskTma : fa::kMaskCopied));
+                } else if (which == 0) {
+                    const fa::SmallArgs a{static_cast<const __half*>(q), static_cast<const __half*>(k), static_cast<const __half*>(v),
+                                          p.mask, p.y, B, L, F, p.R, p.scale_log2, p.mask_to_score};
+                    switch (H) {
+                        case 16: rc = launch_small<16>(*c, a, st, overlap); break;
+                        case 32: rc = launch_small<32>(*c, a, st, overlap); break;
+                        case 64: rc = launch_small<64>(*c, a, st, overlap); break;
+                        default: rc = launch_small<128>(*c, a, st, overlap); break;
+                    }
                 } else if (mask) {
                     switch (H) {
                         case 16: rc = launch_simple<16, true>(*c, 4, mq, mk, mv, p, st, overlap); break;
@@ -885,11 +943,11 @@ int fa_b200_attention_forward_host(const void* q, const void* k, const void* v, 
         // the result has the same bits as one device-pointer call on the full tensors with
         // FA_B200_FLAG_NO_SPLIT
         // (plain launches: a chunk's kernel is ordered behind copies on other streams, not behind a kernel)
+        // (the kernel for short sequences is chosen by length and head_dim alone, so a chunk gets it as the whole does)
+        const int whole = select_kernel(B, L, F, H, mask_or_null != nullptr, flags, c->sm_count);
         const uint32_t chunk_flags =
             (flags & ~static_cast<uint32_t>(FA_B200_FLAG_SYNC | FA_B200_FLAG_FORCE_SIMPLE | FA_B200_FLAG_FORCE_PIPELINED)) |
-            FA_B200_FLAG_NO_OVERLAP | FA_B200_FLAG_NO_SPLIT |
-            (select_kernel(B, L, F, H, mask_or_null != nullptr, flags, c->sm_count) == 2 ? FA_B200_FLAG_FORCE_PIPELINED
-                                                                                       : FA_B200_FLAG_FORCE_SIMPLE);
+            FA_B200_FLAG_NO_OVERLAP | FA_B200_FLAG_NO_SPLIT | (whole == 0 ? 0u : (whole == 2 ? FA_B200_FLAG_FORCE_PIPELINED : FA_B200_FLAG_FORCE_SIMPLE));
         if (mbytes && !by_batch) {   // the mask is shared by all heads: one copy ahead of everything
             e = cudaMemcpyAsync(c->stage[4], mask_or_null, mbytes, cudaMemcpyHostToDevice, s_in);
             if (e != cudaSuccess) rc = static_cast<int>(e);
@@ -1081,7 +1139,8 @@ int fa_b200_describe_schedule(uint32_t B, uint32_t L, uint32_t F, uint32_t head_
     const uint32_t n = (L + fa::kTile - 1) / fa::kTile;
     const uint32_t n_items = ((L + 2 * fa::kTile - 1) / (2 * fa::kTile)) * (F / head_dim) * B;
     // (head_dim 16 and 32: reported as one CTA per query tile, see the header)
-    const int which = head_dim < 64 ? 1 : select_kernel(B, L, F, head_dim, false, flags, static_cast<int>(sm_count));
+    const int chosen = head_dim < 64 ? 1 : select_kernel(B, L, F, head_dim, false, flags, static_cast<int>(sm_count));
+    const int which = chosen == 0 ? 1 : chosen;   // (short sequences: reported as one CTA per query tile, which it is)
     out[0] = static_cast<uint32_t>(which);
     out[5] = n;
     if (which != 2) {
@@ -1122,7 +1181,7 @@ int fa_b200_select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t head_dim,
         sms = 148;
     }
     const int which = head_dim < 64 ? 1 : select_kernel(B, L, F, head_dim, has_mask != 0, flags, sms);
-    if (which != 2) return which;
+    if (which != 2) return 1;
     const uint32_t n = (L + fa::kTile - 1) / fa::kTile, q_pairs = (L + 2 * fa::kTile - 1) / (2 * fa::kTile);
     const Schedule s = make_schedule(q_pairs * (F / head_dim) * B, n, static_cast<uint32_t>(sms),
                                      (flags & (FA_B200_FLAG_NO_SPLIT | FA_B200_FLAG_FORCE_PAIR)) == 0);

@@ -299,6 +299,16 @@ __device__ __forceinline__ void cp_async_4_part(uint32_t dst, uint64_t src, uint
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
+// 16 bytes; zeros instead of the source when `in` is false (nothing is read then)
+__device__ __forceinline__ void cp_async_16_zero(uint32_t dst, const void* src, bool in) {
+    const uint32_t n = in ? 16u : 0u;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void cp_async_wait_group() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
 __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
@@ -312,6 +322,14 @@ __device__ __forceinline__ uint32_t ld_shared_u32(uint32_t addr) {
     uint32_t w;
     asm volatile("ld.shared.b32 %0, [%1];" : "=r"(w) : "r"(addr));
     return w;
+}
+__device__ __forceinline__ float ld_shared_half(uint32_t addr) {
+    uint16_t w;
+    asm volatile("ld.shared.b16 %0, [%1];" : "=h"(w) : "r"(addr));
+    return __half2float(__ushort_as_half(w));
+}
+__device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v) {
+    asm volatile("st.shared.b32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 __device__ __forceinline__ void st_shared_u16(uint32_t addr, uint16_t v) {
     asm volatile("st.shared.b16 [%0], %1;" ::"r"(addr), "h"(v) : "memory");
@@ -531,6 +549,23 @@ __device__ __forceinline__ void tma_load_3d_pair(uint32_t dst, const void* map, 
         "[%0], [%1, {%3, %4, %5}], [%2];" ::"r"(dst),
         "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(z)
         : "memory");
+}
+
+// ----------------------------------------------------------------------------- warp-wide products (fa_small.cuh)
+// Four 8 x 8 matrices of 16-bit values from shared memory, one row address per lane.
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// d[16 x 8] += a[16 x 16] b[16 x 8], fp16 operands, fp32 sums
+__device__ __forceinline__ void mma_m16n8k16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
 // ----------------------------------------------------------------------------- arithmetic

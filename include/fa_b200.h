@@ -210,8 +210,9 @@ int fa_b200_debug_cycles(void* device_buffer_of_256_u64);
 
 /*
  * Which kernel the default heuristics pick for a shape: returns 1 for the one-tile-per-CTA
- * kernel (and always for head_dim 16 and 32, which the flags cannot force onto another one; by
- * default they are served by either), 2 for the warp-specialised kernel, 3 for the warp-specialised kernel on pairs of CTAs
+ * kernel (and for sequences of one query tile, which may go to a kernel of small CTAs, and always
+ * for head_dim 16 and 32, which the flags cannot force onto another one; by default they are
+ * served by any), 2 for the warp-specialised kernel, 3 for the warp-specialised kernel on pairs of CTAs
  * (head_dim 128, whole work items; a mask is taken to start on a 16-byte boundary, its rows then
  * do so whenever L is a multiple of 8), negative status on invalid arguments.
  * No counterpart in the reference.
