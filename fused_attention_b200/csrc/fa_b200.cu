@@ -274,8 +274,14 @@ struct Schedule {
 // built for).  Dividing has a price, measured at about five key steps per CTA (one more segment boundary,
 // the hand-over of a part through L2 and the merge, which reads 128 KB per other part of an item): it is
 // done when what it saves beyond that is at least a twentieth of the CTA's work.
+// With few items, 3 r CTAs at most as many as SMs, every item is cut into three instead, each CTA taking exactly one
+// part (the cuts of 3 r even ranges fall on the items' ends): when that saves two steps over halves, or three at head_dim
+// 128, where a part to be merged is 128 KB, unless the thirds are even.  Measured, us with halves (or undivided) and thirds:
+//   H = 128: R=4 L=3000 31.1 / 27.8, R=1 L=8192 57.2 / 47.6, R=2 L=5000 43.6 / 36.0, R=4 L=1500 22.3 / 19.6;
+//   R=2 L=2048 22.5 / 22.5, R=8 L=1400 21.1 / 21.4.   H = 64: R=1 L=8192 52.4 / 40.3, R=2 L=2048 19.0 / 17.3, R=3
+//   L=1700 18.5 / 17.2.   H = 32: R=4 L=2048 17.6 / 15.9
 constexpr uint32_t kSplitCostSteps = 5;
-Schedule make_schedule(uint32_t n_items, uint32_t n, uint32_t sms, bool allow_split) {
+Schedule make_schedule(uint32_t H, uint32_t n_items, uint32_t n, uint32_t sms, bool allow_split) {
     Schedule s;
     s.grid = n_items < sms ? n_items : sms;
     s.full_rounds = (n_items + s.grid - 1) / s.grid;
@@ -285,7 +291,9 @@ Schedule make_schedule(uint32_t n_items, uint32_t n, uint32_t sms, bool allow_sp
     if (!allow_split || sms == 0 || n < 2) return s;
     const uint32_t r = n_items % sms;
     if (r == 0) return s;
-    const uint32_t tg = 2u * r < sms ? 2u * r : sms;
+    const uint32_t half = (n + 1u) / 2u, third = (n + 2u) / 3u;
+    const bool thirds = 3u * r <= sms && n >= 12u && half - third >= (H == 128 && n % 3u != 0u ? 3u : 2u);
+    const uint32_t tg = thirds ? 3u * r : (2u * r < sms ? 2u * r : sms);
     const uint64_t T = static_cast<uint64_t>(r) * n;
     if (T * tg > 0xFFFFFFFFull) return s;                 // the kernel's range arithmetic is 32-bit
     const uint32_t most = static_cast<uint32_t>((T + tg - 1) / tg);   // key steps of the busiest tail CTA
@@ -293,7 +301,7 @@ Schedule make_schedule(uint32_t n_items, uint32_t n, uint32_t sms, bool allow_sp
     const uint64_t undivided = static_cast<uint64_t>(s.full_rounds) * n;          // key steps of the busiest CTA, whole items
     const uint64_t gain_needed = kSplitCostSteps + (undivided / 20 > 1 ? undivided / 20 : 1);
     if (static_cast<uint64_t>(most) + gain_needed >= n) return s;
-    if (2u * least + 2u <= n) return s;                   // four parts would fit (cannot happen with tail_grid <= 2 r: guard)
+    if (!thirds && 2u * least + 2u <= n) return s;        // four parts would fit (cannot happen with tail_grid <= 2 r: guard)
     s.grid = n_items < sms ? tg : sms;
     s.full_rounds = n_items / sms;
     s.tail_items = r;
@@ -618,7 +626,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                     bool planned = false;
                     if (want_plan && scratch != nullptr)
                         rc = plan_mask(*c, *scratch, k, v, mask_tma, p, st, overlap, &mask_at, &mask_pitch, &planned);
-                    const Schedule sch = make_schedule(p.n_items, p.n_kv_tiles, sms, want_split && scratch != nullptr && !planned);
+                    const Schedule sch = make_schedule(H, p.n_items, p.n_kv_tiles, sms, want_split && scratch != nullptr && !planned);
                     p.full_rounds = sch.full_rounds;
                     p.tail_items = sch.tail_items;
                     p.tail_steps = sch.tail_steps;
@@ -1148,7 +1156,7 @@ int fa_b200_describe_schedule(uint32_t B, uint32_t L, uint32_t F, uint32_t head_
         out[2] = out[3] = out[4] = out[6] = 0;
         return FA_B200_OK;
     }
-    const Schedule s = make_schedule(n_items, n, sm_count,
+    const Schedule s = make_schedule(head_dim, n_items, n, sm_count,
                                      (flags & (FA_B200_FLAG_NO_SPLIT | FA_B200_FLAG_FORCE_PAIR)) == 0);
     const uint32_t q_pairs = (L + 2 * fa::kTile - 1) / (2 * fa::kTile);
     if (use_pair_kernel(head_dim, false, true, q_pairs, (F / head_dim) * B, sm_count, s.tail_steps, flags) && sm_count >= 2) {
@@ -1183,7 +1191,7 @@ int fa_b200_select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t head_dim,
     const int which = head_dim < 64 ? 1 : select_kernel(B, L, F, head_dim, has_mask != 0, flags, sms);
     if (which != 2) return 1;
     const uint32_t n = (L + fa::kTile - 1) / fa::kTile, q_pairs = (L + 2 * fa::kTile - 1) / (2 * fa::kTile);
-    const Schedule s = make_schedule(q_pairs * (F / head_dim) * B, n, static_cast<uint32_t>(sms),
+    const Schedule s = make_schedule(head_dim, q_pairs * (F / head_dim) * B, n, static_cast<uint32_t>(sms),
                                      (flags & (FA_B200_FLAG_NO_SPLIT | FA_B200_FLAG_FORCE_PAIR)) == 0);
     // (a mask is taken to start on a 16-byte boundary here)
     return use_pair_kernel(head_dim, has_mask != 0, (L & 7u) == 0u, q_pairs, (F / head_dim) * B,

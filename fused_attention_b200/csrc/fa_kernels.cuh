@@ -797,8 +797,8 @@ constexpr uint32_t kMaxParts = 3;
 //     steps in all) evenly among the first tg = Params::tail_grid CTAs: CTA c < tg takes the tail key
 //     steps [c*T/tg, (c+1)*T/tg), numbered item by item.  That range is never longer than n, so it
 //     touches at most two items: up to two tail segments, the first ending an item (or lying inside
-//     one), the second starting the next item at step 0; and never shorter than n/2, so no item is
-//     cut into more than three parts.
+//     one), the second starting the next item at step 0; and never shorter than n/2, or exactly a third
+//     of every item with tg = 3 * tail_items, so no item is cut into more than three parts.
 // A segment that does not cover all n key steps is PARTIAL: its epilogue does not write Y but adds
 // its (reference maximum, row sum, numerator) to the item's other parts, see the epilogue role.
 struct Plan {
