@@ -60,7 +60,7 @@ struct DeviceCtx {
     // grow-on-demand staging buffers
     std::mutex host_mu;   // one host-buffer call at a time per device: they share the staging buffers
     cudaStream_t host_stream = nullptr, host_stream2 = nullptr, host_stream3 = nullptr;
-    cudaEvent_t ev_in[8] = {}, ev_cmp[8] = {};
+    cudaEvent_t ev_in[kHostChunks] = {}, ev_cmp[kHostChunks] = {};
     void* stage[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // q k v y mask
     size_t stage_bytes[5] = {0, 0, 0, 0, 0};
 };
@@ -168,10 +168,10 @@ int make_map(CUtensorMap* map, const void* base, uint32_t B, uint32_t L, uint32_
     return r == CUDA_SUCCESS ? FA_B200_OK : FA_B200_ERR_DRIVER;
 }
 
-// 3-D map {L keys, L rows, B} over a [B, L, L] fp16 mask whose rows are `pitch` elements apart; box = 128 rows x 64
+// 3-D map {L keys, Lq rows, B} over a [B, Lq, L] fp16 mask whose rows are `pitch` elements apart; box = 128 rows x 64
 // keys.  Needs rows that start on 16-byte boundaries (pitch a multiple of 8, base aligned); the caller checks.
-int make_mask_map(CUtensorMap* map, const void* base, uint32_t B, uint32_t L, uint32_t pitch) {
-    const cuuint64_t dims[3] = {L, L, B};
+int make_mask_map(CUtensorMap* map, const void* base, uint32_t B, uint32_t Lq, uint32_t L, uint32_t pitch) {
+    const cuuint64_t dims[3] = {L, Lq, B};
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(pitch) * 2ull, static_cast<cuuint64_t>(pitch) * 2ull * L};
     const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(fa::kTile), 1};
     const cuuint32_t estr[3] = {1, 1, 1};
@@ -553,8 +553,9 @@ int launch_small(DeviceCtx& c, const fa::SmallArgs& a, cudaStream_t st, bool ove
     return a.mask ? launch_small<H, true>(c, a, st, overlap) : launch_small<H, false>(c, a, st, overlap);
 }
 
-// Device-pointer launch on `st`.  Caller holds no lock.
-int forward_device(const void* q, const void* k, const void* v, const void* mask, void* y, uint32_t B,
+// Device-pointer launch on `st`.  Caller holds no lock.  With Lq < L (B = 1) the call is for the Lq query rows that q, y
+// and the mask begin with.
+int forward_device(const void* q, const void* k, const void* v, const void* mask, void* y, uint32_t B, uint32_t Lq,
                    uint32_t L, uint32_t F, uint32_t H, int device, cudaStream_t st, uint32_t flags) {
     int prev = -1;
     cudaError_t e = cudaGetDevice(&prev);
@@ -573,7 +574,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
         if (rc == FA_B200_OK && c->cc_major != 10) rc = FA_B200_ERR_ARCH;
         if (rc == FA_B200_OK) {
             CUtensorMap mq, mk, mv;
-            rc = make_map(&mq, q, B, L, F, H);
+            rc = make_map(&mq, q, B, Lq, F, H);
             if (rc == FA_B200_OK) rc = make_map(&mk, k, B, L, F, H);
             if (rc == FA_B200_OK) rc = make_map(&mv, v, B, L, F, H);
             if (rc == FA_B200_OK) {
@@ -586,9 +587,10 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                 p.F = F;
                 p.launch_id = next_launch_id();
                 p.n_kv_tiles = (L + fa::kTile - 1) / fa::kTile;
-                p.n_q_tiles = p.n_kv_tiles;
+                p.Lq = Lq;
+                p.n_q_tiles = (Lq + fa::kTile - 1) / fa::kTile;
                 p.R = F / H;
-                p.q_pairs = (L + 2 * fa::kTile - 1) / (2 * fa::kTile);
+                p.q_pairs = (Lq + 2 * fa::kTile - 1) / (2 * fa::kTile);
                 p.n_items = p.q_pairs * p.R * B;
                 p.scale_log2 = static_cast<float>(1.4426950408889634 / std::sqrt(static_cast<double>(H)));
                 p.mask_to_score = static_cast<float>(std::sqrt(static_cast<double>(H)));
@@ -617,7 +619,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                     // (Planning a mask needs the same scratch, and a planned call is not divided.)
                     const uint32_t sms = static_cast<uint32_t>(c->sm_count);
                     const bool mask_tma = mask && mask_rows_aligned(mask, L);
-                    const bool want_plan = mask && use_mask_plan(H, p.n_items, p.n_kv_tiles, B, p.q_pairs, mask_tma, sms, flags);
+                    const bool want_plan = mask && Lq == L && use_mask_plan(H, p.n_items, p.n_kv_tiles, B, p.q_pairs, mask_tma, sms, flags);
                     const bool want_split = !(flags & (FA_B200_FLAG_NO_SPLIT | FA_B200_FLAG_FORCE_PAIR));
                     const SplitScratch* scratch = want_plan || want_split ? scratch_for_stream(*c, st) : nullptr;
                     const bool pair = use_pair_kernel(H, mask != nullptr, mask_tma, p.q_pairs, p.R * B, sms, 0, flags);
@@ -638,11 +640,11 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                     }
                     // Y as a TMA store target: boxes of 32 rows x 64 columns (one epilogue warp each)
                     CUtensorMap my;
-                    if (rc == FA_B200_OK) rc = make_map(&my, y, B, L, F, H, 32);
+                    if (rc == FA_B200_OK) rc = make_map(&my, y, B, Lq, F, H, 32);
                     // mask tiles through TMA when every mask row (or row of the plan's copy) starts on a 16-byte
                     // boundary; else two of the warps (of the kernel on single CTAs) copy them with cp.async
                     CUtensorMap mm = mq;
-                    if (rc == FA_B200_OK && (mask_tma || planned)) rc = make_mask_map(&mm, mask_at, B, L, mask_pitch);
+                    if (rc == FA_B200_OK && (mask_tma || planned)) rc = make_mask_map(&mm, mask_at, B, Lq, L, mask_pitch);
                     auto launch_single = [&](int kind) {
                         switch (H) {
                             case 16: return launch_pipelined<16>(*c, 12, kind, mq, mk, mv, my, mm, p, sch.grid, st, overlap);
@@ -656,7 +658,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                     // and the plan says which of them finds work (the other leaves at once, 4 to 6 us).
                     if (rc == FA_B200_OK && planned) {
                         const CUtensorMap wide = my;   // (fa::PipeCfg::kStoreCols of the planned kernel at head_dim 128)
-                        if (H == 128) rc = make_map(&my, y, B, L, F, H, 32, fa::PipeCfg<128, fa::kMaskPlanned>::kStoreCols);
+                        if (H == 128) rc = make_map(&my, y, B, Lq, F, H, 32, fa::PipeCfg<128, fa::kMaskPlanned>::kStoreCols);
                         if (rc == FA_B200_OK) rc = launch_single(fa::kMaskPlanned);
                         my = wide;
                     }
@@ -835,6 +837,7 @@ int fa_b200_attention_forward_noalloc(const void* q, const void* k, const void* 
         p.L = L;
         p.F = F;
         p.n_kv_tiles = n_q_tiles;
+        p.Lq = L;
         p.n_q_tiles = n_q_tiles;
         p.R = F / H;
         p.q_pairs = (L + 2 * fa::kTile - 1) / (2 * fa::kTile);
@@ -890,7 +893,7 @@ int fa_b200_attention_forward(const void* q, const void* k, const void* v, const
                               uint32_t chunk_hint, int device, void* cuda_stream, uint32_t flags) {
     const int rc = validate(q, k, v, mask_or_null, y, B, L, F, head_dim, chunk_hint, flags);
     if (rc != FA_B200_OK) return rc;
-    return forward_device(q, k, v, mask_or_null, y, B, L, F, head_dim, device,
+    return forward_device(q, k, v, mask_or_null, y, B, L, L, F, head_dim, device,
                           static_cast<cudaStream_t>(cuda_stream), flags);
 }
 
@@ -936,17 +939,20 @@ int fa_b200_attention_forward_host(const void* q, const void* k, const void* v, 
         if (rc == FA_B200_OK && mbytes) rc = grow(*c, 4, mbytes);
     }
     if (rc == FA_B200_OK) {
-        // Chunked pipeline over three streams: while chunk c computes, chunk c+1 is copied in and
-        // chunk c-1 is copied out (PCIe carries both directions at once).  Chunks are groups of
-        // batch entries (contiguous in host memory) when B >= 2, otherwise groups of heads moved
-        // with pitched copies into compact [B, L, heads*H] device slices.
+        // Chunked pipeline over three streams: while chunk c computes, chunk c+1 is copied in and chunk c-1 is copied
+        // out.  Chunks are groups of batch entries where there are enough of
+        // them; otherwise K and V of an entry go ahead and its queries (with their rows of the mask) follow in blocks
+        // of rows, so that what is left behind the last copy in is one block's product and copy out.  Every copy is one
+        // contiguous run: the 2-D copies that a division by heads needs move 44 GB/s with rows of 2 KB and 38 with 1 KB
+        // against 54 here.  Measured, pinned buffers, us by heads and by rows: B=1 R=8 L=256 H=64 165 / 81, B=1 R=16
+        // L=1000 H=128 449 / 339, B=1 R=32 L=1024 H=128 683 / 632; B=2 R=32 L=1024 H=128 (by batch entries before) 1187 /
+        // 1178, where the two directions together move 57 GB/s, all that the box gives.  Sixteen chunks are no better.
         cudaStream_t s_in = c->host_stream, s_cmp = c->host_stream2, s_out = c->host_stream3;
-        const uint32_t H = head_dim, R = F / H;
-        const bool by_batch = B >= 2;
-        const uint32_t units = by_batch ? B : R;
-        const uint32_t n_chunks = units < kHostChunks ? units : kHostChunks;
-        const __half* hsrc[3] = {static_cast<const __half*>(q), static_cast<const __half*>(k),
-                                 static_cast<const __half*>(v)};
+        const uint32_t H = head_dim;
+        const __half *hq = static_cast<const __half*>(q), *hk = static_cast<const __half*>(k), *hv = static_cast<const __half*>(v);
+        const __half* hm = static_cast<const __half*>(mask_or_null);
+        __half *dq = static_cast<__half*>(c->stage[0]), *dk = static_cast<__half*>(c->stage[1]), *dv = static_cast<__half*>(c->stage[2]);
+        __half *dy = static_cast<__half*>(c->stage[3]), *dm = static_cast<__half*>(c->stage[4]);
         // every chunk runs the kernel the whole problem would get, with every work item undivided, so
         // the result has the same bits as one device-pointer call on the full tensors with
         // FA_B200_FLAG_NO_SPLIT
@@ -956,61 +962,49 @@ int fa_b200_attention_forward_host(const void* q, const void* k, const void* v, 
         const uint32_t chunk_flags =
             (flags & ~static_cast<uint32_t>(FA_B200_FLAG_SYNC | FA_B200_FLAG_FORCE_SIMPLE | FA_B200_FLAG_FORCE_PIPELINED)) |
             FA_B200_FLAG_NO_OVERLAP | FA_B200_FLAG_NO_SPLIT | (whole == 0 ? 0u : (whole == 2 ? FA_B200_FLAG_FORCE_PIPELINED : FA_B200_FLAG_FORCE_SIMPLE));
-        if (mbytes && !by_batch) {   // the mask is shared by all heads: one copy ahead of everything
-            e = cudaMemcpyAsync(c->stage[4], mask_or_null, mbytes, cudaMemcpyHostToDevice, s_in);
-            if (e != cudaSuccess) rc = static_cast<int>(e);
-        }
-        size_t dev_off = 0;   // elements into the staging buffers
-        for (uint32_t ch = 0; ch < n_chunks && rc == FA_B200_OK; ++ch) {
-            const uint32_t u0 = static_cast<uint32_t>(static_cast<uint64_t>(units) * ch / n_chunks);
-            const uint32_t u1 = static_cast<uint32_t>(static_cast<uint64_t>(units) * (ch + 1) / n_chunks);
-            const uint32_t nu = u1 - u0;
-            if (nu == 0) continue;
-            const uint32_t cB = by_batch ? nu : B, cF = by_batch ? F : nu * H;
-            const size_t elems = static_cast<size_t>(cB) * L * cF;
-            __half* d[4];
-            for (int i = 0; i < 4; ++i) d[i] = static_cast<__half*>(c->stage[i]) + dev_off;
-            const __half* dmask = nullptr;
-            for (int i = 0; i < 3 && rc == FA_B200_OK; ++i) {
-                if (by_batch)
-                    e = cudaMemcpyAsync(d[i], hsrc[i] + static_cast<size_t>(u0) * L * F, elems * sizeof(__half),
-                                        cudaMemcpyHostToDevice, s_in);
-                else
-                    e = cudaMemcpy2DAsync(d[i], static_cast<size_t>(cF) * sizeof(__half), hsrc[i] + static_cast<size_t>(u0) * H,
-                                          static_cast<size_t>(F) * sizeof(__half), static_cast<size_t>(cF) * sizeof(__half),
-                                          static_cast<size_t>(B) * L, cudaMemcpyHostToDevice, s_in);
-                if (e != cudaSuccess) rc = static_cast<int>(e);
+        auto in = [&](__half* dst, const __half* src, size_t at, size_t elems) {
+            if (rc != FA_B200_OK) return;
+            const cudaError_t err = cudaMemcpyAsync(dst + at, src + at, elems * sizeof(__half), cudaMemcpyHostToDevice, s_in);
+            if (err != cudaSuccess) rc = static_cast<int>(err);
+        };
+        const uint32_t groups = B < kHostChunks ? B : kHostChunks;   // of batch entries
+        // blocks of query rows per group: whole work items (256 rows), no smaller than half a megabyte, eight chunks in all
+        uint32_t blocks = 1, block_rows = L;
+        if (whole != 0 && B < kHostChunks) {
+            const uint32_t pairs = (L + 2 * fa::kTile - 1) / (2 * fa::kTile), most = kHostChunks / B;
+            const size_t pair_bytes = static_cast<size_t>(2 * fa::kTile) * F * sizeof(__half), least = (1u << 19) / pair_bytes + 1;
+            uint32_t per = (pairs + most - 1) / most;
+            if (per < least) per = static_cast<uint32_t>(least);
+            if (per < pairs) {
+                block_rows = per * 2 * fa::kTile;
+                blocks = (pairs + per - 1) / per;
             }
-            if (rc == FA_B200_OK && mbytes) {
-                if (by_batch) {
-                    const size_t moff = static_cast<size_t>(u0) * L * L;
-                    e = cudaMemcpyAsync(static_cast<__half*>(c->stage[4]) + moff,
-                                        static_cast<const __half*>(mask_or_null) + moff,
-                                        static_cast<size_t>(nu) * L * L * sizeof(__half), cudaMemcpyHostToDevice, s_in);
+        }
+        uint32_t ch = 0;   // chunk: an event pair each
+        for (uint32_t gr = 0; gr < groups && rc == FA_B200_OK; ++gr) {
+            const uint32_t b0 = static_cast<uint32_t>(static_cast<uint64_t>(B) * gr / groups);
+            const uint32_t nb = static_cast<uint32_t>(static_cast<uint64_t>(B) * (gr + 1) / groups) - b0;
+            const size_t kv_at = static_cast<size_t>(b0) * L * F;
+            in(dk, hk, kv_at, static_cast<size_t>(nb) * L * F);
+            in(dv, hv, kv_at, static_cast<size_t>(nb) * L * F);
+            for (uint32_t bl = 0; bl < blocks && rc == FA_B200_OK; ++bl, ++ch) {
+                const uint32_t r0 = bl * block_rows, rows = blocks == 1 ? L : (L - r0 < block_rows ? L - r0 : block_rows);
+                const size_t at = kv_at + static_cast<size_t>(r0) * F, elems = (blocks == 1 ? static_cast<size_t>(nb) * L : rows) * F;
+                const size_t m_at = (static_cast<size_t>(b0) * L + r0) * L;
+                in(dq, hq, at, elems);
+                if (hm) in(dm, hm, m_at, elems / F * L);
+                if (rc == FA_B200_OK && (e = cudaEventRecord(c->ev_in[ch], s_in)) != cudaSuccess) rc = static_cast<int>(e);
+                if (rc == FA_B200_OK && (e = cudaStreamWaitEvent(s_cmp, c->ev_in[ch], 0)) != cudaSuccess) rc = static_cast<int>(e);
+                if (rc == FA_B200_OK)
+                    rc = forward_device(dq + at, dk + kv_at, dv + kv_at, hm ? dm + m_at : nullptr, dy + at, nb, rows, L, F, H,
+                                        device, s_cmp, chunk_flags);
+                if (rc == FA_B200_OK && (e = cudaEventRecord(c->ev_cmp[ch], s_cmp)) != cudaSuccess) rc = static_cast<int>(e);
+                if (rc == FA_B200_OK && (e = cudaStreamWaitEvent(s_out, c->ev_cmp[ch], 0)) != cudaSuccess) rc = static_cast<int>(e);
+                if (rc == FA_B200_OK) {
+                    e = cudaMemcpyAsync(static_cast<__half*>(y) + at, dy + at, elems * sizeof(__half), cudaMemcpyDeviceToHost, s_out);
                     if (e != cudaSuccess) rc = static_cast<int>(e);
-                    dmask = static_cast<const __half*>(c->stage[4]) + moff;
-                } else {
-                    dmask = static_cast<const __half*>(c->stage[4]);
                 }
             }
-            if (rc == FA_B200_OK && (e = cudaEventRecord(c->ev_in[ch], s_in)) != cudaSuccess) rc = static_cast<int>(e);
-            if (rc == FA_B200_OK && (e = cudaStreamWaitEvent(s_cmp, c->ev_in[ch], 0)) != cudaSuccess) rc = static_cast<int>(e);
-            if (rc == FA_B200_OK)
-                rc = forward_device(d[0], d[1], d[2], dmask, d[3], cB, L, cF, head_dim, device, s_cmp, chunk_flags);
-            if (rc == FA_B200_OK && (e = cudaEventRecord(c->ev_cmp[ch], s_cmp)) != cudaSuccess) rc = static_cast<int>(e);
-            if (rc == FA_B200_OK && (e = cudaStreamWaitEvent(s_out, c->ev_cmp[ch], 0)) != cudaSuccess) rc = static_cast<int>(e);
-            if (rc == FA_B200_OK) {
-                __half* hy = static_cast<__half*>(y);
-                if (by_batch)
-                    e = cudaMemcpyAsync(hy + static_cast<size_t>(u0) * L * F, d[3], elems * sizeof(__half),
-                                        cudaMemcpyDeviceToHost, s_out);
-                else
-                    e = cudaMemcpy2DAsync(hy + static_cast<size_t>(u0) * H, static_cast<size_t>(F) * sizeof(__half), d[3],
-                                          static_cast<size_t>(cF) * sizeof(__half), static_cast<size_t>(cF) * sizeof(__half),
-                                          static_cast<size_t>(B) * L, cudaMemcpyDeviceToHost, s_out);
-                if (e != cudaSuccess) rc = static_cast<int>(e);
-            }
-            dev_off += elems;
         }
         // all three streams drain before the staging buffers may be reused or the result read
         cudaError_t e1 = cudaStreamSynchronize(s_in), e2 = cudaStreamSynchronize(s_cmp), e3 = cudaStreamSynchronize(s_out);

@@ -41,6 +41,7 @@ struct Params {
     uint32_t launch_id;   // non-zero and different for every launch of the process
     uint32_t n_q_tiles;   // ceil(L / 128)
     uint32_t B, L, F;
+    uint32_t Lq;          // query rows: L, or with B = 1 those of a block that q, y and the mask begin with
     uint32_t n_kv_tiles;  // ceil(L / 128)
     uint32_t R;           // heads = F / H
     uint32_t q_pairs;     // ceil(L / 256): pairs of query tiles per (batch, head)
@@ -444,7 +445,7 @@ struct MaskRows {
 __device__ __forceinline__ MaskRows mask_rows(const Params& p) {
     MaskRows m;
     m.base = reinterpret_cast<uint64_t>(p.mask);
-    m.end = m.base + 2ull * p.B * p.L * p.L;
+    m.end = m.base + 2ull * (static_cast<uint64_t>(p.B - 1u) * p.L + p.Lq) * p.L;
     m.wide = (((p.L * 2u) | static_cast<uint32_t>(m.base)) & 7u) == 0u;
     m.shifted = (((p.L * 2u) | static_cast<uint32_t>(m.base)) & 2u) != 0u;
     return m;
@@ -461,7 +462,7 @@ __device__ __forceinline__ void copy_mask_rows(const Params& p, const MaskRows& 
                                                uint32_t batch, uint32_t q0, uint32_t key0, uint32_t r0, uint32_t lane) {
     const uint64_t first = m.base + 2ull * ((static_cast<uint64_t>(batch) * p.L + q0 + r0) * p.L + key0);
     const uint64_t pitch = 2ull * p.L;
-    const uint32_t n = q0 + r0 < p.L ? min(kRows, p.L - q0 - r0) : 0u;
+    const uint32_t n = q0 + r0 < p.Lq ? min(kRows, p.Lq - q0 - r0) : 0u;
 #pragma unroll 1
     for (uint32_t g = 0; g < n; g += 8u) {
         const uint64_t at = first + g * pitch;
@@ -613,7 +614,7 @@ fa_fwd_simple(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
 
     float m = -INFINITY, l = 0.f;
     const uint32_t q_row = q_tile * kTile + tid;
-    const bool row_valid = q_row < p.L;
+    const bool row_valid = q_row < p.Lq;
 
     for (uint32_t j = 0; j < n_tiles; ++j) {
         const uint32_t ph = j & 1u;
@@ -1523,7 +1524,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 seen = __shfl_sync(0xffffffffu, seen, 0);
                 bool last = seen + 1u == po.parts;
                 if (last && po.parts == 2u) {
-                    merge_two<H>(p, tail_item, po.c_first, i, row, mine, tO, m, l, y_row, q_row < p.L, wait_for_o);
+                    merge_two<H>(p, tail_item, po.c_first, i, row, mine, tO, m, l, y_row, q_row < p.Lq, wait_for_o);
                 } else {
                     wait_for_o();
                     if (!last) {
@@ -1537,7 +1538,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         if (last) __threadfence();
                     }
                     if (last)
-                        merge_parts<H>(p, tail_item, i, row, mine, tO, m, l, y_row, q_row < p.L);
+                        merge_parts<H>(p, tail_item, i, row, mine, tO, m, l, y_row, q_row < p.Lq);
                 }
                 if (last) {
                     __syncwarp();
@@ -1560,7 +1561,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             stage_o_row<H, C::kStoreCols>(tO, 1.f / l, stage, lane);
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0 && row0 < static_cast<int32_t>(p.L)) {
+            if (lane == 0 && row0 < static_cast<int32_t>(p.Lq)) {
 #pragma unroll
                 for (int half = 0; half < H / C::kStoreCols; ++half)
                     tma_store_3d(&tmY, stage + half * (64u * C::kStoreCols), static_cast<int32_t>((bh % p.R) * H + half * C::kStoreCols),
@@ -1580,7 +1581,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 __half* y_row = p.y + (static_cast<size_t>(bh / p.R) * p.L + q_row) * p.F + (bh % p.R) * H;
                 const uint32_t tail_item = seg_tail_item(pl_s, t0, t0);
                 __threadfence();
-                merge_parts<H>(p, tail_item, i, row, kMaxParts, tO, 0.f, 0.f, y_row, q_row < p.L);
+                merge_parts<H>(p, tail_item, i, row, kMaxParts, tO, 0.f, 0.f, y_row, q_row < p.Lq);
                 __syncwarp();
                 if (lane == 0) atomicExch(p.part_cnt + (tail_item * 2u + i) * 4u + wq, 0u);
             }
@@ -1655,7 +1656,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         }
                         fence_proxy_async_smem();
                         __syncwarp();
-                        if (lane == 0 && row0 < static_cast<int32_t>(p.L)) {   // rows past L are clipped by the store
+                        if (lane == 0 && row0 < static_cast<int32_t>(p.Lq)) {   // rows past Lq are clipped by the store
                             tma_store_3d(&tmY, stage, static_cast<int32_t>(head * H + half * W), row0,
                                          static_cast<int32_t>(batch));
                             bulk_commit_group();

@@ -300,7 +300,7 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
             stage_o_row<H>(tO, 1.f / l_last, stage, lane);
             fence_proxy_async_smem();
             __syncwarp();
-            if (lane == 0 && row0 < static_cast<int32_t>(p.L)) {
+            if (lane == 0 && row0 < static_cast<int32_t>(p.Lq)) {
 #pragma unroll
                 for (int half = 0; half < H / 64; ++half)
                     tma_store_3d(&tmY, stage + half * 4096u, static_cast<int32_t>((bh % p.R) * H + half * 64), row0,
@@ -361,7 +361,7 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
                     }
                     fence_proxy_async_smem();
                     __syncwarp();
-                    if (lane == 0 && row0 < static_cast<int32_t>(p.L)) {
+                    if (lane == 0 && row0 < static_cast<int32_t>(p.Lq)) {
                         tma_store_3d(&tmY, stage, static_cast<int32_t>(head * H + half * 64), row0,
                                      static_cast<int32_t>(batch));
                         bulk_commit_group();

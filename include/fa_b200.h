@@ -99,7 +99,7 @@ int fa_b200_attention_forward(const void* q, const void* k, const void* v,
 /*
  * Same operator with HOST buffers: copies q, k, v (and mask) to the device, runs the kernel and
  * copies y back, and returns when y is complete.  The work is cut into up to 8 chunks (batch
- * entries, or heads when B = 1) that flow through three internal streams, so the copy-in of one
+ * entries, or blocks of query rows of one where there are few) that flow through three internal streams, so the copy-in of one
  * chunk, the kernel of the previous and the copy-out of the one before overlap; pinned host
  * buffers are needed for that overlap.  Device staging buffers are cached per device and grow on
  * demand.  This is the call a torch-free
