@@ -59,6 +59,8 @@ class LibraryNotBuilt(RuntimeError):
 def load() -> ctypes.CDLL:
     """Return the loaded library, loading it on first use.  Raises if it is missing."""
     global _lib
+    if _lib is not None:   # (set once, when everything else about it is set up)
+        return _lib
     with _lock:
         if _lib is not None:
             return _lib
