@@ -510,8 +510,10 @@ int plan_mask(DeviceCtx& c, const SplitScratch& scratch, const void* k, const vo
     a.copy_pitch = pitch;
     a.stamp = p.launch_id;
     a.dense_allowed = mask_tma ? 1u : 0u;
-    const uint64_t most = static_cast<uint64_t>(fa::kPlanCtasPerSm) * c.sm_count, wide = tiles > jobs ? tiles : jobs;
-    cudaError_t e = launch_kernel(fa::fa_mask_plan, dim3(static_cast<unsigned>(wide < most ? wide : most)), fa::kPlanThreads, 0, st, overlap, a);
+    const uint64_t most = static_cast<uint64_t>(mask_tma ? fa::kPlanCtasPerSm : fa::kPlanCopyCtasPerSm) * c.sm_count;
+    const uint64_t wide = tiles > jobs ? tiles : jobs;
+    cudaError_t e = launch_kernel(mask_tma ? fa::fa_mask_plan<false> : fa::fa_mask_plan<true>,
+                                  dim3(static_cast<unsigned>(wide < most ? wide : most)), fa::kPlanThreads, 0, st, overlap, a);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return static_cast<int>(e);
     p.plan_head = a.head;

@@ -33,12 +33,15 @@ struct PlanArgs {
 };
 constexpr uint8_t kTileNeg = 0, kTileZero = 1, kTileMixed = 2;
 constexpr uint32_t kPlanThreads = 256;
-constexpr uint32_t kPlanCtasPerSm = 4;      // 128 KB of loads in flight per SM
+// CTAs per SM, 32 KB of loads in flight each; the instance that copies keeps a tile in registers, which fewer leave room for
+// (B=4 R=12 L=1021 H=64, the whole call: 40.5 us with four, 39.2 with three, 40.8 with two).
+constexpr uint32_t kPlanCtasPerSm = 4, kPlanCopyCtasPerSm = 3;
 constexpr uint32_t kPlanCols = 128;         // columns of K or V that are looked through at a time
 constexpr uint32_t kPlanMaxTiles = 256;     // key tiles per sequence,
 constexpr uint32_t kPlanMaxGroups = 1024;   // and pairs of query tiles of all batch entries that the lists are built for
 
 // One 128 x 128 tile of the mask: its class, and its copy.
+template <bool kCopy>
 __device__ __forceinline__ void plan_mask_tile(const PlanArgs& a, uint32_t tile) {
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t kt = tile % a.n, qt = (tile / a.n) % a.n, b = tile / (a.n * a.n);
@@ -47,14 +50,18 @@ __device__ __forceinline__ void plan_mask_tile(const PlanArgs& a, uint32_t tile)
     const uint32_t rows = row0 < a.L ? min(16u, a.L - row0) : 0u;   // of this warp
     const uint32_t keys = min(kTile + 0u, a.L - key0);
     uint32_t not_neg = 0, not_zero = 0;
-    // rows on no 16-byte boundary: two keys at a time, keys 2 * lane and 64 + 2 * lane of row r
+    // Rows on no 16-byte boundary: this warp's 16 rows in whole words where all of them, and a word more, lie inside the
+    // mask (B=4 R=12 L=1021 H=64, the whole call 46 us with values one by one, 39 with words), else value by value.
+    const uint64_t mask0 = reinterpret_cast<uint64_t>(a.mask), first = reinterpret_cast<uint64_t>(base), pitch = 2ull * a.L;
+    const bool words = (first & ~3ull) >= mask0 && first + 15u * pitch + 260u <= mask0 + 2ull * a.B * a.L * a.L;
+    uint32_t w[16][2], extra = 0;
     auto two_keys = [&](uint32_t r, uint32_t col) -> uint32_t {
         const uint16_t* at = base + static_cast<size_t>(r) * a.L + col;
         const uint32_t lo = r < rows && col < keys ? __ldg(at) : 0u;
         const uint32_t hi = r < rows && col + 1u < keys ? __ldg(at + 1) : 0u;
         return lo | (hi << 16);
     };
-    if (a.copy == nullptr) {   // rows on 16-byte boundaries: two rows a load, eight keys a lane (L is a multiple of 8)
+    if constexpr (!kCopy) {   // rows on 16-byte boundaries: two rows a load, eight keys a lane (L is a multiple of 8)
         const uint32_t col = (lane & 15u) * 8u;
         uint4 x[8];
 #pragma unroll
@@ -70,29 +77,65 @@ __device__ __forceinline__ void plan_mask_tile(const PlanArgs& a, uint32_t tile)
                 not_zero |= (x[i].x | x[i].y | x[i].z | x[i].w) & 0x7FFF7FFFu;
             }
         }
-    } else {
-#pragma unroll 8
+    } else if (words) {
+        // Whole aligned words: word j of a row that starts in the middle of one holds its keys 2 j - 1 and 2 j.
+#pragma unroll
         for (uint32_t r = 0; r < 16; ++r)
 #pragma unroll
+            for (uint32_t h = 0; h < 2; ++h)
+                w[r][h] = __ldg(reinterpret_cast<const uint32_t*>((first + r * pitch) & ~3ull) + h * 32u + lane);
+        extra = __ldg(reinterpret_cast<const uint32_t*>((first + (lane & 15u) * pitch) & ~3ull) + 64u);   // of row `lane`
+#pragma unroll
+        for (uint32_t r = 0; r < 16; ++r) {
+            const uint32_t sh = static_cast<uint32_t>((first + r * pitch) >> 1) & 1u;
+#pragma unroll
             for (uint32_t h = 0; h < 2; ++h) {
-                const uint32_t col = h * 64u + lane * 2u, w = two_keys(r, col);
+                const uint32_t lo = (h * 32u + lane) * 2u - sh;   // key of the low half (wraps below 0)
+                const uint32_t valid = r < rows ? (lo < keys ? 0xFFFFu : 0u) | (lo + 1u < keys ? 0xFFFF0000u : 0u) : 0u;
+                not_neg |= (w[r][h] ^ 0xFC00FC00u) & valid;
+                not_zero |= w[r][h] & 0x7FFF7FFFu & valid;
+            }
+        }
+        const uint32_t valid = lane < rows && ((first + lane * pitch) & 2u) != 0u && keys == kTile ? 0xFFFFu : 0u;   // key 127
+        not_neg |= (extra ^ 0xFC00FC00u) & valid;
+        not_zero |= extra & 0x7FFF7FFFu & valid;
+    } else {
+#pragma unroll 1
+        for (uint32_t r = 0; r < rows; ++r)
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+                const uint32_t col = h * 64u + lane * 2u, v = two_keys(r, col);
                 const uint32_t valid = r < rows ? (col + 1u < keys ? 0xFFFFFFFFu : (col < keys ? 0xFFFFu : 0u)) : 0u;
-                not_neg |= (w ^ 0xFC00FC00u) & valid;
-                not_zero |= w & 0x7FFF7FFFu & valid;
+                not_neg |= (v ^ 0xFC00FC00u) & valid;
+                not_zero |= v & 0x7FFF7FFFu & valid;
             }
     }
     const bool any_not_neg = __syncthreads_or(not_neg != 0u), any_not_zero = __syncthreads_or(not_zero != 0u);
     if (tid == 0) a.cls[tile] = !any_not_neg ? kTileNeg : (any_not_zero ? kTileMixed : kTileZero);
-    if (a.copy != nullptr && any_not_neg && any_not_zero) {   // (the values again, from L1)
+    if constexpr (kCopy) {
+        if (!any_not_neg || !any_not_zero) return;
         uint16_t* dst = reinterpret_cast<uint16_t*>(a.copy) + (static_cast<size_t>(b) * a.L + row0) * a.copy_pitch + key0;
-#pragma unroll 4
-        for (uint32_t r = 0; r < 16; ++r)
+        auto put = [&](uint32_t r, uint32_t h, uint32_t v) {
+            const uint32_t col = h * 64u + lane * 2u;
+            if (r < rows && col < keys)   // (the pitch is even: the second key has a place)
+                *reinterpret_cast<uint32_t*>(dst + static_cast<size_t>(r) * a.copy_pitch + col) = v;
+        };
+        if (words) {
 #pragma unroll
-            for (uint32_t h = 0; h < 2; ++h) {
-                const uint32_t col = h * 64u + lane * 2u, w = two_keys(r, col);
-                if (r < rows && col < keys)   // (the pitch is even: the second key has a place)
-                    *reinterpret_cast<uint32_t*>(dst + static_cast<size_t>(r) * a.copy_pitch + col) = w;
+            for (uint32_t r = 0; r < 16; ++r) {   // the word behind each, from the next lane, and the two put together
+                const uint32_t sh = (static_cast<uint32_t>((first + r * pitch) >> 1) & 1u) * 16u;
+                const uint32_t n0 = __shfl_sync(0xffffffffu, w[r][0], (lane + 1u) & 31u), n1 = __shfl_sync(0xffffffffu, w[r][1], (lane + 1u) & 31u);
+                const uint32_t head1 = __shfl_sync(0xffffffffu, w[r][1], 0), tail = __shfl_sync(0xffffffffu, extra, r);
+                put(r, 0, __funnelshift_r(w[r][0], lane == 31u ? head1 : n0, sh));
+                put(r, 1, __funnelshift_r(w[r][1], lane == 31u ? tail : n1, sh));
             }
+        } else {
+#pragma unroll 1
+            for (uint32_t r = 0; r < rows; ++r) {
+                put(r, 0, two_keys(r, lane * 2u));
+                put(r, 1, two_keys(r, 64u + lane * 2u));
+            }
+        }
     }
 }
 
@@ -123,9 +166,10 @@ __device__ __forceinline__ void plan_finite(const PlanArgs& a, const __half* x, 
     if (bits & 0x80008000u) a.bad[b * a.n + kt] = a.stamp;
 }
 
-// grid: at most kPlanCtasPerSm CTAs per SM.  The tiles of the mask round-robin, then a run of the parts of K and V; the
+// kCopy: the mask's rows start on no 16-byte boundary and are copied.  grid: at most the launch bound's CTAs per SM.  The tiles of the mask round-robin, then a run of the parts of K and V; the
 // CTA that is through last writes the lists, one group of 8, 16 or 32 lanes per pair of query tiles.
-__global__ void __launch_bounds__(kPlanThreads, kPlanCtasPerSm) fa_mask_plan(const PlanArgs a) {
+template <bool kCopy>
+__global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPlanCtasPerSm) fa_mask_plan(const PlanArgs a) {
     __shared__ uint32_t hist[kPlanMaxTiles + 1], cost[2];
     __shared__ uint16_t lens[kPlanMaxGroups];
     __shared__ bool last;
@@ -150,7 +194,7 @@ __global__ void __launch_bounds__(kPlanThreads, kPlanCtasPerSm) fa_mask_plan(con
             return;
         }
     }
-    for (uint32_t t = blockIdx.x; t < a.B * n * n; t += gridDim.x) plan_mask_tile(a, t);
+    for (uint32_t t = blockIdx.x; t < a.B * n * n; t += gridDim.x) plan_mask_tile<kCopy>(a, t);
     const uint32_t chunks = (a.F + kPlanCols - 1u) / kPlanCols, jobs = a.B * n * 2u * chunks;   // (launcher: below 2^31 / gridDim.x)
     uint32_t job = static_cast<uint32_t>(static_cast<uint64_t>(jobs) * blockIdx.x / gridDim.x);
     const uint32_t job_end = static_cast<uint32_t>(static_cast<uint64_t>(jobs) * (blockIdx.x + 1u) / gridDim.x);
