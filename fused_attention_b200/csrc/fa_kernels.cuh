@@ -4,7 +4,7 @@
 //   fa_fwd_simple<H, kHasMask>  one 128-row query tile per CTA, 128 threads, every step in program
 //                               order.  Covers every head_dim (16, 32, 64, 128), the additive mask
 //                               and tiny problems; several CTAs per SM overlap one another.
-//   fa_fwd_pipelined<H, kHasMask>  two 128-row query tiles per CTA, 512 threads split into roles
+//   fa_fwd_pipelined<H, kMask>  two 128-row query tiles per CTA, 512 threads split into roles
 //                               (2 softmax warpgroups, 1 epilogue warpgroup, 1 or 2 MMA warps, 1 TMA
 //                               warp, 1 warp for the mask tiles); K/V stream through a shared-memory
 //                               ring; the softmax of one tile overlaps the MMAs of the other.
