@@ -1318,14 +1318,22 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // will stop at this same point: the overlap is never deeper than one launch).
     grid_dep_wait();
     grid_dep_launch();
+    // A planned kernel ahead of this launch may have taken the call: no segments here then.  The producer thread finds out
+    // before it asks for anything, because with no segments no role would wait for a copy and the CTA would leave with it
+    // still landing in its shared memory.
+    if constexpr (kMask == kMaskTma) {
+        if (first_known && p.plan_head != nullptr && __ldg(p.plan_head) != 0u) {
+            plan_smem = Plan{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
+            first_known = false;
+        }
+    }
     if (first_known) {   // the producer thread only
         load_tile<H>(sQ, &tmQ, bar(BAR_QFULL0), first_col0, first_q_row0, first_batch);
         load_tile<H>(sRing, &tmK, bar(BAR_FULL), first_col0, first_key0, first_batch);
     }
     if (tid == 15 * 32) leave_early_if_launch_failed(ctl);
-    if constexpr (kMask == kMaskTma) {   // the planned kernel before this one has taken the call: no segments here
-        if (p.plan_head != nullptr && tid == 13 * 32 && __ldg(p.plan_head) != 0u) plan_smem = Plan{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-        if (p.plan_head != nullptr) __syncthreads();
+    if constexpr (kMask == kMaskTma) {
+        if (p.plan_head != nullptr) __syncthreads();   // plan_smem may have been emptied
     }
     if constexpr (kPlanned) {
         // the lists were written by the kernel before this one, so this CTA's plan is made behind the wait for it

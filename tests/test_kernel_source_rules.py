@@ -1,0 +1,26 @@
+"""Rules that the kernels keep by the order or the kind of their instructions, and that no run can be made to show."""
+import os
+import re
+
+import fused_attention_b200 as fa
+
+CSRC = os.path.join(os.path.dirname(fa.__file__), "csrc")
+
+
+def source(name):
+    with open(os.path.join(CSRC, name)) as f:
+        return re.sub(r"//[^\n]*", "", f.read())
+
+
+def body_behind_the_wait(name, kernel):
+    text = source(name)
+    text = text[text.index(f"\n{kernel}("):]
+    return text[text.index("grid_dep_wait();"):]
+
+
+def test_a_launch_without_work_asks_for_no_copies():
+    """A kernel that stands behind a planned one reads whether that one took the call before its first copy: with nothing
+    to do no role waits for a copy, and the CTA would leave with it still landing in shared memory."""
+    for name, kernel in (("fa_kernels.cuh", "fa_fwd_pipelined"), ("fa_pair.cuh", "fa_fwd_pair")):
+        text = body_behind_the_wait(name, kernel)
+        assert text.index("p.plan_head") < re.search(r"\b(load_tile|tma_load_3d)\w*[<(]", text).start(), kernel
