@@ -150,6 +150,22 @@ int ensure_ctx(int device, DeviceCtx** out) {
     return FA_B200_OK;
 }
 
+// The driver's encoder over a 3-D fp16 array.  It needs a current context, and a thread that has not called the runtime
+// yet has none, although the device is set up (the launches bind it, but come after the maps): bind the device's context
+// to the thread then.
+CUresult encode_3d(CUtensorMap* map, const void* base, const cuuint64_t (&dims)[3], const cuuint64_t (&strides)[2],
+                   const cuuint32_t (&box)[3], CUtensorMapSwizzle swz) {
+    const cuuint32_t estr[3] = {1, 1, 1};
+    auto encode = [&] {
+        return g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr,
+                        CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    };
+    CUresult r = encode();
+    int device = 0;
+    if (r == CUDA_ERROR_INVALID_CONTEXT && cudaGetDevice(&device) == cudaSuccess && cudaSetDevice(device) == cudaSuccess) r = encode();
+    return r;
+}
+
 // 3-D map {F, L, B} over a contiguous [B, L, F] fp16 array; box = 128 rows x min(H, 64) columns.
 int make_map(CUtensorMap* map, const void* base, uint32_t B, uint32_t L, uint32_t F, uint32_t H,
              uint32_t box_rows = static_cast<uint32_t>(fa::kTile), uint32_t max_cols = 64) {
@@ -158,14 +174,10 @@ int make_map(CUtensorMap* map, const void* base, uint32_t B, uint32_t L, uint32_
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(F) * 2ull,
                                    static_cast<cuuint64_t>(F) * 2ull * L};
     const cuuint32_t box[3] = {box_cols, box_rows, 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
     const CUtensorMapSwizzle swz = box_cols == 64   ? CU_TENSOR_MAP_SWIZZLE_128B
                                    : box_cols == 32 ? CU_TENSOR_MAP_SWIZZLE_64B
                                                     : CU_TENSOR_MAP_SWIZZLE_32B;
-    const CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims,
-                                strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? FA_B200_OK : FA_B200_ERR_DRIVER;
+    return encode_3d(map, base, dims, strides, box, swz) == CUDA_SUCCESS ? FA_B200_OK : FA_B200_ERR_DRIVER;
 }
 
 // 3-D map {L keys, Lq rows, B} over a [B, Lq, L] fp16 mask whose rows are `pitch` elements apart; box = 128 rows x 64
@@ -174,11 +186,7 @@ int make_mask_map(CUtensorMap* map, const void* base, uint32_t B, uint32_t Lq, u
     const cuuint64_t dims[3] = {L, Lq, B};
     const cuuint64_t strides[2] = {static_cast<cuuint64_t>(pitch) * 2ull, static_cast<cuuint64_t>(pitch) * 2ull * L};
     const cuuint32_t box[3] = {64, static_cast<cuuint32_t>(fa::kTile), 1};
-    const cuuint32_t estr[3] = {1, 1, 1};
-    const CUresult r = g_encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void*>(base), dims, strides, box,
-                                estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
-                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-    return r == CUDA_SUCCESS ? FA_B200_OK : FA_B200_ERR_DRIVER;
+    return encode_3d(map, base, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B) == CUDA_SUCCESS ? FA_B200_OK : FA_B200_ERR_DRIVER;
 }
 
 bool is_pow2(uint32_t x) { return x != 0 && (x & (x - 1)) == 0; }

@@ -608,6 +608,27 @@ def test_concurrent_callers_from_several_threads():
         assert torch.equal(results[idx], expected if idx < 2 else expected_whole)
 
 
+def test_first_call_of_a_thread():
+    """A thread that has called nothing of the CUDA runtime yet has no context; its first call has the same result."""
+    import threading
+    q, k, v = (t.cuda() for t in make_inputs(2, 300, 256, 1.0, 92))
+    expected = fa.attention_forward(64, 64, q, k, v)
+    results = []
+
+    def call():
+        try:
+            results.append(fa.attention_forward(64, 64, q, k, v))
+        except Exception as exc:  # noqa: BLE001
+            results.append(exc)
+
+    for _ in range(2):
+        t = threading.Thread(target=call)
+        t.start()
+        t.join()
+    torch.cuda.synchronize()
+    assert all(torch.is_tensor(y) and torch.equal(y, expected) for y in results), results
+
+
 def test_non_default_stream_and_output_placement():
     q, k, v = (t.cuda() for t in make_inputs(1, 512, 256, 1.0, 31))
     s = torch.cuda.Stream()
