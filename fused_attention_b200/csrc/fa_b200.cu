@@ -40,6 +40,10 @@ struct SplitScratch {
     float4* o = nullptr;       // fa::Params::part_o
     float2* ml = nullptr;      // fa::Params::part_ml
     uint32_t* cnt = nullptr;   // fa::Params::part_cnt
+    // Held from the first launch of a call that uses the buffer to its last one.  The launches of a planned call pass
+    // the plan on through the buffer, and stream order keeps them together only as long as no other thread that
+    // works on the same stream can put a launch that uses it in between.
+    std::mutex mu;
 };
 constexpr int kSplitPool = 4;
 
@@ -382,7 +386,7 @@ int launch_pipelined(DeviceCtx& c, int slot, int mask_kind, const CUtensorMap& m
 
 // The split-scratch buffer of `st` on this device: the one it already has, else a free one, else none.
 // None also while the stream is being captured.
-const SplitScratch* scratch_for_stream(DeviceCtx& c, cudaStream_t st) {
+SplitScratch* scratch_for_stream(DeviceCtx& c, cudaStream_t st) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -631,19 +635,23 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                     const bool mask_tma = mask && mask_rows_aligned(mask, L);
                     const bool want_plan = mask && Lq == L && use_mask_plan(H, p.n_items, p.n_kv_tiles, B, p.q_pairs, mask_tma, sms, flags);
                     const bool want_split = !(flags & (FA_B200_FLAG_NO_SPLIT | FA_B200_FLAG_FORCE_PAIR));
-                    const SplitScratch* scratch = want_plan || want_split ? scratch_for_stream(*c, st) : nullptr;
+                    SplitScratch* scratch = want_plan || want_split ? scratch_for_stream(*c, st) : nullptr;
+                    std::unique_lock<std::mutex> launches;   // see SplitScratch::mu; given back when the last one is made
                     const bool pair = use_pair_kernel(H, mask != nullptr, mask_tma, p.q_pairs, p.R * B, sms, 0, flags);
                     const void* mask_at = mask;
                     uint32_t mask_pitch = L;
                     bool planned = false;
-                    if (want_plan && scratch != nullptr)
+                    if (want_plan && scratch != nullptr) {
+                        launches = std::unique_lock<std::mutex>(scratch->mu);
                         rc = plan_mask(*c, *scratch, k, v, mask_tma, p, st, overlap, &mask_at, &mask_pitch, &planned);
+                    }
                     const Schedule sch = make_schedule(H, p.n_items, p.n_kv_tiles, sms, want_split && scratch != nullptr && !planned);
                     p.full_rounds = sch.full_rounds;
                     p.tail_items = sch.tail_items;
                     p.tail_steps = sch.tail_steps;
                     p.tail_grid = sch.tail_grid;
                     if (sch.tail_steps != 0) {
+                        if (!launches.owns_lock()) launches = std::unique_lock<std::mutex>(scratch->mu);
                         p.part_o = scratch->o;
                         p.part_ml = scratch->ml;
                         p.part_cnt = scratch->cnt;
