@@ -368,7 +368,7 @@ __device__ __forceinline__ void add_mask_row(float (&s)[kTile], const __half* mr
         for (int i0 = 0; i0 < kTile; i0 += 16) {
             if (i0 + 16 <= valid) {
                 uint32_t w[8];
-                ldg_256(mrow + i0, w);
+                ld_global_256(mrow + i0, w);
 #pragma unroll
                 for (int e = 0; e < 8; ++e) {
                     const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[e]));
@@ -385,7 +385,7 @@ __device__ __forceinline__ void add_mask_row(float (&s)[kTile], const __half* mr
 #pragma unroll
         for (int i0 = 0; i0 < kTile; i0 += 8) {
             if (i0 + 8 <= valid) {
-                const uint4 w = __ldg(reinterpret_cast<const uint4*>(mrow + i0));
+                const uint4 w = *reinterpret_cast<const uint4*>(mrow + i0);
                 const uint32_t ws[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
                 for (int e = 0; e < 4; ++e) {
@@ -886,14 +886,14 @@ __device__ __forceinline__ uint32_t planned_count(const Params& p) {
     const uint32_t full = p.n_items / gridDim.x, rest = p.n_items % gridDim.x;
     return full + (((full & 1u) ? gridDim.x - 1u - blockIdx.x : blockIdx.x) < rest ? 1u : 0u);
 }
-__device__ __forceinline__ Planned planned_item(const Params& p, uint32_t k) {
+__device__ __forceinline__ Planned planned_item(const Params& p, uint32_t zero, uint32_t k) {   // zero: zero_behind_the_wait()
     const uint32_t idx = k * gridDim.x + ((k & 1u) ? gridDim.x - 1u - blockIdx.x : blockIdx.x);
     if (idx >= p.n_items) return Planned{0u, 0u, 0u};
-    const uint32_t o = __ldg(p.plan_order + idx / p.R);
+    const uint32_t o = ld_settled(p.plan_order + idx / p.R + zero);
     return Planned{o & ((1u << kPlanLenShift) - 1u), idx % p.R, o >> kPlanLenShift};
 }
-__device__ __forceinline__ Seg planned_seg(const Params& p, uint32_t k) {
-    const Planned it = planned_item(p, k);
+__device__ __forceinline__ Seg planned_seg(const Params& p, uint32_t zero, uint32_t k) {
+    const Planned it = planned_item(p, zero, k);
     Seg s;
     s.item = (it.pair / p.q_pairs * p.R + it.head) * p.q_pairs + it.pair % p.q_pairs;
     s.j0 = 0;
@@ -1213,13 +1213,14 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t q_pairs = p.q_pairs;
     __shared__ Plan plan_smem;
     volatile Plan& pl_s = plan_smem;
+    uint32_t settled = 0;   // for what is read behind the wait for the previous kernel, see zero_behind_the_wait()
     auto seg_of = [&](uint32_t t_first, uint32_t k) {
-        if constexpr (kPlanned) return planned_seg(p, k);
+        if constexpr (kPlanned) return planned_seg(p, settled, k);
         else return get_seg(pl_s, t_first, p, k);
     };
     // key tile of step jj of a segment (with what the mask is there, if it is planned)
     auto step_of = [&](const Seg& sg, uint32_t jj) -> uint32_t {
-        if constexpr (kPlanned) return __ldg(p.plan_list + sg.list + jj);
+        if constexpr (kPlanned) return ld_settled(p.plan_list + sg.list + jj + settled);
         else return sg.j0 + jj;
     };
     auto step_tile = [](uint32_t e) -> uint32_t { return kPlanned ? e & ((1u << kStepShift0) - 1u) : e; };
@@ -1322,7 +1323,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // before it asks for anything, because with no segments no role would wait for a copy and the CTA would leave with it
     // still landing in its shared memory.
     if constexpr (kMask == kMaskTma) {
-        if (first_known && p.plan_head != nullptr && __ldg(p.plan_head) != 0u) {
+        if (first_known && p.plan_head != nullptr && *p.plan_head != 0u) {
             plan_smem = Plan{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
             first_known = false;
         }
@@ -1336,12 +1337,13 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if (p.plan_head != nullptr) __syncthreads();   // plan_smem may have been emptied
     }
     if constexpr (kPlanned) {
+        settled = zero_behind_the_wait();
         // the lists were written by the kernel before this one, so this CTA's plan is made behind the wait for it
         if (warp == 13) {
-            const bool runs = __ldg(p.plan_head) != 0u;   // else the kernel launched behind this one takes the call
+            const bool runs = *p.plan_head != 0u;   // else the kernel launched behind this one takes the call
             const uint32_t mine = planned_count(p);
             uint32_t sum = 0;
-            for (uint32_t k = lane; k < mine; k += 32u) sum += planned_item(p, k).len;
+            for (uint32_t k = lane; k < mine; k += 32u) sum += planned_item(p, settled, k).len;
             sum = __reduce_add_sync(0xffffffffu, sum);
             if (lane == 0) plan_smem = runs ? Plan{mine, 0u, mine, sum, 0u, 0u, 0u, 0u} : Plan{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
         }
@@ -1736,7 +1738,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             // ring item 2g is the K tile of global step g, item 2g+1 its V tile
             // (k, j, len): segment of the step a loop is working on, its position in it, its length
             auto seg_len_of = [&](uint32_t kk) {
-                if constexpr (kPlanned) return planned_item(p, kk).len;
+                if constexpr (kPlanned) return planned_item(p, settled, kk).len;
                 else return seg_len(pl, p, kk);
             };
             uint32_t k = 0, j = 0, len = seg_len_of(0);

@@ -57,9 +57,16 @@ __device__ __forceinline__ void plan_mask_tile(const PlanArgs& a, uint32_t tile)
     uint32_t w[16][2], extra = 0;
     auto two_keys = [&](uint32_t r, uint32_t col) -> uint32_t {
         const uint16_t* at = base + static_cast<size_t>(r) * a.L + col;
-        const uint32_t lo = r < rows && col < keys ? __ldg(at) : 0u;
-        const uint32_t hi = r < rows && col + 1u < keys ? __ldg(at + 1) : 0u;
+        const uint32_t lo = r < rows && col < keys ? ld_settled(at) : 0u;
+        const uint32_t hi = r < rows && col + 1u < keys ? ld_settled(at + 1) : 0u;
         return lo | (hi << 16);
+    };
+    // (four rows in flight together: one after the other, such a warp's way is what the whole plan waits for)
+    auto four_rows = [&](uint32_t r0, uint32_t (&v)[4][2]) {
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u)
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) v[u][h] = two_keys(r0 + u, h * 64u + lane * 2u);
     };
     if constexpr (!kCopy) {   // rows on 16-byte boundaries: two rows a load, eight keys a lane (L is a multiple of 8)
         const uint32_t col = (lane & 15u) * 8u;
@@ -67,7 +74,7 @@ __device__ __forceinline__ void plan_mask_tile(const PlanArgs& a, uint32_t tile)
 #pragma unroll
         for (uint32_t i = 0; i < 8; ++i) {
             const uint32_t r = 2u * i + (lane >> 4);
-            if (r < rows && col < keys) x[i] = __ldg(reinterpret_cast<const uint4*>(base + static_cast<size_t>(r) * a.L + col));
+            if (r < rows && col < keys) x[i] = ld_settled(reinterpret_cast<const uint4*>(base + static_cast<size_t>(r) * a.L + col));
         }
 #pragma unroll
         for (uint32_t i = 0; i < 8; ++i) {
@@ -83,8 +90,8 @@ __device__ __forceinline__ void plan_mask_tile(const PlanArgs& a, uint32_t tile)
         for (uint32_t r = 0; r < 16; ++r)
 #pragma unroll
             for (uint32_t h = 0; h < 2; ++h)
-                w[r][h] = __ldg(reinterpret_cast<const uint32_t*>((first + r * pitch) & ~3ull) + h * 32u + lane);
-        extra = __ldg(reinterpret_cast<const uint32_t*>((first + (lane & 15u) * pitch) & ~3ull) + 64u);   // of row `lane`
+                w[r][h] = ld_settled(reinterpret_cast<const uint32_t*>((first + r * pitch) & ~3ull) + h * 32u + lane);
+        extra = ld_settled(reinterpret_cast<const uint32_t*>((first + (lane & 15u) * pitch) & ~3ull) + 64);   // of row `lane`
 #pragma unroll
         for (uint32_t r = 0; r < 16; ++r) {
             const uint32_t sh = static_cast<uint32_t>((first + r * pitch) >> 1) & 1u;
@@ -101,14 +108,19 @@ __device__ __forceinline__ void plan_mask_tile(const PlanArgs& a, uint32_t tile)
         not_zero |= extra & 0x7FFF7FFFu & valid;
     } else {
 #pragma unroll 1
-        for (uint32_t r = 0; r < rows; ++r)
+        for (uint32_t r0 = 0; r0 < rows; r0 += 4u) {
+            uint32_t v[4][2];
+            four_rows(r0, v);
 #pragma unroll
-            for (uint32_t h = 0; h < 2; ++h) {
-                const uint32_t col = h * 64u + lane * 2u, v = two_keys(r, col);
-                const uint32_t valid = r < rows ? (col + 1u < keys ? 0xFFFFFFFFu : (col < keys ? 0xFFFFu : 0u)) : 0u;
-                not_neg |= (v ^ 0xFC00FC00u) & valid;
-                not_zero |= v & 0x7FFF7FFFu & valid;
-            }
+            for (uint32_t u = 0; u < 4; ++u)
+#pragma unroll
+                for (uint32_t h = 0; h < 2; ++h) {
+                    const uint32_t col = h * 64u + lane * 2u;
+                    const uint32_t valid = r0 + u < rows ? (col + 1u < keys ? 0xFFFFFFFFu : (col < keys ? 0xFFFFu : 0u)) : 0u;
+                    not_neg |= (v[u][h] ^ 0xFC00FC00u) & valid;
+                    not_zero |= v[u][h] & 0x7FFF7FFFu & valid;
+                }
+        }
     }
     const bool any_not_neg = __syncthreads_or(not_neg != 0u), any_not_zero = __syncthreads_or(not_zero != 0u);
     if (tid == 0) a.cls[tile] = !any_not_neg ? kTileNeg : (any_not_zero ? kTileMixed : kTileZero);
@@ -131,9 +143,13 @@ __device__ __forceinline__ void plan_mask_tile(const PlanArgs& a, uint32_t tile)
             }
         } else {
 #pragma unroll 1
-            for (uint32_t r = 0; r < rows; ++r) {
-                put(r, 0, two_keys(r, lane * 2u));
-                put(r, 1, two_keys(r, 64u + lane * 2u));
+            for (uint32_t r0 = 0; r0 < rows; r0 += 4u) {
+                uint32_t v[4][2];
+                four_rows(r0, v);
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u)
+#pragma unroll
+                    for (uint32_t h = 0; h < 2; ++h) put(r0 + u, h, v[u][h]);
             }
         }
     }
@@ -143,7 +159,7 @@ __device__ __forceinline__ void plan_mask_tile(const PlanArgs& a, uint32_t tile)
 __device__ __forceinline__ bool plan_maybe_left_out(const PlanArgs& a, uint32_t b, uint32_t kt) {
     bool neg = false;
     for (uint32_t qt = threadIdx.x; qt < a.n; qt += kPlanThreads)
-        neg |= __ldg(reinterpret_cast<const uint16_t*>(a.mask) + (static_cast<size_t>(b) * a.L + qt * kTile) * a.L + kt * kTile) == 0xFC00u;
+        neg |= ld_settled(reinterpret_cast<const uint16_t*>(a.mask) + (static_cast<size_t>(b) * a.L + qt * kTile) * a.L + kt * kTile) == 0xFC00u;
     return __syncthreads_or(neg);
 }
 
@@ -157,7 +173,7 @@ __device__ __forceinline__ void plan_finite(const PlanArgs& a, const __half* x, 
 #pragma unroll
     for (uint32_t u = 0; u < 8; ++u) {
         const uint32_t r = u * 16u + (tid >> 4);
-        w[u] = r < rows && c < a.F ? __ldg(reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * a.F)) : make_uint4(0, 0, 0, 0);
+        w[u] = r < rows && c < a.F ? ld_settled(reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * a.F)) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (uint32_t u = 0; u < 8; ++u)   // an exponent of all ones carries into the sign's place
@@ -169,12 +185,15 @@ __device__ __forceinline__ void plan_finite(const PlanArgs& a, const __half* x, 
 // kCopy: the mask's rows start on no 16-byte boundary and are copied.  grid: at most the launch bound's CTAs per SM.  The tiles of the mask round-robin, then a run of the parts of K and V; the
 // CTA that is through last writes the lists, one group of 8, 16 or 32 lanes per pair of query tiles.
 template <bool kCopy>
-__global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPlanCtasPerSm) fa_mask_plan(const PlanArgs a) {
+__global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPlanCtasPerSm) fa_mask_plan(const PlanArgs args) {
     __shared__ uint32_t hist[kPlanMaxTiles + 1], cost[2];
     __shared__ uint16_t lens[kPlanMaxGroups];
     __shared__ bool last;
     grid_dep_wait();
     grid_dep_launch();
+    PlanArgs a = args;   // (the inputs' addresses, for ld_settled)
+    const uint32_t settled = zero_behind_the_wait();
+    a.mask += settled, a.k += settled, a.v += settled;
     const uint32_t tid = threadIdx.x, n = a.n;
     if (a.dense_allowed) {
         // A tile that is -inf throughout begins with -inf.  Where fewer than a fifth of the tiles do, every CTA finds so
@@ -182,7 +201,7 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
         uint32_t neg = 0;
         for (uint32_t t = tid; t < a.B * n * n; t += kPlanThreads) {
             const uint32_t kt = t % n, qt = (t / n) % n, b = t / (n * n);
-            neg += __ldg(reinterpret_cast<const uint16_t*>(a.mask) + (static_cast<size_t>(b) * a.L + qt * kTile) * a.L + kt * kTile) == 0xFC00u;
+            neg += ld_settled(reinterpret_cast<const uint16_t*>(a.mask) + (static_cast<size_t>(b) * a.L + qt * kTile) * a.L + kt * kTile) == 0xFC00u;
         }
         if (tid == 0) cost[0] = 0;
         __syncthreads();

@@ -239,8 +239,36 @@ __device__ __forceinline__ bool dbg_tmem_ok(uint32_t taddr, uint32_t ncols) {
 // returns at once in a launch without the attribute).  grid_dep_launch() tells the scheduler that
 // the kernel after this one may be made resident as SMs fall free; it fires once every CTA of
 // this grid has executed it.
+// What a kernel reads behind the wait may have been written while it was resident already, so nothing here is loaded
+// as read-only data (ld.global.nc, __ldg): such a load is for memory that nobody writes during the kernel's life, and
+// need not stay behind the wait.
 __device__ __forceinline__ void grid_dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dep_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Loads of what was complete when grid_dep_wait() returned and is not written again while the kernel runs.  The compiler
+// may move them past stores, barriers and waits and combine them, as it may a read-only load, but for the hardware they
+// are ordinary, coherent loads.  What holds them behind grid_dep_wait() is their address, which zero_behind_the_wait()
+// is added to: 0, but not known before that point of the program.
+__device__ __forceinline__ uint32_t zero_behind_the_wait() {
+    uint32_t zero;
+    asm volatile("mov.u32 %0, 0;" : "=r"(zero)::"memory");
+    return zero;
+}
+__device__ __forceinline__ uint32_t ld_settled(const uint16_t* ptr) {
+    uint16_t v;
+    asm("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(ptr));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_settled(const uint32_t* ptr) {
+    uint32_t v;
+    asm("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(ptr));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_settled(const uint4* ptr) {
+    uint4 v;
+    asm("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(ptr));
+    return v;
+}
 
 // ----------------------------------------------------------------------------- TMA
 __device__ __forceinline__ void prefetch_tensormap(const void* map) {
@@ -614,9 +642,9 @@ __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* ptr) {
     return v;
 }
 
-// 32 bytes of read-only global memory with one instruction (the address must be 32-byte aligned)
-__device__ __forceinline__ void ldg_256(const void* ptr, uint32_t (&w)[8]) {
-    asm volatile("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+// 32 bytes of global memory with one instruction (the address must be 32-byte aligned)
+__device__ __forceinline__ void ld_global_256(const void* ptr, uint32_t (&w)[8]) {
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                  : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
                  : "l"(ptr));
 }

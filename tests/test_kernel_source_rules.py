@@ -24,3 +24,10 @@ def test_a_launch_without_work_asks_for_no_copies():
     for name, kernel in (("fa_kernels.cuh", "fa_fwd_pipelined"), ("fa_pair.cuh", "fa_fwd_pair")):
         text = body_behind_the_wait(name, kernel)
         assert text.index("p.plan_head") < re.search(r"\b(load_tile|tma_load_3d)\w*[<(]", text).start(), kernel
+
+
+def test_no_load_of_read_only_data():
+    """Every kernel may be resident while the kernel before it still writes: what it loads is not read-only for its life,
+    which ld.global.nc asks for, and such a load need not stay behind the wait for that kernel."""
+    names = [n for n in os.listdir(CSRC) if n.endswith((".cu", ".cuh"))]
+    assert names and not [n for n in names if re.search(r"__ldg\b|ld\.global\.nc", source(n))]
