@@ -40,6 +40,10 @@ struct SplitScratch {
     float4* o = nullptr;       // fa::Params::part_o
     float2* ml = nullptr;      // fa::Params::part_ml
     uint32_t* cnt = nullptr;   // fa::Params::part_cnt
+    // fa::PlanArgs::ticket: a word of its own.  Every CTA of the planning kernel comes to its end, so it is zero between
+    // launches whatever became of the others; the part counters may be left half counted by a launch that gave up, and
+    // are zeroed with its report while other streams work.
+    uint32_t* ticket = nullptr;
     // Held from the first launch of a call that uses the buffer to its last one.  The launches of a planned call pass
     // the plan on through the buffer, and stream order keeps them together only as long as no other thread that
     // works on the same stream can put a launch that uses it in between.
@@ -130,12 +134,13 @@ int ensure_ctx(int device, DeviceCtx** out) {
         for (int i = 0; i < kSplitPool; ++i) {
             char* base = nullptr;
             const size_t ob = split_o_bytes(c.sm_count), mb = split_ml_bytes(c.sm_count), cb = split_cnt_bytes(c.sm_count);
-            e = cudaMalloc(reinterpret_cast<void**>(&base), ob + mb + cb);
+            e = cudaMalloc(reinterpret_cast<void**>(&base), ob + mb + cb + sizeof(uint32_t));
             if (e != cudaSuccess) return static_cast<int>(e);
             c.split[i].o = reinterpret_cast<float4*>(base);
             c.split[i].ml = reinterpret_cast<float2*>(base + ob);
             c.split[i].cnt = reinterpret_cast<uint32_t*>(base + ob + mb);
-            e = cudaMemset(c.split[i].cnt, 0, cb);
+            c.split[i].ticket = reinterpret_cast<uint32_t*>(base + ob + mb + cb);
+            e = cudaMemset(c.split[i].cnt, 0, cb + sizeof(uint32_t));
             if (e != cudaSuccess) return static_cast<int>(e);
         }
         c.ready = true;
@@ -509,7 +514,7 @@ int plan_mask(DeviceCtx& c, const SplitScratch& scratch, const void* k, const vo
     a.v = static_cast<const __half*>(v);
     a.copy = mask_tma ? nullptr : reinterpret_cast<__half*>(base);
     a.head = reinterpret_cast<uint32_t*>(base + copy_bytes);
-    a.ticket = scratch.cnt;
+    a.ticket = scratch.ticket;
     a.order = reinterpret_cast<uint32_t*>(base + order_at);
     a.bad = reinterpret_cast<uint32_t*>(base + bad_at);
     a.list = reinterpret_cast<uint16_t*>(base + list_at);

@@ -31,3 +31,12 @@ def test_no_load_of_read_only_data():
     which ld.global.nc asks for, and such a load need not stay behind the wait for that kernel."""
     names = [n for n in os.listdir(CSRC) if n.endswith((".cu", ".cuh"))]
     assert names and not [n for n in names if re.search(r"__ldg\b|ld\.global\.nc", source(n))]
+
+
+def test_the_plan_counts_its_ctas_in_a_word_of_its_own():
+    """The part counters of divided calls can be left half counted by a launch that gave up, and are zeroed with its
+    report at any time; a plan that counted there would never find its last CTA and leave old lists in place."""
+    text = source("fa_b200.cu")
+    assert re.search(r"a\.ticket = scratch\.ticket;", text)
+    report = text[text.index("int fold_ctx_status"):text.index("uint32_t next_launch_id")]
+    assert "ticket" not in report and ".cnt" in report
