@@ -620,7 +620,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                 p.part_slots = static_cast<uint32_t>(2 * c->sm_count);
 #ifdef FA_DEBUG
                 // checked build: rows the kernel fails to write stay NaN
-                if ((e = cudaMemsetAsync(y, 0xFF, static_cast<size_t>(B) * L * F * sizeof(__half), st)) != cudaSuccess)
+                if ((e = cudaMemsetAsync(y, 0xFF, static_cast<size_t>(B) * Lq * F * sizeof(__half), st)) != cudaSuccess)
                     rc = static_cast<int>(e);
 #endif
                 p.part_o = nullptr;

@@ -705,6 +705,8 @@ def _checked_lib():
     u32, vp, i32 = ctypes.c_uint32, ctypes.c_void_p, ctypes.c_int
     lib.fa_b200_attention_forward.restype = i32
     lib.fa_b200_attention_forward.argtypes = [vp, vp, vp, vp, vp, u32, u32, u32, u32, u32, i32, vp, u32]
+    lib.fa_b200_attention_forward_host.restype = i32
+    lib.fa_b200_attention_forward_host.argtypes = [vp, vp, vp, vp, vp, u32, u32, u32, u32, u32, i32, u32]
     lib.fa_b200_read_status.restype = i32
     lib.fa_b200_read_status.argtypes = [i32, ctypes.POINTER(u32)]
     lib.fa_b200_selftest_debug_checks.restype = i32
@@ -745,6 +747,24 @@ def test_checked_build_runs_clean_and_gives_the_same_bits(H, B, R, L, flags, mas
     assert lib.fa_b200_read_status(0, w) == 0 and (w[0], w[1]) == (0, 0), hex(w[0])
     assert torch.isfinite(y).all()
     assert torch.equal(y, fa.attention_forward(H, 16 if H < 128 else 32, q, k, v, mask, flags=flags | _lib.FLAG_SYNC))
+
+
+@pytest.mark.parametrize("B,R,L,H,masked", [(1, 24, 1025, 128, False), (2, 32, 600, 64, True), (3, 40, 1300, 32, True), (1, 40, 513, 64, False),
+                                            (9, 4, 100, 64, True)])
+def test_checked_build_host_calls(B, R, L, H, masked):
+    """Host buffers under the checked build: calls cut into blocks of query rows, each with rows of Y of its own."""
+    lib = _checked_lib()
+    q, k, v = make_inputs(B, L, R * H, 1.0, L + H)
+    mask = None
+    if masked:
+        mask = torch.triu(torch.full((L, L), float("-inf")), diagonal=1).half().unsqueeze(0).repeat(B, 1, 1)
+    y = torch.empty_like(q)
+    rc = lib.fa_b200_attention_forward_host(q.data_ptr(), k.data_ptr(), v.data_ptr(), None if mask is None else mask.data_ptr(),
+                                            y.data_ptr(), B, L, R * H, H, 0, 0, 0)
+    assert rc == 0, rc
+    w = (ctypes.c_uint32 * 2)()
+    assert lib.fa_b200_read_status(0, w) == 0 and (w[0], w[1]) == (0, 0), hex(w[0])
+    assert torch.equal(y, fa.attention_forward_host(H, 16 if H < 128 else 32, q, k, v, mask))
 
 
 @pytest.mark.parametrize("flags", [ONE, PAIR])
