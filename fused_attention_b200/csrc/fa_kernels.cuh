@@ -1574,7 +1574,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             if (lane == 0 && row0 < static_cast<int32_t>(p.Lq)) {
 #pragma unroll
                 for (int half = 0; half < H / C::kStoreCols; ++half)
-                    tma_store_3d(&tmY, stage + half * (64u * C::kStoreCols), static_cast<int32_t>((bh % p.R) * H + half * C::kStoreCols),
+                    tma_store_3d<64u * C::kStoreCols>(&tmY, stage + half * (64u * C::kStoreCols), static_cast<int32_t>((bh % p.R) * H + half * C::kStoreCols),
                                  row0, static_cast<int32_t>(bh / p.R));
                 bulk_commit_group();
             }
@@ -1667,7 +1667,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         fence_proxy_async_smem();
                         __syncwarp();
                         if (lane == 0 && row0 < static_cast<int32_t>(p.Lq)) {   // rows past Lq are clipped by the store
-                            tma_store_3d(&tmY, stage, static_cast<int32_t>(head * H + half * W), row0,
+                            tma_store_3d<64u * C::kStoreCols>(&tmY, stage, static_cast<int32_t>(head * H + half * W), row0,
                                          static_cast<int32_t>(batch));
                             bulk_commit_group();
                         }

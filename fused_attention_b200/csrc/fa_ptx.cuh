@@ -296,8 +296,10 @@ __device__ __forceinline__ void tma_prefetch_l2_3d(const void* map, int32_t x, i
 
 // 3-D tiled store shared -> global as one bulk group; the box is clipped at the tensor's bounds.
 // Coordinates must not be negative; x * sizeof(element) must be a multiple of 16 bytes.
+// kBytes: of the box, for the checked build.
+template <uint32_t kBytes = 4096u>
 __device__ __forceinline__ void tma_store_3d(const void* map, uint32_t src, int32_t x, int32_t y, int32_t z) {
-    FA_DBG_COPY(src, 4096u, x, y, z, true);
+    FA_DBG_COPY(src, kBytes, x, y, z, true);
     asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
                      reinterpret_cast<uint64_t>(map)),
                  "r"(src), "r"(x), "r"(y), "r"(z)

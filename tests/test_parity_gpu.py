@@ -726,9 +726,14 @@ def test_checked_build_refuses_bad_operands_without_touching_memory():
 @pytest.mark.parametrize("H,B,R,L,flags,masked", [
     (16, 2, 3, 200, SIMPLE, False), (64, 2, 3, 300, SIMPLE, True), (64, 3, 5, 700, ONE, False), (64, 2, 2, 520, ONE, True),
     (128, 2, 3, 1000, ONE, False), (128, 2, 4, 2048, PAIR, False), (128, 1, 4, 2048 + 77, 0, False), (128, 1, 2, 650, ONE, True),
-    (128, 20, 10, 300, PAIR, False), (128, 2, 3, 1000, PAIR, True), (128, 3, 4, 2048, PAIR, True)])
+    (128, 20, 10, 300, PAIR, False), (128, 2, 3, 1000, PAIR, True), (128, 3, 4, 2048, PAIR, True),
+    # planned, several items per CTA: rows that TMA can fetch (two launches behind the plan), and rows that are copied
+    (128, 2, 20, 2048, 0, True), (128, 3, 20, 1101, 0, True), (64, 2, 30, 2048, 0, True), (64, 3, 20, 1021, 0, True),
+    (32, 2, 30, 2048, 0, True), (16, 3, 50, 515, 0, True),
+    # mask rows that warps of the CTA copy (two key tiles are not planned), and head_dim 16 and 32
+    (128, 2, 4, 201, 0, True), (64, 2, 4, 201, 0, True), (16, 2, 4, 201, 0, True), (16, 2, 4, 1000, 0, False), (32, 1, 4, 2048, 0, False)])
 def test_checked_build_runs_clean_and_gives_the_same_bits(H, B, R, L, flags, masked):
-    """Every kernel under the checked build: each TMA copy and tensor-memory access is checked against the
+    """The kernels that copy with TMA and multiply in tensor memory, under the checked build: each TMA copy and tensor-memory access is checked against the
     CTA's tile area, the tensor's extent and the CTA's tensor-memory allocation, tile buffers and Y are
     filled with NaN beforehand.  No check may fire, no NaN may survive, and the bits are the normal build's."""
     lib = _checked_lib()
