@@ -97,6 +97,7 @@ __device__ __forceinline__ void dbg_begin(const Params& p, const WaitCtl& ctl, u
         g_dbg.smem_hi = smem_base + bytes;
         g_dbg.F = p.F;
         g_dbg.L = p.L;
+        g_dbg.Lq = p.Lq;
         g_dbg.B = p.B;
         g_dbg.tmem_base = 0;
         g_dbg.tmem_cols = 512;
@@ -2092,7 +2093,8 @@ __global__ void fa_selftest_debug_checks(uint32_t* status) {
         g_dbg.smem_lo = 0x4000;
         g_dbg.smem_hi = 0x4000 + 64 * 1024;
         g_dbg.F = 512;
-        g_dbg.L = 300;
+        g_dbg.L = 700;
+        g_dbg.Lq = 300;
         g_dbg.B = 2;
         g_dbg.tmem_base = 0;
         g_dbg.tmem_cols = 256;

@@ -198,7 +198,7 @@ enum : uint32_t {
 };
 struct DbgCtx {
     uint32_t smem_lo, smem_hi;   // the CTA's tile area in shared memory (shared-window addresses)
-    uint32_t F, L, B;            // extent of the tensors in elements / rows / batch entries
+    uint32_t F, L, Lq, B;        // extent of the tensors in elements / rows (of Y: Lq) / batch entries
     uint32_t tmem_base, tmem_cols;
     WaitCtl ctl;
 };
@@ -215,7 +215,7 @@ __device__ __forceinline__ bool dbg_copy_ok(uint32_t saddr, uint32_t bytes, int3
     ok &= dbg_ok((x & 7) == 0, kDbgTmaX);
     const uint32_t x_extent = (g_dbg.F > g_dbg.L ? g_dbg.F : g_dbg.L) + (store ? 0u : 128u);   // a load may start in the zero fill
     ok &= dbg_ok(x >= 0 && static_cast<uint32_t>(x) < x_extent && z >= 0 && static_cast<uint32_t>(z) < g_dbg.B, kDbgTmaCoord);
-    if (store) ok &= dbg_ok(y >= 0 && static_cast<uint32_t>(y) < g_dbg.L, kDbgStoreRow);
+    if (store) ok &= dbg_ok(y >= 0 && static_cast<uint32_t>(y) < g_dbg.Lq, kDbgStoreRow);
     else ok &= dbg_ok(y >= 0, kDbgTmaCoord);   // a load may run past the last row (zero fill), never start before the first
     return ok;
 }
