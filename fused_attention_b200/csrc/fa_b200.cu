@@ -573,9 +573,9 @@ int launch_small(DeviceCtx& c, const fa::SmallArgs& a, cudaStream_t st, bool ove
 }
 
 // Device-pointer launch on `st`.  Caller holds no lock.  With Lq < L (B = 1) the call is for the Lq query rows that q, y
-// and the mask begin with.
+// and the mask begin with.  `may_plan`: a masked call may be planned, for which it takes scratch for its stream.
 int forward_device(const void* q, const void* k, const void* v, const void* mask, void* y, uint32_t B, uint32_t Lq,
-                   uint32_t L, uint32_t F, uint32_t H, int device, cudaStream_t st, uint32_t flags) {
+                   uint32_t L, uint32_t F, uint32_t H, int device, cudaStream_t st, uint32_t flags, bool may_plan) {
     int prev = -1;
     cudaError_t e = cudaGetDevice(&prev);
     if (e != cudaSuccess) return static_cast<int>(e);
@@ -638,7 +638,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                     // (Planning a mask needs the same scratch, and a planned call is not divided.)
                     const uint32_t sms = static_cast<uint32_t>(c->sm_count);
                     const bool mask_tma = mask && mask_rows_aligned(mask, L);
-                    const bool want_plan = mask && Lq == L && use_mask_plan(H, p.n_items, p.n_kv_tiles, B, p.q_pairs, mask_tma, sms, flags);
+                    const bool want_plan = mask && may_plan && use_mask_plan(H, p.n_items, p.n_kv_tiles, B, p.q_pairs, mask_tma, sms, flags);
                     const bool want_split = !(flags & (FA_B200_FLAG_NO_SPLIT | FA_B200_FLAG_FORCE_PAIR));
                     SplitScratch* scratch = want_plan || want_split ? scratch_for_stream(*c, st) : nullptr;
                     std::unique_lock<std::mutex> launches;   // see SplitScratch::mu; given back when the last one is made
@@ -917,7 +917,7 @@ int fa_b200_attention_forward(const void* q, const void* k, const void* v, const
     const int rc = validate(q, k, v, mask_or_null, y, B, L, F, head_dim, chunk_hint, flags);
     if (rc != FA_B200_OK) return rc;
     return forward_device(q, k, v, mask_or_null, y, B, L, L, F, head_dim, device,
-                          static_cast<cudaStream_t>(cuda_stream), flags);
+                          static_cast<cudaStream_t>(cuda_stream), flags, true);
 }
 
 int fa_b200_attention_forward_host(const void* q, const void* k, const void* v, const void* mask_or_null,
@@ -981,6 +981,7 @@ int fa_b200_attention_forward_host(const void* q, const void* k, const void* v, 
         // FA_B200_FLAG_NO_SPLIT
         // (plain launches: a chunk's kernel is ordered behind copies on other streams, not behind a kernel)
         // (the kernel for short sequences is chosen by length and head_dim alone, so a chunk gets it as the whole does)
+        // (not planned: the copies bound the call, and the scratch a plan lies in belongs to the callers' streams)
         const int whole = select_kernel(B, L, F, H, mask_or_null != nullptr, flags, c->sm_count);
         const uint32_t chunk_flags =
             (flags & ~static_cast<uint32_t>(FA_B200_FLAG_SYNC | FA_B200_FLAG_FORCE_SIMPLE | FA_B200_FLAG_FORCE_PIPELINED)) |
@@ -1020,7 +1021,7 @@ int fa_b200_attention_forward_host(const void* q, const void* k, const void* v, 
                 if (rc == FA_B200_OK && (e = cudaStreamWaitEvent(s_cmp, c->ev_in[ch], 0)) != cudaSuccess) rc = static_cast<int>(e);
                 if (rc == FA_B200_OK)
                     rc = forward_device(dq + at, dk + kv_at, dv + kv_at, hm ? dm + m_at : nullptr, dy + at, nb, rows, L, F, H,
-                                        device, s_cmp, chunk_flags);
+                                        device, s_cmp, chunk_flags, false);
                 if (rc == FA_B200_OK && (e = cudaEventRecord(c->ev_cmp[ch], s_cmp)) != cudaSuccess) rc = static_cast<int>(e);
                 if (rc == FA_B200_OK && (e = cudaStreamWaitEvent(s_out, c->ev_cmp[ch], 0)) != cudaSuccess) rc = static_cast<int>(e);
                 if (rc == FA_B200_OK) {
