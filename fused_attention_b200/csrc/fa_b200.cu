@@ -37,6 +37,7 @@ size_t split_cnt_bytes(int sms) { return static_cast<size_t>(sms) * 2 * 4 * size
 struct SplitScratch {
     bool taken = false;
     cudaStream_t stream = nullptr;
+    unsigned long long stream_id = 0;   // of cudaStreamPerThread, a handle that is another stream in every thread
     float4* o = nullptr;       // fa::Params::part_o
     float2* ml = nullptr;      // fa::Params::part_ml
     uint32_t* cnt = nullptr;   // fa::Params::part_cnt
@@ -398,13 +399,19 @@ SplitScratch* scratch_for_stream(DeviceCtx& c, cudaStream_t st) {
         return nullptr;
     }
     if (cap != cudaStreamCaptureStatusNone) return nullptr;
+    unsigned long long id = 0;
+    if (st == cudaStreamPerThread && cudaStreamGetId(st, &id) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
     std::lock_guard<std::mutex> lk(c.split_mu);
     for (int i = 0; i < kSplitPool; ++i)
-        if (c.split[i].taken && c.split[i].stream == st) return &c.split[i];
+        if (c.split[i].taken && c.split[i].stream == st && c.split[i].stream_id == id) return &c.split[i];
     for (int i = 0; i < kSplitPool; ++i)
         if (!c.split[i].taken) {
             c.split[i].taken = true;
             c.split[i].stream = st;
+            c.split[i].stream_id = id;
             return &c.split[i];
         }
     return nullptr;

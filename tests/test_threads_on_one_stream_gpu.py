@@ -1,5 +1,8 @@
 """Several threads that call on one stream: a planned call is two or three launches, which hand the plan on through
 scratch memory that belongs to the stream, and a divided call puts its parts there."""
+import os
+import subprocess
+import sys
 import threading
 
 import pytest
@@ -57,3 +60,37 @@ def test_results_do_not_depend_on_the_other_threads_of_the_stream(kinds):
         t.join()
     assert wrong == []
     assert fa.read_status(0) == (0, 0)
+
+
+PER_THREAD = """
+import threading, torch, fused_attention_b200 as fa
+from fused_attention_b200 import _lib
+from fused_attention_b200.workloads import make_inputs
+B, R, L, H = 1, 4, 3000, 128
+lib = _lib.load()
+def call(x, y, stream):
+    _lib.check(lib.fa_b200_attention_forward(x[0].data_ptr(), x[1].data_ptr(), x[2].data_ptr(), None, y.data_ptr(),
+                                             B, L, R * H, H, 0, 0, stream, 0))
+xs = [[t.cuda() for t in make_inputs(B, L, R * H, 1.0, seed)] for seed in range(3)]
+ys = [[torch.empty_like(xs[0][0]) for _ in range(30)] for _ in xs]
+alone = [torch.empty_like(xs[0][0]) for _ in xs]
+for x, y in zip(xs, alone):
+    call(x, y, 0)
+torch.cuda.synchronize()
+def work(i):
+    for y in ys[i]:
+        call(xs[i], y, 2)            # cudaStreamPerThread
+threads = [threading.Thread(target=work, args=(i,)) for i in range(3)]
+for t in threads: t.start()
+for t in threads: t.join()
+torch.cuda.synchronize()
+assert all(torch.equal(alone[i], y) for i in range(3) for y in ys[i])
+assert fa.read_status(0) == (0, 0)
+"""
+
+
+def test_the_per_thread_stream_is_another_stream_in_every_thread():
+    """One handle, a stream per thread: divided calls of three threads do not share scratch (a process of its own, where
+    the four buffers are free)."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    subprocess.run([sys.executable, "-c", PER_THREAD], check=True, cwd=root, timeout=300)
