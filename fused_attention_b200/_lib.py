@@ -20,6 +20,8 @@ EXPORTED_SYMBOLS = (
     "fa_b200_strerror",
     "fa_b200_query",
     "fa_b200_read_status",
+    "fa_b200_describe_call",
+    "fa_b200_stream_has_scratch",
     "fa_b200_select_kernel",
     "fa_b200_describe_schedule",
     "fa_b200_selftest_bounded_wait",
@@ -85,6 +87,10 @@ def load() -> ctypes.CDLL:
         lib.fa_b200_read_status.argtypes = [i32, ctypes.POINTER(ctypes.c_uint32)]
         lib.fa_b200_selftest_bounded_wait.restype = i32
         lib.fa_b200_selftest_bounded_wait.argtypes = [i32, ctypes.POINTER(ctypes.c_uint32)]
+        lib.fa_b200_describe_call.restype = i32
+        lib.fa_b200_describe_call.argtypes = [u32, u32, u32, u32, u32, u32, u32, ctypes.POINTER(ctypes.c_uint32)]
+        lib.fa_b200_stream_has_scratch.restype = i32
+        lib.fa_b200_stream_has_scratch.argtypes = [i32, vp, ctypes.POINTER(ctypes.c_uint32)]
         lib.fa_b200_select_kernel.restype = i32
         lib.fa_b200_select_kernel.argtypes = [u32, u32, u32, u32, i32, u32]
         lib.fa_b200_describe_schedule.restype = i32

@@ -177,6 +177,22 @@ def query(device: int = 0) -> dict:
     return {"cc_major": o[0], "cc_minor": o[1], "sm_count": o[2], "smem_optin": o[3]}
 
 
+def describe_call(B: int, L: int, F: int, head_dim: int, mask_alignment: int = 0, flags: int = 0, sm_count: int = 148) -> dict:
+    """What a call launches (``fa_b200_describe_call``): ``kernel``, whether it is ``planned`` on a stream that has scratch,
+    and the number of ``launches`` then.  ``mask_alignment``: 0 without a mask, else what its address is a multiple of."""
+    o = (ctypes.c_uint32 * 3)()
+    _lib.check(_lib.load().fa_b200_describe_call(B, L, F, head_dim, int(mask_alignment), int(flags), int(sm_count), o))
+    return {"kernel": ("short sequences", "simple", "pipelined", "pipelined on pairs of CTAs")[o[0]], "planned": bool(o[1]),
+            "launches": int(o[2])}
+
+
+def stream_has_scratch(stream: int = 0, device: int = 0) -> bool:
+    """Whether a call on a stream (its handle) would find scratch for a divided or planned call."""
+    o = (ctypes.c_uint32 * 1)()
+    _lib.check(_lib.load().fa_b200_stream_has_scratch(int(device), int(stream), o))
+    return bool(o[0])
+
+
 def select_kernel(B: int, L: int, F: int, head_dim: int, has_mask: bool = False, flags: int = 0) -> str:
     rc = _lib.load().fa_b200_select_kernel(B, L, F, head_dim, int(has_mask), flags)
     if rc < 0:

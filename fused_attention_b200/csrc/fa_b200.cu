@@ -390,9 +390,9 @@ int launch_pipelined(DeviceCtx& c, int slot, int mask_kind, const CUtensorMap& m
     }
 }
 
-// The split-scratch buffer of `st` on this device: the one it already has, else a free one, else none.
-// None also while the stream is being captured.
-SplitScratch* scratch_for_stream(DeviceCtx& c, cudaStream_t st) {
+// The split-scratch buffer of `st` on this device: the one it already has, else a free one (which is its own from now on
+// with `take`), else none.  None also while the stream is being captured.
+SplitScratch* scratch_for_stream(DeviceCtx& c, cudaStream_t st, bool take = true) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
         (void)cudaGetLastError();
@@ -409,9 +409,11 @@ SplitScratch* scratch_for_stream(DeviceCtx& c, cudaStream_t st) {
         if (c.split[i].taken && c.split[i].stream == st && c.split[i].stream_id == id) return &c.split[i];
     for (int i = 0; i < kSplitPool; ++i)
         if (!c.split[i].taken) {
-            c.split[i].taken = true;
-            c.split[i].stream = st;
-            c.split[i].stream_id = id;
+            if (take) {
+                c.split[i].taken = true;
+                c.split[i].stream = st;
+                c.split[i].stream_id = id;
+            }
             return &c.split[i];
         }
     return nullptr;
@@ -484,6 +486,37 @@ int launch_pair(DeviceCtx& c, const CUtensorMap& mq, const CUtensorMap& mkh, con
     return static_cast<int>(e != cudaSuccess ? e : cudaGetLastError());
 }
 
+// Where a plan lies in the scratch, and how much there is to look through.
+struct PlanLayout {
+    uint32_t groups, pitch;   // pairs of query tiles of all batch entries; elements between rows of the mask's copy
+    size_t copy_bytes, order_at, bad_at, list_at, cls_at, bytes;
+    uint64_t jobs, tiles;     // parts of K and V; tiles of the mask
+};
+PlanLayout plan_layout(uint32_t B, uint32_t L, uint32_t F, bool mask_tma) {
+    auto up = [](size_t x) { return (x + 255u) & ~static_cast<size_t>(255u); };
+    const uint32_t n = (L + fa::kTile - 1) / fa::kTile;
+    PlanLayout l;
+    l.groups = B * ((L + 2 * fa::kTile - 1) / (2 * fa::kTile));
+    l.pitch = (L + 7u) & ~7u;
+    l.copy_bytes = mask_tma ? 0 : up(static_cast<size_t>(B) * L * l.pitch * 2u);
+    l.order_at = l.copy_bytes + 256;
+    l.bad_at = l.order_at + up(l.groups * 4ull);
+    l.list_at = l.bad_at + up(static_cast<size_t>(B) * n * 4u);
+    l.cls_at = l.list_at + up(static_cast<size_t>(l.groups) * n * 2u);
+    l.bytes = l.cls_at + up(static_cast<size_t>(B) * n * n);
+    l.jobs = static_cast<uint64_t>(B) * n * 2u * ((F + fa::kPlanCols - 1u) / fa::kPlanCols);
+    l.tiles = static_cast<uint64_t>(B) * n * n;
+    return l;
+}
+
+// Whether the lists and the scratch are large enough for a plan of this call.
+bool plan_fits(uint32_t B, uint32_t L, uint32_t F, bool mask_tma, uint32_t sms) {
+    const uint64_t q_pairs = (L + 2 * fa::kTile - 1) / (2 * fa::kTile);
+    if ((L + fa::kTile - 1) / fa::kTile > fa::kPlanMaxTiles || B * q_pairs > fa::kPlanMaxGroups) return false;
+    const PlanLayout l = plan_layout(B, L, F, mask_tma);
+    return l.bytes <= split_o_bytes(static_cast<int>(sms)) && l.jobs <= 0x7FFFFFFFull;
+}
+
 // Whether a masked call of the pipelined kernel is planned (fa_mask_plan.cuh).  The plan is a launch and a pass over the
 // mask, K and V ahead of the attention kernel, 6 us at least, and 13 in all where it finds that too little can be left
 // out; what it saves is up to half of the key steps where there is more than one round of them.  Measured, us without
@@ -495,47 +528,42 @@ int launch_pair(DeviceCtx& c, const CUtensorMap& mq, const CUtensorMap& mkh, con
 // spares every head the copies inside the kernel, and it pays much sooner:
 //   H = 64: B=32 R=16 L=201 36 / 46, B=1 R=8 L=301 15 / 18, B=32 R=12 L=301 82 / 63, B=2 R=8 L=511 26 / 21,
 //           B=4 R=12 L=1021 72 / 38;   H = 128: B=1 R=8 L=301 25 / 19, B=2 R=32 L=1021 125 / 51
-bool use_mask_plan(uint32_t H, uint32_t n_items, uint32_t n, uint32_t B, uint32_t q_pairs, bool mask_tma, uint32_t sms, uint32_t flags) {
-    if ((flags & FA_B200_FLAG_FORCE_PAIR) || n > fa::kPlanMaxTiles || static_cast<uint64_t>(B) * q_pairs > fa::kPlanMaxGroups) return false;
-    const uint64_t steps = static_cast<uint64_t>(n_items) * n;
+bool use_mask_plan(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool mask_tma, uint32_t sms, uint32_t flags) {
+    if ((flags & FA_B200_FLAG_FORCE_PAIR) || !plan_fits(B, L, F, mask_tma, sms)) return false;
+    const uint32_t n = (L + fa::kTile - 1) / fa::kTile;
+    const uint64_t steps = static_cast<uint64_t>((L + 2 * fa::kTile - 1) / (2 * fa::kTile)) * (F / H) * B * n;
     if (mask_tma) return n >= 16u && steps >= 48ull * sms;
     return n >= 4u || (n == 3u && (H == 128 || steps >= 4ull * sms));
 }
 
 // Launches the kernel that plans a masked call, into the scratch of the call's stream (a planned call is not divided,
 // so the scratch is free): on return p's plan_ fields are set, and the mask's rows are at *mask_rows, *mask_pitch
-// elements apart.  *planned stays false when the copy of the mask does not fit.
+// elements apart.
 int plan_mask(DeviceCtx& c, const SplitScratch& scratch, const void* k, const void* v, bool mask_tma,
-              Params& p, cudaStream_t st, bool overlap, const void** mask_rows, uint32_t* mask_pitch, bool* planned) {
-    const uint32_t n = p.n_kv_tiles, groups = p.B * p.q_pairs, pitch = (p.L + 7u) & ~7u;
-    auto up = [](size_t x) { return (x + 255u) & ~static_cast<size_t>(255u); };
-    const size_t copy_bytes = mask_tma ? 0 : up(static_cast<size_t>(p.B) * p.L * pitch * 2u);
-    const size_t order_at = copy_bytes + 256, bad_at = order_at + up(groups * 4ull), list_at = bad_at + up(static_cast<size_t>(p.B) * n * 4u);
-    const size_t cls_at = list_at + up(static_cast<size_t>(groups) * n * 2u), bytes = cls_at + up(static_cast<size_t>(p.B) * n * n);
-    const uint64_t jobs = static_cast<uint64_t>(p.B) * n * 2u * ((p.F + fa::kPlanCols - 1u) / fa::kPlanCols), tiles = static_cast<uint64_t>(p.B) * n * n;
-    if (bytes > split_o_bytes(c.sm_count) || jobs > 0x7FFFFFFFull) return FA_B200_OK;
+              Params& p, cudaStream_t st, bool overlap, const void** mask_rows, uint32_t* mask_pitch) {
+    const PlanLayout l = plan_layout(p.B, p.L, p.F, mask_tma);
     char* base = reinterpret_cast<char*>(scratch.o);
     fa::PlanArgs a;
     a.mask = p.mask;
     a.k = static_cast<const __half*>(k);
     a.v = static_cast<const __half*>(v);
     a.copy = mask_tma ? nullptr : reinterpret_cast<__half*>(base);
-    a.head = reinterpret_cast<uint32_t*>(base + copy_bytes);
+    a.head = reinterpret_cast<uint32_t*>(base + l.copy_bytes);
     a.ticket = scratch.ticket;
-    a.order = reinterpret_cast<uint32_t*>(base + order_at);
-    a.bad = reinterpret_cast<uint32_t*>(base + bad_at);
-    a.list = reinterpret_cast<uint16_t*>(base + list_at);
-    a.cls = reinterpret_cast<uint8_t*>(base + cls_at);
+    a.order = reinterpret_cast<uint32_t*>(base + l.order_at);
+    a.bad = reinterpret_cast<uint32_t*>(base + l.bad_at);
+    a.list = reinterpret_cast<uint16_t*>(base + l.list_at);
+    a.cls = reinterpret_cast<uint8_t*>(base + l.cls_at);
     a.B = p.B;
     a.L = p.L;
     a.F = p.F;
-    a.n = n;
+    a.n = p.n_kv_tiles;
     a.q_pairs = p.q_pairs;
-    a.copy_pitch = pitch;
+    a.copy_pitch = l.pitch;
     a.stamp = p.launch_id;
     a.dense_allowed = mask_tma ? 1u : 0u;
     const uint64_t most = static_cast<uint64_t>(mask_tma ? fa::kPlanCtasPerSm : fa::kPlanCopyCtasPerSm) * c.sm_count;
-    const uint64_t wide = tiles > jobs ? tiles : jobs;
+    const uint64_t wide = l.tiles > l.jobs ? l.tiles : l.jobs;
     cudaError_t e = launch_kernel(mask_tma ? fa::fa_mask_plan<false> : fa::fa_mask_plan<true>,
                                   dim3(static_cast<unsigned>(wide < most ? wide : most)), fa::kPlanThreads, 0, st, overlap, a);
     if (e == cudaSuccess) e = cudaGetLastError();
@@ -544,8 +572,7 @@ int plan_mask(DeviceCtx& c, const SplitScratch& scratch, const void* k, const vo
     p.plan_order = a.order;
     p.plan_list = a.list;
     *mask_rows = mask_tma ? static_cast<const void*>(p.mask) : a.copy;
-    *mask_pitch = mask_tma ? p.L : pitch;
-    *planned = true;
+    *mask_pitch = mask_tma ? p.L : l.pitch;
     return FA_B200_OK;
 }
 
@@ -645,17 +672,17 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                     // (Planning a mask needs the same scratch, and a planned call is not divided.)
                     const uint32_t sms = static_cast<uint32_t>(c->sm_count);
                     const bool mask_tma = mask && mask_rows_aligned(mask, L);
-                    const bool want_plan = mask && may_plan && use_mask_plan(H, p.n_items, p.n_kv_tiles, B, p.q_pairs, mask_tma, sms, flags);
+                    const bool want_plan = mask && may_plan && use_mask_plan(B, L, F, H, mask_tma, sms, flags);
                     const bool want_split = !(flags & (FA_B200_FLAG_NO_SPLIT | FA_B200_FLAG_FORCE_PAIR));
                     SplitScratch* scratch = want_plan || want_split ? scratch_for_stream(*c, st) : nullptr;
                     std::unique_lock<std::mutex> launches;   // see SplitScratch::mu; given back when the last one is made
                     const bool pair = use_pair_kernel(H, mask != nullptr, mask_tma, p.q_pairs, p.R * B, sms, 0, flags);
                     const void* mask_at = mask;
                     uint32_t mask_pitch = L;
-                    bool planned = false;
-                    if (want_plan && scratch != nullptr) {
+                    const bool planned = want_plan && scratch != nullptr;
+                    if (planned) {
                         launches = std::unique_lock<std::mutex>(scratch->mu);
-                        rc = plan_mask(*c, *scratch, k, v, mask_tma, p, st, overlap, &mask_at, &mask_pitch, &planned);
+                        rc = plan_mask(*c, *scratch, k, v, mask_tma, p, st, overlap, &mask_at, &mask_pitch);
                     }
                     const Schedule sch = make_schedule(H, p.n_items, p.n_kv_tiles, sms, want_split && scratch != nullptr && !planned);
                     p.full_rounds = sch.full_rounds;
@@ -1199,6 +1226,47 @@ int fa_b200_describe_schedule(uint32_t B, uint32_t L, uint32_t F, uint32_t head_
     out[4] = s.tail_steps;
     out[6] = s.tail_grid;
     return FA_B200_OK;
+}
+
+int fa_b200_describe_call(uint32_t B, uint32_t L, uint32_t F, uint32_t head_dim, uint32_t mask_alignment,
+                          uint32_t flags, uint32_t sm_count, uint32_t out[3]) {
+    if (!out) return FA_B200_ERR_NULL_POINTER;
+    alignas(16) static const char d[32] = {0};
+    const bool has_mask = mask_alignment != 0;
+    const void* m = has_mask ? d + (mask_alignment & 15u) : nullptr;   // an address of that alignment
+    const int rc = validate(d, d, d, m, d, B, L, F, head_dim, 0, flags);
+    if (rc != FA_B200_OK) return rc;
+    const bool mask_tma = has_mask && mask_rows_aligned(m, L);
+    const int which = select_kernel(B, L, F, head_dim, has_mask, flags, static_cast<int>(sm_count));
+    out[0] = static_cast<uint32_t>(which);
+    out[1] = 0;
+    out[2] = 1;
+    if (which != 2) return FA_B200_OK;
+    const uint32_t n = (L + fa::kTile - 1) / fa::kTile, q_pairs = (L + 2 * fa::kTile - 1) / (2 * fa::kTile);
+    const bool planned = has_mask && use_mask_plan(B, L, F, head_dim, mask_tma, sm_count, flags);
+    const Schedule s = make_schedule(head_dim, q_pairs * (F / head_dim) * B, n, sm_count,
+                                     (flags & (FA_B200_FLAG_NO_SPLIT | FA_B200_FLAG_FORCE_PAIR)) == 0 && !planned);
+    if (use_pair_kernel(head_dim, has_mask, mask_tma, q_pairs, (F / head_dim) * B, sm_count, s.tail_steps, flags)) out[0] = 3;
+    out[1] = planned ? 1u : 0u;
+    out[2] = planned ? (mask_tma ? 3u : 2u) : 1u;
+    return FA_B200_OK;
+}
+
+int fa_b200_stream_has_scratch(int device, void* cuda_stream, uint32_t out[1]) {
+    if (!out) return FA_B200_ERR_NULL_POINTER;
+    int prev = -1;
+    cudaError_t e = cudaGetDevice(&prev);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (prev != device && (e = cudaSetDevice(device)) != cudaSuccess) return static_cast<int>(e);
+    DeviceCtx* c = nullptr;
+    int rc;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        rc = ensure_ctx(device, &c);
+    }
+    if (rc == FA_B200_OK) out[0] = scratch_for_stream(*c, static_cast<cudaStream_t>(cuda_stream), false) != nullptr ? 1u : 0u;
+    if (prev != device) (void)cudaSetDevice(prev);
+    return rc;
 }
 
 int fa_b200_select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t head_dim, int has_mask,

@@ -209,26 +209,51 @@ int fa_b200_debug_cycles(void* device_buffer_of_256_u64);
 #endif
 
 /*
- * Which kernel the default heuristics pick for a shape: returns 1 for the one-tile-per-CTA
- * kernel (and for sequences of one query tile, which may go to a kernel of small CTAs, and always
- * for head_dim 16 and 32, which the flags cannot force onto another one; by default they are
- * served by any), 2 for the warp-specialised kernel, 3 for the warp-specialised kernel on pairs of CTAs
- * (head_dim 128, whole work items; a mask is taken to start on a 16-byte boundary, its rows then
- * do so whenever L is a multiple of 8), negative status on invalid arguments.
- * No counterpart in the reference.
+ * What a call launches on a device with `sm_count` SMs.  `mask_alignment`: 0 without a mask, else what the
+ * mask's address is a multiple of, in bytes (2, 4, 8 or 16).
+ * out[0] = the kernel: 0 the one for short sequences, 1 the one with a query tile per CTA, 2 the
+ *          warp-specialised one, 3 the warp-specialised one on pairs of CTAs,
+ * out[1] = 1 if the call is planned on a stream that has scratch (fa_b200_stream_has_scratch): a kernel
+ *          finds out first what the mask leaves to do, and the warp-specialised kernel follows its lists;
+ *          for a mask whose rows all start on 16-byte boundaries the kernel of out[0] is launched behind
+ *          the two and does the call where the mask leaves too little out.  Without scratch it is
+ *          launched alone,
+ * out[2] = how many kernels that are (1, 2 or 3).
+ * Pure arithmetic, no CUDA call; it is what the launcher itself uses.  No counterpart in the reference.
+ */
+int fa_b200_describe_call(uint32_t B, uint32_t L, uint32_t F, uint32_t head_dim,
+                          uint32_t mask_alignment, uint32_t flags, uint32_t sm_count, uint32_t out[3]);
+
+/*
+ * out[0] = 1 if a call on `cuda_stream` would find scratch for a divided or a planned call, 0 if not: four
+ * streams of a device get some, the first four that ask, and keep it; a stream that is being captured
+ * gets none.  Takes none itself.  No counterpart in the reference.
+ */
+int fa_b200_stream_has_scratch(int device, void* cuda_stream, uint32_t out[1]);
+
+/*
+ * The family a call belongs to, as harnesses ask for it: 1 for the kernel with a query tile per CTA, for
+ * every sequence that the kernel for short sequences takes, and for every call at head_dim 16 and 32
+ * (whichever kernel serves those: FA_B200_FLAG_FORCE_PIPELINED is refused there), 2 for the
+ * warp-specialised kernel, 3 for the warp-specialised kernel on pairs of CTAs (head_dim 128, whole work
+ * items; a mask is taken to start on a 16-byte boundary, its rows then do so whenever L is a multiple of
+ * 8, and not to be planned), negative status on invalid arguments.  fa_b200_describe_call says what a
+ * call launches.  No counterpart in the reference.
  */
 int fa_b200_select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t head_dim,
                           int has_mask, uint32_t flags);
 
 /*
  * How the warp-specialised kernel would spread a call's work over its CTAs on a device with
- * `sm_count` SMs (head_dim 64 and 128; smaller ones are described as one CTA per query tile):
+ * `sm_count` SMs, without a mask (head_dim 64 and 128; smaller ones are described as one CTA per query
+ * tile, whichever kernel serves them, see fa_b200_select_kernel):
  * out[0] = kernel (1, 2 or 3, as fa_b200_select_kernel; for 3 a work item is 512 query
  * rows and out[1] CTAs form out[1]/2 pairs, nothing is divided), out[1] = CTAs launched,
  * out[2] = rounds of whole work items (a work item is 256 query rows of one (batch, head) against
  * all keys; CTA c takes items c, c + out[1], ...), out[3] = work items of the last, partial round
  * whose key steps are divided evenly among the first out[6] CTAs (0 = nothing is divided; a range
- * is at least half a work item, so a work item has at most three parts), out[4] = key steps of
+ * is at least half a work item, or exactly a third of each with out[6] = 3 * out[3]: a work item has
+ * at most three parts), out[4] = key steps of
  * those items in all, out[5] = key steps (tiles of 128 keys) per work item.  Pure arithmetic, no
  * CUDA call; it is what the launcher itself uses (FA_B200_FLAG_NO_SPLIT in `flags` is honoured).
  * No counterpart in the reference, whose grid is one CTA per (batch, query chunk, head)

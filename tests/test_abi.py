@@ -136,6 +136,20 @@ def test_kernel_selection(lib):
     assert sel(1 << 20, 128 * 2048, 64, 64, 0, 0) == _lib.ERR_SHAPE   # 2^31 CTAs: too many for one grid axis
 
 
+@pytest.mark.parametrize("call,kernel,planned,launches", [
+    ((8, 49, 256, 32, 2), 0, 0, 1), ((1, 160, 64, 16, 0), 0, 0, 1), ((8, 100, 768, 64, 0), 0, 0, 1), ((8, 128, 768, 64, 0), 1, 0, 1),
+    ((8, 1024, 512, 32, 0), 2, 0, 1), ((1, 256, 256, 64, 0), 1, 0, 1), ((1, 256, 256, 64, 16), 2, 0, 1),
+    ((8, 512, 768, 64, 16), 2, 0, 1), ((4, 1021, 768, 64, 16), 2, 1, 2), ((4, 1024, 768, 64, 16), 2, 0, 1),
+    ((4, 1024, 768, 64, 8), 2, 1, 2), ((8, 2048, 2048, 64, 16), 2, 1, 3), ((4, 2048, 4096, 128, 16), 3, 1, 3),
+    ((4, 2048, 4096, 128, 0), 3, 0, 1), ((1, 16384, 512, 128, 0), 2, 0, 1), ((1, 40000, 64, 64, 2), 2, 0, 1)])
+def test_what_a_call_launches(lib, call, kernel, planned, launches):
+    out = (ctypes.c_uint32 * 3)()
+    assert lib.fa_b200_describe_call(*call, 0, 148, out) == 0
+    assert tuple(out) == (kernel, planned, launches)
+    assert lib.fa_b200_describe_call(*call[:3], 48, call[4], 0, 148, out) == _lib.ERR_HEAD_DIM
+    assert lib.fa_b200_describe_call(*call[:4], 1, 0, 148, out) == _lib.ERR_ALIGNMENT
+
+
 def test_missing_library_is_loud(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "_lib", None)
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))

@@ -112,6 +112,9 @@ def _block_mask(B, L, kind):
 def test_planned_masks(B, R, L, H, kind):
     """Calls that are planned: key tiles that the mask takes away are left out, tiles that are zero or -inf are not
     fetched, rows on no 16-byte boundary are copied.  The same bits as without a plan, and the oracle's values."""
+    route = fa.describe_call(B, L, R * H, H, 16)
+    assert route["planned"] == (L != 201) and fa.stream_has_scratch()      # (two key tiles are not worth a plan)
+    assert route["launches"] == (1 if L == 201 else 3 if L % 8 == 0 else 2)
     q, k, v = make_inputs(B, L, R * H, 1.0, L)
     mask = _block_mask(B, L, kind)
     dev = [t.cuda() for t in (q, k, v, mask)]
@@ -128,6 +131,7 @@ def test_masked_keys_that_are_not_finite_are_not_left_out(where, value, B, R, L)
     """0 * inf and inf - inf are NaN: a masked key with an infinity or a NaN in K or V reaches the result with a plan
     exactly as it does without one."""
     H = 64
+    assert fa.describe_call(B, L, R * H, H, 16)["planned"] and fa.stream_has_scratch()
     q, k, v = (t.cuda() for t in make_inputs(B, L, R * H, 1.0, L))
     mask = torch.zeros(B, L, L, dtype=torch.float16)
     mask[:, :, 200:] = float("-inf")
