@@ -660,9 +660,6 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                 p.part_o = nullptr;
                 p.part_ml = nullptr;
                 p.part_cnt = nullptr;
-                p.plan_head = nullptr;
-                p.plan_order = nullptr;
-                p.plan_list = nullptr;
                 const int which = select_kernel(B, L, F, H, mask != nullptr, flags, c->sm_count);
                 const bool overlap = (flags & FA_B200_FLAG_NO_OVERLAP) == 0;
                 if (which == 2) {
@@ -906,9 +903,6 @@ int fa_b200_attention_forward_noalloc(const void* q, const void* k, const void* 
         p.part_o = nullptr;
         p.part_ml = nullptr;
         p.part_cnt = nullptr;
-        p.plan_head = nullptr;
-        p.plan_order = nullptr;
-        p.plan_list = nullptr;
 #ifdef FA_CYCLES
         p.cycles = nullptr;
 #endif

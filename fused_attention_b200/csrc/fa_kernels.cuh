@@ -53,14 +53,23 @@ struct Params {
     uint32_t tail_items;   // items after the full rounds whose key steps are divided among the CTAs
     uint32_t tail_steps;   // tail_items * n_kv_tiles, or 0 when nothing is divided
     uint32_t tail_grid;    // the first tail_grid CTAs share the tail key steps (at most the grid)
-    float4* part_o;        // [2 * grid slots][2 tiles][H/4][128 rows] numerators of partial segments, fp32
-    float2* part_ml;       // [2 * grid slots][2 tiles][128 rows] {reference maximum, row sum}
-    uint32_t* part_cnt;    // [tail item][2 tiles][4 warps] parts counted in; zero between launches
+    // A planned call is not divided, so what its mask leaves to do (fa_mask_plan.cuh) takes the places of the parts; with
+    // tail_steps == 0, plan_head is null or {1 = the planned kernel runs, 0 = the one that the call has without a plan}.
+    // (Three words more in here, and what the rescaling of masked rows does in the instances without a mask, made the
+    // compiler lay out the unmasked kernel at H = 64 worse: B=37 R=4 L=2048 194.6 us, 191.1 without either.)
+    union {
+        float4* part_o;    // [2 * grid slots][2 tiles][H/4][128 rows] numerators of partial segments, fp32
+        const uint32_t* plan_order;   // pairs of query tiles of a batch entry, longest first: index | key steps << kPlanLenShift
+    };
+    union {
+        float2* part_ml;   // [2 * grid slots][2 tiles][128 rows] {reference maximum, row sum}
+        const uint16_t* plan_list;    // [pair][n_kv_tiles]: the key steps that are left, see kStepShift0
+    };
+    union {
+        uint32_t* part_cnt;   // [tail item][2 tiles][4 warps] parts counted in; zero between launches
+        const uint32_t* plan_head;
+    };
     uint32_t part_slots;   // scratch slots behind part_o / part_ml (two per CTA of the largest grid)
-    // what the mask leaves to do (fa_mask_plan.cuh), or null: {1 = the planned kernel runs, 0 = the kernel behind it}
-    const uint32_t* plan_head;
-    const uint32_t* plan_order;   // pairs of query tiles of a batch entry, longest first: index | key steps << kPlanLenShift
-    const uint16_t* plan_list;    // [pair][n_kv_tiles]: the key steps that are left, see kStepShift0
 #ifdef FA_CYCLES
     unsigned long long* cycles;  // 64 records (launch_id % 64) of CTA 0: {globaltimer at entry, globaltimer after the
                                  // wait for the previous kernel, globaltimer at the end, clock64 from that wait to the end}
@@ -1324,7 +1333,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // before it asks for anything, because with no segments no role would wait for a copy and the CTA would leave with it
     // still landing in its shared memory.
     if constexpr (kMask == kMaskTma) {
-        if (first_known && p.plan_head != nullptr && *p.plan_head != 0u) {
+        if (first_known && p.tail_steps == 0u && p.plan_head != nullptr && *p.plan_head != 0u) {
             plan_smem = Plan{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
             first_known = false;
         }
@@ -1335,7 +1344,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
     if (tid == 15 * 32) leave_early_if_launch_failed(ctl);
     if constexpr (kMask == kMaskTma) {
-        if (p.plan_head != nullptr) __syncthreads();   // plan_smem may have been emptied
+        if (p.tail_steps == 0u && p.plan_head != nullptr) __syncthreads();   // plan_smem may have been emptied
     }
     if constexpr (kPlanned) {
         settled = zero_behind_the_wait();
@@ -1473,9 +1482,13 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         float nmc2 = -m * c;
                         if constexpr (kHasMask) nmc2 = (m == -INFINITY) ? 0.f : nmc2;
                         float unused[4];
-                        // (the sum in the order of the common path: it does not matter on which of them a row took its reference)
-                        const float sum2 = exp_chunks<0, C::kHeldChunks, false>(s, c, nmc2, tP, unused);
-                        l = l * alpha + (sum2 + exp_chunks<C::kHeldChunks, 4, false>(s, c, nmc2, tP, unused));
+                        if constexpr (kHasMask) {
+                            // (the sum in the order of the common path: it does not matter on which of them a row took its reference)
+                            const float sum2 = exp_chunks<0, C::kHeldChunks, false>(s, c, nmc2, tP, unused);
+                            l = l * alpha + (sum2 + exp_chunks<C::kHeldChunks, 4, false>(s, c, nmc2, tP, unused));
+                        } else {
+                            l = l * alpha + exp_chunks<0, 4, false>(s, c, nmc2, tP, unused);
+                        }
                         // (This wait returns at once.  It is here because with a branch point at this
                         // place of the rare path the compiler allocates the common path without spills.)
                         if (g > 0) mbar_wait(bar(BAR_PV0 + i), (g - 1u) & 1u, ctl, kRoleSoftmax | (BAR_PV0 + i));

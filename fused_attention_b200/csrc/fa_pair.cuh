@@ -259,9 +259,13 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
                         float nmc2 = -m * c;
                         if constexpr (kHasMask) nmc2 = (m == -INFINITY) ? 0.f : nmc2;
                         float unused[4];
-                        // (the sum in the order of the common path: it does not matter on which of them a row took its reference)
-                        const float sum2 = exp_chunks<0, C::kHeldChunks, false>(s, c, nmc2, tP, unused);
-                        l = l * alpha + (sum2 + exp_chunks<C::kHeldChunks, 4, false>(s, c, nmc2, tP, unused));
+                        if constexpr (kHasMask) {
+                            // (the sum in the order of the common path: it does not matter on which of them a row took its reference)
+                            const float sum2 = exp_chunks<0, C::kHeldChunks, false>(s, c, nmc2, tP, unused);
+                            l = l * alpha + (sum2 + exp_chunks<C::kHeldChunks, 4, false>(s, c, nmc2, tP, unused));
+                        } else {
+                            l = l * alpha + exp_chunks<0, 4, false>(s, c, nmc2, tP, unused);
+                        }
                         if (g > 0) mbar_wait(bar(BAR_PV0 + i), (g - 1u) & 1u, ctl, kRoleSoftmax | (BAR_PV0 + i));
                         tc_fence_after();
                         __syncwarp();
