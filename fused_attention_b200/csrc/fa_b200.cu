@@ -235,24 +235,42 @@ int validate(const void* q, const void* k, const void* v, const void* mask, cons
     return FA_B200_OK;
 }
 
-// Whether a call goes to the kernel for short sequences (fa_small.cuh): by length, head_dim and mask alone, never by how
-// many problems there are.  Measured, us on the kernel that would have the call otherwise and on this one:
+// Whether a call goes to the kernel for short sequences (fa_small.cuh).  Measured, us on the kernel that would have the call otherwise and on this one:
 //   H = 16 and 32: ahead up to 160 keys: H = 32, B=256 R=8 L=49 29 / 12 (with a mask 44 / 12), L=121 32 / 26, L=144
 //   58 / 54 (88 / 68), B=64 R=8 L=144 18.5 / 15.0.
 //   H = 64: B=256 R=8 L=49 31 / 11, L=121 41 / 39, but L=128, where the 128-row tile wastes nothing, B=32 R=16 10.1 /
 //   11.2, and behind that (L=144) 62 / 85, the scores of ten key tiles leaving the SM too few warps; with a mask L=121
 //   95 / 61, L=128 62 / 56, L=144 102 / 92, L=129 119 / 133 (a row that starts anywhere costs its reader twice the loads).
 //   H = 128: B=64 R=16 L=50 21 / 11, L=100 16 / 23; with a mask that TMA cannot fetch L=121 141 / 109.
-bool use_small_kernel(uint32_t H, uint32_t L, bool has_mask) {
-    const bool even_rows = (L & 7u) == 0u;
+// Near the last lengths at H = 64 and 128 the two kernels are level, and the number of problems decides: both go in rounds
+// of two CTAs per SM, and where the last round is more than half full the one-tile kernel's larger CTAs, of which two
+// share an SM better, are ahead, until there are four rounds.  Measured with 192, 384, 512, 768, 1024 and 1600 problems,
+// one-tile kernel / this one:
+//   H = 64, L=128, aligned mask: 8.2 / 9.1, 14.3 / 13.5, 15.0 / 16.9, 21.9 / 24.4, 29.0 / 28.3, 51 / 46
+//   H = 64, L=112, no mask: 6.0 / 6.2, 9.9 / 9.3, 11.1 / 11.4, 15.6 / 16.3, 19.4 / 19.6, 30.8 / 30.2
+//   H = 128, L=100, rows on no 16-byte boundary: 14.4 / 15.2, 24.8 / 22.6, 26.6 / 29.7, 39.1 / 43.8, 54.3 / 53.4, 92 / 83
+//   (rows that start in the middle of a word, which the one-tile kernel reads value by value: L=121 18.1 / 16.5, 30.4 /
+//   24.8, 33.5 / 32.6, 54.4 / 48.6, 77 / 59, 115 / 90)
+// The two differ in their last bits, so with FA_B200_FLAG_NO_SPLIT (and in host calls, which make chunks of a call) the
+// number of problems is not looked at.
+bool use_small_kernel(uint32_t H, uint32_t L, bool has_mask, bool mask_tma, uint64_t problems, uint32_t sms, uint32_t flags) {
     if (H <= 32) return L <= 160;
-    if (H == 64) return has_mask ? L <= 128 || (L <= 160 && even_rows) : L < 128;
-    return L <= 64 || (has_mask && !even_rows && L <= 128);
+    const bool even_rows = (L & 7u) == 0u;
+    bool takes, level;
+    if (H == 64) {
+        takes = has_mask ? L <= 128 || (L <= 160 && even_rows) : L < 128;
+        level = has_mask ? L == 128 && mask_tma : L > 96;
+    } else {
+        takes = L <= 64 || (has_mask && !even_rows && L <= 128);
+        level = L > 96 && (L & 1u) == 0u;
+    }
+    if (!takes || !level || (flags & FA_B200_FLAG_NO_SPLIT)) return takes;
+    return problems >= 8ull * sms || (problems - 1u) % (2ull * sms) < sms;
 }
 
 // 0 = the kernel for short sequences, 1 = simple kernel, 2 = pipelined kernel (or the one on pairs of CTAs, see
 // use_pair_kernel).
-int select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool has_mask, uint32_t flags,
+int select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool has_mask, bool mask_tma, uint32_t flags,
                   int sm_count) {
     if (flags & FA_B200_FLAG_FORCE_SIMPLE) return 1;
     if (flags & (FA_B200_FLAG_FORCE_PIPELINED | FA_B200_FLAG_FORCE_PAIR)) return 2;
@@ -268,7 +286,8 @@ int select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool has_mask,
     // With a mask the pipelined kernel is ahead from the second tile on: its other warps bring the mask in
     // (H = 32, B=1 R=4 L=129 9.7 vs 11.6 us, L=256 7.7 vs 10.1 us, L=1024 17.6 vs 34.9 us).
     const uint64_t pairs = static_cast<uint64_t>((L + 255) / 256) * (F / H) * B;
-    if (use_small_kernel(H, L, has_mask)) return 0;
+    const uint64_t problems = static_cast<uint64_t>(F / H) * B;
+    if (use_small_kernel(H, L, has_mask, mask_tma, problems, static_cast<uint32_t>(sm_count), flags)) return 0;
     if (L <= 128) return 1;
     if (has_mask || L > (H >= 64 ? 5u : 2u) * 128u) return 2;
     if (pairs * 2 < static_cast<uint64_t>(sm_count)) return 1;
@@ -660,7 +679,8 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                 p.part_o = nullptr;
                 p.part_ml = nullptr;
                 p.part_cnt = nullptr;
-                const int which = select_kernel(B, L, F, H, mask != nullptr, flags, c->sm_count);
+                const bool mask_tma = mask && mask_rows_aligned(mask, L);
+                const int which = select_kernel(B, L, F, H, mask != nullptr, mask_tma, flags, c->sm_count);
                 const bool overlap = (flags & FA_B200_FLAG_NO_OVERLAP) == 0;
                 if (which == 2) {
                     // Dividing the last round needs scratch that no other launch is using: the buffer that
@@ -668,7 +688,6 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                     // could later be replayed next to anything).
                     // (Planning a mask needs the same scratch, and a planned call is not divided.)
                     const uint32_t sms = static_cast<uint32_t>(c->sm_count);
-                    const bool mask_tma = mask && mask_rows_aligned(mask, L);
                     const bool want_plan = mask && may_plan && use_mask_plan(B, L, F, H, mask_tma, sms, flags);
                     const bool want_split = !(flags & (FA_B200_FLAG_NO_SPLIT | FA_B200_FLAG_FORCE_PAIR));
                     SplitScratch* scratch = want_plan || want_split ? scratch_for_stream(*c, st) : nullptr;
@@ -1008,9 +1027,10 @@ int fa_b200_attention_forward_host(const void* q, const void* k, const void* v, 
         // the result has the same bits as one device-pointer call on the full tensors with
         // FA_B200_FLAG_NO_SPLIT
         // (plain launches: a chunk's kernel is ordered behind copies on other streams, not behind a kernel)
-        // (the kernel for short sequences is chosen by length and head_dim alone, so a chunk gets it as the whole does)
+        // (with NO_SPLIT the kernel for short sequences is chosen by length, head_dim and mask alone, so a chunk gets it as the
+        // whole does; the mask lies in the staging buffer, where its rows are aligned whenever L is a multiple of 8)
         // (not planned: the copies bound the call, and the scratch a plan lies in belongs to the callers' streams)
-        const int whole = select_kernel(B, L, F, H, mask_or_null != nullptr, flags, c->sm_count);
+        const int whole = select_kernel(B, L, F, H, mask_or_null != nullptr, (L & 7u) == 0u, flags | FA_B200_FLAG_NO_SPLIT, c->sm_count);
         const uint32_t chunk_flags =
             (flags & ~static_cast<uint32_t>(FA_B200_FLAG_SYNC | FA_B200_FLAG_FORCE_SIMPLE | FA_B200_FLAG_FORCE_PIPELINED)) |
             FA_B200_FLAG_NO_OVERLAP | FA_B200_FLAG_NO_SPLIT | (whole == 0 ? 0u : (whole == 2 ? FA_B200_FLAG_FORCE_PIPELINED : FA_B200_FLAG_FORCE_SIMPLE));
@@ -1193,7 +1213,7 @@ int fa_b200_describe_schedule(uint32_t B, uint32_t L, uint32_t F, uint32_t head_
     const uint32_t n = (L + fa::kTile - 1) / fa::kTile;
     const uint32_t n_items = ((L + 2 * fa::kTile - 1) / (2 * fa::kTile)) * (F / head_dim) * B;
     // (head_dim 16 and 32: reported as one CTA per query tile, see the header)
-    const int chosen = head_dim < 64 ? 1 : select_kernel(B, L, F, head_dim, false, flags, static_cast<int>(sm_count));
+    const int chosen = head_dim < 64 ? 1 : select_kernel(B, L, F, head_dim, false, false, flags, static_cast<int>(sm_count));
     const int which = chosen == 0 ? 1 : chosen;   // (short sequences: reported as one CTA per query tile, which it is)
     out[0] = static_cast<uint32_t>(which);
     out[5] = n;
@@ -1231,7 +1251,7 @@ int fa_b200_describe_call(uint32_t B, uint32_t L, uint32_t F, uint32_t head_dim,
     const int rc = validate(d, d, d, m, d, B, L, F, head_dim, 0, flags);
     if (rc != FA_B200_OK) return rc;
     const bool mask_tma = has_mask && mask_rows_aligned(m, L);
-    const int which = select_kernel(B, L, F, head_dim, has_mask, flags, static_cast<int>(sm_count));
+    const int which = select_kernel(B, L, F, head_dim, has_mask, mask_tma, flags, static_cast<int>(sm_count));
     out[0] = static_cast<uint32_t>(which);
     out[1] = 0;
     out[2] = 1;
@@ -1275,7 +1295,7 @@ int fa_b200_select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t head_dim,
         (void)cudaGetLastError();
         sms = 148;
     }
-    const int which = head_dim < 64 ? 1 : select_kernel(B, L, F, head_dim, has_mask != 0, flags, sms);
+    const int which = head_dim < 64 ? 1 : select_kernel(B, L, F, head_dim, has_mask != 0, (L & 7u) == 0u, flags, sms);
     if (which != 2) return 1;
     const uint32_t n = (L + fa::kTile - 1) / fa::kTile, q_pairs = (L + 2 * fa::kTile - 1) / (2 * fa::kTile);
     const Schedule s = make_schedule(head_dim, q_pairs * (F / head_dim) * B, n, static_cast<uint32_t>(sms),

@@ -150,6 +150,22 @@ def test_what_a_call_launches(lib, call, kernel, planned, launches):
     assert lib.fa_b200_describe_call(*call[:4], 1, 0, 148, out) == _lib.ERR_ALIGNMENT
 
 
+@pytest.mark.parametrize("H,L,alignment,takes", [(64, 128, 16, False), (64, 128, 2, True), (64, 112, 0, False), (64, 96, 0, True),
+                                                 (128, 100, 2, False), (128, 99, 2, True), (128, 95, 2, True), (128, 64, 0, True), (32, 160, 0, True)])
+def test_short_sequences_whose_number_decides(lib, H, L, alignment, takes):
+    """Rounds of 296 problems on 148 SMs: the kernel for short sequences up to half a round, the one-tile kernel beyond,
+    the former again from four rounds on; with NO_SPLIT the number of problems is not looked at."""
+    out = (ctypes.c_uint32 * 3)()
+
+    def kernel(problems, flags=0):
+        assert lib.fa_b200_describe_call(problems, L, H, H, alignment, flags, 148, out) == 0
+        return out[0]
+
+    assert [kernel(n) for n in (1, 148, 297, 444, 1184, 5000)] == [0] * 6
+    assert [kernel(n) for n in (149, 296, 445, 592, 1183)] == [0 if takes else 1] * 5
+    assert [kernel(n, _lib.FLAG_NO_SPLIT) for n in (1, 149, 296, 592, 1183)] == [0] * 5
+
+
 def test_missing_library_is_loud(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "_lib", None)
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
