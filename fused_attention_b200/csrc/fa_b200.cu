@@ -281,15 +281,26 @@ int select_kernel(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool has_mask,
     // With few items the two are level up to about five key steps (7-14 us, mostly launch); from
     // there on the pipelined kernel wins however few items there are (measured: B=1 R=16 L=1024 H=128
     // 20.5 vs 24.6 us, B=1 R=4 L=2048 32.8 vs 41.9 us, B=1 R=2 L=4096 57 vs 79 us).
-    // At H = 16 and 32, where a tile is cheap to load, they are level up to two key steps only (H = 32, B=1 R=4 L=256
-    // 7.7 vs 7.4 us, L=512 8.5 vs 9.2 us; H = 16, B=8 R=16 L=1024 49.0 vs 67.6 us).
+    // At H = 16 and 32, where a tile is cheap to load, the pipelined kernel is ahead from four key steps on (H = 32, R=1 L=512
+    // 8.4 vs 9.0 us, 92 heads 15.5 vs 19.7 us; H = 16, B=8 R=16 L=1024 49.0 vs 67.6 us).  Below that the rounds decide, of
+    // two tiles per SM here and of one item there.  H = 32, us here and there: L=256, one round here: 74 heads 5.8 / 6.5,
+    // 148 heads 7.3 / 7.4; two: 200 heads 11.9 / 10.0.  L=300, a tile per SM: 49 heads 8.1 / 8.7; a round each: 74 heads 9.7
+    // / 8.9; one round and two: 92 heads 9.8 / 13.2; two each: 111 heads 16.1 / 13.6; two and three (H = 16): 180 heads
+    // 17.3 / 18.3; more: 400 heads 39.9 / 33.1.
     // With a mask the pipelined kernel is ahead from the second tile on: its other warps bring the mask in
     // (H = 32, B=1 R=4 L=129 9.7 vs 11.6 us, L=256 7.7 vs 10.1 us, L=1024 17.6 vs 34.9 us).
     const uint64_t pairs = static_cast<uint64_t>((L + 255) / 256) * (F / H) * B;
     const uint64_t problems = static_cast<uint64_t>(F / H) * B;
     if (use_small_kernel(H, L, has_mask, mask_tma, problems, static_cast<uint32_t>(sm_count), flags)) return 0;
     if (L <= 128) return 1;
-    if (has_mask || L > (H >= 64 ? 5u : 2u) * 128u) return 2;
+    if (has_mask) return 2;
+    if (H < 64) {
+        const uint64_t n = (L + 127u) / 128u, sms = static_cast<uint64_t>(sm_count), tiles = n * problems;
+        const uint64_t waves = (tiles + 2u * sms - 1u) / (2u * sms), rounds = (pairs + sms - 1u) / sms;
+        if (n > 3u) return 2;
+        return (n == 2u ? waves == 1u : tiles <= sms || (waves < rounds && waves <= 2u)) ? 1 : 2;
+    }
+    if (L > 5u * 128u) return 2;
     if (pairs * 2 < static_cast<uint64_t>(sm_count)) return 1;
     return 2;
 }

@@ -166,6 +166,20 @@ def test_short_sequences_whose_number_decides(lib, H, L, alignment, takes):
     assert [kernel(n, _lib.FLAG_NO_SPLIT) for n in (1, 149, 296, 592, 1183)] == [0] * 5
 
 
+@pytest.mark.parametrize("H", [16, 32])
+def test_two_and_three_tiles_at_small_head_dims(lib, H):
+    """Rounds of 296 tiles on the one-tile kernel against rounds of 148 pairs of tiles on the warp-specialised one."""
+    out = (ctypes.c_uint32 * 3)()
+
+    def kernel(heads, L):
+        assert lib.fa_b200_describe_call(heads, L, H, H, 0, 0, 148, out) == 0
+        return out[0]
+
+    assert [kernel(n, 256) for n in (1, 74, 148, 149, 400)] == [1, 1, 1, 2, 2]
+    assert [kernel(n, 300) for n in (1, 49, 50, 74, 75, 98, 99, 148, 149, 197, 198, 400)] == [1, 1, 2, 2, 1, 1, 2, 2, 1, 1, 2, 2]
+    assert [kernel(n, 385) for n in (1, 50, 400)] == [2, 2, 2]
+
+
 def test_missing_library_is_loud(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "_lib", None)
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
