@@ -315,8 +315,9 @@ def other_workloads(torch, fa, dev, peaks: dict, skip: str) -> dict:
 
 def masked_run(torch, fa, dev, w, peaks: dict, unmasked_ms: float) -> dict:
     """The same workload with an additive causal mask [B, L, L] (0 on and below the diagonal, -inf above), one
-    GPU: the mask costs B*L*L*2 bytes of reads on top of Q, K, V, Y, and no work is skipped (the operator's mask
-    is data, not a causal flag), so the FLOP count is the unmasked one."""
+    GPU: the mask costs B*L*L*2 bytes of reads on top of Q, K, V, Y.  The mask is data, not a causal flag; a planned
+    call finds out on the device that key tiles are taken away whole and leaves them out, so the FLOPs counted are
+    those of the pairs of a query and a key that the mask leaves in."""
     host = __import__("fused_attention_b200.workloads", fromlist=["workload_inputs"]).workload_inputs(w)
     bufs, n, one = device_copies(torch, host, dev, 2 * L2_BYTES, max_copies=8)
     mask = torch.triu(torch.full((w.L, w.L), float("-inf"), device=dev, dtype=torch.float16), diagonal=1)
@@ -345,14 +346,16 @@ def masked_run(torch, fa, dev, w, peaks: dict, unmasked_ms: float) -> dict:
     ms_plain_after = timed(without)
     ms_plain = 0.5 * (ms_plain_before + ms_plain_after)
     mask_bytes = w.B * w.L * w.L * 2
-    t_tensor = w.flops / (float(peaks["bf16_tflops"]) * 1e12)
+    flops = w.flops * (w.L + 1) / (2 * w.L)   # L (L + 1) / 2 pairs of L * L
+    route = fa.describe_call(w.B, w.L, w.F, w.H, 16, sm_count=fa.query(dev.index or 0)["sm_count"])
+    t_tensor = flops / (float(peaks["bf16_tflops"]) * 1e12)
     t_hbm = (w.bytes + mask_bytes) / (float(peaks["hbm_gbs"]) * 1e9)
-    return {"mask": "causal, additive fp16 [B, L, L]", "ms_per_launch": ms, "tflops": w.flops / (ms * 1e-3) / 1e12,
-            "algorithmic_bytes": w.bytes + mask_bytes, "algorithmic_gbs": (w.bytes + mask_bytes) / (ms * 1e-3) / 1e9,
+    return {"mask": "causal, additive fp16 [B, L, L]", "ms_per_launch": ms, "tflops": flops / (ms * 1e-3) / 1e12,
+            "flops_counted": "pairs that the mask leaves in", "algorithmic_bytes": w.bytes + mask_bytes, "algorithmic_gbs": (w.bytes + mask_bytes) / (ms * 1e-3) / 1e9,
             "bound": "tensor" if t_tensor >= t_hbm else "hbm", "frac_of_bound": max(t_tensor, t_hbm) / (ms * 1e-3),
             "unmasked_ms_per_launch_before_and_after": [ms_plain_before, ms_plain_after],
             "time_over_unmasked": ms / ms_plain, "time_over_the_timed_region": ms / unmasked_ms,
-            "kernel": fa.select_kernel(w.B, w.L, w.F, w.H, has_mask=True)}
+            "kernel": "pipelined, planned" if route["planned"] else route["kernel"], "launches_per_call": route["launches"]}
 
 
 def run_ours(args, workload, rank: int, world: int, local_rank: int) -> dict | None:
