@@ -554,7 +554,9 @@ bool plan_fits(uint32_t B, uint32_t L, uint32_t F, bool mask_tma, uint32_t sms) 
 //   H = 64: B=8 R=12 L=512 21.8 / 24.2, B=32 R=12 L=512 58 / 73, B=8 R=16 L=1024 70 / 65, B=8 R=32 L=2048 430 / 320
 //   H = 32: B=8 R=16 L=2048 255 / 160
 //   H = 128: B=4 R=32 L=1024 77 / 97, B=2 R=32 L=2048 141 / 138, B=4 R=32 L=2048 291 / 254, B=1 R=40 L=4096 385 / 227
-// so from sixteen key tiles and some fifty key steps per SM on.  Where TMA cannot fetch the rows the plan's copy also
+// so from sixteen key tiles and some fifty key steps per SM on.  (A mask that leaves nothing out pays for the plan and the
+// planned kernel's launch all the same: H = 128, B=2 R=32 L=2048 139 / 151, B=4 R=32 L=2048 265 / 277; at H = 64 B=4 R=32
+// L=2048 it is 248 with both.  What the mask holds is known on the device only.)  Where TMA cannot fetch the rows the plan's copy also
 // spares every head the copies inside the kernel, and it pays much sooner:
 //   H = 64: B=32 R=16 L=201 36 / 46, B=1 R=8 L=301 15 / 18, B=32 R=12 L=301 82 / 63, B=2 R=8 L=511 26 / 21,
 //           B=4 R=12 L=1021 72 / 38;   H = 128: B=1 R=8 L=301 25 / 19, B=2 R=32 L=1021 125 / 51
@@ -1020,14 +1022,14 @@ int fa_b200_attention_forward_host(const void* q, const void* k, const void* v, 
         if (rc == FA_B200_OK && mbytes) rc = grow(*c, 4, mbytes);
     }
     if (rc == FA_B200_OK) {
-        // Chunked pipeline over three streams: while chunk c computes, chunk c+1 is copied in and chunk c-1 is copied
-        // out.  Chunks are groups of batch entries where there are enough of
-        // them; otherwise K and V of an entry go ahead and its queries (with their rows of the mask) follow in blocks
-        // of rows, so that what is left behind the last copy in is one block's product and copy out.  Every copy is one
-        // contiguous run: the 2-D copies that a division by heads needs move 44 GB/s with rows of 2 KB and 38 with 1 KB
-        // against 54 here.  Measured, pinned buffers, us by heads and by rows: B=1 R=8 L=256 H=64 165 / 81, B=1 R=16
-        // L=1000 H=128 449 / 339, B=1 R=32 L=1024 H=128 683 / 632; B=2 R=32 L=1024 H=128 (by batch entries before) 1187 /
-        // 1178, where the two directions together move 57 GB/s, all that the box gives.  Sixteen chunks are no better.
+        // Chunked pipeline over three streams: while chunk c computes, chunk c+1 is copied in and chunk c-1 is copied out.
+        // Chunks are groups of batch entries where there are enough of them; otherwise K and V of an entry go ahead and its
+        // queries (with their rows of the mask) follow in blocks of rows, so that what is left behind the last copy in is
+        // one block's product and copy out.  Every copy is one contiguous run: the 2-D copies that a division by heads
+        // needs move 44 GB/s with rows of 2 KB and 38 with 1 KB against 54 here.  Measured, pinned buffers, us by heads and
+        // by rows: B=1 R=8 L=256 H=64 165 / 81, B=1 R=16 L=1000 H=128 449 / 339, B=1 R=32 L=1024 H=128 683 / 632; B=2 R=32
+        // L=1024 H=128, which went by batch entries before, 1187 / 1178, no more than its runs differ.  Sixteen chunks are
+        // no better.
         cudaStream_t s_in = c->host_stream, s_cmp = c->host_stream2, s_out = c->host_stream3;
         const uint32_t H = head_dim;
         const __half *hq = static_cast<const __half*>(q), *hk = static_cast<const __half*>(k), *hv = static_cast<const __half*>(v);

@@ -761,7 +761,7 @@ struct PipeCfg {
     static constexpr int kRingBytes = kStages * G::kTileBytes;
     static constexpr int kMaskBoxBytes = kTile * 64 * 2;                  // 128 rows x 64 keys
     static constexpr int kMaskBytes = kHasMask ? kMaskBoxes * kMaskBoxBytes : 0;   // one buffer
-    static constexpr int kMaskExtraBytes = kMask == kMaskCopied ? kTile * 4 : 0;  // of one buffer:     // one word per row, see copy_mask_rows
+    static constexpr int kMaskExtraBytes = kMask == kMaskCopied ? kTile * 4 : 0;   // of one buffer: a word per row, see copy_mask_rows
     // Columns of one TMA store of Y: with the mask's box the whole ring leaves room for staging buffers of 32 only.
     static constexpr int kStoreCols = kMaskBoxes == 1 ? 32 : G::kBoxCols;
     static constexpr int kStageWarpBytes = kMaskBoxes == 1 ? 2048 : 4096;   // per epilogue warp 32 rows x kStoreCols fp16
@@ -1414,7 +1414,8 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 if constexpr (kHasMask) {
                     const uint32_t what = step_mask(step, i);
                     if (what == kStepMask) {
-                        // The mask tile of this tile and step, brought in by TMA or by the copying warps; its buffer is handed back as soon as it has been read.
+                        // The mask tile of this tile and step, brought in by TMA or by the copying warps; its buffer is handed
+                        // back as soon as it has been read.
                         mbar_wait(bar(BAR_MFULL0 + i), gm & 1u, ctl, kRoleSoftmax | (BAR_MFULL0 + i));
                         ++gm;
                         if constexpr (C::kMaskBoxes == 1) {   // the second box follows the first in the same place
@@ -2019,8 +2020,8 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         } else if ((kMask == kMaskTma || kPlanned) && warp == 15 && elect_one()) {
             // -------------------------------------------------------------- TMA producer of the mask tiles
             // Tile 0 and tile 1 of every key step in turn (where the step needs them; box by box where a buffer holds one
-            // box), each as soon as the softmax warps that had the buffer before have read it.  Boxes that lie beyond the end of the
-            // sequence (keys or rows) arrive as zeros.
+            // box), each as soon as the softmax warps that had the buffer before have read it.  Boxes that lie beyond the
+            // end of the sequence (keys or rows) arrive as zeros.
             uint32_t asked[2] = {0, 0};   // mask tiles (or boxes) asked for so far for tile i
             uint32_t before = 0;          // the tile that was asked for last
             bool stop = false;

@@ -182,8 +182,9 @@ __device__ __forceinline__ void plan_finite(const PlanArgs& a, const __half* x, 
     if (bits & 0x80008000u) a.bad[b * a.n + kt] = a.stamp;
 }
 
-// kCopy: the mask's rows start on no 16-byte boundary and are copied.  grid: at most the launch bound's CTAs per SM.  The tiles of the mask round-robin, then a run of the parts of K and V; the
-// CTA that is through last writes the lists, one group of 8, 16 or 32 lanes per pair of query tiles.
+// kCopy: the mask's rows start on no 16-byte boundary and are copied.  grid: at most the launch bound's CTAs per SM.  The
+// tiles of the mask round-robin, then a run of the parts of K and V; the CTA that is through last writes the lists, one
+// group of 8, 16 or 32 lanes per pair of query tiles.
 template <bool kCopy>
 __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPlanCtasPerSm) fa_mask_plan(const PlanArgs args) {
     __shared__ uint32_t hist[kPlanMaxTiles + 1], cost[2];
