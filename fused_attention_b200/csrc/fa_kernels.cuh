@@ -702,6 +702,7 @@ fa_fwd_simple(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ C
     }
     tc_fence_before();
     __syncthreads();
+    if (tid == 0) report_expired(ctl);
     if (warp == 0) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kTmemCols);
@@ -1353,6 +1354,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const bool runs = *p.plan_head != 0u;   // else the kernel launched behind this one takes the call
             const uint32_t mine = planned_count(p);
             uint32_t sum = 0;
+#pragma unroll 1
             for (uint32_t k = lane; k < mine; k += 32u) sum += planned_item(p, settled, k).len;
             sum = __reduce_add_sync(0xffffffffu, sum);
             if (lane == 0) plan_smem = runs ? Plan{mine, 0u, mine, sum, 0u, 0u, 0u, 0u} : Plan{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
@@ -1382,6 +1384,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         uint32_t g = 0;   // global step
         uint32_t gm = 0;  // mask tiles (or boxes) taken so far
         float m = -INFINITY, l = 0.f;
+#pragma unroll 1
         for (uint32_t k = 0; k < nseg; ++k) {
             const Seg sg = seg_of(t0, k);
             m = -INFINITY;
@@ -1390,6 +1393,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             uint32_t mask_sh = 0;
             if constexpr (kMask == kMaskCopied)
                 mask_sh = mask_row_shift(p, (sg.item / q_pairs) / p.R, ((sg.item % q_pairs) * 2u + i) * kTile + row);
+#pragma unroll 1
             for (uint32_t jj = 0; jj < sg.len; ++jj, ++g) {
                 const uint32_t step = step_of(sg, jj), j = step_tile(step);
                 mbar_wait(bar(BAR_S0 + i), g & 1u, ctl, kRoleSoftmax | (BAR_S0 + i));
@@ -1621,12 +1625,15 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         // Part of a divided item that is not the CTA's last segment: the rows go to this CTA's scratch
         // slot as they are (fp32, not normalised) together with (reference maximum, row sum), and the
         // warp counts itself in on the item's counter (see store_part, merge_parts).
+        // (Loops over tiles, halves and columns stay loops: this role is not in a hurry, and its code would push the other
+        // roles' out of the instruction cache.)
         setmaxnreg_dec<64>();
         const uint32_t row = tid & 127u;
         const uint32_t wq = warp & 3u;
         const uint32_t lane_off = (wq * 32u) << 16;
         const uint32_t stage = sStage + wq * C::kStageWarpBytes;
         uint32_t g_end = 0;   // global steps up to and including the current segment
+#pragma unroll 1
         for (uint32_t k = 0; k < nseg; ++k) {
             const Seg sg = seg_of(t0, k);
             // the softmax warps finish a final part themselves, and with kSoftmaxWritesLast a final whole item too
@@ -1634,7 +1641,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             g_end += sg.len;
             const uint32_t q_pair = sg.item % q_pairs, bh = sg.item / q_pairs;
             const uint32_t head = bh % p.R, batch = bh / p.R;
-#pragma unroll
+#pragma unroll 1
             for (uint32_t i = 0; i < 2; ++i) {
                 // this wait lasts for a whole segment: poll every 100 ns
                 mbar_wait_relaxed(bar(BAR_A0 + i), k & 1u, ctl, kRoleEpilogue | (BAR_A0 + i), 100);
@@ -1651,12 +1658,12 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     const float inv_l = 1.f / l_row;
                     constexpr int W = C::kStoreCols;   // columns of one staging buffer and store
                     constexpr uint32_t kRow = W * 2;
-#pragma unroll
+#pragma unroll 1
                     for (int half = 0; half < H / W; ++half) {
                         // the previous store out of this staging buffer must have read it completely
                         if (lane == 0) bulk_wait_read_all();
                         __syncwarp();
-#pragma unroll
+#pragma unroll 1
                         for (int c = 0; c < W / 16; ++c) {   // 16 columns at a time keeps this role within 64 registers
                             float o[16];
                             tmem_ld16(tO + half * W + c * 16, o);
@@ -1786,6 +1793,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     // softmax warps have read what the S buffer holds.  That K has landed is known long
                     // before; it is tested ahead of the previous step's last MMAs and the answer read
                     // after them (mbar_poll_begin).
+#pragma unroll 1
                     for (uint32_t q = 1; q < steps; ++q) {
                         bool new_seg = false;            // step q opens segment k
                         if (++j == len) { j = 0; ++k; len = seg_len_of(k); new_seg = true; }
@@ -1819,6 +1827,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     }
                 } else {
                     // P V stream: for every step the products of tile 0 and tile 1 as their P arrive.
+#pragma unroll 1
                     for (uint32_t g = 0; g < steps; ++g) {
                         const uint32_t tv = 2 * g + 1;
                         const uint32_t acc = j > 0 ? 1u : 0u;
@@ -1854,6 +1863,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 // (mbar_poll_begin); only the waits for P block.
                 mbar_poll_declare();
                 bool polled = false;   // predicates 0-2 hold answers for this step
+#pragma unroll 1
                 for (uint32_t g = 0; g < steps; ++g) {
                     const uint32_t tv = 2 * g + 1, tk = 2 * g + 2;
                     const bool more = g + 1 < steps;            // a next global step exists
@@ -1936,6 +1946,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             uint32_t k = 0;           // segment
             bool stop = false;
             uint32_t q_asked[2] = {0, 0};   // for how many segments query tile tt has been asked for
+#pragma unroll 1
             for (; k < nseg && !stop; ++k) {
                 const Seg sg = seg_of(t0, k);
 #ifdef FA_DEBUG
@@ -1948,6 +1959,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 const int32_t batch = static_cast<int32_t>(bh / p.R);
                 const int32_t q_row0 = static_cast<int32_t>(q_pair * 2u * kTile);
                 uint32_t key_tile = 0;
+#pragma unroll 1
                 for (uint32_t tt = 0; tt < 2 * sg.len; ++tt, ++t) {
                     if ((tt & 1u) == 0u) key_tile = step_tile(step_of(sg, tt >> 1));
                     const bool asked_already = !kPlanned && t == 0u;   // query tile 0 and K tile 0 of the first segment: see above
@@ -1979,6 +1991,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     }
                 }
                 // the query tiles asked for last (with two buffers, those of the last two segments)
+#pragma unroll 1
                 for (uint32_t tt = 0; tt < 2; ++tt) {
                     const uint32_t first_q = q_asked[tt] > static_cast<uint32_t>(C::kQBufs) ? q_asked[tt] - C::kQBufs : 0u;
                     for (uint32_t kk = first_q; kk < q_asked[tt]; ++kk) {
@@ -1996,9 +2009,11 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const MaskRows mr = mask_rows(p);
             uint32_t g = 0;
             bool stop = false;
+#pragma unroll 1
             for (uint32_t k = 0; k < nseg && !stop; ++k) {
                 const Seg sg = seg_of(t0, k);
                 const uint32_t batch = (sg.item / q_pairs) / p.R, q0 = (sg.item % q_pairs) * 2u * kTile;
+#pragma unroll 1
                 for (uint32_t jj = 0; jj < sg.len && !stop; ++jj, ++g) {
                     for (uint32_t i = 0; i < 2; ++i) {
                         bool ok = true;
@@ -2025,10 +2040,12 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             uint32_t asked[2] = {0, 0};   // mask tiles (or boxes) asked for so far for tile i
             uint32_t before = 0;          // the tile that was asked for last
             bool stop = false;
+#pragma unroll 1
             for (uint32_t k = 0; k < nseg && !stop; ++k) {
                 const Seg sg = seg_of(t0, k);
                 const int32_t batch = static_cast<int32_t>((sg.item / q_pairs) / p.R);
                 const int32_t q_row0 = static_cast<int32_t>((sg.item % q_pairs) * 2u * kTile);
+#pragma unroll 1
                 for (uint32_t jj = 0; jj < sg.len && !stop; ++jj) {
                     const uint32_t step = step_of(sg, jj);
                     const int32_t key0 = static_cast<int32_t>(step_tile(step) * kTile);
@@ -2072,6 +2089,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         p.cycles[4 * (p.launch_id & 63u) + 3] = static_cast<unsigned long long>(clock64() - cyc0);
     }
 #endif
+    if (tid == 0) report_expired(ctl);
     if (warp == 12) {
         tc_fence_after();
         tmem_dealloc(tmem_base, C::kTmemCols);
@@ -2093,6 +2111,7 @@ __global__ void fa_selftest_bounded_wait(uint32_t* status, uint32_t code, long l
     const WaitCtl ctl{status, &abort_flag, cap_cycles};
     const bool ok = mbar_wait(smem_u32(&bar_mem), 0, ctl, code);
     __syncthreads();
+    if (threadIdx.x == 0) report_expired(ctl);
     if (threadIdx.x == 0) *returned = ok ? 1u : 2u;  // 2 = gave up, as it must
 }
 
@@ -2125,6 +2144,7 @@ __global__ void fa_selftest_debug_checks(uint32_t* status) {
         bits |= dbg_copy_ok(0x4000, 4096, 0, 0, 2, false) ? 0u : 256u;           // batch entry outside the tensor
         bits |= dbg_tmem_ok(240u, 32u) ? 0u : 512u;                              // columns beyond the allocation
         bits |= dbg_tmem_ok((32u << 16) | 0u, 16u) ? 0u : 1024u;                 // another warp's lanes
+        report_expired(g_dbg.ctl);
         status[3] = bits;
     }
 }

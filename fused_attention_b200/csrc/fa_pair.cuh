@@ -193,8 +193,10 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
         const float c = p.scale_log2;
         uint32_t g = 0;   // global step
         float l_last = 1.f;
+#pragma unroll 1
         for (uint32_t k = 0; k < my_items; ++k) {
             float m = -INFINITY, l = 0.f;
+#pragma unroll 1
             for (uint32_t j = 0; j < n; ++j, ++g) {
                 // (time line, softmax warp of rows 0-31: 0 looks for S, 1 S there, 2 S in registers, 3 first 32
                 // exponentials taken, 4 P buffer free, 5 all exponentials taken and P stored, 6 P handed over)
@@ -322,10 +324,11 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
         const uint32_t stage = sStage + wq * 4096u;
         uint32_t k = 0;
         // (the CTA's last item is written by the softmax warps)
+#pragma unroll 1
         for (uint32_t item = cluster; k + 1u < my_items; item += n_clusters, ++k) {
             const uint32_t q_quad = item % q_quads, bh = item / q_quads;
             const uint32_t head = bh % p.R, batch = bh / p.R;
-#pragma unroll
+#pragma unroll 1
             for (uint32_t i = 0; i < 2; ++i) {
                 mbar_wait_relaxed(bar(BAR_A0 + i), k & 1u, ctl, kRoleEpilogue | (BAR_A0 + i), 100);
                 const float inv_l = 1.f / l_buf[k & 1u][i][row];
@@ -334,11 +337,11 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
                 __syncwarp();
                 const uint32_t tO = tmem_base + lane_off + (i ? C::kColO1 : C::kColO0);
                 const int32_t row0 = static_cast<int32_t>(((q_quad * 2u + rank) * 2u + i) * kTile + wq * 32u);
-#pragma unroll
+#pragma unroll 1
                 for (int half = 0; half < 2; ++half) {
                     if (lane == 0) bulk_wait_read_all();
                     __syncwarp();
-#pragma unroll
+#pragma unroll 1
                     for (int c = 0; c < 4; ++c) {
                         float o[16];
                         tmem_ld16(tO + half * 64 + c * 16, o);
@@ -398,6 +401,7 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
                 // Q K^T stream.  Uses of the one S buffer are numbered 2g + i; use u needs use u - 1 to have been read.
                 bool polled = false;
                 uint32_t k = 0, j = 0;
+#pragma unroll 1
                 for (uint32_t g = 0; g < steps; ++g) {
                     const bool new_item = j == 0;
                     const bool last_of_item = j + 1 == n;
@@ -439,6 +443,7 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
                 // P V stream
                 bool polled = false;
                 uint32_t k = 0, j = 0;
+#pragma unroll 1
                 for (uint32_t g = 0; g < steps; ++g) {
                     const uint32_t tv = 2 * g + 1;
                     const uint32_t acc = j > 0 ? 1u : 0u;
@@ -486,11 +491,13 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
             uint32_t t = 0, k = 0;
             bool stop = false;
             bool q_pending[2] = {false, false};
+#pragma unroll 1
             for (uint32_t item = cluster; item < n_items && !stop; item += n_clusters, ++k) {
                 const uint32_t q_quad = item % q_quads, bh = item / q_quads;
                 const int32_t col0 = static_cast<int32_t>((bh % p.R) * H);
                 const int32_t batch = static_cast<int32_t>(bh / p.R);
                 const int32_t q_row0 = static_cast<int32_t>((q_quad * 2u + rank) * 2u * kTile);
+#pragma unroll 1
                 for (uint32_t tt = 0; tt < 2 * n; ++tt, ++t) {
                     if (tt < 2) {
                         if (k > 0 && !mbar_wait(bar(BAR_QEMPTY0 + tt), (k - 1u) & 1u, ctl,
@@ -532,10 +539,12 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
             uint32_t g = 0;   // global step
             uint32_t asked[2] = {0, 0};   // for how many key steps tile i's mask tile has been asked for
             bool stop = false;
+#pragma unroll 1
             for (uint32_t item = cluster; item < n_items && !stop; item += n_clusters) {
                 const uint32_t q_quad = item % q_quads, bh = item / q_quads;
                 const int32_t batch = static_cast<int32_t>(bh / p.R);
                 const int32_t q_row0 = static_cast<int32_t>((q_quad * 2u + rank) * 2u * kTile);
+#pragma unroll 1
                 for (uint32_t j = 0; j < n && !stop; ++j, ++g) {
                     const int32_t key0 = static_cast<int32_t>(j * kTile);
                     for (uint32_t i = 0; i < 2; ++i) {
@@ -576,6 +585,7 @@ fa_fwd_pair(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUt
         p.cycles[4 * (p.launch_id & 63u) + 3] = static_cast<unsigned long long>(clock64() - cyc0);
     }
 #endif
+    if (tid == 0) report_expired(ctl);
     if (warp == 12) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, C::kTmemCols);
