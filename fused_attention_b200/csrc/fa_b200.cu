@@ -519,21 +519,22 @@ int launch_pair(DeviceCtx& c, const CUtensorMap& mq, const CUtensorMap& mkh, con
 // Where a plan lies in the scratch, and how much there is to look through.
 struct PlanLayout {
     uint32_t groups, pitch;   // pairs of query tiles of all batch entries; elements between rows of the mask's copy
-    size_t copy_bytes, order_at, bad_at, list_at, cls_at, bytes;
+    size_t copy_bytes, order_at, bad_at, list_at, cls_at, bytes;   // (the runs lie right behind the head's block)
     uint64_t jobs, tiles;     // parts of K and V; tiles of the mask
 };
-PlanLayout plan_layout(uint32_t B, uint32_t L, uint32_t F, bool mask_tma) {
+PlanLayout plan_layout(uint32_t B, uint32_t L, uint32_t F, bool mask_tma, bool with_runs) {
     auto up = [](size_t x) { return (x + 255u) & ~static_cast<size_t>(255u); };
     const uint32_t n = (L + fa::kTile - 1) / fa::kTile;
     PlanLayout l;
     l.groups = B * ((L + 2 * fa::kTile - 1) / (2 * fa::kTile));
     l.pitch = (L + 7u) & ~7u;
     l.copy_bytes = mask_tma ? 0 : up(static_cast<size_t>(B) * L * l.pitch * 2u);
-    l.order_at = l.copy_bytes + 256;
+    const size_t tiles = static_cast<size_t>(B) * n * n, runs = tiles * fa::kTile * sizeof(uint16_t);
+    l.order_at = l.copy_bytes + fa::kPlanHeadWords * sizeof(uint32_t) + (with_runs ? runs : 0);
     l.bad_at = l.order_at + up(l.groups * 4ull);
     l.list_at = l.bad_at + up(static_cast<size_t>(B) * n * 4u);
     l.cls_at = l.list_at + up(static_cast<size_t>(l.groups) * n * 2u);
-    l.bytes = l.cls_at + up(static_cast<size_t>(B) * n * n);
+    l.bytes = l.cls_at + up(tiles);
     l.jobs = static_cast<uint64_t>(B) * n * 2u * ((F + fa::kPlanCols - 1u) / fa::kPlanCols);
     l.tiles = static_cast<uint64_t>(B) * n * n;
     return l;
@@ -543,7 +544,7 @@ PlanLayout plan_layout(uint32_t B, uint32_t L, uint32_t F, bool mask_tma) {
 bool plan_fits(uint32_t B, uint32_t L, uint32_t F, bool mask_tma, uint32_t sms) {
     const uint64_t q_pairs = (L + 2 * fa::kTile - 1) / (2 * fa::kTile);
     if ((L + fa::kTile - 1) / fa::kTile > fa::kPlanMaxTiles || B * q_pairs > fa::kPlanMaxGroups) return false;
-    const PlanLayout l = plan_layout(B, L, F, mask_tma);
+    const PlanLayout l = plan_layout(B, L, F, mask_tma, false);
     return l.bytes <= split_o_bytes(static_cast<int>(sms)) && l.jobs <= 0x7FFFFFFFull;
 }
 
@@ -573,7 +574,9 @@ bool use_mask_plan(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool mask_tma
 // elements apart.
 int plan_mask(DeviceCtx& c, const SplitScratch& scratch, const void* k, const void* v, bool mask_tma,
               Params& p, cudaStream_t st, bool overlap, const void** mask_rows, uint32_t* mask_pitch) {
-    const PlanLayout l = plan_layout(p.B, p.L, p.F, mask_tma);
+    // (without the runs where there is no room for them: rows that are runs are then mask tiles like any other)
+    const bool with_runs = plan_layout(p.B, p.L, p.F, mask_tma, true).bytes <= split_o_bytes(c.sm_count);
+    const PlanLayout l = plan_layout(p.B, p.L, p.F, mask_tma, with_runs);
     char* base = reinterpret_cast<char*>(scratch.o);
     fa::PlanArgs a;
     a.mask = p.mask;
@@ -582,6 +585,7 @@ int plan_mask(DeviceCtx& c, const SplitScratch& scratch, const void* k, const vo
     a.copy = mask_tma ? nullptr : reinterpret_cast<__half*>(base);
     a.head = reinterpret_cast<uint32_t*>(base + l.copy_bytes);
     a.ticket = scratch.ticket;
+    a.runs = with_runs ? reinterpret_cast<uint16_t*>(a.head + fa::kPlanHeadWords) : nullptr;
     a.order = reinterpret_cast<uint32_t*>(base + l.order_at);
     a.bad = reinterpret_cast<uint32_t*>(base + l.bad_at);
     a.list = reinterpret_cast<uint16_t*>(base + l.list_at);
@@ -593,7 +597,7 @@ int plan_mask(DeviceCtx& c, const SplitScratch& scratch, const void* k, const vo
     a.q_pairs = p.q_pairs;
     a.copy_pitch = l.pitch;
     a.stamp = p.launch_id;
-    a.dense_allowed = mask_tma ? 1u : 0u;
+    a.dense_allowed = a.items_check = mask_tma ? 1u : 0u;
     const uint64_t most = static_cast<uint64_t>(mask_tma ? fa::kPlanCtasPerSm : fa::kPlanCopyCtasPerSm) * c.sm_count;
     const uint64_t wide = l.tiles > l.jobs ? l.tiles : l.jobs;
     cudaError_t e = launch_kernel(mask_tma ? fa::fa_mask_plan<false> : fa::fa_mask_plan<true>,

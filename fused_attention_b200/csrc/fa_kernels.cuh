@@ -538,6 +538,25 @@ __device__ __forceinline__ void add_mask_tile_row_shifted(float (&s)[kTile], uin
     }
 }
 
+// The same for a row that is zero from key `first` up to key `last` (not included) and -inf elsewhere.  (Added, not put in
+// the scores' place: a score that is NaN or +inf has to give NaN.)
+__device__ __forceinline__ void add_mask_run(float (&s)[kTile], uint32_t first, uint32_t last) {
+#pragma unroll
+    for (uint32_t w = 0; w < kTile / 32u; ++w) {
+        const uint32_t lo = first > w * 32u ? min(first - w * 32u, 32u) : 0u, hi = last > w * 32u ? min(last - w * 32u, 32u) : 0u;
+        const uint32_t in = (hi == 32u ? 0xFFFFFFFFu : (1u << hi) - 1u) & ~(lo == 32u ? 0xFFFFFFFFu : (1u << lo) - 1u);
+#pragma unroll
+        for (uint32_t e = 0; e < 32u; ++e)
+            if (!(in & (1u << e))) s[w * 32u + e] += -INFINITY;
+    }
+}
+
+// Eight fp16 values: is the sign's place of one set where its exponent is all ones (which carries into it)?
+__device__ __forceinline__ uint32_t nonfinite_bits(const uint4& w) {
+    return ((w.x & 0x7C007C00u) + 0x04000400u) | ((w.y & 0x7C007C00u) + 0x04000400u) | ((w.z & 0x7C007C00u) + 0x04000400u) |
+           ((w.w & 0x7C007C00u) + 0x04000400u);
+}
+
 // What every mask row start of a call is aligned to: rows are L fp16 values apart from the base address.
 __device__ __forceinline__ uint32_t mask_row_alignment(const Params& p) {
     const uint32_t bits = (p.L * 2u) | static_cast<uint32_t>(reinterpret_cast<uintptr_t>(p.mask));
@@ -733,7 +752,12 @@ enum : int { kNoMask = 0, kMaskTma = 1, kMaskCopied = 2, kMaskPlanned = 3 };
 constexpr uint32_t kPlanLenShift = 20;
 // an entry of a list: key tile, and what the mask is there for query tile 0 and 1 of the pair
 constexpr uint32_t kStepShift0 = 12, kStepShift1 = 14;
-constexpr uint32_t kStepNoMask = 0, kStepMask = 1, kStepAllNeg = 2;   // zero; a tile of its own; -inf throughout
+constexpr uint32_t kStepNoMask = 0, kStepMask = 1, kStepAllNeg = 2;   // zero; a tile of its own; -inf throughout;
+constexpr uint32_t kStepRows = 3;   // every row a run of zeros with -inf around it: the runs' ends stand behind plan_head
+constexpr uint32_t kStepCheck = 1u << 11;   // this item looks through the key tile's K and V, see fa_mask_plan.cuh
+// plan_head's block: word 0, then from kPlanInputs on the addresses of K and V; the runs of kStepRows stand behind it, 128
+// per tile of the mask ({first zero, key behind the last} in a byte each).
+constexpr uint32_t kPlanInputs = 2, kPlanHeadWords = 64;
 
 template <int H, int kMask = kNoMask>
 struct PipeCfg {
@@ -897,14 +921,19 @@ __device__ __forceinline__ uint32_t planned_count(const Params& p) {
     const uint32_t full = p.n_items / gridDim.x, rest = p.n_items % gridDim.x;
     return full + (((full & 1u) ? gridDim.x - 1u - blockIdx.x : blockIdx.x) < rest ? 1u : 0u);
 }
-__device__ __forceinline__ Planned planned_item(const Params& p, uint32_t zero, uint32_t k) {   // zero: zero_behind_the_wait()
-    const uint32_t idx = k * gridDim.x + ((k & 1u) ? gridDim.x - 1u - blockIdx.x : blockIdx.x);
-    if (idx >= p.n_items) return Planned{0u, 0u, 0u};
-    const uint32_t o = ld_settled(p.plan_order + idx / p.R + zero);
-    return Planned{o & ((1u << kPlanLenShift) - 1u), idx % p.R, o >> kPlanLenShift};
+__device__ __forceinline__ uint32_t planned_index(uint32_t k) {
+    return k * gridDim.x + ((k & 1u) ? gridDim.x - 1u - blockIdx.x : blockIdx.x);
 }
-__device__ __forceinline__ Seg planned_seg(const Params& p, uint32_t zero, uint32_t k) {
-    const Planned it = planned_item(p, zero, k);
+// The word of Params::plan_order of this CTA's segment k, 0 if there is none.  It comes from L2: a role asks for it a segment
+// ahead of its use.
+__device__ __forceinline__ uint32_t planned_order(const Params& p, uint32_t zero, uint32_t k) {   // zero: zero_behind_the_wait()
+    const uint32_t idx = planned_index(k);
+    return idx < p.n_items ? ld_settled(p.plan_order + idx / p.R + zero) : 0u;
+}
+__device__ __forceinline__ uint32_t planned_len(uint32_t order) { return order >> kPlanLenShift; }
+__device__ __forceinline__ uint32_t planned_pair(uint32_t order) { return order & ((1u << kPlanLenShift) - 1u); }
+__device__ __forceinline__ Seg planned_seg(const Params& p, uint32_t order, uint32_t k) {
+    const Planned it{planned_pair(order), planned_index(k) % p.R, planned_len(order)};
     Seg s;
     s.item = (it.pair / p.q_pairs * p.R + it.head) * p.q_pairs + it.pair % p.q_pairs;
     s.j0 = 0;
@@ -912,6 +941,31 @@ __device__ __forceinline__ Seg planned_seg(const Params& p, uint32_t zero, uint3
     s.partial = false;
     s.list = it.pair * p.n_kv_tiles;
     return s;
+}
+
+// The K (x = 0) or V (x = 1) that the plan's block names.
+__device__ __forceinline__ const __half* plan_input(const uint32_t* head, uint32_t x) {
+    const uint64_t at = *reinterpret_cast<const volatile uint64_t*>(head + kPlanInputs + 2u * x);
+    return reinterpret_cast<const __half*>(at);
+}
+// Are all values of a key tile of one head finite?  128 threads: a thread looks at eight columns of every 128 / (H / 8)-th
+// row from its `r` on.
+template <int H>
+__device__ __forceinline__ bool rows_finite(const __half* src, uint32_t r, uint32_t L, uint32_t F) {
+    constexpr uint32_t kRowsApart = kTile / (H / 8), kRows = H / 8, kAtOnce = kRows < 4u ? kRows : 4u;
+    uint32_t bits = 0;
+#pragma unroll 1
+    for (uint32_t u0 = 0; u0 < kRows; u0 += kAtOnce) {
+        uint4 w[kAtOnce];
+#pragma unroll
+        for (uint32_t u = 0; u < kAtOnce; ++u) {
+            const uint32_t at = r + (u0 + u) * kRowsApart;
+            w[u] = at < L ? ld_settled(reinterpret_cast<const uint4*>(src + static_cast<size_t>(at) * F)) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (uint32_t u = 0; u < kAtOnce; ++u) bits |= nonfinite_bits(w[u]);
+    }
+    return (bits & 0x80008000u) == 0u;
 }
 
 // The CTA whose tail range holds tail key step `step` (ranges are [c*T/tg, (c+1)*T/tg)).
@@ -1226,7 +1280,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     volatile Plan& pl_s = plan_smem;
     uint32_t settled = 0;   // for what is read behind the wait for the previous kernel, see zero_behind_the_wait()
     auto seg_of = [&](uint32_t t_first, uint32_t k) {
-        if constexpr (kPlanned) return planned_seg(p, settled, k);
+        if constexpr (kPlanned) return planned_seg(p, planned_order(p, settled, k), k);
         else return get_seg(pl_s, t_first, p, k);
     };
     // key tile of step jj of a segment (with what the mask is there, if it is planned)
@@ -1234,7 +1288,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         if constexpr (kPlanned) return ld_settled(p.plan_list + sg.list + jj + settled);
         else return sg.j0 + jj;
     };
-    auto step_tile = [](uint32_t e) -> uint32_t { return kPlanned ? e & ((1u << kStepShift0) - 1u) : e; };
+    auto step_tile = [](uint32_t e) -> uint32_t { return kPlanned ? e & (kStepCheck - 1u) : e; };
     // what the mask is at a step for query tile i
     auto step_mask = [](uint32_t e, uint32_t i) -> uint32_t {
         return kPlanned ? (e >> (i ? kStepShift1 : kStepShift0)) & 3u : (kHasMask ? kStepMask : kStepNoMask);
@@ -1355,7 +1409,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const uint32_t mine = planned_count(p);
             uint32_t sum = 0;
 #pragma unroll 1
-            for (uint32_t k = lane; k < mine; k += 32u) sum += planned_item(p, settled, k).len;
+            for (uint32_t k = lane; k < mine; k += 32u) sum += planned_len(planned_order(p, settled, k));
             sum = __reduce_add_sync(0xffffffffu, sum);
             if (lane == 0) plan_smem = runs ? Plan{mine, 0u, mine, sum, 0u, 0u, 0u, 0u} : Plan{0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
         }
@@ -1384,9 +1438,29 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
         uint32_t g = 0;   // global step
         uint32_t gm = 0;  // mask tiles (or boxes) taken so far
         float m = -INFINITY, l = 0.f;
+        // kMaskPlanned: what comes next is asked for ahead of its use (it comes from L2): the next segment's order at a
+        // segment's first step, a step's entry a step ahead, the run of this thread's row in the middle of the step before.
+        uint32_t order = 0, order_next = 0, entry = 0, run = 0;
+        auto runs_of = [&](uint32_t ord) {   // of this thread's row, kTile values apart from key tile to key tile
+            const uint32_t pair = planned_pair(ord), tile0 = (pair / q_pairs * p.n_kv_tiles + pair % q_pairs * 2u + i) * p.n_kv_tiles;
+            return reinterpret_cast<const uint16_t*>(p.plan_head + kPlanHeadWords) + static_cast<size_t>(tile0) * kTile + row + settled;
+        };
+        if constexpr (kPlanned) {
+            if (nseg > 0u) {
+                order = planned_order(p, settled, 0);
+                entry = ld_settled(p.plan_list + planned_pair(order) * p.n_kv_tiles + settled);
+                if (step_mask(entry, i) == kStepRows) run = ld_settled(runs_of(order) + step_tile(entry) * kTile);
+            }
+        }
 #pragma unroll 1
         for (uint32_t k = 0; k < nseg; ++k) {
-            const Seg sg = seg_of(t0, k);
+            Seg sg;
+            if constexpr (kPlanned) {
+                sg = planned_seg(p, order, k);
+                order_next = planned_order(p, settled, k + 1u);
+            } else {
+                sg = seg_of(t0, k);
+            }
             m = -INFINITY;
             l = 0.f;
             // how far into its first word this thread's mask row starts
@@ -1395,7 +1469,11 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 mask_sh = mask_row_shift(p, (sg.item / q_pairs) / p.R, ((sg.item % q_pairs) * 2u + i) * kTile + row);
 #pragma unroll 1
             for (uint32_t jj = 0; jj < sg.len; ++jj, ++g) {
-                const uint32_t step = step_of(sg, jj), j = step_tile(step);
+                const uint32_t step = kPlanned ? entry : step_of(sg, jj), j = step_tile(step);
+                const bool more = jj + 1u < sg.len || order_next != 0u;   // (kMaskPlanned: a step follows)
+                if constexpr (kPlanned) {
+                    if (more) entry = ld_settled(p.plan_list + settled + (jj + 1u < sg.len ? sg.list + jj + 1u : planned_pair(order_next) * p.n_kv_tiles));
+                }
                 mbar_wait(bar(BAR_S0 + i), g & 1u, ctl, kRoleSoftmax | (BAR_S0 + i));
                 tc_fence_after();
                 __syncwarp();
@@ -1441,6 +1519,8 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     } else if (what == kStepAllNeg) {
 #pragma unroll
                         for (int e = 0; e < kTile; ++e) s[e] += -INFINITY;
+                    } else if (kPlanned && what == kStepRows) {
+                        add_mask_run(s, run & 0xFFu, run >> 8);
                     }
                 }
                 if (ragged) mask_tail(s, static_cast<int>(p.L - j * kTile));
@@ -1464,6 +1544,10 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     }
 #pragma unroll
                     for (int ch = 0; ch < C::kHeldChunks; ++ch) tmem_st16(tP + ch * 16, held + ch * 16);
+                    if constexpr (kPlanned) {
+                        if (more && step_mask(entry, i) == kStepRows)
+                            run = ld_settled(runs_of(jj + 1u < sg.len ? order : order_next) + step_tile(entry) * kTile);
+                    }
                     sum += exp_chunks<C::kHeldChunks, 4, false>(s, c, nmc, tP, mx4);
                     // The reference has to move when a score exceeds it by more than 2^8 in the exp2 domain, that is
                     // when a P exceeds 2^8.  No P can while the row's sum of P stays below 2^8, so the row maximum is
@@ -1509,6 +1593,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                 __syncwarp();
                 if (lane == 0) mbar_arrive(bar(BAR_P0 + i));
             }
+            if constexpr (kPlanned) order = order_next;
             // Hand the row sums (and the references they are relative to) to the epilogue.  The A
             // barrier may run at most one phase ahead of the epilogue's wait, so the previous segment's
             // O must have been read out first (always true already when a segment has two or more
@@ -1636,6 +1721,23 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll 1
         for (uint32_t k = 0; k < nseg; ++k) {
             const Seg sg = seg_of(t0, k);
+            if constexpr (kPlanned) {
+                // Key tiles whose K and V this item looks through (these warps have nothing else to do until its end): other
+                // items leave them out, which is only right while they are finite.  If not, the kernel behind takes the call.
+                const uint32_t bh = sg.item / q_pairs, piece = row % (H / 8);
+                const size_t at = static_cast<size_t>(bh / p.R) * p.L * p.F + (bh % p.R) * H + piece * 8u;
+                bool finite = true;
+#pragma unroll 1
+                for (uint32_t jj = 0; jj < sg.len; ++jj) {
+                    const uint32_t step = step_of(sg, jj);
+                    if (!(step & kStepCheck)) continue;
+                    const uint32_t first_row = step_tile(step) * kTile + row / (H / 8);
+#pragma unroll 1
+                    for (uint32_t x = 0; x < 2; ++x)
+                        finite &= rows_finite<H>(plan_input(p.plan_head, x) + at, first_row, p.L, p.F);
+                }
+                if (!finite) *const_cast<uint32_t*>(p.plan_head) = 0;
+            }
             // the softmax warps finish a final part themselves, and with kSoftmaxWritesLast a final whole item too
             if (k + 1u == nseg && (sg.partial || C::kSoftmaxWritesLast)) break;
             g_end += sg.len;
@@ -1759,11 +1861,18 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
             const uint32_t steps = pl.steps;   // global steps of this CTA
             // ring item 2g is the K tile of global step g, item 2g+1 its V tile
             // (k, j, len): segment of the step a loop is working on, its position in it, its length
-            auto seg_len_of = [&](uint32_t kk) {
-                if constexpr (kPlanned) return planned_item(p, settled, kk).len;
+            // (a planned item's length is asked for a segment ahead)
+            uint32_t ahead = kPlanned ? planned_order(p, settled, 1u) : 0u;
+            auto next_seg_len = [&](uint32_t kk) {   // of the segment kk behind the one a loop is working on
+                if constexpr (kPlanned) return planned_len(ahead);
                 else return seg_len(pl, p, kk);
             };
-            uint32_t k = 0, j = 0, len = seg_len_of(0);
+            auto enter_seg = [&](uint32_t kk) {
+                const uint32_t l = next_seg_len(kk);
+                if constexpr (kPlanned) ahead = planned_order(p, settled, kk + 1u);
+                return l;
+            };
+            uint32_t k = 0, j = 0, len = kPlanned ? planned_len(planned_order(p, settled, 0u)) : seg_len(pl, p, 0);
             if (steps > 0 && warp == 12) {
                 // S tiles of the very first step
                 mwait(bar_qfull(0, 0), 0, code_qfull(0, 0));
@@ -1796,7 +1905,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 #pragma unroll 1
                     for (uint32_t q = 1; q < steps; ++q) {
                         bool new_seg = false;            // step q opens segment k
-                        if (++j == len) { j = 0; ++k; len = seg_len_of(k); new_seg = true; }
+                        if (++j == len) { j = 0; ++k; len = enter_seg(k); new_seg = true; }
                         const bool last_of_seg = j + 1 == len;   // a segment's last Q K^T is its last use of the query tile
                         const uint32_t tk = 2 * q;
                         if (!(polled && mbar_poll_end<0>())) wait_full(tk);
@@ -1852,7 +1961,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                             tc_commit(bar(BAR_PV1));
                             free_slot(tv);
                         }
-                        if (++j == len) { j = 0; ++k; len = seg_len_of(k); }
+                        if (++j == len) { j = 0; ++k; len = enter_seg(k); }
                     }
                 }
             } else {
@@ -1869,7 +1978,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                     const bool more = g + 1 < steps;            // a next global step exists
                     const bool next_new_seg = j + 1 == len;     // ... and it opens segment k + 1
                     // is the next step the last of its segment (its Q K^T the last use of the query tile)?
-                    const bool next_last_of_seg = next_new_seg ? seg_len_of(k + 1u) == 1u : j + 2 == len;
+                    const bool next_last_of_seg = next_new_seg ? next_seg_len(k + 1u) == 1u : j + 2 == len;
                     const uint32_t acc = j > 0 ? 1u : 0u;
                     const uint32_t kn = next_new_seg ? k + 1u : k;   // the segment of the next step
                     {
@@ -1931,7 +2040,7 @@ fa_fwd_pipelined(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
                         tc_commit(bar(BAR_PV1));
                         free_slot(tv);
                     }
-                    if (++j == len) { j = 0; ++k; len = seg_len_of(k); }
+                    if (++j == len) { j = 0; ++k; len = enter_seg(k); }
                 }
             }
             // Every MMA this warp issued has to retire before the CTA releases tensor memory and shared

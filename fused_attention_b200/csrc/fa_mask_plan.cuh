@@ -2,13 +2,15 @@
 // kMaskPlanned).  The mask is shared by the heads, so one pass over it saves every head's pass over
 //   - key tiles (128 keys) that the mask takes away from all 256 query rows of a work item: half of a causal mask,
 //     the padding of a batch.  They are left out: P would be 0 there, so neither l nor O changes;
-//   - the mask tiles that are zero throughout (nothing is added) or -inf throughout (no tile is fetched).
+//   - the mask tiles that are zero throughout (nothing is added) or -inf throughout (no tile is fetched), and those whose
+//     every row is a run of zeros between -inf, of which only the runs' ends are passed on.
 // A mask whose rows TMA cannot fetch (row starts on no 16-byte boundary) is copied on the way, the tiles that are
 // neither, into rows that it can.
 //
 // Leaving a key tile out is only the same as adding -inf while its K and V are finite: 0 * inf and inf - inf are
-// NaN.  So the K and V rows of every key tile that might be left out for some query tile are looked through as well,
-// and a tile with an infinity or a NaN in it is not left out.  (Q need not be looked at: a row of Q with an infinity
+// NaN.  So the K and V rows of every key tile that might be left out for some query tile are looked through as well (by
+// the plan, or by items of the planned kernel, see plan_looks_through), and a tile with an infinity or a NaN in it is not
+// left out.  (Q need not be looked at: a row of Q with an infinity
 // or a NaN has no finite score, so its result is NaN whatever is left out.)
 #pragma once
 
@@ -21,17 +23,19 @@ struct PlanArgs {
     const __half* k;       // [B, L, F]
     const __half* v;
     __half* copy;          // [B, L, copy_pitch] or nullptr: rows that start on 16-byte boundaries
-    uint8_t* cls;          // [B][n][n] (query tile, key tile): kTileNeg, kTileZero or kTileMixed
-    uint32_t* head;        // {1 = the planned kernel runs, 0 = the one behind it}
+    uint8_t* cls;          // [B][n][n] (query tile, key tile): kTileNeg, kTileZero, kTileMixed or kTileRows
+    uint16_t* runs;        // [B][n][n][128] for a kTileRows tile: first zero | key behind the last << 8; or nullptr
+    uint32_t* head;        // {1 = the planned kernel runs, 0 = the one behind it}, see kPlanInputs
     uint32_t* ticket;      // CTAs that are through; zero between launches
     uint32_t* bad;         // [B][n]: `stamp` if the key tile's K or V is not finite throughout
     uint32_t* order;       // [B * q_pairs]: (query pair of a batch entry) | key steps << kPlanLenShift, longest first
     uint16_t* list;        // [B * q_pairs][n]: key steps, see kStepShift0
     uint32_t B, L, F, n, q_pairs, copy_pitch;
     uint32_t stamp;           // of this call alone (a leftover that equals it costs a step, no more)
-    uint32_t dense_allowed;   // a kernel without a plan stands ready for a mask that leaves little out
+    uint32_t dense_allowed;   // a kernel without a plan stands ready for a mask that leaves little out,
+    uint32_t items_check;     // and for K and V that items of the planned kernel find not to be finite
 };
-constexpr uint8_t kTileNeg = 0, kTileZero = 1, kTileMixed = 2;
+constexpr uint8_t kTileNeg = 0, kTileZero = 1, kTileMixed = 2, kTileRows = 3;
 constexpr uint32_t kPlanThreads = 256;
 // CTAs per SM, 32 KB of loads in flight each; the instance that copies keeps a tile in registers, which fewer leave room for
 // (B=4 R=12 L=1021 H=64, the whole call: 40.5 us with four, 39.2 with three, 40.8 with two).
@@ -40,127 +44,169 @@ constexpr uint32_t kPlanCols = 128;         // columns of K or V that are looked
 constexpr uint32_t kPlanMaxTiles = 256;     // key tiles per sequence,
 constexpr uint32_t kPlanMaxGroups = 1024;   // and pairs of query tiles of all batch entries that the lists are built for
 
-// One 128 x 128 tile of the mask: its class, and its copy.
+// A row whose zeros follow one another and whose other keys are -inf is kept as its run: first zero | key behind the last
+// << 8 (0: no zero).
+constexpr uint32_t kWholeRun = kTile << 8;
+
+// A tile is brought into shared memory with asynchronous copies and looked at there, in loops: a CTA of this kernel meets
+// all of its code for the first time, and its length counts.  (Rows in registers and everything written out over them were
+// 118 KB of code; a tile on the diagonal of B=4 R=12 L=1021 H=64 took 15 us.)
+// Measured, the call: B=4 R=32 L=2048 H=128 causal 232 us with mask tiles on the diagonal and K and V looked through here,
+// 206 with runs and K and V looked through by the items; this kernel alone, cold, 36 and 24.
+// Words of a staged row.  Rows on 16-byte boundaries: 64.  Others in whole aligned words, where word j of a row that starts
+// in the middle of one holds its keys 2 j - 1 and 2 j: 65 (and one so that rows lie an even number of banks apart).
+constexpr uint32_t kPlanRowWords = 66;
+
+// A warp's 16 rows of a 128 x 128 tile of the mask.
+struct PlanRows {
+    uint64_t first, pitch;   // the first of them, and from row to row, in bytes
+    uint32_t b, row0, key0, rows, keys;
+    bool words;   // whole words are only copied where all of them lie inside the mask: not in its first and last rows if it
+                  // begins or ends in the middle of one, which are put into place value by value
+    // how far into its first word a row starts
+    __device__ __forceinline__ uint32_t shift(uint32_t r) const { return words ? static_cast<uint32_t>((first + r * pitch) >> 1) & 1u : 0u; }
+};
+__device__ __forceinline__ PlanRows plan_rows(const PlanArgs& a, uint32_t tile) {
+    const uint32_t kt = tile % a.n, qt = (tile / a.n) % a.n;
+    PlanRows t;
+    t.b = tile / (a.n * a.n);
+    t.row0 = qt * kTile + (threadIdx.x >> 5) * 16u, t.key0 = kt * kTile;
+    t.rows = t.row0 < a.L ? min(16u, a.L - t.row0) : 0u;
+    t.keys = min(kTile + 0u, a.L - t.key0);
+    t.first = reinterpret_cast<uint64_t>(a.mask) + 2ull * ((static_cast<uint64_t>(t.b) * a.L + t.row0) * a.L + t.key0);
+    t.pitch = 2ull * a.L;
+    const uint64_t mask0 = reinterpret_cast<uint64_t>(a.mask);
+    t.words = (t.first & ~3ull) >= mask0 &&
+              ((t.first + (t.rows ? t.rows - 1u : 0u) * t.pitch + 2u * t.keys + 3u) & ~3ull) <= mask0 + 2ull * a.B * a.L * a.L;
+    return t;
+}
+
+// Asks for a tile.  `staged`: this warp's rows.
 template <bool kCopy>
-__device__ __forceinline__ void plan_mask_tile(const PlanArgs& a, uint32_t tile) {
-    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
-    const uint32_t kt = tile % a.n, qt = (tile / a.n) % a.n, b = tile / (a.n * a.n);
-    const uint32_t row0 = qt * kTile + warp * 16u, key0 = kt * kTile;
-    const uint16_t* base = reinterpret_cast<const uint16_t*>(a.mask) + (static_cast<size_t>(b) * a.L + row0) * a.L + key0;
-    const uint32_t rows = row0 < a.L ? min(16u, a.L - row0) : 0u;   // of this warp
-    const uint32_t keys = min(kTile + 0u, a.L - key0);
-    uint32_t not_neg = 0, not_zero = 0;
-    // Rows on no 16-byte boundary: this warp's 16 rows in whole words where all of them, and a word more, lie inside the
-    // mask (B=4 R=12 L=1021 H=64, the whole call 46 us with values one by one, 39 with words), else value by value.
-    const uint64_t mask0 = reinterpret_cast<uint64_t>(a.mask), first = reinterpret_cast<uint64_t>(base), pitch = 2ull * a.L;
-    const bool words = (first & ~3ull) >= mask0 && first + 15u * pitch + 260u <= mask0 + 2ull * a.B * a.L * a.L;
-    uint32_t w[16][2], extra = 0;
-    auto two_keys = [&](uint32_t r, uint32_t col) -> uint32_t {
-        const uint16_t* at = base + static_cast<size_t>(r) * a.L + col;
-        const uint32_t lo = r < rows && col < keys ? ld_settled(at) : 0u;
-        const uint32_t hi = r < rows && col + 1u < keys ? ld_settled(at + 1) : 0u;
-        return lo | (hi << 16);
-    };
-    // (four rows in flight together: one after the other, such a warp's way is what the whole plan waits for)
-    auto four_rows = [&](uint32_t r0, uint32_t (&v)[4][2]) {
-#pragma unroll
-        for (uint32_t u = 0; u < 4; ++u)
-#pragma unroll
-            for (uint32_t h = 0; h < 2; ++h) v[u][h] = two_keys(r0 + u, h * 64u + lane * 2u);
-    };
-    if constexpr (!kCopy) {   // rows on 16-byte boundaries: two rows a load, eight keys a lane (L is a multiple of 8)
-        const uint32_t col = (lane & 15u) * 8u;
-        uint4 x[8];
-#pragma unroll
-        for (uint32_t i = 0; i < 8; ++i) {
-            const uint32_t r = 2u * i + (lane >> 4);
-            if (r < rows && col < keys) x[i] = ld_settled(reinterpret_cast<const uint4*>(base + static_cast<size_t>(r) * a.L + col));
+__device__ __forceinline__ void plan_fetch_tile(const PlanRows& t, uint32_t* staged) {
+    const uint32_t lane = threadIdx.x & 31u;
+    if constexpr (!kCopy) {   // two rows a copy, eight keys a lane (L is a multiple of 8)
+        const uint32_t piece = lane & 15u;
+        const bool in = piece * 8u < t.keys;
+#pragma unroll 2
+        for (uint32_t r = lane >> 4; r < t.rows; r += 2u)
+            cp_async_16_zero(smem_u32(staged + r * 64u + piece * 4u), reinterpret_cast<const void*>(t.first + r * t.pitch + (in ? piece * 16u : 0u)), in);
+    } else if (t.words) {
+#pragma unroll 2
+        for (uint32_t r = 0; r < t.rows; ++r) {   // (behind the word with the row's last key that one again, instead of what lies behind)
+            const uint64_t row = (t.first + r * t.pitch) & ~3ull;
+            const uint32_t last = (t.keys + t.shift(r) - 1u) >> 1, at = smem_u32(staged + r * kPlanRowWords + lane);
+            cp_async_4(at, row + 4u * min(lane, last));
+            cp_async_4(at + 128u, row + 4u * min(32u + lane, last));
+            if (lane == 0) cp_async_4(at + 256u, row + 4u * min(64u, last));
         }
-#pragma unroll
-        for (uint32_t i = 0; i < 8; ++i) {
-            const uint32_t r = 2u * i + (lane >> 4);
-            if (r < rows && col < keys) {
-                not_neg |= (x[i].x ^ 0xFC00FC00u) | (x[i].y ^ 0xFC00FC00u) | (x[i].z ^ 0xFC00FC00u) | (x[i].w ^ 0xFC00FC00u);
-                not_zero |= (x[i].x | x[i].y | x[i].z | x[i].w) & 0x7FFF7FFFu;
-            }
-        }
-    } else if (words) {
-        // Whole aligned words: word j of a row that starts in the middle of one holds its keys 2 j - 1 and 2 j.
-#pragma unroll
-        for (uint32_t r = 0; r < 16; ++r)
-#pragma unroll
-            for (uint32_t h = 0; h < 2; ++h)
-                w[r][h] = ld_settled(reinterpret_cast<const uint32_t*>((first + r * pitch) & ~3ull) + h * 32u + lane);
-        extra = ld_settled(reinterpret_cast<const uint32_t*>((first + (lane & 15u) * pitch) & ~3ull) + 64);   // of row `lane`
-#pragma unroll
-        for (uint32_t r = 0; r < 16; ++r) {
-            const uint32_t sh = static_cast<uint32_t>((first + r * pitch) >> 1) & 1u;
+    } else {
+#pragma unroll 4
+        for (uint32_t r = 0; r < t.rows; ++r) {
+            const uint16_t* row = reinterpret_cast<const uint16_t*>(t.first + r * t.pitch);
 #pragma unroll
             for (uint32_t h = 0; h < 2; ++h) {
-                const uint32_t lo = (h * 32u + lane) * 2u - sh;   // key of the low half (wraps below 0)
-                const uint32_t valid = r < rows ? (lo < keys ? 0xFFFFu : 0u) | (lo + 1u < keys ? 0xFFFF0000u : 0u) : 0u;
-                not_neg |= (w[r][h] ^ 0xFC00FC00u) & valid;
-                not_zero |= w[r][h] & 0x7FFF7FFFu & valid;
-            }
-        }
-        const uint32_t valid = lane < rows && ((first + lane * pitch) & 2u) != 0u && keys == kTile ? 0xFFFFu : 0u;   // key 127
-        not_neg |= (extra ^ 0xFC00FC00u) & valid;
-        not_zero |= extra & 0x7FFF7FFFu & valid;
-    } else {
-#pragma unroll 1
-        for (uint32_t r0 = 0; r0 < rows; r0 += 4u) {
-            uint32_t v[4][2];
-            four_rows(r0, v);
-#pragma unroll
-            for (uint32_t u = 0; u < 4; ++u)
-#pragma unroll
-                for (uint32_t h = 0; h < 2; ++h) {
-                    const uint32_t col = h * 64u + lane * 2u;
-                    const uint32_t valid = r0 + u < rows ? (col + 1u < keys ? 0xFFFFFFFFu : (col < keys ? 0xFFFFu : 0u)) : 0u;
-                    not_neg |= (v[u][h] ^ 0xFC00FC00u) & valid;
-                    not_zero |= v[u][h] & 0x7FFF7FFFu & valid;
-                }
-        }
-    }
-    const bool any_not_neg = __syncthreads_or(not_neg != 0u), any_not_zero = __syncthreads_or(not_zero != 0u);
-    if (tid == 0) a.cls[tile] = !any_not_neg ? kTileNeg : (any_not_zero ? kTileMixed : kTileZero);
-    if constexpr (kCopy) {
-        if (!any_not_neg || !any_not_zero) return;
-        uint16_t* dst = reinterpret_cast<uint16_t*>(a.copy) + (static_cast<size_t>(b) * a.L + row0) * a.copy_pitch + key0;
-        auto put = [&](uint32_t r, uint32_t h, uint32_t v) {
-            const uint32_t col = h * 64u + lane * 2u;
-            if (r < rows && col < keys)   // (the pitch is even: the second key has a place)
-                *reinterpret_cast<uint32_t*>(dst + static_cast<size_t>(r) * a.copy_pitch + col) = v;
-        };
-        if (words) {
-#pragma unroll
-            for (uint32_t r = 0; r < 16; ++r) {   // the word behind each, from the next lane, and the two put together
-                const uint32_t sh = (static_cast<uint32_t>((first + r * pitch) >> 1) & 1u) * 16u;
-                const uint32_t n0 = __shfl_sync(0xffffffffu, w[r][0], (lane + 1u) & 31u), n1 = __shfl_sync(0xffffffffu, w[r][1], (lane + 1u) & 31u);
-                const uint32_t head1 = __shfl_sync(0xffffffffu, w[r][1], 0), tail = __shfl_sync(0xffffffffu, extra, r);
-                put(r, 0, __funnelshift_r(w[r][0], lane == 31u ? head1 : n0, sh));
-                put(r, 1, __funnelshift_r(w[r][1], lane == 31u ? tail : n1, sh));
-            }
-        } else {
-#pragma unroll 1
-            for (uint32_t r0 = 0; r0 < rows; r0 += 4u) {
-                uint32_t v[4][2];
-                four_rows(r0, v);
-#pragma unroll
-                for (uint32_t u = 0; u < 4; ++u)
-#pragma unroll
-                    for (uint32_t h = 0; h < 2; ++h) put(r0 + u, h, v[u][h]);
+                const uint32_t key = h * 64u + lane * 2u;
+                const uint32_t lo = key < t.keys ? ld_settled(row + key) : 0u, hi = key + 1u < t.keys ? ld_settled(row + key + 1u) : 0u;
+                staged[r * kPlanRowWords + h * 32u + lane] = lo | (hi << 16);
             }
         }
     }
 }
 
-// Can any tile of the mask over key tile kt of batch entry b be -inf throughout?  Its first value tells when not.
-__device__ __forceinline__ bool plan_maybe_left_out(const PlanArgs& a, uint32_t b, uint32_t kt) {
-    bool neg = false;
-    for (uint32_t qt = threadIdx.x; qt < a.n; qt += kPlanThreads)
-        neg |= ld_settled(reinterpret_cast<const uint16_t*>(a.mask) + (static_cast<size_t>(b) * a.L + qt * kTile) * a.L + kt * kTile) == 0xFC00u;
-    return __syncthreads_or(neg);
+// What the tile is: its class, its rows as runs or its copy.
+template <bool kCopy>
+__device__ __forceinline__ void plan_look_at_tile(const PlanArgs& a, const PlanRows& t, uint32_t tile, const uint32_t* staged) {
+    const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, rows = t.rows, keys = t.keys;
+    cp_async_wait_all();
+    __syncwarp();
+    // keys 2 j and 2 j + 1 of row r (a key beyond the end: anything)
+    auto two_keys = [&](uint32_t r, uint32_t j) {
+        if constexpr (!kCopy) return staged[r * 64u + j];
+        const uint32_t* at = staged + r * kPlanRowWords + j;
+        return __funnelshift_r(at[0], at[1], t.shift(r) * 16u);
+    };
+    auto valid_of = [&](uint32_t key) { return (key < keys ? 0xFFFFu : 0u) | (key + 1u < keys ? 0xFFFF0000u : 0u); };   // key, key + 1
+    const uint32_t valid0 = valid_of(2u * lane), valid1 = valid_of(64u + 2u * lane);
+    uint32_t not_neg = 0, not_zero = 0;
+#pragma unroll 4
+    for (uint32_t r = 0; r < rows; ++r) {
+        const uint32_t v0 = two_keys(r, lane), v1 = two_keys(r, 32u + lane);
+        not_neg |= ((v0 ^ 0xFC00FC00u) & valid0) | ((v1 ^ 0xFC00FC00u) & valid1);
+        not_zero |= (v0 & 0x7FFF7FFFu & valid0) | (v1 & 0x7FFF7FFFu & valid1);
+    }
+    const bool any_not_neg = __syncthreads_or(not_neg != 0u), any_not_zero = __syncthreads_or(not_zero != 0u);
+    if (!any_not_neg || !any_not_zero) {
+        if (tid == 0) a.cls[tile] = any_not_neg ? kTileZero : kTileNeg;
+        return;
+    }
+    // Neither: rows that are runs of zeros between -inf (a causal mask's diagonal, the end of a padded sequence, a window)
+    // are passed on as the ends of their runs, 256 bytes instead of 32 KB and nothing to be fetched ahead of a step.
+    bool in_runs = a.runs != nullptr;
+    if (in_runs) {
+        // a row and half of its keys per lane (a row per warp with votes is five times the instructions)
+        const uint32_t r = lane >> 1, half = (lane & 1u) * 64u;
+        uint32_t from = kTile, behind = 0, count = 0;
+        bool fits = true;
+        if (r < rows) {
+            const uint32_t* at = staged + r * (kCopy ? kPlanRowWords : 64u) + half / 2u;
+            const uint32_t sh = kCopy ? t.shift(r) * 16u : 0u;
+            uint32_t w = at[0];
+#pragma unroll 4
+            for (uint32_t j = 0; j < 32u; ++j) {
+                uint32_t v = w;
+                if constexpr (kCopy) {
+                    w = at[j + 1u];
+                    v = __funnelshift_r(v, w, sh);
+                } else {
+                    w = at[min(j + 1u, 31u)];
+                }
+                const uint32_t key = half + 2u * j, valid = valid_of(key);
+                const __half2 h = *reinterpret_cast<const __half2*>(&v);
+                const uint32_t zero = __heq2_mask(h, __float2half2_rn(0.f)) & valid, neg = __heq2_mask(h, __float2half2_rn(-INFINITY));
+                fits &= ((zero | neg | ~valid) == 0xFFFFFFFFu);
+                if (zero) {
+                    from = min(from, key + ((zero & 1u) ? 0u : 1u));
+                    behind = key + ((zero >> 16) ? 2u : 1u);
+                    count += (zero & 1u) + (zero >> 31);
+                }
+            }
+        }
+        from = min(from, __shfl_xor_sync(0xffffffffu, from, 1));
+        behind = max(behind, __shfl_xor_sync(0xffffffffu, behind, 1));
+        count += __shfl_xor_sync(0xffffffffu, count, 1);
+        fits &= count == 0u || count == behind - from;
+        in_runs = __syncthreads_and(fits);
+        if (in_runs && half == 0u)
+            a.runs[static_cast<size_t>(tile) * kTile + warp * 16u + r] = static_cast<uint16_t>(r >= rows ? kWholeRun : (count == 0u ? 0u : from | (behind << 8)));
+    }
+    if (tid == 0) a.cls[tile] = in_runs ? kTileRows : kTileMixed;
+    if constexpr (kCopy) {
+        if (in_runs) return;
+        uint16_t* dst = reinterpret_cast<uint16_t*>(a.copy) + (static_cast<size_t>(t.b) * a.L + t.row0) * a.copy_pitch + t.key0;
+#pragma unroll 2
+        for (uint32_t r = 0; r < rows; ++r) {
+#pragma unroll
+            for (uint32_t h = 0; h < 2; ++h) {
+                const uint32_t v = two_keys(r, h * 32u + lane), at = h * 64u + lane * 2u;
+                if (at < keys)   // (the pitch is even: the second key has a place)
+                    *reinterpret_cast<uint32_t*>(dst + static_cast<size_t>(r) * a.copy_pitch + at) = v;
+            }
+        }
+    }
+}
+
+// Does the plan itself look through K and V of key tile kt of batch entry b?  Only tiles that begin with -inf can be -inf
+// throughout.  Where a kernel without a plan stands behind the planned one, it is done here for key tiles that may be left
+// out by every item; of the others an item that works on them looks them through (kStepCheck) while it multiplies: 134 MB
+// of K and V at B=4 R=32 L=2048 H=128 are 25 us for a kernel of their own.
+__device__ __forceinline__ bool plan_looks_through(const PlanArgs& a, uint32_t b, uint32_t kt) {
+    bool any = false, all = true;
+    for (uint32_t qt = threadIdx.x; qt < a.n; qt += kPlanThreads) {
+        const bool neg = ld_settled(reinterpret_cast<const uint16_t*>(a.mask) + (static_cast<size_t>(b) * a.L + qt * kTile) * a.L + kt * kTile) == 0xFC00u;
+        any |= neg, all &= neg;
+    }
+    return a.items_check ? __syncthreads_and(all) : __syncthreads_or(any);
 }
 
 // 128 rows x up to kPlanCols columns of K or V: is every value finite?
@@ -176,9 +222,7 @@ __device__ __forceinline__ void plan_finite(const PlanArgs& a, const __half* x, 
         w[u] = r < rows && c < a.F ? ld_settled(reinterpret_cast<const uint4*>(src + static_cast<size_t>(r) * a.F)) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
-    for (uint32_t u = 0; u < 8; ++u)   // an exponent of all ones carries into the sign's place
-        bits |= ((w[u].x & 0x7C007C00u) + 0x04000400u) | ((w[u].y & 0x7C007C00u) + 0x04000400u) |
-                ((w[u].z & 0x7C007C00u) + 0x04000400u) | ((w[u].w & 0x7C007C00u) + 0x04000400u);
+    for (uint32_t u = 0; u < 8; ++u) bits |= nonfinite_bits(w[u]);
     if (bits & 0x80008000u) a.bad[b * a.n + kt] = a.stamp;
 }
 
@@ -190,43 +234,68 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
     __shared__ uint32_t hist[kPlanMaxTiles + 1], cost[2];
     __shared__ uint16_t lens[kPlanMaxGroups];
     __shared__ bool last;
+    __shared__ __align__(16) uint32_t staged[kPlanThreads / 32u * 16u * kPlanRowWords];
     grid_dep_wait();
     grid_dep_launch();
     PlanArgs a = args;   // (the inputs' addresses, for ld_settled)
     const uint32_t settled = zero_behind_the_wait();
     a.mask += settled, a.k += settled, a.v += settled;
     const uint32_t tid = threadIdx.x, n = a.n;
+    // The first tile is on its way while the CTA finds out whether there is a plan, and looks at its parts of K and V.
+    uint32_t* my_rows = staged + (tid >> 5) * (16u * kPlanRowWords);
+    const uint32_t tiles = a.B * n * n;
+    uint32_t tile = blockIdx.x;
+    PlanRows rows = plan_rows(a, tile);
+    if (tile < tiles) plan_fetch_tile<kCopy>(rows, my_rows);
+    if (tile + gridDim.x < tiles) {   // the next one as far as L2: a row's 256 bytes per two lanes
+        const PlanRows next = plan_rows(a, tile + gridDim.x);
+        const uint32_t lane = tid & 31u, key = (lane & 1u) * 64u;
+        if ((lane >> 1) < next.rows && key < next.keys) prefetch_l2(next.first + (lane >> 1) * next.pitch + 2u * key);
+    }
     if (a.dense_allowed) {
-        // A tile that is -inf throughout begins with -inf.  Where fewer than a fifth of the tiles do, every CTA finds so
-        // for itself, nothing more is read and the kernel without a plan takes the call.
-        uint32_t neg = 0;
-        for (uint32_t t = tid; t < a.B * n * n; t += kPlanThreads) {
-            const uint32_t kt = t % n, qt = (t / n) % n, b = t / (n * n);
-            neg += ld_settled(reinterpret_cast<const uint16_t*>(a.mask) + (static_cast<size_t>(b) * a.L + qt * kTile) * a.L + kt * kTile) == 0xFC00u;
+        // A tile that is -inf throughout begins with -inf.  Where fewer than a fifth of the tiles do (and some tile begins
+        // with neither -inf nor zero, or none with -inf), every CTA finds so for itself, nothing more is read and the kernel
+        // without a plan takes the call.  One tile per thread, evenly spread, is looked at: the 1024 of B=4 L=2048 took
+        // every CTA 5 us.
+        const uint32_t of = min(tiles, kPlanThreads);
+        uint32_t begins = 0;   // with -inf: 1, with zero: 1 << 16
+        if (tid < of) {
+            const uint32_t t = static_cast<uint32_t>(static_cast<uint64_t>(tiles) * tid / of), kt = t % n, qt = (t / n) % n, b = t / (n * n);
+            const uint32_t v = ld_settled(reinterpret_cast<const uint16_t*>(a.mask) + (static_cast<size_t>(b) * a.L + qt * kTile) * a.L + kt * kTile);
+            begins = v == 0xFC00u ? 1u : ((v & 0x7FFFu) == 0u ? 1u << 16 : 0u);
         }
         if (tid == 0) cost[0] = 0;
         __syncthreads();
-        neg = __reduce_add_sync(0xffffffffu, neg);
-        if ((tid & 31u) == 0) atomicAdd(&cost[0], neg);
+        begins = __reduce_add_sync(0xffffffffu, begins);
+        if ((tid & 31u) == 0) atomicAdd(&cost[0], begins);
         __syncthreads();
-        if (5u * cost[0] < a.B * n * n) {
+        const uint32_t neg = cost[0] & 0xFFFFu, zero = cost[0] >> 16;
+        if (5u * neg < of && (neg == 0u || neg + zero < of)) {
             if (tid == 0 && blockIdx.x == 0) a.head[0] = 0;
+            cp_async_wait_all();
             return;
         }
     }
-    for (uint32_t t = blockIdx.x; t < a.B * n * n; t += gridDim.x) plan_mask_tile<kCopy>(a, t);
     const uint32_t chunks = (a.F + kPlanCols - 1u) / kPlanCols, jobs = a.B * n * 2u * chunks;   // (launcher: below 2^31 / gridDim.x)
     uint32_t job = static_cast<uint32_t>(static_cast<uint64_t>(jobs) * blockIdx.x / gridDim.x);
     const uint32_t job_end = static_cast<uint32_t>(static_cast<uint64_t>(jobs) * (blockIdx.x + 1u) / gridDim.x);
-    while (job < job_end) {   // parts of one key tile at a time
+    while (job < job_end) {   // parts of one key tile at a time (while the tile is on its way)
         const uint32_t bk = job / (2u * chunks), end = min(job_end, (bk + 1u) * 2u * chunks), b = bk / n, kt = bk % n;
-        if (plan_maybe_left_out(a, b, kt)) {
+        if (plan_looks_through(a, b, kt)) {
             for (; job < end; ++job) {
                 const uint32_t part = job - bk * 2u * chunks;
                 plan_finite(a, part < chunks ? a.k : a.v, b, kt, (part < chunks ? part : part - chunks) * kPlanCols);
             }
         }
         job = end;
+    }
+    while (tile < tiles) {
+        plan_look_at_tile<kCopy>(a, rows, tile, my_rows);
+        tile += gridDim.x;
+        if (tile >= tiles) break;
+        __syncwarp();   // every lane is through with these rows
+        rows = plan_rows(a, tile);
+        plan_fetch_tile<kCopy>(rows, my_rows);
     }
     __syncthreads();
     if (tid == 0) {   // (the barrier orders what the other threads wrote before this, the fence passes it on)
@@ -237,6 +306,17 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
     __syncthreads();
     if (!last) return;
     const uint32_t groups = a.B * a.q_pairs;
+    // the classes, and which K and V are not finite, all at once where they fit into shared memory: the lists take them in
+    // steps that would each wait for L2
+    const uint8_t* cls = a.cls;
+    const uint32_t* bad_of = a.bad;
+    const uint32_t cls_words = (tiles + 3u) / 4u;   // (the bytes behind the classes are the scratch's own)
+    if (cls_words + a.B * n <= sizeof(staged) / sizeof(uint32_t)) {
+        for (uint32_t i = tid; i < cls_words; i += kPlanThreads) staged[i] = __ldcg(reinterpret_cast<const uint32_t*>(a.cls) + i);
+        for (uint32_t i = tid; i < a.B * n; i += kPlanThreads) staged[cls_words + i] = __ldcg(a.bad + i);
+        cls = reinterpret_cast<const uint8_t*>(staged);
+        bad_of = staged + cls_words;
+    }
     for (uint32_t i = tid; i <= n; i += kPlanThreads) hist[i] = 0;
     if (tid < 2) cost[tid] = 0;
     if (tid == 0) *a.ticket = 0;
@@ -249,7 +329,7 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
         const uint32_t gr = g0 + sub;
         const bool live = gr < groups;
         const uint32_t b = gr / a.q_pairs, q0 = (gr % a.q_pairs) * 2u;
-        const uint8_t* c0 = a.cls + (b * n + q0) * n;
+        const volatile uint8_t* c0 = cls + (b * n + q0) * n;
         const bool two = q0 + 1u < n;   // the second query tile exists
         uint16_t* out = a.list + gr * n;
         uint32_t len = 0;
@@ -257,18 +337,29 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
             const uint32_t kt = k0 + l_in;
             const bool in = live && kt < n;
             uint32_t x = kTileNeg, y = kTileNeg, bad = a.stamp + 1u;
-            if (in) {
-                x = __ldcg(c0 + kt);
-                bad = __ldcg(a.bad + b * n + kt);
-                y = two ? __ldcg(c0 + n + kt) : (x == kTileNeg ? kTileNeg : kTileZero);
+            bool above = false, below = false;   // the pair of query tiles before this one, behind it, leaves the key tile out
+            if (in) {   // (all asked for together)
+                const volatile uint8_t* c = c0 + kt;
+                const bool has_below = q0 + 2u < n, has_above = q0 != 0u;
+                x = *c;
+                bad = *const_cast<const volatile uint32_t*>(bad_of + b * n + kt);
+                y = *(two ? c + n : c);
+                const uint32_t a0 = *(has_above ? c - 2u * n : c), a1 = *(has_above ? c - n : c);
+                const uint32_t b0 = *(has_below ? c + 2u * n : c), b1 = *(q0 + 3u < n ? c + 3u * n : c);
+                if (!two) y = x == kTileNeg ? kTileNeg : kTileZero;
+                above = has_above && (a0 | a1) == kTileNeg;
+                below = has_below && (q0 + 3u < n ? b0 | b1 : b0) == kTileNeg;
             }
             const bool keep = in && (x != kTileNeg || y != kTileNeg || bad == a.stamp);
+            // Looked through by the items that keep it next to items that do not (among those that keep a tile that others
+            // leave out there is such a pair, and every head of it looks at its own columns).
+            const uint32_t check = keep && a.items_check && bad != a.stamp && (above || below) ? kStepCheck : 0u;
             const uint32_t votes = __ballot_sync(0xffffffffu, keep) & sub_mask;
             if (keep) {
-                const uint32_t ex = x == kTileZero ? kStepNoMask : (x == kTileNeg ? kStepAllNeg : kStepMask);
-                const uint32_t ey = y == kTileZero ? kStepNoMask : (y == kTileNeg ? kStepAllNeg : kStepMask);
+                auto what = [](uint32_t c) { return c == kTileZero ? kStepNoMask : (c == kTileNeg ? kStepAllNeg : (c == kTileRows ? kStepRows : kStepMask)); };
+                const uint32_t ex = what(x), ey = what(y);
                 mask_tiles += (ex == kStepMask ? 1u : 0u) + (ey == kStepMask ? 1u : 0u);
-                out[len + __popc(votes & ((1u << lane) - 1u))] = static_cast<uint16_t>(kt | (ex << kStepShift0) | (ey << kStepShift1));
+                out[len + __popc(votes & ((1u << lane) - 1u))] = static_cast<uint16_t>(kt | check | (ex << kStepShift0) | (ey << kStepShift1));
             }
             len += __popc(votes);
         }
@@ -298,6 +389,8 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
         }
         // The planned kernel needs about 1.0 for a step and 0.2 more for each mask tile of it, the one without a plan
         // 1.2 for each step of all.
+        *reinterpret_cast<const __half**>(a.head + kPlanInputs) = a.k;
+        *reinterpret_cast<const __half**>(a.head + kPlanInputs + 2) = a.v;
         a.head[0] = !a.dense_allowed || 5u * cost[0] + cost[1] < 6u * groups * n ? 1u : 0u;
     }
     __syncthreads();

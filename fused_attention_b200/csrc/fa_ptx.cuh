@@ -335,6 +335,7 @@ __device__ __forceinline__ void cp_async_4_part(uint32_t dst, uint64_t src, uint
 __device__ __forceinline__ void cp_async_arrive(uint32_t bar) {
     asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(bar) : "memory");
 }
+__device__ __forceinline__ void prefetch_l2(uint64_t at) { asm volatile("prefetch.global.L2 [%0];" ::"l"(at) : "memory"); }
 // 16 bytes; zeros instead of the source when `in` is false (nothing is read then)
 __device__ __forceinline__ void cp_async_16_zero(uint32_t dst, const void* src, bool in) {
     const uint32_t n = in ? 16u : 0u;

@@ -141,3 +141,40 @@ def test_masked_keys_that_are_not_finite_are_not_left_out(where, value, B, R, L)
     plain = _recorded(q, k, v, H, mask, _lib.FLAG_NO_SPLIT)
     assert torch.equal(torch.isnan(y), torch.isnan(plain)) and bool(torch.isnan(y).any())
     assert torch.equal(torch.nan_to_num(y, nan=9.0), torch.nan_to_num(plain, nan=9.0))
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan")])
+@pytest.mark.parametrize("where", ["k", "v"])
+@pytest.mark.parametrize("H,R,L", [(32, 30, 2048), (64, 30, 2048), (128, 30, 1928), (64, 40, 515)])
+def test_keys_that_only_some_items_leave_out_and_that_are_not_finite(where, value, H, R, L):
+    """Causal: the key tile is worked on by some items and left out by others.  Where its rows start on 16-byte boundaries
+    the items that work on it find the value, and the kernel behind the planned one does the call again."""
+    B = 2
+    assert fa.describe_call(B, L, R * H, H, 16)["planned"] and fa.stream_has_scratch()
+    q, k, v = (t.cuda() for t in make_inputs(B, L, R * H, 1.0, L))
+    mask = torch.full((L, L), float("-inf"), dtype=torch.float16).triu(1).repeat(B, 1, 1).cuda()
+    {"k": k, "v": v}[where][1, L - 70, 7 * H + 3] = value
+    y = fa.attention_forward(H, 32, q, k, v, mask, flags=_lib.FLAG_SYNC)
+    plain = _recorded(q, k, v, H, mask, _lib.FLAG_NO_SPLIT)
+    assert torch.equal(torch.nan_to_num(y, nan=9.0), torch.nan_to_num(plain, nan=9.0))
+    assert bool((~torch.isfinite(plain)).any())
+
+
+@pytest.mark.parametrize("B,R,L,H", [(2, 30, 2048, 64), (2, 30, 1928, 128), (3, 40, 1021, 64), (2, 30, 2048, 32), (2, 9, 389, 128)])
+def test_rows_that_are_runs_of_zeros(B, R, L, H):
+    """Rows of a tile as runs: ends on and beside the edges of words, halves and tiles, rows without a key, -0 in a run; and
+    one row that is no run, which makes its tile a mask tile.  The bits of the call without a plan."""
+    assert fa.describe_call(B, L, R * H, H, 16)["planned"] and fa.stream_has_scratch()
+    q, k, v = (t.cuda() for t in make_inputs(B, L, R * H, 1.0, L))
+    ends = torch.tensor([0, 1, 2, 31, 32, 33, 63, 64, 65, 95, 96, 97, 126, 127, 128, 129, 200, 256, L - 1, L])
+    gen = torch.Generator().manual_seed(L + H)
+    a, b = (ends[torch.randint(0, len(ends), (B, L, 1), generator=gen)] for _ in range(2))
+    keys = torch.arange(L)
+    mask = torch.where((keys >= torch.minimum(a, b)) & (keys < torch.maximum(a, b)), 0.0, float("-inf")).half()
+    mask[:, ::7] = torch.where(mask[:, ::7] == 0, torch.tensor(-0.0, dtype=torch.float16), mask[:, ::7])
+    mask[0, 300, :] = 0.0
+    mask[0, 300, 40:50] = float("-inf")
+    mask = mask.cuda()
+    y = fa.attention_forward(H, 32, q, k, v, mask, flags=_lib.FLAG_SYNC)
+    plain = _recorded(q, k, v, H, mask, _lib.FLAG_NO_SPLIT)
+    assert torch.equal(torch.nan_to_num(y, nan=9.0), torch.nan_to_num(plain, nan=9.0))
