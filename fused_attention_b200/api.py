@@ -12,6 +12,8 @@ applied to every key tile (the reference applies it to the first chunk only,
 from __future__ import annotations
 
 import ctypes
+import importlib.util
+import os
 from typing import Optional
 
 import torch
@@ -78,11 +80,36 @@ def _is_fp16_cuda(t, device: int) -> bool:
     return isinstance(t, torch.Tensor) and t.dtype is torch.float16 and t.is_cuda and t.get_device() == device and t.is_contiguous()
 
 
+def _load_native():
+    """The call in native code, from the extension module where it has been built: checks, allocation and launch without
+    ctypes (B=1 R=4 L=256 H=64: 8.4 us a call through ctypes).  A function that always answers None where there is none."""
+    from .build import ext_path
+    path = os.path.abspath(ext_path())
+    try:
+        spec = importlib.util.spec_from_file_location("fused_attn", path)
+        module = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(module)
+        return module._forward_or_none
+    except (ImportError, AttributeError, OSError):
+        return lambda *args: None
+
+
+_native = None
+
+
 def attention_forward(head_dim: int, chunk_size: int, queries: torch.Tensor, keys: torch.Tensor,
                       values: torch.Tensor, mask: Optional[torch.Tensor] = None, *,
                       flags: int = _lib.FLAG_DEFAULT) -> torch.Tensor:
     """Fused multi-head attention forward ``softmax(Q K^T / sqrt(head_dim)) V`` on the GPU."""
+    global _native
     lib = _lib.load()  # raises when the CUDA library is missing: no fallback
+    if _native is None:
+        _native = _load_native()
+    out = _native(head_dim, chunk_size, queries, keys, values, mask, flags)
+    if out is not None:
+        if out.__class__ is int:
+            _lib.check(out)
+        return out
     # All preconditions in one expression, nothing formatted and no device object built while they hold; what does not
     # pass goes through the checks one by one (measured on B=1 R=4 L=256: 8.3 us a call, 13.8 with the checks in a row
     # and their messages formatted on every call).
