@@ -552,12 +552,12 @@ bool plan_fits(uint32_t B, uint32_t L, uint32_t F, bool mask_tma, uint32_t sms) 
 // mask, K and V ahead of the attention kernel, 6 us at least, and 13 in all where it finds that too little can be left
 // out; what it saves is up to half of the key steps where there is more than one round of them.  Measured, us without
 // and with a plan, causal masks:
-//   H = 64: B=8 R=12 L=512 21.8 / 24.2, B=32 R=12 L=512 58 / 73, B=8 R=16 L=1024 70 / 65, B=8 R=32 L=2048 430 / 320
-//   H = 32: B=8 R=16 L=2048 255 / 160
-//   H = 128: B=4 R=32 L=1024 77 / 97, B=2 R=32 L=2048 141 / 138, B=4 R=32 L=2048 291 / 254, B=1 R=40 L=4096 385 / 227
-// so from sixteen key tiles and some fifty key steps per SM on.  (A mask that leaves nothing out pays for the plan and the
-// planned kernel's launch all the same: H = 128, B=2 R=32 L=2048 139 / 151, B=4 R=32 L=2048 265 / 277; at H = 64 B=4 R=32
-// L=2048 it is 248 with both.  What the mask holds is known on the device only.)  Where TMA cannot fetch the rows the plan's copy also
+//   H = 64: B=8 R=12 L=512 19.8 / 33.5, B=32 R=12 L=512 50 / 70, B=8 R=16 L=1024 63 / 67, B=2 R=12 L=2048 50 / 51
+//   H = 32: B=8 R=16 L=1024 73 / 65;   H = 128: B=4 R=32 L=1024 69 / 78, B=2 R=32 L=1536 82 / 79
+// so from sixteen key tiles and some fifty key steps per SM on, where it is far ahead (B=4 R=32 L=2048 H=128 with mask tiles
+// 250, planned 206; B=8 R=32 L=2048 H=64 430 and 270).  (A mask that leaves nothing out pays for the plan and the planned
+// kernel's launch all the same: H = 64, B=8 R=16 L=1024 63 / 81, B=2 R=16 L=2048 63 / 80.  What the mask holds is known on the
+// device only.)  Where TMA cannot fetch the rows the plan's copy also
 // spares every head the copies inside the kernel, and it pays much sooner:
 //   H = 64: B=32 R=16 L=201 36 / 46, B=1 R=8 L=301 15 / 18, B=32 R=12 L=301 82 / 63, B=2 R=8 L=511 26 / 21,
 //           B=4 R=12 L=1021 72 / 38;   H = 128: B=1 R=8 L=301 25 / 19, B=2 R=32 L=1021 125 / 51
