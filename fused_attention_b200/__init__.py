@@ -10,14 +10,14 @@ The compute path is the CUDA library ``lib/libfa_b200.so`` behind the C ABI of
 ``include/fa_b200.h``; there is no CPU path.
 """
 from . import _lib
-from .api import (attention_forward, attention_forward_host, bind_forward, cta_segments, describe_call, describe_schedule, query,
+from .api import (attention_forward, attention_forward_host, bind_forward, cta_segments, describe_call, describe_schedule, plan_taken, query,
                   read_status, select_kernel, stream_has_scratch)
 from .sharding import (Shard, aggregate_throughput, attention_bytes, attention_flops, shard_units,
                        slice_tensor)
 
 __all__ = [
     "attention_forward", "attention_forward_host", "bind_forward", "query", "read_status", "select_kernel",
-    "describe_call", "describe_schedule", "cta_segments", "stream_has_scratch",
+    "describe_call", "describe_schedule", "cta_segments", "plan_taken", "stream_has_scratch",
     "Shard", "shard_units", "slice_tensor", "attention_flops", "attention_bytes", "aggregate_throughput",
     "_lib",
 ]

@@ -22,6 +22,8 @@ EXPORTED_SYMBOLS = (
     "fa_b200_read_status",
     "fa_b200_describe_call",
     "fa_b200_stream_has_scratch",
+    "fa_b200_describe_plan_sample",
+    "fa_b200_plan_taken",
     "fa_b200_select_kernel",
     "fa_b200_describe_schedule",
     "fa_b200_selftest_bounded_wait",
@@ -91,6 +93,10 @@ def load() -> ctypes.CDLL:
         lib.fa_b200_describe_call.argtypes = [u32, u32, u32, u32, u32, u32, u32, ctypes.POINTER(ctypes.c_uint32)]
         lib.fa_b200_stream_has_scratch.restype = i32
         lib.fa_b200_stream_has_scratch.argtypes = [i32, vp, ctypes.POINTER(ctypes.c_uint32)]
+        lib.fa_b200_describe_plan_sample.restype = i32
+        lib.fa_b200_describe_plan_sample.argtypes = [u32, u32, u32, ctypes.POINTER(ctypes.c_uint32)]
+        lib.fa_b200_plan_taken.restype = i32
+        lib.fa_b200_plan_taken.argtypes = [i32, vp, ctypes.POINTER(ctypes.c_uint32)]
         lib.fa_b200_select_kernel.restype = i32
         lib.fa_b200_select_kernel.argtypes = [u32, u32, u32, u32, i32, u32]
         lib.fa_b200_describe_schedule.restype = i32

@@ -220,6 +220,14 @@ def stream_has_scratch(stream: int = 0, device: int = 0) -> bool:
     return bool(o[0])
 
 
+def plan_taken(stream: int = 0, device: int = 0) -> Optional[bool]:
+    """Whether the planned kernel had the last planned call on a stream (its handle), or the kernel behind it; None where
+    that is not known (``fa_b200_plan_taken``).  Synchronises the stream."""
+    o = (ctypes.c_uint32 * 2)()
+    _lib.check(_lib.load().fa_b200_plan_taken(int(device), int(stream), o))
+    return bool(o[1]) if o[0] else None
+
+
 def select_kernel(B: int, L: int, F: int, head_dim: int, has_mask: bool = False, flags: int = 0) -> str:
     rc = _lib.load().fa_b200_select_kernel(B, L, F, head_dim, int(has_mask), flags)
     if rc < 0:

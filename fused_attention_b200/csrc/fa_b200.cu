@@ -45,6 +45,9 @@ struct SplitScratch {
     // launches whatever became of the others; the part counters may be left half counted by a launch that gave up, and
     // are zeroed with its report while other streams work.
     uint32_t* ticket = nullptr;
+    // Where the plan of the last planned call that used the buffer says which kernel has the call (fa::PlanArgs::head);
+    // nullptr if something else may lie there now.
+    const uint32_t* plan_head = nullptr;
     // Held from the first launch of a call that uses the buffer to its last one.  The launches of a planned call pass
     // the plan on through the buffer, and stream order keeps them together only as long as no other thread that
     // works on the same stream can put a launch that uses it in between.
@@ -572,7 +575,7 @@ bool use_mask_plan(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool mask_tma
 // Launches the kernel that plans a masked call, into the scratch of the call's stream (a planned call is not divided,
 // so the scratch is free): on return p's plan_ fields are set, and the mask's rows are at *mask_rows, *mask_pitch
 // elements apart.
-int plan_mask(DeviceCtx& c, const SplitScratch& scratch, const void* k, const void* v, bool mask_tma,
+int plan_mask(DeviceCtx& c, SplitScratch& scratch, const void* k, const void* v, bool mask_tma,
               Params& p, cudaStream_t st, bool overlap, const void** mask_rows, uint32_t* mask_pitch) {
     // (without the runs where there is no room for them: rows that are runs are then mask tiles like any other)
     const bool with_runs = plan_layout(p.B, p.L, p.F, mask_tma, true).bytes <= split_o_bytes(c.sm_count);
@@ -600,11 +603,12 @@ int plan_mask(DeviceCtx& c, const SplitScratch& scratch, const void* k, const vo
     a.dense_allowed = a.items_check = mask_tma ? 1u : 0u;
     const uint64_t most = static_cast<uint64_t>(mask_tma ? fa::kPlanCtasPerSm : fa::kPlanCopyCtasPerSm) * c.sm_count;
     const uint64_t wide = l.tiles > l.jobs ? l.tiles : l.jobs;
+    scratch.plan_head = nullptr;
     cudaError_t e = launch_kernel(mask_tma ? fa::fa_mask_plan<false> : fa::fa_mask_plan<true>,
                                   dim3(static_cast<unsigned>(wide < most ? wide : most)), fa::kPlanThreads, 0, st, overlap, a);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return static_cast<int>(e);
-    p.plan_head = a.head;
+    p.plan_head = scratch.plan_head = a.head;
     p.plan_order = a.order;
     p.plan_list = a.list;
     *mask_rows = mask_tma ? static_cast<const void*>(p.mask) : a.copy;
@@ -727,6 +731,7 @@ int forward_device(const void* q, const void* k, const void* v, const void* mask
                         p.part_o = scratch->o;
                         p.part_ml = scratch->ml;
                         p.part_cnt = scratch->cnt;
+                        scratch->plan_head = nullptr;
                     }
                     // Y as a TMA store target: boxes of 32 rows x 64 columns (one epilogue warp each)
                     CUtensorMap my;
@@ -1296,6 +1301,47 @@ int fa_b200_stream_has_scratch(int device, void* cuda_stream, uint32_t out[1]) {
         rc = ensure_ctx(device, &c);
     }
     if (rc == FA_B200_OK) out[0] = scratch_for_stream(*c, static_cast<cudaStream_t>(cuda_stream), false) != nullptr ? 1u : 0u;
+    if (prev != device) (void)cudaSetDevice(prev);
+    return rc;
+}
+
+int fa_b200_describe_plan_sample(uint32_t B, uint32_t L, uint32_t index, uint32_t out[4]) {
+    if (!out) return FA_B200_ERR_NULL_POINTER;
+    const uint32_t n = L / fa::kTile + (L % fa::kTile != 0u);
+    if (B == 0 || L == 0 || n > fa::kPlanMaxTiles || B > fa::kPlanMaxGroups) return FA_B200_ERR_SHAPE;
+    out[3] = fa::plan_samples(B, n);
+    if (index >= out[3]) return FA_B200_ERR_SHAPE;
+    const fa::PlanSample s = fa::plan_sample(index, B, n);
+    out[0] = s.b;
+    out[1] = s.qt;
+    out[2] = s.kt;
+    return FA_B200_OK;
+}
+
+int fa_b200_plan_taken(int device, void* cuda_stream, uint32_t out[2]) {
+    if (!out) return FA_B200_ERR_NULL_POINTER;
+    out[0] = out[1] = 0;
+    int prev = -1;
+    cudaError_t e = cudaGetDevice(&prev);
+    if (e != cudaSuccess) return static_cast<int>(e);
+    if (prev != device && (e = cudaSetDevice(device)) != cudaSuccess) return static_cast<int>(e);
+    DeviceCtx* c = nullptr;
+    int rc;
+    {
+        std::lock_guard<std::mutex> lk(g_mu);
+        rc = ensure_ctx(device, &c);
+    }
+    cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
+    SplitScratch* scratch = rc == FA_B200_OK ? scratch_for_stream(*c, st, false) : nullptr;   // (a free buffer has no plan_head)
+    if (scratch != nullptr) {
+        std::lock_guard<std::mutex> lk(scratch->mu);
+        if (scratch->plan_head != nullptr) {
+            e = cudaStreamSynchronize(st);
+            if (e == cudaSuccess) e = cudaMemcpy(out + 1, scratch->plan_head, sizeof(uint32_t), cudaMemcpyDeviceToHost);
+            if (e == cudaSuccess) out[0] = 1;
+            else rc = static_cast<int>(e);
+        }
+    }
     if (prev != device) (void)cudaSetDevice(prev);
     return rc;
 }

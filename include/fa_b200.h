@@ -216,8 +216,8 @@ int fa_b200_debug_cycles(void* device_buffer_of_256_u64);
  * out[1] = 1 if the call is planned on a stream that has scratch (fa_b200_stream_has_scratch): a kernel
  *          finds out first what the mask leaves to do, and the warp-specialised kernel follows its lists;
  *          for a mask whose rows all start on 16-byte boundaries the kernel of out[0] is launched behind
- *          the two and does the call where the mask leaves too little out.  Without scratch it is
- *          launched alone,
+ *          the two and does the call where the mask leaves too little out (fa_b200_plan_taken).  Without
+ *          scratch it is launched alone,
  * out[2] = how many kernels that are (1, 2 or 3).
  * Pure arithmetic, no CUDA call; it is what the launcher itself uses.  No counterpart in the reference.
  */
@@ -230,6 +230,25 @@ int fa_b200_describe_call(uint32_t B, uint32_t L, uint32_t F, uint32_t head_dim,
  * gets none.  Takes none itself.  No counterpart in the reference.
  */
 int fa_b200_stream_has_scratch(int device, void* cuda_stream, uint32_t out[1]);
+
+/*
+ * A planned call whose mask's rows all start on 16-byte boundaries is given to the kernel behind the
+ * planned one where too little of the mask is -inf.  That is judged first by the beginnings of at most 256
+ * of its 128 x 128 tiles: out[0] = batch entry, out[1] = query tile, out[2] = key tile of the one with the
+ * given index, out[3] = how many are looked at.  FA_B200_ERR_SHAPE for an index beyond them, or sizes that
+ * are not planned.  Pure arithmetic, no CUDA call; it is what the kernel itself uses.  No counterpart in the
+ * reference.
+ */
+int fa_b200_describe_plan_sample(uint32_t B, uint32_t L, uint32_t index, uint32_t out[4]);
+
+/*
+ * Which kernel had the last planned call on `cuda_stream`: out[0] = 1 if that is known (the stream's scratch
+ * still holds the plan: no call with a divided last round came behind it), out[1] = 1 if it was the planned
+ * kernel, 0 if the one behind it.  Synchronises the stream.  A diagnostic, for tests and harnesses: what the
+ * mask holds is only known on the device, so fa_b200_describe_call cannot tell.  No counterpart in the
+ * reference.
+ */
+int fa_b200_plan_taken(int device, void* cuda_stream, uint32_t out[2]);
 
 /*
  * The family a call belongs to, as harnesses ask for it: 1 for the kernel with a query tile per CTA, for

@@ -124,6 +124,19 @@ def test_planned_masks(B, R, L, H, kind):
     assert_close(y[..., cols].float().cpu(), oracle(*(t[..., cols].contiguous() for t in (q, k, v)), H, mask))
 
 
+@pytest.mark.parametrize("B,R,L,H", [(16, 4, 2048, 64), (32, 2, 1928, 32), (8, 2, 4096, 128), (4, 1, 8192, 64), (12, 6, 2048, 64)])
+@pytest.mark.parametrize("kind", ["causal", "padding"])
+def test_large_batches_keep_their_plan(B, R, L, H, kind):
+    """Numbers of batch entries and of key tiles whose product is a multiple of 256, and one whose is not: what is looked at to
+    find out whether a mask leaves enough out has to come from all of its key tiles."""
+    assert fa.describe_call(B, L, R * H, H, 16)["planned"] and fa.stream_has_scratch()
+    q, k, v = (t.cuda() for t in make_inputs(B, L, R * H, 1.0, L))
+    mask = _block_mask(B, L, kind).cuda()
+    y = fa.attention_forward(H, 32, q, k, v, mask, flags=_lib.FLAG_SYNC)
+    assert fa.plan_taken() is True
+    assert torch.equal(y, _recorded(q, k, v, H, mask, _lib.FLAG_NO_SPLIT))
+
+
 @pytest.mark.parametrize("value", [float("inf"), float("nan")])
 @pytest.mark.parametrize("where", ["k", "v", "q"])
 @pytest.mark.parametrize("B,R,L", [(2, 30, 2048), (3, 40, 515)])
