@@ -77,6 +77,7 @@ def load() -> ctypes.CDLL:
         u32, vp, i32 = ctypes.c_uint32, ctypes.c_void_p, ctypes.c_int
         lib.fa_b200_attention_forward.restype = i32
         lib.fa_b200_attention_forward.argtypes = [vp, vp, vp, vp, vp, u32, u32, u32, u32, u32, i32, vp, u32]
+        lib.forward_entry = ctypes.cast(lib.fa_b200_attention_forward, vp).value   # for the extension module's call
         lib.fa_b200_attention_forward_noalloc.restype = i32
         lib.fa_b200_attention_forward_noalloc.argtypes = [vp, vp, vp, vp, vp, u32, u32, u32, u32, u32, i32, vp, u32]
         lib.fa_b200_attention_forward_host.restype = i32

@@ -89,7 +89,7 @@ def _load_native():
         spec = importlib.util.spec_from_file_location("fused_attn", path)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
-        return module._forward_or_none
+        return module._forward_through
     except (ImportError, AttributeError, OSError):
         return lambda *args: None
 
@@ -105,7 +105,7 @@ def attention_forward(head_dim: int, chunk_size: int, queries: torch.Tensor, key
     lib = _lib.load()  # raises when the CUDA library is missing: no fallback
     if _native is None:
         _native = _load_native()
-    out = _native(head_dim, chunk_size, queries, keys, values, mask, flags)
+    out = _native(lib.forward_entry, head_dim, chunk_size, queries, keys, values, mask, flags)
     if out is not None:
         if out.__class__ is int:
             _lib.check(out)

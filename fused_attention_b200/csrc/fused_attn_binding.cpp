@@ -64,10 +64,12 @@ torch::Tensor attention_forward(int head_dim, int chunk_size, torch::Tensor quer
     return output;
 }
 
-// The call behind the package's Python function (fused_attention_b200.attention_forward), positional arguments (head_dim,
-// chunk_size, queries, keys, values, mask or None, flags): the output, the status of a launch that failed, or None for
-// everything that is not a plain call with every precondition met, which Python then looks at with its own checks (and their
-// messages).  Checks, allocation and call took 8.4 us in Python on B=1 R=4 L=256 H=64, more than the kernel.
+// The call behind the package's Python function (fused_attention_b200.attention_forward), positional arguments (entry,
+// head_dim, chunk_size, queries, keys, values, mask or None, flags): the output, the status of a launch that failed, or None
+// for everything that is not a plain call with every precondition met, which Python then looks at with its own checks (and
+// their messages).  `entry` is the address of fa_b200_attention_forward in the library that Python has loaded, which need not
+// be the one that this module links (the checked and the clock-counting build).  Checks, allocation and call took 8.4 us in
+// Python on B=1 R=4 L=256 H=64, more than the kernel.
 bool plain_tensor(PyObject* o, at::Tensor& t) {
     if (!THPVariable_CheckExact(o)) return false;   // a subclass may have its own idea of every operation
     t = THPVariable_Unpack(o);
@@ -77,9 +79,16 @@ bool plain_tensor(PyObject* o, at::Tensor& t) {
     return t.defined() && !t.key_set().has_any(wrapped) && t.scalar_type() == at::kHalf && t.is_cuda() && t.dim() == 3 && t.is_contiguous();
 }
 
-PyObject* forward_or_none(PyObject*, PyObject* const* args, Py_ssize_t n) {
+PyObject* forward_through(PyObject*, PyObject* const* args, Py_ssize_t n) {
     HANDLE_TH_ERRORS
-    if (n != 7 || !PyLong_CheckExact(args[0]) || !PyLong_CheckExact(args[1]) || !PyLong_CheckExact(args[6]) ||
+    if (n != 8 || !PyLong_CheckExact(args[0])) Py_RETURN_NONE;
+    auto* const entry = reinterpret_cast<decltype(&fa_b200_attention_forward)>(PyLong_AsVoidPtr(args[0]));
+    if (entry == nullptr) {
+        PyErr_Clear();
+        Py_RETURN_NONE;
+    }
+    ++args;
+    if (!PyLong_CheckExact(args[0]) || !PyLong_CheckExact(args[1]) || !PyLong_CheckExact(args[6]) ||
         at::impl::PythonTorchFunctionTLS::stack_len() > 0)
         Py_RETURN_NONE;
     int over = 0;
@@ -104,14 +113,14 @@ PyObject* forward_or_none(PyObject*, PyObject* const* args, Py_ssize_t n) {
     void *py = out.data_ptr(), *stream = static_cast<void*>(c10::cuda::getCurrentCUDAStream(device).stream());
     int rc = 0;
     Py_BEGIN_ALLOW_THREADS   // (a call that waits for the stream must not hold other threads up)
-    rc = fa_b200_attention_forward(pq, pk, pv, pm, py, static_cast<uint32_t>(B), static_cast<uint32_t>(L), static_cast<uint32_t>(F),
-                                   static_cast<uint32_t>(H), static_cast<uint32_t>(C), device, stream, static_cast<uint32_t>(flags));
+    rc = entry(pq, pk, pv, pm, py, static_cast<uint32_t>(B), static_cast<uint32_t>(L), static_cast<uint32_t>(F),
+               static_cast<uint32_t>(H), static_cast<uint32_t>(C), device, stream, static_cast<uint32_t>(flags));
     Py_END_ALLOW_THREADS
     if (rc != FA_B200_OK) return PyLong_FromLong(rc);
     return THPVariable_Wrap(std::move(out));
     END_HANDLE_TH_ERRORS
 }
-PyMethodDef forward_or_none_def = {"_forward_or_none", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(forward_or_none)),
+PyMethodDef forward_through_def = {"_forward_through", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(forward_through)),
                                    METH_FASTCALL, nullptr};
 
 }  // namespace
@@ -120,5 +129,5 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("attention_forward", &attention_forward, py::arg("head_dim"), py::arg("chunk_size"), py::arg("queries"),
           py::arg("keys"), py::arg("values"), py::arg("mask") = torch::optional<torch::Tensor>(),
           "Fused multihead attention");
-    m.add_object("_forward_or_none", PyCFunction_New(&forward_or_none_def, nullptr));
+    m.add_object("_forward_through", PyCFunction_New(&forward_through_def, nullptr));
 }
