@@ -14,6 +14,7 @@ from __future__ import annotations
 import ctypes
 import importlib.util
 import os
+import warnings
 from typing import Optional
 
 import torch
@@ -82,15 +83,20 @@ def _is_fp16_cuda(t, device: int) -> bool:
 
 def _load_native():
     """The call in native code, from the extension module where it has been built: checks, allocation and launch without
-    ctypes (B=1 R=4 L=256 H=64: 5.7 us a call, 8.4 through ctypes).  A function that always answers None where there is none."""
+    ctypes (B=1 R=4 L=256 H=64: 5.7 us a call, 8.4 through ctypes).  A function that always answers None where there is none,
+    or, with a warning, one that cannot be loaded (built for another torch, or from older sources)."""
     from .build import ext_path
     path = os.path.abspath(ext_path())
+    if not os.path.exists(path):
+        return lambda *args: None
     try:
         spec = importlib.util.spec_from_file_location("fused_attn", path)
         module = importlib.util.module_from_spec(spec)
         spec.loader.exec_module(module)
         return module._forward_through
-    except (ImportError, AttributeError, OSError):
+    except (ImportError, AttributeError, OSError) as e:
+        warnings.warn(f"{path} cannot be used, so calls go through ctypes, which takes some 3 us more each: {e}; rebuild it with "
+                      "python -m fused_attention_b200.build --ext", RuntimeWarning, stacklevel=3)
         return lambda *args: None
 
 

@@ -191,3 +191,17 @@ def test_time_line_words_are_parsed():
     assert r["pv_warp"]["wait_for_P0"] == 1000.0
     assert r["S_finished_before_its_tile_looks"]["tile0_issue_to_seen"] == 10_000 + 120 - (10_000 + 900 - 600)
     assert cycles.parse_timeline([0] * cycles.TIMELINE_WORDS)["step_period"] is None
+
+
+@pytest.mark.parametrize("content", [b"not a library", None])
+def test_an_extension_module_that_cannot_be_loaded_is_reported(monkeypatch, tmp_path, content, recwarn):
+    """Calls then go through ctypes, which is slower: with a warning if there is a file, without one if none was built."""
+    from fused_attention_b200 import api, build
+    path = tmp_path / os.path.basename(build.ext_path())
+    if content is not None:
+        path.write_bytes(content)
+    monkeypatch.setattr(build, "ext_path", lambda: str(path))
+    native = api._load_native()
+    assert native(0, 64, 64, None, None, None, None, 0) is None
+    warned = [str(w.message) for w in recwarn if issubclass(w.category, RuntimeWarning)]
+    assert len(warned) == (0 if content is None else 1) and all(str(path) in w and "--ext" in w for w in warned)
