@@ -23,6 +23,7 @@ EXPORTED_SYMBOLS = (
     "fa_b200_describe_call",
     "fa_b200_stream_has_scratch",
     "fa_b200_describe_plan_sample",
+    "fa_b200_describe_plan_check",
     "fa_b200_plan_taken",
     "fa_b200_select_kernel",
     "fa_b200_describe_schedule",
@@ -96,6 +97,8 @@ def load() -> ctypes.CDLL:
         lib.fa_b200_stream_has_scratch.argtypes = [i32, vp, ctypes.POINTER(ctypes.c_uint32)]
         lib.fa_b200_describe_plan_sample.restype = i32
         lib.fa_b200_describe_plan_sample.argtypes = [u32, u32, u32, ctypes.POINTER(ctypes.c_uint32)]
+        lib.fa_b200_describe_plan_check.restype = i32
+        lib.fa_b200_describe_plan_check.argtypes = [u32, ctypes.c_char_p, u32, ctypes.POINTER(ctypes.c_uint32)]
         lib.fa_b200_plan_taken.restype = i32
         lib.fa_b200_plan_taken.argtypes = [i32, vp, ctypes.POINTER(ctypes.c_uint32)]
         lib.fa_b200_select_kernel.restype = i32

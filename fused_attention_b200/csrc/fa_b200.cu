@@ -1318,6 +1318,14 @@ int fa_b200_describe_plan_sample(uint32_t B, uint32_t L, uint32_t index, uint32_
     return FA_B200_OK;
 }
 
+int fa_b200_describe_plan_check(uint32_t tiles, const uint8_t* works, uint32_t key_tile, uint32_t out[1]) {
+    if (!works || !out) return FA_B200_ERR_NULL_POINTER;
+    if (tiles == 0 || tiles > fa::kPlanMaxTiles || key_tile >= tiles) return FA_B200_ERR_SHAPE;
+    static_assert(fa::kTileNeg == 0, "`works` is 0 for a tile that is -inf throughout");
+    out[0] = fa::plan_checker(works, 1u, tiles, key_tile);
+    return FA_B200_OK;
+}
+
 int fa_b200_plan_taken(int device, void* cuda_stream, uint32_t out[2]) {
     if (!out) return FA_B200_ERR_NULL_POINTER;
     out[0] = out[1] = 0;

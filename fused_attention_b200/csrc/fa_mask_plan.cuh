@@ -198,7 +198,7 @@ __device__ __forceinline__ void plan_look_at_tile(const PlanArgs& a, const PlanR
 
 // Does the plan itself look through K and V of key tile kt of batch entry b?  Only tiles that begin with -inf can be -inf
 // throughout.  Where a kernel without a plan stands behind the planned one, it is done here for key tiles that may be left
-// out by every item; of the others an item that works on them looks them through (kStepCheck) while it multiplies: 134 MB
+// out by every item; of the others an item that works on them (plan_checker) looks them through while it multiplies: 134 MB
 // of K and V at B=4 R=32 L=2048 H=128 are 25 us for a kernel of their own.
 __device__ __forceinline__ bool plan_looks_through(const PlanArgs& a, uint32_t b, uint32_t kt) {
     bool any = false, all = true;
@@ -226,7 +226,6 @@ __device__ __forceinline__ void plan_finite(const PlanArgs& a, const __half* x, 
     if (bits & 0x80008000u) a.bad[b * a.n + kt] = a.stamp;
 }
 
-// kCopy: the mask's rows start on no 16-byte boundary and are copied.  grid: at most the launch bound's CTAs per SM.  The
 // The tiles of the mask, of all batch entries, that are looked at to find out whether enough of it is -inf: all of them, or
 // one per thread.  Those are points of Roberts' sequence in three dimensions (multiples of the powers of the root of
 // x^4 = x + 1, without their whole parts), one coordinate each for batch entry, query tile and key tile, so that they are
@@ -245,12 +244,34 @@ __host__ __device__ inline PlanSample plan_sample(uint32_t i, uint32_t B, uint32
     return PlanSample{coordinate(3518319155u, B), coordinate(2882110345u, n), coordinate(2360945575u, n)};
 }
 
+// Which pair of query tiles looks through the K and V of a key tile that some pairs leave out and others work on: one that
+// works on it, kNoChecker if none does or none leaves it out.  The first one from the diagonal on, so that every pair has
+// about two key tiles of its own to look through, whatever the mask.  (Every pair next to one that leaves the tile out: with
+// blocks of 256 x 128 of which half are -inf B=1 R=40 L=4096 H=128 took 253 us; 189 with K and V looked through by the plan.)
+constexpr uint32_t kNoChecker = 0xFFFFu;
+// cls: the classes of the key tile's tiles, `pitch` apart from query tile to query tile.
+__host__ __device__ inline uint32_t plan_checker(const volatile uint8_t* cls, uint32_t pitch, uint32_t n, uint32_t kt) {
+    const uint32_t q_pairs = (n + 1u) / 2u;
+    uint32_t pair = kt / 2u, checker = kNoChecker;
+    bool left_out = false;
+#pragma unroll 4
+    for (uint32_t d = 0; d < q_pairs; ++d) {
+        const volatile uint8_t* at = cls + 2u * pair * pitch;
+        const uint32_t x = *at, y = *(2u * pair + 1u < n ? at + pitch : at);
+        if ((x | y) == kTileNeg) left_out = true;
+        else if (checker == kNoChecker) checker = pair;
+        pair = pair + 1u == q_pairs ? 0u : pair + 1u;
+    }
+    return left_out ? checker : kNoChecker;
+}
+
+// kCopy: the mask's rows start on no 16-byte boundary and are copied.  grid: at most the launch bound's CTAs per SM.  The
 // tiles of the mask round-robin, then a run of the parts of K and V; the CTA that is through last writes the lists, one
 // group of 8, 16 or 32 lanes per pair of query tiles.
 template <bool kCopy>
 __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPlanCtasPerSm) fa_mask_plan(const PlanArgs args) {
     __shared__ uint32_t hist[kPlanMaxTiles + 1], cost[2];
-    __shared__ uint16_t lens[kPlanMaxGroups];
+    __shared__ uint16_t lens[kPlanMaxGroups], checkers[2 * kPlanMaxGroups];   // B n is at most twice the groups
     __shared__ bool last;
     __shared__ __align__(16) uint32_t staged[kPlanThreads / 32u * 16u * kPlanRowWords];
     grid_dep_wait();
@@ -339,6 +360,11 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
     if (tid < 2) cost[tid] = 0;
     if (tid == 0) *a.ticket = 0;
     __syncthreads();
+    if (a.items_check) {
+        for (uint32_t i = tid; i < a.B * n; i += kPlanThreads)
+            checkers[i] = static_cast<uint16_t>(plan_checker(cls + (i / n) * n * n + i % n, n, n, i % n));
+        __syncthreads();
+    }
     const uint32_t width = n <= 8u ? 8u : (n <= 16u ? 16u : 32u), per_warp = 32u / width;
     const uint32_t lane = tid & 31u, sub = lane / width, l_in = lane % width;
     const uint32_t sub_mask = (width == 32u ? 0xFFFFFFFFu : (1u << width) - 1u) << (sub * width);
@@ -355,23 +381,18 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
             const uint32_t kt = k0 + l_in;
             const bool in = live && kt < n;
             uint32_t x = kTileNeg, y = kTileNeg, bad = a.stamp + 1u;
-            bool above = false, below = false;   // the pair of query tiles before this one, behind it, leaves the key tile out
+            uint32_t checker = kNoChecker;
             if (in) {   // (all asked for together)
                 const volatile uint8_t* c = c0 + kt;
-                const bool has_below = q0 + 2u < n, has_above = q0 != 0u;
                 x = *c;
                 bad = *const_cast<const volatile uint32_t*>(bad_of + b * n + kt);
                 y = *(two ? c + n : c);
-                const uint32_t a0 = *(has_above ? c - 2u * n : c), a1 = *(has_above ? c - n : c);
-                const uint32_t b0 = *(has_below ? c + 2u * n : c), b1 = *(q0 + 3u < n ? c + 3u * n : c);
+                if (a.items_check) checker = checkers[b * n + kt];
                 if (!two) y = x == kTileNeg ? kTileNeg : kTileZero;
-                above = has_above && (a0 | a1) == kTileNeg;
-                below = has_below && (q0 + 3u < n ? b0 | b1 : b0) == kTileNeg;
             }
             const bool keep = in && (x != kTileNeg || y != kTileNeg || bad == a.stamp);
-            // Looked through by the items that keep it next to items that do not (among those that keep a tile that others
-            // leave out there is such a pair, and every head of it looks at its own columns).
-            const uint32_t check = keep && a.items_check && bad != a.stamp && (above || below) ? kStepCheck : 0u;
+            // (every head of the pair that looks a key tile through looks at its own columns)
+            const uint32_t check = checker == gr % a.q_pairs && bad != a.stamp ? kStepCheck : 0u;
             const uint32_t votes = __ballot_sync(0xffffffffu, keep) & sub_mask;
             if (keep) {
                 auto what = [](uint32_t c) { return c == kTileZero ? kStepNoMask : (c == kTileNeg ? kStepAllNeg : (c == kTileRows ? kStepRows : kStepMask)); };

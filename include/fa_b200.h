@@ -242,6 +242,16 @@ int fa_b200_stream_has_scratch(int device, void* cuda_stream, uint32_t out[1]);
 int fa_b200_describe_plan_sample(uint32_t B, uint32_t L, uint32_t index, uint32_t out[4]);
 
 /*
+ * Leaving a key tile out is only right while its K and V are finite.  Where the rows of a planned call's
+ * mask all start on 16-byte boundaries, a key tile that some pairs of query tiles leave out and others work
+ * on is looked through by one of the latter: out[0] = which, 0xFFFF if no pair works on it or none leaves it
+ * out.  `works`: for each of the `tiles` query tiles of a batch entry 0 if the mask is -inf throughout for it
+ * and the key tile, anything else if not.  Pure arithmetic, no CUDA call; it is what the kernel itself uses.
+ * No counterpart in the reference.
+ */
+int fa_b200_describe_plan_check(uint32_t tiles, const uint8_t* works, uint32_t key_tile, uint32_t out[1]);
+
+/*
  * Which kernel had the last planned call on `cuda_stream`: out[0] = 1 if that is known (the stream's scratch
  * still holds the plan: no call with a divided last round came behind it), out[1] = 1 if it was the planned
  * kernel, 0 if the one behind it.  Synchronises the stream.  A diagnostic, for tests and harnesses: what the
