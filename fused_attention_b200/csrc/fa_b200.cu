@@ -600,7 +600,6 @@ int plan_mask(DeviceCtx& c, SplitScratch& scratch, const void* k, const void* v,
     a.q_pairs = p.q_pairs;
     a.copy_pitch = l.pitch;
     a.stamp = p.launch_id;
-    a.dense_allowed = a.items_check = mask_tma ? 1u : 0u;
     const uint64_t most = static_cast<uint64_t>(mask_tma ? fa::kPlanCtasPerSm : fa::kPlanCopyCtasPerSm) * c.sm_count;
     const uint64_t wide = l.tiles > l.jobs ? l.tiles : l.jobs;
     scratch.plan_head = nullptr;

@@ -31,9 +31,7 @@ struct PlanArgs {
     uint32_t* order;       // [B * q_pairs]: (query pair of a batch entry) | key steps << kPlanLenShift, longest first
     uint16_t* list;        // [B * q_pairs][n]: key steps, see kStepShift0
     uint32_t B, L, F, n, q_pairs, copy_pitch;
-    uint32_t stamp;           // of this call alone (a leftover that equals it costs a step, no more)
-    uint32_t dense_allowed;   // a kernel without a plan stands ready for a mask that leaves little out,
-    uint32_t items_check;     // and for K and V that items of the planned kernel find not to be finite
+    uint32_t stamp;        // of this call alone (a leftover that equals it costs a step, no more)
 };
 constexpr uint8_t kTileNeg = 0, kTileZero = 1, kTileMixed = 2, kTileRows = 3;
 constexpr uint32_t kPlanThreads = 256;
@@ -206,13 +204,14 @@ __device__ __forceinline__ void plan_look_at_tile(const PlanArgs& a, const PlanR
 // throughout.  Where a kernel without a plan stands behind the planned one, it is done here for key tiles that may be left
 // out by every item; of the others an item that works on them (plan_checker) looks them through while it multiplies: 134 MB
 // of K and V at B=4 R=32 L=2048 H=128 are 25 us for a kernel of their own.
+template <bool kCopy>
 __device__ __forceinline__ bool plan_looks_through(const PlanArgs& a, uint32_t b, uint32_t kt) {
     bool any = false, all = true;
     for (uint32_t qt = threadIdx.x; qt < a.n; qt += kPlanThreads) {
         const bool neg = ld_settled(reinterpret_cast<const uint16_t*>(a.mask) + (static_cast<size_t>(b) * a.L + qt * kTile) * a.L + kt * kTile) == 0xFC00u;
         any |= neg, all &= neg;
     }
-    return a.items_check ? __syncthreads_and(all) : __syncthreads_or(any);
+    return kCopy ? __syncthreads_or(any) : __syncthreads_and(all);
 }
 
 // 128 rows x up to kPlanCols columns of K or V: is every value finite?
@@ -271,7 +270,9 @@ __host__ __device__ inline uint32_t plan_checker(const volatile uint8_t* cls, ui
     return left_out ? checker : kNoChecker;
 }
 
-// kCopy: the mask's rows start on no 16-byte boundary and are copied.  grid: at most the launch bound's CTAs per SM.  The
+// kCopy: the mask's rows start on no 16-byte boundary and are copied.  Else a kernel without a plan stands ready for a mask
+// that leaves little out, and for K and V that items of the planned kernel find not to be finite.  grid: at most the launch
+// bound's CTAs per SM.  The
 // tiles of the mask round-robin, then a run of the parts of K and V; the CTA that is through last writes the lists, one
 // group of 8, 16 or 32 lanes per pair of query tiles.
 template <bool kCopy>
@@ -297,7 +298,7 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
         const uint32_t lane = tid & 31u, key = (lane & 1u) * 64u;
         if ((lane >> 1) < next.rows && key < next.keys) prefetch_l2(next.first + (lane >> 1) * next.pitch + 2u * key);
     }
-    if (a.dense_allowed) {
+    if constexpr (!kCopy) {
         // A tile that is -inf throughout begins with -inf.  Where fewer than a fifth of the tiles looked at do (and some of
         // them begins with neither -inf nor zero, or none with -inf), every CTA finds so for itself, nothing more is read
         // and the kernel without a plan takes the call.  One tile per thread is looked at (plan_sample): the 1024 of B=4
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
     const uint32_t job_end = static_cast<uint32_t>(static_cast<uint64_t>(jobs) * (blockIdx.x + 1u) / gridDim.x);
     while (job < job_end) {   // parts of one key tile at a time (while the tile is on its way)
         const uint32_t bk = job / (2u * chunks), end = min(job_end, (bk + 1u) * 2u * chunks), b = bk / n, kt = bk % n;
-        if (plan_looks_through(a, b, kt)) {
+        if (plan_looks_through<kCopy>(a, b, kt)) {
             for (; job < end; ++job) {
                 const uint32_t part = job - bk * 2u * chunks;
                 plan_finite(a, part < chunks ? a.k : a.v, b, kt, (part < chunks ? part : part - chunks) * kPlanCols);
@@ -351,30 +352,37 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
     __syncthreads();
     if (!last) return;
     const uint32_t groups = a.B * a.q_pairs;
-    // the classes, and which K and V are not finite, all at once where they fit into shared memory: the lists take them in
-    // steps that would each wait for L2
+    const uint32_t width = n <= 8u ? 8u : (n <= 16u ? 16u : 32u), per_warp = 32u / width;
+    const uint32_t lane = tid & 31u, sub = lane / width, l_in = lane % width;
+    const uint32_t sub_mask = (width == 32u ? 0xFFFFFFFFu : (1u << width) - 1u) << (sub * width);
+    // Where the lists (or plan_checker) take more than one step, each of which would wait for L2, the classes, and which K and V
+    // are not finite, are brought into shared memory all at once, if they fit.  (All loops from here on stay loops: one CTA
+    // goes through this code, once, and meets all of it for the first time.  Written out, and with what only the other
+    // instance needs, the plan of B=8 R=12 L=387 H=16 causal took 9.8 us instead of 8.5, and the call of B=4 R=12 L=1021 H=64
+    // 1 us more.)
     const uint8_t* cls = a.cls;
     const uint32_t* bad_of = a.bad;
     const uint32_t cls_words = (tiles + 3u) / 4u;   // (the bytes behind the classes are the scratch's own)
-    if (cls_words + a.B * n <= sizeof(staged) / sizeof(uint32_t)) {
+    if ((!kCopy || groups > kPlanThreads / 32u * per_warp || n > width) && cls_words + a.B * n <= sizeof(staged) / sizeof(uint32_t)) {
+#pragma unroll 1
         for (uint32_t i = tid; i < cls_words; i += kPlanThreads) staged[i] = __ldcg(reinterpret_cast<const uint32_t*>(a.cls) + i);
+#pragma unroll 1
         for (uint32_t i = tid; i < a.B * n; i += kPlanThreads) staged[cls_words + i] = __ldcg(a.bad + i);
         cls = reinterpret_cast<const uint8_t*>(staged);
         bad_of = staged + cls_words;
     }
+#pragma unroll 1
     for (uint32_t i = tid; i <= n; i += kPlanThreads) hist[i] = 0;
     if (tid < 2) cost[tid] = 0;
     if (tid == 0) *a.ticket = 0;
     __syncthreads();
-    if (a.items_check) {
+    if constexpr (!kCopy) {
         for (uint32_t i = tid; i < a.B * n; i += kPlanThreads)
             checkers[i] = static_cast<uint16_t>(plan_checker(cls + (i / n) * n * n + i % n, n, n, i % n));
         __syncthreads();
     }
-    const uint32_t width = n <= 8u ? 8u : (n <= 16u ? 16u : 32u), per_warp = 32u / width;
-    const uint32_t lane = tid & 31u, sub = lane / width, l_in = lane % width;
-    const uint32_t sub_mask = (width == 32u ? 0xFFFFFFFFu : (1u << width) - 1u) << (sub * width);
     uint32_t mask_tiles = 0, steps = 0;
+#pragma unroll 1
     for (uint32_t g0 = (tid >> 5) * per_warp; g0 < groups; g0 += kPlanThreads / 32u * per_warp) {
         const uint32_t gr = g0 + sub;
         const bool live = gr < groups;
@@ -383,6 +391,7 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
         const bool two = q0 + 1u < n;   // the second query tile exists
         uint16_t* out = a.list + gr * n;
         uint32_t len = 0;
+#pragma unroll 1
         for (uint32_t k0 = 0; k0 < n; k0 += width) {
             const uint32_t kt = k0 + l_in;
             const bool in = live && kt < n;
@@ -393,7 +402,7 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
                 x = *c;
                 bad = *const_cast<const volatile uint32_t*>(bad_of + b * n + kt);
                 y = *(two ? c + n : c);
-                if (a.items_check) checker = checkers[b * n + kt];
+                if constexpr (!kCopy) checker = checkers[b * n + kt];
                 if (!two) y = x == kTileNeg ? kTileNeg : kTileZero;
             }
             const bool keep = in && (x != kTileNeg || y != kTileNeg || bad == a.stamp);
@@ -427,6 +436,7 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
     __syncthreads();
     if (tid == 0) {   // places, longest first
         uint32_t at = 0;
+#pragma unroll 1
         for (uint32_t len = n; len >= 1u; --len) {
             const uint32_t c = hist[len];
             hist[len] = at;
@@ -436,9 +446,10 @@ __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPl
         // 1.2 for each step of all.
         *reinterpret_cast<const __half**>(a.head + kPlanInputs) = a.k;
         *reinterpret_cast<const __half**>(a.head + kPlanInputs + 2) = a.v;
-        a.head[0] = !a.dense_allowed || 5u * cost[0] + cost[1] < 6u * groups * n ? 1u : 0u;
+        a.head[0] = kCopy || 5u * cost[0] + cost[1] < 6u * groups * n ? 1u : 0u;
     }
     __syncthreads();
+#pragma unroll 1
     for (uint32_t gr = tid; gr < groups; gr += kPlanThreads)
         a.order[atomicAdd(&hist[lens[gr]], 1u)] = gr | (static_cast<uint32_t>(lens[gr]) << kPlanLenShift);
 }
