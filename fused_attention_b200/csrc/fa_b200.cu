@@ -577,8 +577,14 @@ bool use_mask_plan(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool mask_tma
 // elements apart.
 int plan_mask(DeviceCtx& c, SplitScratch& scratch, const void* k, const void* v, bool mask_tma,
               Params& p, cudaStream_t st, bool overlap, const void** mask_rows, uint32_t* mask_pitch) {
-    // (without the runs where there is no room for them: rows that are runs are then mask tiles like any other)
-    const bool with_runs = plan_layout(p.B, p.L, p.F, mask_tma, true).bytes <= split_o_bytes(c.sm_count);
+    // Finding the runs is 1 us of the plan of an unaligned mask, and what they save is a copied tile's way into shared memory
+    // once per item.  Where there are fewer than two rounds of items, and no mask tile to wait for at every step (H = 128),
+    // rows that are runs are mask tiles like any other, as they are where there is no room for the runs.  Measured, us with and
+    // without, padding and windows: 1.3 rounds, B=8 R=12 L=387 H=16 24.4 / 23.1 and 28.2 / 28.0, B=4 R=12 L=1021 H=64 32.4 /
+    // 31.7 and 36.8 / 36.4; 2.2 rounds, B=4 R=40 L=389 H=16 27.1 / 25.5 and 35.8 / 36.5; 2.6, B=8 R=16 L=515 H=32 31.6 / 31.1 and
+    // 36.3 / 37.0; 3.5, B=8 R=32 L=389 H=64 39.8 / 39.6 and 55.0 / 57.3; H = 128, B=2 R=32 L=389 22.8 / 24.
+    const bool worth = mask_tma || p.F / p.R == 128u || p.n_items >= 2u * static_cast<uint32_t>(c.sm_count);
+    const bool with_runs = worth && plan_layout(p.B, p.L, p.F, mask_tma, true).bytes <= split_o_bytes(c.sm_count);
     const PlanLayout l = plan_layout(p.B, p.L, p.F, mask_tma, with_runs);
     char* base = reinterpret_cast<char*>(scratch.o);
     fa::PlanArgs a;
