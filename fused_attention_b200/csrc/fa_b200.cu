@@ -552,18 +552,21 @@ bool plan_fits(uint32_t B, uint32_t L, uint32_t F, bool mask_tma, uint32_t sms) 
 }
 
 // Whether a masked call of the pipelined kernel is planned (fa_mask_plan.cuh).  The plan is a launch and a pass over the
-// mask, K and V ahead of the attention kernel, 6 us at least, and 13 in all where it finds that too little can be left
-// out; what it saves is up to half of the key steps where there is more than one round of them.  Measured, us without
-// and with a plan, causal masks:
-//   H = 64: B=8 R=12 L=512 19.8 / 33.5, B=32 R=12 L=512 50 / 70, B=8 R=16 L=1024 63 / 67, B=2 R=12 L=2048 50 / 51
-//   H = 32: B=8 R=16 L=1024 73 / 65;   H = 128: B=4 R=32 L=1024 69 / 78, B=2 R=32 L=1536 82 / 79
-// so from sixteen key tiles and some fifty key steps per SM on, where it is far ahead (B=4 R=32 L=2048 H=128 with mask tiles
-// 250, planned 206; B=8 R=32 L=2048 H=64 430 and 270).  (A mask that leaves nothing out pays for the plan and the planned
-// kernel's launch all the same: H = 64, B=8 R=16 L=1024 63 / 81, B=2 R=16 L=2048 63 / 80.  What the mask holds is known on the
-// device only.)  Where TMA cannot fetch the rows the plan's copy also
-// spares every head the copies inside the kernel, and it pays much sooner:
-//   H = 64: B=32 R=16 L=201 36 / 46, B=1 R=8 L=301 15 / 18, B=32 R=12 L=301 82 / 63, B=2 R=8 L=511 26 / 21,
-//           B=4 R=12 L=1021 72 / 38;   H = 128: B=1 R=8 L=301 25 / 19, B=2 R=32 L=1021 125 / 51
+// mask, K and V ahead of the attention kernel; what it saves is up to half of the key steps where there is more than one
+// round of them.  What the mask holds is known on the device only: one that leaves nothing out pays for the plan and the
+// planned kernel's launch all the same.  Measured, us without and with a plan, causal masks, then dense ones:
+//   H = 64: B=8 R=12 L=512 19.3 / 32.5, 19.3 / 28.0; B=32 R=12 L=512 49.5 / 69, 53 / 67; B=8 R=16 L=1024 69 / 67, 69 / 78;
+//           B=2 R=12 L=2048 52.6 / 50, 52.8 / 74; B=2 R=16 L=2048 63 / 53.5, 63 / 75.5; B=4 R=32 L=2048 201 / 148, 201 / 228;
+//           B=8 R=32 L=2048 400 / 268, 445 / 465
+//   H = 32: B=8 R=16 L=1024 78 / 67, 75 / 80; B=4 R=32 L=1024 73 / 62, 69 / 74; B=8 R=16 L=2048 245 / 154, 241 / 246
+//   H = 128: B=4 R=32 L=1024 71 / 75.5, 74.5 / 81; B=2 R=32 L=1536 76 / 72, 80 / 87.5; B=2 R=32 L=2048 145 / 97, 148 / 154;
+//           B=4 R=32 L=2048 253 / 190, 278 / 276; B=1 R=40 L=4096 405 / 203, 390 / 367
+// so from sixteen key tiles and some fifty key steps per SM on: below, a causal mask gains 15 % at most and a dense one loses
+// up to 40; above, up to 50 and 14.  Where TMA cannot fetch the rows the plan's copy also spares every head the copies inside
+// the kernel, and it pays much sooner:
+//   H = 64: B=32 R=16 L=201 39 / 44, 36 / 40; B=1 R=8 L=301 14.8 / 17.0, 14.8 / 18.3; B=32 R=12 L=301 73.5 / 55.6, 73.7 / 63.8;
+//           B=2 R=8 L=511 25.8 / 19.6, 25.8 / 20.1; B=4 R=12 L=1021 72 / 31, 72.5 / 51
+//   H = 128: B=1 R=8 L=301 24.6 / 17.9, 24.6 / 21.9; B=2 R=32 L=1021 123 / 47, 123 / 71
 bool use_mask_plan(uint32_t B, uint32_t L, uint32_t F, uint32_t H, bool mask_tma, uint32_t sms, uint32_t flags) {
     if ((flags & FA_B200_FLAG_FORCE_PAIR) || !plan_fits(B, L, F, mask_tma, sms)) return false;
     const uint32_t n = (L + fa::kTile - 1) / fa::kTile;

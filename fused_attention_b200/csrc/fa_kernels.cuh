@@ -78,7 +78,7 @@ struct Params {
 
 constexpr int kTile = 128;  // rows of a query tile and of a key/value tile
 
-// role << 8 | barrier id, written to the status word when a bounded wait expires
+// role << 8 | barrier id, which the status word receives from a CTA in which a bounded wait has expired
 enum : uint32_t {
     kRoleSimple = 0x100u,
     kRoleProducer = 0x200u,

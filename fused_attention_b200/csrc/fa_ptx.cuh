@@ -88,18 +88,19 @@ __device__ __forceinline__ uint32_t mbar_poll_end() {
 
 // Where a bounded wait reports: a device status block and a CTA-wide abort flag.
 struct WaitCtl {
-    uint32_t* status;              // global: [0] first failure code, [1] number of reporting CTAs
+    uint32_t* status;              // global: [0] first failure code, [1] number of reporting CTAs (report_expired)
     volatile uint32_t* abort_flag; // shared: non-zero once any wait of this CTA has expired
     long long cap_cycles;          // how long one wait may spin
-    uint32_t* launch_word;         // global, may be null: receives launch_id when a wait expires, so that
-    uint32_t launch_id;            // CTAs of the same launch that start later leave at once
+    uint32_t* launch_word;         // global, may be null: receives launch_id at the end of a CTA in which a wait has
+    uint32_t launch_id;            // expired, so that CTAs of the same launch that start after that leave at once
 };
 
 // About two seconds at 2 GHz; a whole launch of the largest supported problem takes milliseconds.
 constexpr long long kWaitCapCycles = 4000000000LL;
 
 // A wait that gives up leaves its code in the CTA's abort flag (the first one stays); one thread passes it on at the end of
-// the kernel (report_expired).  Waits are inlined in some fifty places, most of which run into their loop once in a while,
+// the CTA (report_expired), which comes soon: all further waits return at once, but for those for what is in flight.  CTAs
+// that are running by then wait until their own caps.  Waits are inlined in some fifty places, most of which run into their loop once in a while,
 // and the roles of a CTA share one instruction cache, so what they do there is kept short.  With the report, the spin
 // counting and 64-bit clocks in every one of them, and the epilogue's loops unrolled, 22 % of the instruction fetches of the
 // ViT-shaped call (B=64 R=16 L=197 H=64) missed that cache; now 10 %, and the call went from 35.8 to 32.2 us, B=8 R=12 L=512
@@ -185,9 +186,9 @@ __device__ __forceinline__ bool mbar_wait_certain(uint32_t bar, uint32_t parity,
 // the shared-memory side lies inside the CTA's tile area and on a 1024-byte boundary, the innermost
 // coordinate is a multiple of 8 elements (16 bytes) and all coordinates lie inside the tensor, a store does
 // not start at a negative or out-of-range row, a tensor-memory access stays inside the CTA's allocation and
-// on the lanes of the issuing warp.  A failed check records kRoleDebug | <what> in the device status word,
-// sets the CTA's abort flag and SKIPS the access (nothing faults; the bounded waits then return at once and
-// the CTA leaves).  The kernels also fill their tile area with NaN before the first copy, and the launcher
+// on the lanes of the issuing warp.  A failed check leaves kRoleDebug | <what> in the CTA's abort flag, from
+// where it goes to the device status word at the CTA's end, and SKIPS the access (nothing faults; the
+// bounded waits then return at once and the CTA leaves).  The kernels also fill their tile area with NaN before the first copy, and the launcher
 // fills Y with NaN before the launch, so that anything consumed before it has landed, or never written,
 // shows in the result.  Normal builds contain none of this.
 #ifdef FA_DEBUG

@@ -165,8 +165,8 @@ int fa_b200_query(int device, int32_t out[4]);
  * The word is shared by every launch on the device and stays set until it is read here, or
  * returned by a call with FA_B200_FLAG_SYNC or by fa_b200_attention_forward_host (both clear it
  * when they return FA_B200_ERR_DEVICE_TIMEOUT).  An asynchronous call never looks at it: after a
- * launch whose wait expired its output is garbage and only this word says so.  Once one CTA of a
- * launch has given up, the CTAs of that launch that start later leave at once.
+ * launch whose wait expired its output is garbage and only this word says so.  A CTA reports as it
+ * ends; the CTAs of its launch that start after that leave at once.
  * No counterpart in the reference (it has no device-side error reporting).
  */
 int fa_b200_read_status(int device, uint32_t out[2]);
@@ -182,8 +182,8 @@ int fa_b200_selftest_bounded_wait(int device, uint32_t out[3]);
 
 /*
  * The checked build of the library (compiled with -DFA_DEBUG: every TMA copy and tensor-memory access
- * checks its shared-memory operand, its coordinates and its columns first, records a failed check in
- * the device status word and skips the access; tile buffers and Y are filled with NaN beforehand) can
+ * checks its shared-memory operand, its coordinates and its columns first, reports a failed check in
+ * the device status word at the CTA's end and skips the access; tile buffers and Y are filled with NaN beforehand) can
  * test its own predicates: they are asked about operands that are in order and operands that are not,
  * with no copy made.  out[0] = status code recorded by the first refusal (expected 0x703: innermost
  * coordinate not a multiple of 8 elements), out[1] = 1, out[2] = 1 in a checked build and 0 in a normal
