@@ -49,8 +49,8 @@ constexpr uint32_t kWholeRun = kTile << 8;
 // A tile is brought into shared memory with asynchronous copies and looked at there, in loops: a CTA of this kernel meets
 // all of its code for the first time, and its length counts.  (Rows in registers and everything written out over them were
 // 118 KB of code; a tile on the diagonal of B=4 R=12 L=1021 H=64 took 15 us.)
-// Measured, the call: B=4 R=32 L=2048 H=128 causal 232 us with mask tiles on the diagonal and K and V looked through here,
-// 206 with runs and K and V looked through by the items; this kernel alone, cold, 36 and 24.
+// Measured, the call: B=4 R=32 L=2048 H=128 causal 243 us with mask tiles on the diagonal and K and V looked through here,
+// 209 with runs and K and V looked through by the items; this kernel alone 38 and 23.
 // Words of a staged row.  Rows on 16-byte boundaries: 64.  Others in whole aligned words, where word j of a row that starts
 // in the middle of one holds its keys 2 j - 1 and 2 j: 65 (and one so that rows lie an even number of banks apart).
 constexpr uint32_t kPlanRowWords = 66;

@@ -100,11 +100,11 @@ constexpr long long kWaitCapCycles = 4000000000LL;
 
 // A wait that gives up leaves its code in the CTA's abort flag (the first one stays); one thread passes it on at the end of
 // the CTA (report_expired), which comes soon: all further waits return at once, but for those for what is in flight.  CTAs
-// that are running by then wait until their own caps.  Waits are inlined in some fifty places, most of which run into their loop once in a while,
-// and the roles of a CTA share one instruction cache, so what they do there is kept short.  With the report, the spin
-// counting and 64-bit clocks in every one of them, and the epilogue's loops unrolled, 22 % of the instruction fetches of the
-// ViT-shaped call (B=64 R=16 L=197 H=64) missed that cache; now 10 %, and the call went from 35.8 to 32.2 us, B=8 R=12 L=512
-// H=64 from 16.1 to 15.4, the same with a mask from 21.2 to 19.3.
+// that are running by then wait until their own caps.  Waits are inlined in some fifty places, most of which run into their
+// loop once in a while, and the roles of a CTA share one instruction cache, so what they do there is kept short.  With the
+// report, the spin counting and 64-bit clocks in every one of them, and the epilogue's loops unrolled, 21 % of the
+// instruction fetches of the ViT-shaped call (B=64 R=16 L=197 H=64) missed that cache; now 10 %, and the call went from 35.1
+// to 31.6 us, B=8 R=12 L=512 H=64 from 16.0 to 15.4, the same with a mask from 21.0 to 19.2.
 constexpr uint32_t kLeftEarly = 0xFFFFFFFFu;
 __device__ __forceinline__ void wait_expired(const WaitCtl& ctl, uint32_t code) {
     atomicCAS(const_cast<uint32_t*>(ctl.abort_flag), 0u, code);
