@@ -272,9 +272,8 @@ __host__ __device__ inline uint32_t plan_checker(const volatile uint8_t* cls, ui
 
 // kCopy: the mask's rows start on no 16-byte boundary and are copied.  Else a kernel without a plan stands ready for a mask
 // that leaves little out, and for K and V that items of the planned kernel find not to be finite.  grid: at most the launch
-// bound's CTAs per SM.  The
-// tiles of the mask round-robin, then a run of the parts of K and V; the CTA that is through last writes the lists, one
-// group of 8, 16 or 32 lanes per pair of query tiles.
+// bound's CTAs per SM.  The tiles of the mask round-robin, then a run of the parts of K and V; the CTA that is through last
+// writes the lists, one group of 8, 16 or 32 lanes per pair of query tiles.
 template <bool kCopy>
 __global__ void __launch_bounds__(kPlanThreads, kCopy ? kPlanCopyCtasPerSm : kPlanCtasPerSm) fa_mask_plan(const PlanArgs args) {
     __shared__ uint32_t hist[kPlanMaxTiles + 1], cost[2];
